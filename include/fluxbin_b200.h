@@ -354,6 +354,28 @@ int fb_tp_argmax(void* keys, int world, int64_t* best, const int64_t* forced_nex
                  int vocab, int in_features, unsigned* status, uint64_t wait_ns, fb_stream_t stream);
 
 /*
+ * Many-token path (prefill, dense fallback): the packed weights as dense 16-bit rows, and the
+ * element-wise steps between the dense GEMMs.  No counterparts in the reference, which restores weights
+ * and runs these steps as tensor operations (w3_lut_deployment.py:343-359, stock HF modules).
+ *
+ * fb_w3_dequant: rows row_begin .. row_begin + row_count - 1 (row_count 0: all from row_begin) of up to four
+ *   matrices of equal K, `out` of each a row-major [rows, K] buffer (16-byte aligned) of out_dtype, columns in
+ *   the layout's (group-sorted) order: T_out(T_scale(scale * (code - zero))).
+ * fb_gather_columns: out[t, k] = x[t, perm[k]], the activations that go with that order.
+ * fb_qknorm_rope_prompt: rows of qkv [tokens, q_heads + 2 kv_heads, 128] -> per-head RMSNorm of q and k,
+ *   rotary embedding with cos / sin [tokens, 128]; q to q_out [q_heads, tokens, 128], k and v to
+ *   positions 0 .. tokens - 1 of the caches [kv_heads, max_positions, 128].
+ * fb_silu_mul_rows: out[t, i] = T(silu(gate_up[t, i])) * gate_up[t, width + i]; out rows out_stride apart.
+ */
+int fb_w3_dequant(const fb_w3_matrix_t* matrices, int n_matrices, int row_begin, int row_count, int scale_dtype, int in_features,
+                  int out_dtype, fb_stream_t stream);
+int fb_gather_columns(const void* x, const int16_t* perm, void* out, int rows, int in_features, fb_stream_t stream);
+int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, const void* k_weight, const void* cosv, const void* sinv, void* q_out,
+                          void* k_cache, void* v_cache, int tokens, int q_heads, int kv_heads, int head_dim, int max_positions, float eps,
+                          int dtype, fb_stream_t stream);
+int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int width, int out_stride, int dtype, fb_stream_t stream);
+
+/*
  * fb_w3_gemv without a scratch argument, for callers that cannot allocate device memory where
  * they call this library (all memory already handed to a pool, a framework allocator that must
  * not be bypassed, a CUDA graph capture in progress).  The split-K scratch is a fixed array of

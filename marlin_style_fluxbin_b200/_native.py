@@ -128,6 +128,14 @@ def library() -> ctypes.CDLL:
                                           ctypes.c_int] + [ctypes.c_void_p] * 6 + [ctypes.c_size_t, ctypes.c_void_p]
         lib.fb_embed_row.restype = ctypes.c_int
         lib.fb_embed_row.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+        lib.fb_w3_dequant.restype = ctypes.c_int
+        lib.fb_w3_dequant.argtypes = [ctypes.POINTER(W3Matrix)] + [ctypes.c_int] * 6 + [ctypes.c_void_p]
+        lib.fb_gather_columns.restype = ctypes.c_int
+        lib.fb_gather_columns.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 2 + [ctypes.c_void_p]
+        lib.fb_qknorm_rope_prompt.restype = ctypes.c_int
+        lib.fb_qknorm_rope_prompt.argtypes = [ctypes.c_void_p] * 8 + [ctypes.c_int] * 5 + [ctypes.c_float, ctypes.c_int, ctypes.c_void_p]
+        lib.fb_silu_mul_rows.restype = ctypes.c_int
+        lib.fb_silu_mul_rows.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int] * 4 + [ctypes.c_void_p]
         lib.fb_w3_gemv_static.restype = ctypes.c_int
         lib.fb_w3_gemv_static.argtypes = lib.fb_w3_gemv.argtypes[:11] + [ctypes.c_uint, ctypes.c_void_p]
         _lib = lib
@@ -529,3 +537,34 @@ def embed_row(embedding, token, out) -> None:
     vocab, k = embedding.shape
     with torch.cuda.device(out.device):
         check(library().fb_embed_row(ptr(embedding), ptr(token), ptr(out), vocab, k, stream_handle(out.device)))
+
+
+def w3_dequant(entries, out_dtype, *, row_begin: int = 0, row_count: int = 0) -> None:
+    """Dense 16-bit rows of one to four W3 matrices of equal K in one launch: ``entries`` are ``(layout, out)`` pairs,
+    ``out`` a contiguous ``[rows, K]`` tensor; columns stay in the layout's group-sorted order (see the header)."""
+    matrices = w3_matrix_list([(layout["planes"], layout["scales"], layout.get("zeros"), out, None) for layout, out in entries])
+    layout = entries[0][0]
+    device = layout["planes"].device
+    with torch.cuda.device(device):
+        check(library().fb_w3_dequant(matrices, len(entries), row_begin, row_count, dtype_tag(layout["scales"].dtype), layout["planes"].shape[0] * 128,
+                                      dtype_tag(out_dtype), stream_handle(device)))
+
+
+def gather_columns(x, perm, out) -> None:
+    """``out[t, k] = x[t, perm[k]]`` for contiguous 16-bit ``x`` ``[T,K]``."""
+    with torch.cuda.device(x.device):
+        check(library().fb_gather_columns(ptr(x), ptr(perm), ptr(out), x.shape[0], x.shape[1], stream_handle(x.device)))
+
+
+def qknorm_rope_prompt(qkv, q_weight, k_weight, cos, sin, q_out, k_cache, v_cache, eps: float) -> None:
+    """q/k RMSNorm, rotary embedding and cache rows of a prompt: ``qkv`` ``[T, (q_heads + 2 kv_heads) * 128]``, ``q_out`` ``[q_heads, T, 128]``."""
+    with torch.cuda.device(qkv.device):
+        check(library().fb_qknorm_rope_prompt(ptr(qkv), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(q_out), ptr(k_cache), ptr(v_cache),
+                                              qkv.shape[0], q_out.shape[0], k_cache.shape[-3], q_out.shape[-1], k_cache.shape[-2], float(eps),
+                                              dtype_tag(qkv.dtype), stream_handle(qkv.device)))
+
+
+def silu_mul_rows(gate_up, out) -> None:
+    """``out[t, i] = silu(gate_up[t, i]) * gate_up[t, width + i]``; ``out`` may be a column slice of a wider buffer."""
+    with torch.cuda.device(out.device):
+        check(library().fb_silu_mul_rows(ptr(gate_up), ptr(out), out.shape[0], out.shape[1], out.stride(0), dtype_tag(out.dtype), stream_handle(out.device)))

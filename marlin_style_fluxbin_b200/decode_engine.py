@@ -27,6 +27,7 @@ from torch.nn import functional as F
 
 from . import _native
 from .gptq_deployment import restore_planar_w3
+from .w3_lut_deployment import DENSE_CHUNK_BYTES
 
 
 @dataclass(frozen=True)
@@ -80,6 +81,12 @@ def shard_groups(layout, rank, size):
     lo, hi = rank * g // size, (rank + 1) * g // size
     return {"planes": layout["planes"][lo:hi].contiguous(), "scales": layout["scales"][lo:hi].contiguous(),
             "zeros": layout["zeros"][lo:hi].contiguous(), "perm": torch.arange((hi - lo) * 128, dtype=torch.int16, device=layout["perm"].device)}
+
+
+def _chunk_rows(rows, k):
+    """Rows of a ``[rows, k]`` 16-bit weight per chunk: equal chunks of at most ``DENSE_CHUNK_BYTES``, multiples of 128 rows."""
+    chunks = -(-rows * k * 2 // DENSE_CHUNK_BYTES)
+    return min(rows, -(-(-(-rows // chunks)) // 128) * 128)
 
 
 def head_key(logit: float, row: int) -> int:
@@ -185,9 +192,19 @@ class DecodeEngine:
     # ------------------------------------------------------------------ weights
     def _dense(self, layer):
         """Dequantised 16-bit weights of this rank's shards (fused q/k/v and gate/up)."""
-        d = lambda lay: restore_planar_w3(lay, dtype=self.dtype)  # noqa: E731
-        return {"qkv": torch.cat((d(layer.q), d(layer.k), d(layer.v)), 0), "o": d(layer.o),
-                "gate_up": torch.cat((d(layer.gate), d(layer.up)), 0), "down": d(layer.down)}
+        return {name: self._dense_rows(layouts) for name, layouts in (("qkv", (layer.q, layer.k, layer.v)), ("o", (layer.o,)),
+                                                                      ("gate_up", (layer.gate, layer.up)), ("down", (layer.down,)))}
+
+    def _dense_rows(self, layouts, begin=0, count=0, into=None):
+        """Rows ``begin .. begin + count`` (0: all) of each layout, dequantised, one below the other."""
+        heights = [count or lay["planes"].shape[2] - begin for lay in layouts]
+        dense = torch.empty(sum(heights), layouts[0]["planes"].shape[0] * 128, device=self.device, dtype=self.dtype) if into is None else into
+        entries, at = [], 0
+        for lay, height in zip(layouts, heights):
+            entries.append((lay, dense[at:at + height]))
+            at += height
+        _native.w3_dequant(entries, self.dtype, row_begin=begin, row_count=count)
+        return dense[:at]
 
     def _build_matrix_lists(self):
         first = self.tp_rank == 0  # the residual is added by exactly one rank before the allreduce
@@ -238,43 +255,88 @@ class DecodeEngine:
         if self.tp_size > 1:
             torch.distributed.all_reduce(tensor, group=self.group)
 
-    # ------------------------------------------------------------------ prefill (dense, not timed)
+    # ------------------------------------------------------------------ prefill (many tokens)
+    def _prompt_linear(self, x, layouts, dense, addend=None):
+        """``x`` ``[T,K]`` times the stacked rows of ``layouts`` (``dense``: the same rows as one dense matrix, or None
+        on the packed arm), plus ``addend``.  The packed arm keeps up to 4 tokens packed; for more it forms the weight
+        in chunks that stay in the L2 between the dequantising launch and the GEMM."""
+        if dense is not None:
+            return torch.mm(x, dense.t()) if addend is None else torch.addmm(addend, x, dense.t())
+        t, k = x.shape
+        if t <= 4:
+            parts = [torch.empty(t, lay["planes"].shape[2], device=self.device, dtype=self.dtype) for lay in layouts]
+            for lay, part in zip(layouts, parts):
+                _native.w3_gemv(x, lay["planes"], lay["scales"], lay["zeros"], None, part)
+            y = parts[0] if len(parts) == 1 else torch.cat(parts, dim=1)
+            return y if addend is None else y.add_(addend)
+        rows = sum(lay["planes"].shape[2] for lay in layouts)
+        if len(layouts) > 1 or rows * k * 2 <= DENSE_CHUNK_BYTES:
+            weight = self._dense_rows(layouts)
+            return torch.mm(x, weight.t()) if addend is None else torch.addmm(addend, x, weight.t())
+        step = _chunk_rows(rows, k)
+        weight, y = torch.empty(step, k, device=self.device, dtype=self.dtype), torch.empty(t, rows, device=self.device, dtype=self.dtype)
+        for begin in range(0, rows, step):
+            end = min(rows, begin + step)
+            part = self._dense_rows(layouts, begin, end - begin, into=weight)
+            if addend is None:
+                torch.mm(x, part.t(), out=y[:, begin:end])
+            else:
+                torch.addmm(addend[:, begin:end], x, part.t(), out=y[:, begin:end])
+        return y
+
+    def _prompt_mlp_input(self, x, layer):
+        """``silu(x gate^T) * (x up^T)`` ``[T, inter]``; the packed arm takes matching rows of gate and up together."""
+        t, k = x.shape
+        act = torch.empty(t, self.inter, device=self.device, dtype=self.dtype)
+        if layer.dense is not None or t <= 4:
+            _native.silu_mul_rows(self._prompt_linear(x, (layer.gate, layer.up), None if layer.dense is None else layer.dense["gate_up"]), act)
+            return act
+        step = _chunk_rows(2 * self.inter, k) // 2
+        weight = torch.empty(2 * min(step, self.inter), k, device=self.device, dtype=self.dtype)
+        for begin in range(0, self.inter, step):
+            count = min(step, self.inter - begin)
+            part = self._dense_rows((layer.gate, layer.up), begin, count, into=weight)
+            _native.silu_mul_rows(torch.mm(x, part.t()), act[:, begin:begin + count])
+        return act
+
     @torch.inference_mode()
     def prefill(self, input_ids: torch.Tensor) -> torch.Tensor:
-        """Run the prompt through dense (dequantised) weights with plain tensor operations, fill
-        the KV cache for positions ``0..T-1`` and return the logits of the last position."""
-        s = self.shape
+        """Run the prompt through dense (dequantised) weights, fill the KV cache for positions ``0..T-1`` and
+        return the logits of the last position.  GEMMs and attention are library calls; dequantisation and
+        the element-wise steps between them are one launch each."""
+        s, nat = self.shape, _native
         tokens = input_ids.reshape(-1).to(self.device)
         t = tokens.numel()
         if not 1 <= t < self.max_positions:
             raise ValueError("prompt does not fit the KV cache")
         h = self.embedding[tokens]
-        cos, sin = self.cos[:t].unsqueeze(0), self.sin[:t].unsqueeze(0)
-        rotate = lambda x: torch.cat((-x[..., s.head_dim // 2:], x[..., :s.head_dim // 2]), dim=-1)  # noqa: E731
-        norm = lambda x, w: (w * (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + s.eps)).to(self.dtype))  # noqa: E731
+        xn = torch.empty_like(h)
+        q_rot = torch.empty(self.q_heads, t, s.head_dim, device=self.device, dtype=self.dtype)
+        alone = self.tp_size == 1
         for index, layer in enumerate(self.layers):
-            dense = layer.dense if layer.dense is not None else self._dense(layer)
-            x = norm(h, layer.ln1)
-            qkv = F.linear(x, dense["qkv"])
-            q, k, v = qkv.split((self.q_heads * s.head_dim, self.kv_heads * s.head_dim, self.kv_heads * s.head_dim), dim=-1)
-            q = norm(q.reshape(t, self.q_heads, s.head_dim), layer.q_norm).transpose(0, 1)
-            k = norm(k.reshape(t, self.kv_heads, s.head_dim), layer.k_norm).transpose(0, 1)
-            v = v.reshape(t, self.kv_heads, s.head_dim).transpose(0, 1)
-            q = q * cos + rotate(q) * sin
-            k = k * cos + rotate(k) * sin
-            self.k_cache[index, :, :t] = k
-            self.v_cache[index, :, :t] = v
-            attn = F.scaled_dot_product_attention(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), is_causal=True, enable_gqa=True)
-            y = F.linear(attn[0].transpose(0, 1).reshape(t, -1), dense["o"])
-            self._allreduce(y)
-            h = h + y
-            x = norm(h, layer.ln2)
-            gate, up = F.linear(x, dense["gate_up"]).split(self.inter, dim=-1)
-            y = F.linear(F.silu(gate) * up, dense["down"])
-            self._allreduce(y)
-            h = h + y
-            del dense
-        last = norm(h[-1:], self.final_norm)
+            dense = layer.dense or {}
+            nat.rmsnorm(h, layer.ln1, xn, s.eps)
+            qkv = self._prompt_linear(xn, (layer.q, layer.k, layer.v), dense.get("qkv"))
+            nat.qknorm_rope_prompt(qkv, layer.q_norm, layer.k_norm, self.cos, self.sin, q_rot, self.k_cache[index], self.v_cache[index], s.eps)
+            k, v = self.k_cache[index, :, :t], self.v_cache[index, :, :t]
+            attn = F.scaled_dot_product_attention(q_rot.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), is_causal=True, enable_gqa=True)
+            x = attn[0].transpose(0, 1).reshape(t, -1)
+            if alone:
+                h = self._prompt_linear(x, (layer.o,), dense.get("o"), addend=h)
+            else:
+                y = self._prompt_linear(x, (layer.o,), dense.get("o"))
+                self._allreduce(y)
+                h = h + y
+            nat.rmsnorm(h, layer.ln2, xn, s.eps)
+            act = self._prompt_mlp_input(xn, layer)
+            if alone:
+                h = self._prompt_linear(act, (layer.down,), dense.get("down"), addend=h)
+            else:
+                y = self._prompt_linear(act, (layer.down,), dense.get("down"))
+                self._allreduce(y)
+                h = h + y
+        last = torch.empty_like(h[-1:])
+        nat.rmsnorm(h[-1:], self.final_norm, last, s.eps)
         return F.linear(last, self.lm_head)
 
     # ------------------------------------------------------------------ one decode step

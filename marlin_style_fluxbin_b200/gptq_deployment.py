@@ -284,6 +284,12 @@ def restore_planar_w3(layout: Mapping[str, torch.Tensor], *, dtype: torch.dtype 
     rounding, as a GPTQ module loaded in that dtype computes it) and then cast to ``dtype``.
     """
     out_features, in_features = validate_planar_w3(layout)
+    if layout["planes"].is_cuda and dtype in (torch.float16, torch.bfloat16):
+        from . import _native
+
+        ordered = torch.empty(out_features, in_features, device=layout["planes"].device, dtype=dtype)
+        _native.w3_dequant([(layout, ordered)], dtype)
+        return ordered if is_identity_perm(layout["perm"]) else ordered.index_select(1, torch.argsort(layout["perm"].long()))
     signed = _signed_codes(layout)  # [G,128,O]
     product = layout["scales"].unsqueeze(1) * signed  # 16-bit float * int16 -> 16-bit float
     ordered = product.permute(2, 0, 1).reshape(out_features, in_features)

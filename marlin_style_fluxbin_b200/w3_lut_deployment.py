@@ -11,6 +11,7 @@ own tiling, reduces its K split internally and leaves a caller's workspace untou
 """
 from __future__ import annotations
 
+import weakref
 from types import SimpleNamespace
 
 import torch
@@ -19,6 +20,10 @@ from torch.nn import functional as F
 
 from . import _native
 from .gptq_deployment import FIELDS, OPTIONAL_FIELDS, restore_planar_w3, validate_planar_w3
+
+# A dense weight is formed and multiplied in row chunks of at most this size: the GEMM then reads the
+# chunk out of the L2 (126 MB), and the next chunk overwrites it there before it is written back.
+DENSE_CHUNK_BYTES = 52 << 20
 
 ROW_TILES = (256, 512, 1024)
 EXPERIMENTAL_ROW_TILES = ROW_TILES + (2048,)
@@ -114,21 +119,25 @@ def load_w3_lut_extension(row_tile: int, uniform_index_probe: bool = False):
                            finish=finish, m1_out=m1_out)
 
 
-# perm tensors that were checked to be the identity: the kernel then skips the gather
-_IDENTITY_PERMS: dict[tuple[int, int], bool] = {}
+# perm tensors that were checked to be the identity: the kernel then skips the gather.  Keyed by address, and an
+# entry holds only while the tensor it was made for lives unchanged (another one may get the address later).
+_IDENTITY_PERMS: dict[tuple[int, int], tuple] = {}
 
 
 def _perm_or_none(perm: torch.Tensor):
     """``None`` when ``perm`` is the identity (decided once per tensor, outside capture)."""
     key = (perm.data_ptr(), perm.numel())
-    known = _IDENTITY_PERMS.get(key)
-    if known is None:
-        if torch.cuda.is_current_stream_capturing():
-            return perm  # cannot inspect values now; the general gather path is always valid
-        known = bool(torch.equal(perm, torch.arange(perm.numel(), device=perm.device, dtype=perm.dtype)))
-        if len(_IDENTITY_PERMS) > 4096:
-            _IDENTITY_PERMS.clear()
-        _IDENTITY_PERMS[key] = known
+    owner = perm if perm._base is None else perm._base
+    version = None if perm.is_inference() else perm._version
+    entry = _IDENTITY_PERMS.get(key)
+    if entry is not None and entry[0]() is owner and entry[1] == version:
+        return None if entry[2] else perm
+    if torch.cuda.is_current_stream_capturing():
+        return perm  # cannot inspect values now; the general gather path is always valid
+    known = bool(torch.equal(perm, torch.arange(perm.numel(), device=perm.device, dtype=perm.dtype)))
+    if len(_IDENTITY_PERMS) > 4096:
+        _IDENTITY_PERMS.clear()
+    _IDENTITY_PERMS[key] = (weakref.ref(owner), version, known)
     return None if known else perm
 
 
@@ -253,6 +262,37 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
     return out
 
 
+def dense_linear(x, layout, bias=None):
+    """``x`` ``[T,K]`` (16-bit, CUDA) times the dequantised weight, without the table kernels' row limit: up to 16 rows
+    without a bias stay packed (the tensor-core kernel rounds the weights as a dense weight would be rounded), the rest goes
+    through dense chunks of the weight in group-sorted column order, with the activations gathered into that order."""
+    planes, scales, zeros, perm = _layout_args(layout)
+    rows, (out_features, in_features) = x.shape[0], (planes.shape[2], x.shape[1])
+    y = torch.empty(rows, out_features, device=x.device, dtype=x.dtype)
+    x = x.contiguous()
+    # the tensor-core kernel rounds a scale to x's dtype first, so bf16 rows with fp16 scales would lose bits there; a bias
+    # added to its rounded output would round twice
+    if rows <= 16 and bias is None and out_features % 32 == 0 and x.data_ptr() % 16 == 0 and x.dtype in (scales.dtype, torch.float16):
+        _native.w3_gemm_small(x, planes, scales, zeros, perm, y)
+        return y
+    if perm is not None:
+        ordered = torch.empty_like(x)
+        _native.gather_columns(x, perm, ordered)
+        x = ordered
+    chunks = -(-out_features * in_features * 2 // DENSE_CHUNK_BYTES)
+    step = -(-(-(-out_features // chunks)) // 64) * 64
+    weight = torch.empty(min(step, out_features), in_features, device=x.device, dtype=x.dtype)
+    for begin in range(0, out_features, step):
+        count = min(step, out_features - begin)
+        _native.w3_dequant([(layout, weight)], x.dtype, row_begin=begin, row_count=count)
+        target = y[:, begin:begin + count]
+        if bias is None:
+            torch.mm(x, weight[:count].t(), out=target)
+        else:
+            torch.addmm(bias[begin:begin + count], x, weight[:count].t(), out=target)
+    return y
+
+
 def qwen3_row_tile(out_features: int, in_features: int) -> int:
     try:
         return QWEN3_ROW_TILE_BY_SHAPE[(out_features, in_features)]
@@ -304,6 +344,7 @@ class PackedW3Linear(nn.Module):
         self.last_route = "not_called"
         self._decode_binding = None
         self._decode_audit = False
+        self._valid_values = None
         self._fields = tuple(name for name in FIELDS + OPTIONAL_FIELDS if name in layout)
         for name in self._fields:
             self.register_buffer(name, layout[name].detach().clone())
@@ -313,6 +354,13 @@ class PackedW3Linear(nn.Module):
 
     def layout(self) -> dict[str, torch.Tensor]:
         return {name: getattr(self, name) for name in self._fields}
+
+    def _require_valid_values(self, layout) -> None:
+        """The value checks of ``validate_planar_w3`` (they synchronise), once per state of the buffers."""
+        stamp = None if any(t.is_inference() for t in layout.values()) else tuple((t.data_ptr(), t._version) for t in layout.values())
+        if stamp is None or stamp != self._valid_values:
+            validate_planar_w3(layout)
+            self._valid_values = stamp
 
     def clear_prepared_decode(self) -> None:
         self._decode_binding = None
@@ -379,7 +427,10 @@ class PackedW3Linear(nn.Module):
                 raise ValueError("unsupported input; enable explicit dense fallback if needed")
             self.last_route = "dense_fallback"
             self.route_counts["dense_fallback"] += 1
-            return F.linear(x, restore_planar_w3(layout, dtype=x.dtype), self.bias)
+            if not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16) or x.device != self.planes.device or rows == 0:
+                return F.linear(x, restore_planar_w3(layout, dtype=x.dtype), self.bias)
+            self._require_valid_values(layout)
+            return dense_linear(x.reshape(rows, self.in_features), layout, self.bias).reshape(*x.shape[:-1], self.out_features)
         self.last_route = "packed_m1"
         self.route_counts["packed_m1"] += 1
         shape = workspace_shape(self.out_features, self.in_features, self.groups_per_split)
