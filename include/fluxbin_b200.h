@@ -376,6 +376,19 @@ int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, const void* k_w
 int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int width, int out_stride, int dtype, fb_stream_t stream);
 
 /*
+ * Checkpoint preparation on the host (plain host memory, no CUDA call): the reference's converter
+ * (gptq_deployment.py:25-205) without tensors of single codes.
+ * fb_host_w3_order: stable order of the input columns by group; FB_ELIMIT if the group indexes do not span
+ *   0 .. K/128 - 1, FB_EINVAL if a group does not hold exactly 128 columns.
+ * fb_host_w3_planes: qweight [3K/32, O] and that order -> planes [K/128, 3, O, 16] (high plane inverted), on at most
+ *   `threads` threads.
+ * fb_host_w3_zeros: qzeros [G, 3O/32] -> zero points [G, O], (code + plus) & 7; bit z of *seen: z occurs.
+ */
+int fb_host_w3_order(const int32_t* g_idx, int in_features, int64_t* order);
+int fb_host_w3_planes(const uint32_t* qweight, const int64_t* order, int in_features, int out_features, uint8_t* planes, int threads);
+int fb_host_w3_zeros(const uint32_t* qzeros, int groups, int out_features, int plus, uint8_t* zeros, unsigned* seen);
+
+/*
  * fb_w3_gemv without a scratch argument, for callers that cannot allocate device memory where
  * they call this library (all memory already handed to a pool, a framework allocator that must
  * not be bypassed, a CUDA graph capture in progress).  The split-K scratch is a fixed array of

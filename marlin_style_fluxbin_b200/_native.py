@@ -128,6 +128,12 @@ def library() -> ctypes.CDLL:
                                           ctypes.c_int] + [ctypes.c_void_p] * 6 + [ctypes.c_size_t, ctypes.c_void_p]
         lib.fb_embed_row.restype = ctypes.c_int
         lib.fb_embed_row.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+        lib.fb_host_w3_order.restype = ctypes.c_int
+        lib.fb_host_w3_order.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+        lib.fb_host_w3_planes.restype = ctypes.c_int
+        lib.fb_host_w3_planes.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_void_p, ctypes.c_int]
+        lib.fb_host_w3_zeros.restype = ctypes.c_int
+        lib.fb_host_w3_zeros.argtypes = [ctypes.c_void_p] + [ctypes.c_int] * 3 + [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint)]
         lib.fb_w3_dequant.restype = ctypes.c_int
         lib.fb_w3_dequant.argtypes = [ctypes.POINTER(W3Matrix)] + [ctypes.c_int] * 6 + [ctypes.c_void_p]
         lib.fb_gather_columns.restype = ctypes.c_int

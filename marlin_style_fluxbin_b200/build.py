@@ -32,19 +32,19 @@ def _nvcc() -> str:
 
 
 def sources() -> list[Path]:
-    return sorted(CSRC.glob("*.cu"))
+    return sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cpp")])
 
 
 def _fingerprint() -> str:
     digest = hashlib.sha256()
-    for path in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [PACKAGE.parent / "include" / "fluxbin_b200.h", Path(__file__)]):
+    for path in sorted(sources() + list(CSRC.glob("*.cuh")) + [PACKAGE.parent / "include" / "fluxbin_b200.h", Path(__file__)]):
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
     return digest.hexdigest()
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` for sm_100a and link the shared library."""
+    """Compile every ``csrc/*.cu`` for sm_100a (and the host-only ``*.cpp``) and link the shared library."""
     fingerprint = _fingerprint()
     if not force and LIBRARY.exists() and STAMP.exists() and STAMP.read_text() == fingerprint:
         return LIBRARY

@@ -18,6 +18,7 @@ general=True)`` produces it.  All conversions are lossless.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Mapping
 
 import torch
@@ -132,8 +133,56 @@ def _bytes_to_bits(values: torch.Tensor) -> torch.Tensor:
     return ((values.to(torch.int32).unsqueeze(-1) >> position) & 1).to(torch.uint8).flatten(-2)
 
 
-def inspect_gptq_checkpoint(tensors: Mapping[str, torch.Tensor], *, qzero_format: int = 1) -> dict[str, object]:
-    """Validate one Linear's raw GPTQ tensors and report its structure (no conversion)."""
+def _native_host():
+    """The library, or None where it is not built (checkpoint preparation needs no GPU and no nvcc then)."""
+    from . import _native
+
+    return _native.library() if _native.LIBRARY.exists() else None
+
+
+def _decoded_zeros(qzeros: torch.Tensor, qzero_format: int) -> tuple[torch.Tensor, list[int]]:
+    """Zero points ``[G,O]`` and the values that occur."""
+    lib = _native_host()
+    if lib is None or qzeros.shape[1] % 3 or qzero_format not in (1, 2) or qzeros.numel() == 0:
+        zeros = unpack_gptq_w3_qzeros(qzeros, qzero_format=qzero_format)
+        return zeros, sorted(int(v) for v in torch.unique(zeros).tolist())
+    groups, out_features = qzeros.shape[0], qzeros.shape[1] // 3 * 32
+    zeros, seen = torch.empty(groups, out_features, dtype=torch.uint8), ctypes.c_uint()
+    if lib.fb_host_w3_zeros(qzeros.data_ptr(), groups, out_features, int(qzero_format == 1), zeros.data_ptr(), ctypes.byref(seen)):
+        raise RuntimeError(lib.fb_last_error().decode())
+    return zeros, [v for v in range(8) if seen.value >> v & 1]
+
+
+def _group_order(g_idx: torch.Tensor, in_features: int) -> torch.Tensor:
+    """Stable order of the columns by group; every group must hold exactly 128 of them."""
+    groups = in_features // GROUP_SIZE
+    lib = _native_host()
+    if tuple(g_idx.shape) == (in_features,) and lib is not None and groups:
+        order = torch.empty(in_features, dtype=torch.int64)
+        code = lib.fb_host_w3_order(g_idx.data_ptr(), in_features, order.data_ptr())
+        if code == 0:
+            return order
+        raise ValueError("g_idx shape or range drifted" if code == -2 else "each g_idx group must contain exactly 128 input columns")
+    if tuple(g_idx.shape) != (in_features,) or int(g_idx.min()) != 0 or int(g_idx.max()) != groups - 1:
+        raise ValueError("g_idx shape or range drifted")
+    if not bool((torch.bincount(g_idx.long(), minlength=groups) == GROUP_SIZE).all()):
+        raise ValueError("each g_idx group must contain exactly 128 input columns")
+    return torch.argsort(g_idx, stable=True)
+
+
+def _sorted_planes(qweight: torch.Tensor, order: torch.Tensor) -> torch.Tensor:
+    """Packed words -> planes ``[G,3,O,16]`` in group-sorted column order."""
+    lib = _native_host()
+    if lib is None:
+        return planes_from_sorted_codes(unpack_gptq_w3_qweight(qweight)[order])
+    in_features, out_features = order.numel(), qweight.shape[1]
+    planes = torch.empty(in_features // GROUP_SIZE, 3, out_features, 16, dtype=torch.uint8)
+    if lib.fb_host_w3_planes(qweight.data_ptr(), order.data_ptr(), in_features, out_features, planes.data_ptr(), torch.get_num_threads()):
+        raise RuntimeError(lib.fb_last_error().decode())
+    return planes
+
+
+def _inspect(tensors: Mapping[str, torch.Tensor], qzero_format: int):
     wanted = {"qweight", "qzeros", "scales", "g_idx"}
     if set(tensors) != wanted:
         raise ValueError(f"expected exactly {sorted(wanted)}")
@@ -143,24 +192,19 @@ def inspect_gptq_checkpoint(tensors: Mapping[str, torch.Tensor], *, qzero_format
     _require_cpu_int32("g_idx", g_idx, 1)
     if scales.device.type != "cpu" or scales.dtype != torch.float16 or scales.ndim != 2:
         raise ValueError("scales must be contiguous CPU float16 [G,O]")
-    if not scales.is_contiguous() or not bool(torch.isfinite(scales).all()):
+    if not scales.is_contiguous() or bool((scales.view(torch.int16) & 0x7C00).eq(0x7C00).any()):  # an all-ones exponent: infinity or NaN
         raise ValueError("scales must be contiguous and finite")
-    codes = unpack_gptq_w3_qweight(qweight)
-    zeros = unpack_gptq_w3_qzeros(qzeros, qzero_format=qzero_format)
-    in_features, out_features = codes.shape
+    if qweight.shape[0] % 3:
+        raise ValueError("packed row count must be divisible by three")
+    in_features, out_features = qweight.shape[0] // 3 * 32, qweight.shape[1]
+    zeros, zero_values = _decoded_zeros(qzeros, qzero_format)
     if in_features % GROUP_SIZE or in_features > MAX_IN_FEATURES:
         raise ValueError("v1 requires K divisible by 128 and representable by int16")
     groups = in_features // GROUP_SIZE
     if tuple(scales.shape) != (groups, out_features) or tuple(zeros.shape) != (groups, out_features):
         raise ValueError("qzero/scale shape does not match qweight")
-    if tuple(g_idx.shape) != (in_features,) or int(g_idx.min()) != 0 or int(g_idx.max()) != groups - 1:
-        raise ValueError("g_idx shape or range drifted")
-    if not bool((torch.bincount(g_idx.long(), minlength=groups) == GROUP_SIZE).all()):
-        raise ValueError("each g_idx group must contain exactly 128 input columns")
-    order = torch.argsort(g_idx, stable=True)
-    if not torch.equal(g_idx[order].long(), torch.arange(in_features) // GROUP_SIZE):
-        raise ValueError("sorted g_idx is not canonical group128")
-    return {
+    order = _group_order(g_idx, in_features)
+    facts = {
         "bits": BITS,
         "group_size": GROUP_SIZE,
         "qweight_shape": list(qweight.shape),
@@ -171,9 +215,15 @@ def inspect_gptq_checkpoint(tensors: Mapping[str, torch.Tensor], *, qzero_format
         "out_features": out_features,
         "groups": groups,
         "qzero_format": qzero_format,
-        "decoded_zero_unique": sorted(int(v) for v in torch.unique(zeros).tolist()),
+        "decoded_zero_unique": zero_values,
         "permutation_identity": bool(torch.equal(order, torch.arange(in_features))),
     }
+    return facts, zeros, order
+
+
+def inspect_gptq_checkpoint(tensors: Mapping[str, torch.Tensor], *, qzero_format: int = 1) -> dict[str, object]:
+    """Validate one Linear's raw GPTQ tensors and report its structure (no conversion)."""
+    return _inspect(tensors, qzero_format)[0]
 
 
 def validate_planar_w3(layout: Mapping[str, torch.Tensor], *, check_values: bool = True) -> tuple[int, int]:
@@ -236,21 +286,19 @@ def convert_gptq_w3_to_planar(
     ``general=True`` the fp16 scales are kept as they are and, unless all zero points are
     4, a ``zeros`` field carries them.
     """
-    facts = inspect_gptq_checkpoint(tensors, qzero_format=qzero_format)
+    facts, zeros, order = _inspect(tensors, qzero_format)
     if not general and facts["decoded_zero_unique"] != [ZERO]:
         raise ValueError(f"v1 constant-zero fast path requires decoded zero=4, got {facts['decoded_zero_unique']}")
-    codes = unpack_gptq_w3_qweight(tensors["qweight"])
-    order = torch.argsort(tensors["g_idx"], stable=True)
     layout = {
-        "planes": planes_from_sorted_codes(codes[order]),
+        "planes": _sorted_planes(tensors["qweight"], order),
         # A checkpoint loaded with dtype=bfloat16 casts its fp16 scales before
         # dequantising; the three-field layout stores exactly that value.
         "scales": (tensors["scales"] if general else tensors["scales"].to(torch.bfloat16)).contiguous(),
-        "perm": order.to(torch.int16).contiguous(),
+        "perm": order.to(torch.int16),
     }
     if general and facts["decoded_zero_unique"] != [ZERO]:
-        layout["zeros"] = unpack_gptq_w3_qzeros(tensors["qzeros"], qzero_format=qzero_format)
-    validate_planar_w3(layout)
+        layout["zeros"] = zeros
+    validate_planar_w3(layout, check_values=False)  # the values were checked above, on the way in
     return layout
 
 
