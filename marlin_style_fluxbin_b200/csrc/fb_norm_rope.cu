@@ -12,20 +12,35 @@ namespace {
 
 using namespace fb;
 
-// One warp per row when LANES == 32, one 256-thread CTA per row otherwise.
+// One warp per row when LANES == 32, one 256-thread CTA per row otherwise.  Bound: one round trip to the row,
+// so all of a thread's elements are requested before the first use (up to kHeld of them; the rest of a longer row
+// in a second pass).
+constexpr int kHeld = 16;
 template <int LANES>
 __global__ void rmsnorm_kernel(const unsigned short* __restrict__ x, const unsigned short* __restrict__ weight,
                                unsigned short* __restrict__ out, int rows, int dim, float eps, int dtype) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int row = LANES == 32 ? (int)(blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) : (int)blockIdx.x;
   const int t = LANES == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
   if (row >= rows) return;
   const unsigned short* xr = x + (size_t)row * dim;
+  unsigned short w[kHeld], v[kHeld];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j) {
+    const bool in = t + j * LANES < dim;
+    v[j] = in ? xr[t + j * LANES] : (unsigned short)0;
+    w[j] = in ? weight[t + j * LANES] : (unsigned short)0;
+  }
   float ss = 0.f;
-  for (int i = t; i < dim; i += LANES) {
-    const float v = bits_to_float(xr[i], dtype);
-    ss += v * v;
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j) {
+    const float f = bits_to_float(v[j], dtype);  // zeros past the end add nothing
+    ss += f * f;
+  }
+  for (int i = t + kHeld * LANES; i < dim; i += LANES) {
+    const float f = bits_to_float(xr[i], dtype);
+    ss += f * f;
   }
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
@@ -35,15 +50,18 @@ __global__ void rmsnorm_kernel(const unsigned short* __restrict__ x, const unsig
     __syncthreads();
     ss = 0.f;
 #pragma unroll
-    for (int w = 0; w < LANES / 32; ++w) ss += part[w];
+    for (int q = 0; q < LANES / 32; ++q) ss += part[q];
   }
   const float inv = rsqrtf(ss / (float)dim + eps);
-  for (int i = t; i < dim; i += LANES) {
-    const float normed = round_to(bits_to_float(xr[i], dtype) * inv, dtype);
-    const float y = bits_to_float(weight[i], dtype) * normed;
+  auto put = [&](int i, unsigned short xv, unsigned short wv) {
+    const float y = bits_to_float(wv, dtype) * round_to(bits_to_float(xv, dtype) * inv, dtype);
     out[(size_t)row * dim + i] = dtype == FB_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y))
                                                   : __half_as_ushort(__float2half_rn(y));
-  }
+  };
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j)
+    if (t + j * LANES < dim) put(t + j * LANES, v[j], w[j]);
+  for (int i = t + kHeld * LANES; i < dim; i += LANES) put(i, xr[i], weight[i]);
 }
 
 __global__ void rope_kernel(const unsigned short* __restrict__ q, const unsigned short* __restrict__ k,
