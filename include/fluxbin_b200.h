@@ -86,7 +86,8 @@ size_t fb_w3_gemv_scratch_bytes(int m, int out_features, int in_features);
  *                             8 input positions per byte, LSB first (G = K/128)
  *   scales  f16|bf16 [G,O]
  *   zeros   uint8 [G,O] zero points, or NULL for the constant zero point 4
- *   perm    int16 [K] sorted position -> input column (desc_act), or NULL for identity
+ *   perm    int16 [K] sorted position -> input column (desc_act), or NULL for identity; like the planes it is
+ *           read ahead of the wait on the launch ahead in the stream
  * W[o, perm[k]] = scale[k/128, o] * (code - zero); accumulation in fp32.  The split over K
  * (up to 16 partial sums per output) is combined inside the kernel by 64-bit integer adds of
  * the partial sums in fixed point (steps of 2^-26), so results do not depend on arrival order:
@@ -101,6 +102,25 @@ int fb_w3_gemv(const void* x, int act_dtype, int m, const uint8_t* planes, const
                int scale_dtype, const uint8_t* zeros, const int16_t* perm, void* out,
                int out_features, int in_features, void* scratch, size_t scratch_bytes,
                unsigned flags, fb_stream_t stream);
+
+/*
+ * Prepared launches: everything about a call that does not change is checked and laid out once (in host
+ * memory, which these entry points do allocate), and a call from then on is one short function.  The weights
+ * must stay where they are until the release.  fb_prepared_run takes x, out and scratch under the rules of the plain
+ * entry point (flags: FB_W3_SAME_INPUT, FB_W3_NO_PDL); it may run on several threads and streams at once,
+ * with a scratch for each.  No counterpart in the reference.
+ */
+typedef struct fb_prepared fb_prepared_t;
+int fb_w3_prepare(int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype, const uint8_t* zeros,
+                  const int16_t* perm, int out_features, int in_features, unsigned flags, fb_prepared_t** launch);
+int fb_w3_prepare_small(int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype, const uint8_t* zeros,
+                        const int16_t* perm, int out_features, int in_features, fb_prepared_t** launch);
+int fb_bb_prepare(int act_dtype, const uint8_t* codes, int planar, const float* rows, const float* cols, const uint8_t* sparse_codes,
+                  const float* sparse_rows, const float* sparse_cols, const int16_t* indices, int out_features, int in_features,
+                  fb_prepared_t** launch);
+int fb_prepared_run(const fb_prepared_t* launch, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags,
+                    fb_stream_t stream);
+void fb_prepared_release(fb_prepared_t* launch);
 
 /*
  * Several W3 matrices that share the activations x and K (q/k/v, or gate/up) in ONE launch:
@@ -365,10 +385,12 @@ int fb_tp_argmax(void* keys, int world, int64_t* best, const int64_t* forced_nex
  * fb_qknorm_rope_prompt: rows of qkv [tokens, q_heads + 2 kv_heads, 128] -> per-head RMSNorm of q and k,
  *   rotary embedding with cos / sin [tokens, 128]; q to q_out [q_heads, tokens, 128], k and v to
  *   positions 0 .. tokens - 1 of the caches [kv_heads, max_positions, 128].
+ * fb_identity_order: writes 1 to *flag (pinned host memory that the device can reach) if perm[k] == k for all k, else 0.
  * fb_silu_mul_rows: out[t, i] = T(silu(gate_up[t, i])) * gate_up[t, width + i]; out rows out_stride apart.
  */
 int fb_w3_dequant(const fb_w3_matrix_t* matrices, int n_matrices, int row_begin, int row_count, int scale_dtype, int in_features,
                   int out_dtype, fb_stream_t stream);
+int fb_identity_order(const int16_t* perm, int in_features, int* flag, fb_stream_t stream);
 int fb_gather_columns(const void* x, const int16_t* perm, void* out, int rows, int in_features, fb_stream_t stream);
 int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, const void* k_weight, const void* cosv, const void* sinv, void* q_out,
                           void* k_cache, void* v_cache, int tokens, int q_heads, int kv_heads, int head_dim, int max_positions, float eps,

@@ -128,6 +128,14 @@ def library() -> ctypes.CDLL:
                                           ctypes.c_int] + [ctypes.c_void_p] * 6 + [ctypes.c_size_t, ctypes.c_void_p]
         lib.fb_embed_row.restype = ctypes.c_int
         lib.fb_embed_row.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+        lib.fb_w3_prepare.restype = lib.fb_w3_prepare_small.restype = lib.fb_bb_prepare.restype = lib.fb_prepared_run.restype = ctypes.c_int
+        lib.fb_w3_prepare.argtypes = [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int] + [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [
+            ctypes.c_uint, ctypes.POINTER(ctypes.c_void_p)]
+        lib.fb_w3_prepare_small.argtypes = lib.fb_w3_prepare.argtypes[:9] + [ctypes.POINTER(ctypes.c_void_p)]
+        lib.fb_bb_prepare.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_int] + [ctypes.c_void_p] * 6 + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_void_p)]
+        lib.fb_prepared_run.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_size_t, ctypes.c_uint, ctypes.c_void_p]
+        lib.fb_prepared_release.restype = None
+        lib.fb_prepared_release.argtypes = [ctypes.c_void_p]
         lib.fb_host_w3_order.restype = ctypes.c_int
         lib.fb_host_w3_order.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
         lib.fb_host_w3_planes.restype = ctypes.c_int
@@ -136,6 +144,8 @@ def library() -> ctypes.CDLL:
         lib.fb_host_w3_zeros.argtypes = [ctypes.c_void_p] + [ctypes.c_int] * 3 + [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint)]
         lib.fb_w3_dequant.restype = ctypes.c_int
         lib.fb_w3_dequant.argtypes = [ctypes.POINTER(W3Matrix)] + [ctypes.c_int] * 6 + [ctypes.c_void_p]
+        lib.fb_identity_order.restype = ctypes.c_int
+        lib.fb_identity_order.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
         lib.fb_gather_columns.restype = ctypes.c_int
         lib.fb_gather_columns.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 2 + [ctypes.c_void_p]
         lib.fb_qknorm_rope_prompt.restype = ctypes.c_int
@@ -172,7 +182,8 @@ def ptr(tensor):
 
 
 def stream_handle(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    index = device.index
+    return ctypes.c_void_p(_raw_stream(_current_device() if index is None else index))
 
 
 def query(key: str) -> int:
@@ -241,6 +252,94 @@ def check_status(device: torch.device | None = None) -> None:
         raise NativeError(f"a device-side wait expired: {bad}; scratch re-zeroed")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_W3_SLOTS = ("w3", "w3#1", "w3#2")
+_NO_PDL, _NO_SAME_INPUT = bool(_os.environ.get("FB_NO_PDL")), bool(_os.environ.get("FB_NO_SAME_INPUT"))
+
+
+def _w3_slot(key, here) -> int:
+    """Which of the three scratches the next plain W3 launch on ``key`` = (device, stream) uses; above 0 it follows a
+    launch on the same activations and need not wait for it.
+
+    Consecutive Linears on the SAME activations (k_proj and v_proj behind q_proj, up_proj behind gate_proj): the launch
+    ahead is a W3 GEMV that read this very buffer, so the buffer was complete before that launch began and this one need
+    not wait for it (FB_W3_SAME_INPUT).  Such launches may overlap, so each takes its own scratch (three rotate; a fourth
+    launch in a row waits again).  Any other call into the library in between, a scratch chosen by the caller, or several
+    rows switch this off, and so does a capture on a stream whose next scratch no warm-up call has allocated."""
+    ahead = _same_input.get(key)
+    if ahead is None or ahead[1] >= 3 or ahead[0] != here or _NO_SAME_INPUT or _NO_PDL:
+        return 0
+    slot = ahead[1]
+    if (*key, _W3_SLOTS[slot]) not in _scratch and torch.cuda.is_current_stream_capturing():
+        return 0
+    return slot
+
+
+class Launch:
+    """A prepared launch of the library: constant arguments checked and laid out once, then one short call each time.
+
+    Holds the tensors whose addresses it keeps, unless told not to (``hold``).  ``kind``: ``"w3"`` (M = 1..4, table kernel), ``"small"`` (M = 1..16,
+    tensor cores) or ``"bb"`` (two-base)."""
+
+    __slots__ = ("kind", "rows", "_handle", "_tensors", "_index", "_follows", "_need", "_width", "_run", "_release")
+
+    def __init__(self, kind, act_dtype, tensors, out_features, in_features, rows=1, decoded=False, hold=True):
+        lib = library()
+        handle, device = ctypes.c_void_p(), tensors[0].device
+        tag = dtype_tag(act_dtype)
+        with torch.cuda.device(device):
+            if kind == "bb":
+                codes, *rest = tensors
+                code = lib.fb_bb_prepare(tag, codes.data_ptr(), int(codes.ndim == 4), *(t.data_ptr() for t in rest), out_features, in_features, ctypes.byref(handle))
+                self._need = bb_scratch_bytes(out_features, in_features, False)
+            else:
+                planes, scales, zeros, perm = tensors
+                args = (tag, rows, planes.data_ptr(), scales.data_ptr(), dtype_tag(scales.dtype), _addr(zeros), _addr(perm), out_features, in_features)
+                if kind == "w3":
+                    code = lib.fb_w3_prepare(*args, FB_W3_DECODED_BF16 if decoded else 0, ctypes.byref(handle))
+                    self._need = w3_scratch_bytes(rows, out_features, in_features)
+                else:
+                    code = lib.fb_w3_prepare_small(*args, ctypes.byref(handle))
+                    self._need = int(lib.fb_w3_gemm_small_scratch_bytes(rows, out_features, in_features))
+        if code:
+            raise NativeError(lib.fb_last_error().decode())
+        self.kind, self.rows, self._handle, self._tensors = kind, rows, handle.value, tensors if hold else None
+        self._index = device.index if device.index is not None else torch.cuda.current_device()
+        self._follows = kind == "w3" and rows == 1
+        self._width, self._run, self._release = in_features, lib.fb_prepared_run, lib.fb_prepared_release
+
+    def __del__(self):
+        if getattr(self, "_release", None) is not None:  # absent when the launch was refused
+            self._release(self._handle)
+
+    def __call__(self, x, out) -> None:
+        """``x`` and ``out`` as the plain entry point takes them, contiguous on the launch's device (the caller checks)."""
+        index = self._index
+        stream = _raw_stream(index)
+        x_ptr = x.data_ptr()
+        flags = FB_W3_NO_PDL if _NO_PDL else 0
+        family = "bb" if self.kind == "bb" else ("w3mma" if self.kind == "small" else "w3")
+        if self._follows:
+            key, here = (index, stream), (x_ptr, (1, self._width), x.dtype)
+            slot = _w3_slot(key, here)
+            if slot:
+                family, flags = _W3_SLOTS[slot], FB_W3_SAME_INPUT
+        buf = _scratch.get((index, stream, family))
+        if buf is None or buf.numel() < self._need:
+            buf = scratch_for(x.device, self._need, family)
+        if _current_device() == index:
+            code = self._run(self._handle, x_ptr, out.data_ptr(), buf.data_ptr(), buf.numel(), flags, stream)
+        else:
+            with torch.cuda.device(index):
+                code = self._run(self._handle, x_ptr, out.data_ptr(), buf.data_ptr(), buf.numel(), flags, stream)
+        _same_input.clear()
+        if code:
+            raise NativeError(library().fb_last_error().decode() or f"native call failed with code {code}")
+        if self._follows and not _NO_PDL:
+            _same_input[key] = (here, slot + 1)
+
+
 def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_partials=False,
             pdl=True, scratch=None) -> None:
     """Raw launch: x [M,K], planes [G,3,O,16], scales [G,O], out [M,O]; see the header.
@@ -248,31 +347,22 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
     With ``group_partials`` ``out`` is the fp32 ``[G,O]`` workspace of the two-call form."""
     m, k = x.shape
     o = planes.shape[2]
-    need = w3_scratch_bytes(m, o, k)
-    if _os.environ.get("FB_NO_PDL"):
-        pdl = False
-    # Consecutive Linears on the SAME activations (k_proj and v_proj behind q_proj, up_proj behind gate_proj): the
-    # launch ahead is a W3 GEMV that read this very buffer, so the buffer was complete before that launch began and
-    # this one need not wait for it (FB_W3_SAME_INPUT).  Such launches may overlap, so each takes its own scratch
-    # (three rotate; a fourth launch in a row waits again).  Any other call into the library in between, a scratch
-    # or a column order chosen by the caller, or several rows switch this off.
-    key = (x.device.index if x.device.index is not None else torch.cuda.current_device(), torch.cuda.current_stream(x.device).cuda_stream)
-    ahead = _same_input.get(key)
-    here = (x.data_ptr(), tuple(x.shape), x.dtype)
-    follow = (ahead is not None and ahead[0] == here and ahead[1] < 3 and scratch is None and pdl and m == 1 and perm is None
-              and not group_partials and not _os.environ.get("FB_NO_SAME_INPUT"))
-    slot = ahead[1] if follow else 0
+    pdl = pdl and not _NO_PDL
+    index = x.get_device()
+    stream = _raw_stream(index)
+    key, here = (index, stream), (x.data_ptr(), (m, k), x.dtype)
     own_scratch = scratch is None
+    slot = _w3_slot(key, here) if own_scratch and pdl and m == 1 and not group_partials else 0  # see _w3_slot
     if own_scratch:
-        scratch = scratch_for(x.device, need, "w3" if slot == 0 else f"w3#{slot}")
+        scratch = scratch_for(x.device, w3_scratch_bytes(m, o, k), _W3_SLOTS[slot])
     flags = (FB_W3_DECODED_BF16 if decoded_bf16 else 0) | (0 if pdl else FB_W3_NO_PDL) | (
-        FB_W3_GROUP_PARTIALS if group_partials else 0) | (FB_W3_SAME_INPUT if follow else 0)
-    with torch.cuda.device(x.device):
+        FB_W3_GROUP_PARTIALS if group_partials else 0) | (FB_W3_SAME_INPUT if slot else 0)
+    with torch.cuda.device(index):
         check(library().fb_w3_gemv(
-            ptr(x), dtype_tag(x.dtype), m, ptr(planes), ptr(scales), dtype_tag(scales.dtype),
-            ptr(zeros), ptr(perm), ptr(out), o, k, ptr(scratch), scratch.numel() * scratch.element_size(),
-            flags, stream_handle(x.device)))
-    if own_scratch and pdl and m == 1 and perm is None and not group_partials:
+            x.data_ptr(), dtype_tag(x.dtype), m, planes.data_ptr(), scales.data_ptr(), dtype_tag(scales.dtype),
+            _addr(zeros), _addr(perm), out.data_ptr(), o, k, scratch.data_ptr(), scratch.numel() * scratch.element_size(),
+            flags, stream))
+    if own_scratch and pdl and m == 1 and not group_partials:
         _same_input[key] = (here, slot + 1)
 
 

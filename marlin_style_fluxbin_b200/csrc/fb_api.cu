@@ -143,6 +143,18 @@ bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, CUtens
 
 extern "C" const char* fb_last_error(void) { return fb::g_error; }
 
+extern "C" int fb_prepared_run(const fb_prepared_t* launch, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags,
+                               fb_stream_t stream) {
+  const fb::Prepared* self = reinterpret_cast<const fb::Prepared*>(launch);
+  if (!self || !x || !out) return fb::fail(FB_EINVAL, "fb_prepared_run: launch, x and out must be non-null");
+  return self->run(self, x, out, scratch, scratch_bytes, flags, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" void fb_prepared_release(fb_prepared_t* launch) {
+  fb::Prepared* self = reinterpret_cast<fb::Prepared*>(launch);
+  if (self) self->destroy(self);
+}
+
 extern "C" int64_t fb_query(const char* key) {
   if (!key) return fb::fail(FB_EINVAL, "fb_query: null key");
   if (!strcmp(key, "version")) return 1;

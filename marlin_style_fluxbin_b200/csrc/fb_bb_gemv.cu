@@ -21,6 +21,7 @@
 //    residual columns): the per-base sums are kept separate through the K split and the row
 //    scales and the residual are applied once, by whoever reduces a row.
 #include <mutex>
+#include <new>
 
 #include "fb_common.cuh"
 
@@ -447,6 +448,20 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   return launch<false, false, 1>(p, grid, smem, info->max_smem_optin, pdl, s);
 }
 
+struct BBPrepared : Prepared {
+  BBParams p;
+};
+
+int run_prepared(const Prepared* base, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags, cudaStream_t stream) {
+  BBParams p = static_cast<const BBPrepared*>(base)->p;
+  if (overlaps(out, (size_t)p.O * 2, x, (size_t)p.K * 2)) return fail(FB_EALIAS, "fb_bb_gemv: out overlaps an input");
+  if (!aligned(x, 16)) return fail(FB_EINVAL, "fb_bb_gemv: x must be 16-byte aligned");
+  if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_gemv: unknown flag bits 0x%x", flags);
+  p.x = x;
+  p.out = out;
+  return run(p, scratch, scratch_bytes, flags, stream, "fb_bb_gemv");
+}
+
 int check_common(const char* who, const void* x, int act_dtype, const uint8_t* codes, void* out, int O, int K) {
   if (!x || !codes || !out) return fail(FB_EINVAL, "%s: x, codes and out must be non-null", who);
   if (act_dtype != FB_F16 && act_dtype != FB_BF16) return fail(FB_EINVAL, "%s: activation dtype must be FB_F16 or FB_BF16", who);
@@ -466,22 +481,51 @@ extern "C" size_t fb_bb_gemv_scratch_bytes(int out_features, int in_features, in
   return kCombineOffset + (size_t)out_features * sizeof(unsigned long long);
 }
 
-extern "C" int fb_bb_gemv(const void* x, int act_dtype, const uint8_t* codes, int planar, const float* rows,
-                          const float* cols, const uint8_t* sparse_codes, const float* sparse_rows,
-                          const float* sparse_cols, const int16_t* indices, void* out, int out_features,
-                          int in_features, void* scratch, size_t scratch_bytes, unsigned flags, fb_stream_t stream) {
+namespace {
+int fill(BBParams& p, const void* x, int act_dtype, const uint8_t* codes, int planar, const float* rows, const float* cols, const uint8_t* sparse_codes,
+         const float* sparse_rows, const float* sparse_cols, const int16_t* indices, void* out, int out_features, int in_features) {
   int rc = check_common("fb_bb_gemv", x, act_dtype, codes, out, out_features, in_features);
   if (rc) return rc;
   if (!rows || !cols || !sparse_codes || !sparse_rows || !sparse_cols || !indices)
     return fail(FB_EINVAL, "fb_bb_gemv: every payload tensor must be non-null");
   if (!aligned(rows, 8) || !aligned(sparse_rows, 8) || !aligned(sparse_codes, 2) || !aligned(cols, 4) || !aligned(sparse_cols, 4))
     return fail(FB_EINVAL, "fb_bb_gemv: scale tensors are misaligned");
-  if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_gemv: unknown flag bits 0x%x", flags);
-  BBParams p = {};
+  p = {};
   p.x = x; p.codes = codes; p.rows = rows; p.cols = cols; p.sparse = sparse_codes; p.srows = sparse_rows;
   p.scols = sparse_cols; p.indices = indices; p.out = out; p.O = out_features; p.K = in_features;
   p.G = in_features / 128; p.act_dtype = act_dtype; p.interleaved = planar ? 0 : 1; p.global_mode = 0;
+  return FB_OK;
+}
+}  // namespace
+
+extern "C" int fb_bb_gemv(const void* x, int act_dtype, const uint8_t* codes, int planar, const float* rows,
+                          const float* cols, const uint8_t* sparse_codes, const float* sparse_rows,
+                          const float* sparse_cols, const int16_t* indices, void* out, int out_features,
+                          int in_features, void* scratch, size_t scratch_bytes, unsigned flags, fb_stream_t stream) {
+  BBParams p;
+  const int rc = fill(p, x, act_dtype, codes, planar, rows, cols, sparse_codes, sparse_rows, sparse_cols, indices, out, out_features, in_features);
+  if (rc) return rc;
+  if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_gemv: unknown flag bits 0x%x", flags);
   return run(p, scratch, scratch_bytes, flags, stream, "fb_bb_gemv");
+}
+
+extern "C" int fb_bb_prepare(int act_dtype, const uint8_t* codes, int planar, const float* rows, const float* cols, const uint8_t* sparse_codes,
+                             const float* sparse_rows, const float* sparse_cols, const int16_t* indices, int out_features, int in_features,
+                             fb_prepared_t** launch) {
+  if (!launch) return fail(FB_EINVAL, "fb_bb_prepare: null result pointer");
+  auto* made = new (std::nothrow) BBPrepared;
+  if (!made) return fail(FB_ELIMIT, "fb_bb_prepare: out of host memory");
+  // addresses that no tensor has stand in for x and out, which come with each run
+  const int rc = fill(made->p, reinterpret_cast<const void*>((uintptr_t)1 << 20), act_dtype, codes, planar, rows, cols, sparse_codes, sparse_rows, sparse_cols, indices,
+                      reinterpret_cast<void*>(64), out_features, in_features);
+  if (rc != FB_OK) {
+    delete made;
+    return rc;
+  }
+  made->run = run_prepared;
+  made->destroy = [](Prepared* self) { delete static_cast<BBPrepared*>(self); };
+  *launch = reinterpret_cast<fb_prepared_t*>(static_cast<Prepared*>(made));
+  return FB_OK;
 }
 
 extern "C" int fb_bb_global_gemv(const void* x, int act_dtype, const uint8_t* codes, const void* row_scales,

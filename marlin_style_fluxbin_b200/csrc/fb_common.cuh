@@ -56,6 +56,13 @@ int launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s
   return FB_OK;
 }
 
+// A launch whose constant arguments were checked and laid out once (fb_w3_prepare and its kin): what changes from
+// call to call comes with run().
+struct Prepared {
+  int (*run)(const Prepared* self, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags, cudaStream_t stream);
+  void (*destroy)(Prepared* self);
+};
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 inline bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
   auto pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);

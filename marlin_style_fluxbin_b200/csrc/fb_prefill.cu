@@ -6,6 +6,7 @@
 //   fb_gather_columns       x[:, perm]: the activations in that order (cheaper than permuting the weight)
 //   fb_qknorm_rope_prompt   per-head RMSNorm of q and k, rotary embedding, k / v into the cache, T tokens
 //   fb_silu_mul_rows        SwiGLU gate of T rows whose gate and up halves lie side by side
+//   fb_identity_order       whether a column order is the identity, told to the host without a wait
 //
 // Without them a 12288 x 4096 weight went through int32 and int64 tensors of its 50 M codes: 2.2 ms
 // measured, against 0.02 ms for its 120 MB of traffic at the copy rate.
@@ -178,6 +179,17 @@ __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const unsigned short
   *reinterpret_cast<uint4*>(out + (size_t)t * out_stride + i) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
+// *flag (device-visible host memory): 1 if perm is the identity, else 0.
+__global__ void __launch_bounds__(1024) identity_order_kernel(const int16_t* __restrict__ perm, int K, int* flag) {
+  int same = 1;
+  for (int k = threadIdx.x; k < K; k += 1024) same &= perm[k] == k;
+  same = __syncthreads_and(same);
+  if (threadIdx.x == 0) {
+    *flag = same;
+    __threadfence_system();
+  }
+}
+
 int launched(const char* what) {
   const cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? FB_OK : cuda_fail(err, what);
@@ -245,4 +257,11 @@ extern "C" int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int wi
   const long long blocks = ((long long)rows * (width / 8) + 255) / 256;
   silu_mul_rows_kernel<<<(int)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(u16(gate_up), u16(out), rows, width, out_stride, dtype);
   return launched("silu_mul_rows launch");
+}
+
+extern "C" int fb_identity_order(const int16_t* perm, int in_features, int* flag, fb_stream_t stream) {
+  if (!perm || !flag) return fail(FB_EINVAL, "fb_identity_order: null pointer");
+  if (in_features < 1 || in_features > 32767) return fail(FB_ELIMIT, "fb_identity_order: K=%d outside 1..32767", in_features);
+  identity_order_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(perm, in_features, flag);
+  return launched("identity_order launch");
 }

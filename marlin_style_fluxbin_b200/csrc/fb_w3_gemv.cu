@@ -25,8 +25,8 @@
 //  * M = 1: scales and zero points of a unit ride with its planes (two more small tiled copies
 //    into the same ring slot), so HBM latency never sits between a unit's lookups and its
 //    result.  M > 1 (no room in the ring): coalesced global loads requested one task ahead.
-//  * Fused producers of x (M = 1): RMSNorm, the SwiGLU gate, or the merge of the attention
-//    launch's per-split pieces.  Every thread transforms ONE of the K block's 256 activations and
+//  * Fused producers of x (M = 1): RMSNorm, the SwiGLU gate, the merge of the attention launch's per-split
+//    pieces, or the gather through a column order (its indexes, constants, are read ahead of the wait).  Every thread transforms ONE of the K block's 256 activations and
 //    shares it through shared memory; the tables are built from the shared values.
 //  * Two lookups are accumulated by one packed fp32x2 add or multiply-add (an even-step and an
 //    odd-step partial sum share a 64-bit register pair; the plane weights 1, 2, -4 ride in the
@@ -49,6 +49,7 @@
 // correction of the dequantised-weight arithmetic (csrc/w3_lut.cu:105-122) is extended to zero
 // points 3 and 4, the two for which +/-3 are the only inexact products.
 #include <mutex>
+#include <new>
 #include <type_traits>
 
 #include "fb_common.cuh"
@@ -214,7 +215,8 @@ __device__ __forceinline__ void emit_combined(const W3Params& p, int m, int ru, 
   p.combine[(size_t)m * p.O + ru * kUnitRows + lane] = 0ull;
 }
 
-template <int M, bool CORRECT>
+// GATHER (M = 1): x is read through the column order p.perm.
+template <int M, bool CORRECT, bool GATHER>
 __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_gemv_kernel(const __grid_constant__ W3Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   using G_ = Geom<M>;
@@ -376,6 +378,14 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
       for (int b = 0; b < 4; ++b) asm volatile("" : "+r"(xl[jh][jw][b]));
     }
 
+  // The column order is part of the weights: this thread's index for the first K block needs no wait.
+  int el_idx = 0;
+  auto fetch_idx = [&](int kb_) {
+    const int e = kb_ * 256 + (int)threadIdx.x;
+    el_idx = threadIdx.x < 256 && e < p.K ? (int)p.perm[e] : 0;
+  };
+  if (GATHER) fetch_idx(kb_begin);
+
   // Everything below reads activations and writes scratch / outputs of this stream.
   if (!p.same_input) {
     pdl_wait_prior_grid();
@@ -384,7 +394,7 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
 
   // Raw 16-bit activations of one lane's table (8 values); the next K block's are fetched while
   // the current one is being computed.
-  const bool fast_x = M == 1 && !p.perm;
+  const bool fast_x = M == 1 && !GATHER && !p.perm;
   auto fetch_x = [&](int kb_, uint4& raw) {
     const int g = 2 * kb_ + (lane >> 4);
     raw = make_uint4(0u, 0u, 0u, 0u);
@@ -393,16 +403,17 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
   // With a fused input transform every thread owns ONE of the K block's 256 activations: it loads
   // the raw value and the operand, transforms them once and shares the result through shared
   // memory, instead of every warp transforming all 256 for itself.
-  const bool shared_x = fast_x && p.prologue != 0;
+  const bool shared_x = GATHER || (fast_x && p.prologue != 0);
   __shared__ __align__(16) float xs[M == 1 ? 256 : 4];
   uint32_t el_raw = 0u, el_op = 0u;
   auto fetch_el = [&](int kb_) {
     const int e = kb_ * 256 + (int)threadIdx.x;
     el_raw = el_op = 0u;
     if (p.prologue != 3 && threadIdx.x < 256 && e < p.K) {
-      el_raw = reinterpret_cast<const unsigned short*>(p.x)[e];
-      el_op = reinterpret_cast<const unsigned short*>(p.prologue_arg)[e];
+      el_raw = reinterpret_cast<const unsigned short*>(p.x)[GATHER ? el_idx : e];
+      if (!GATHER) el_op = reinterpret_cast<const unsigned short*>(p.prologue_arg)[e];
     }
+    if (GATHER) fetch_idx(kb_ + 1);
   };
   // requested before the RMS reduction below, so that the two round trips overlap
   uint4 raw_next = make_uint4(0u, 0u, 0u, 0u);
@@ -500,7 +511,8 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
           // same roundings as the separate kernels: RMSNorm casts before the weight multiply,
           // SwiGLU rounds silu(gate) before the product
           const float v = bits_to_float((unsigned short)el_raw, p.act_dtype), other = bits_to_float((unsigned short)el_op, p.act_dtype);
-          xs[M == 1 ? threadIdx.x : 0] = p.prologue == 1 ? round_to(other * round_to(v * inv_rms, p.act_dtype), p.act_dtype)
+          xs[M == 1 ? threadIdx.x : 0] = GATHER            ? v
+                                         : p.prologue == 1 ? round_to(other * round_to(v * inv_rms, p.act_dtype), p.act_dtype)
                                                            : round_to(round_to(v / (1.f + __expf(-v)), p.act_dtype) * other, p.act_dtype);
         }
         if (kb_ + 1 < kb_begin + nS) fetch_el(kb_ + 1);
@@ -806,8 +818,8 @@ Plan make_plan(int m, int nKB, int nRU, const DeviceInfo& info) {
   return plan;
 }
 
-template <int M, bool CORRECT>
-int launch(const W3Params& p, const Plan& plan, bool pdl, cudaStream_t stream) {
+template <int M, bool CORRECT, bool GATHER>
+int launch_one(const W3Params& p, const Plan& plan, bool pdl, cudaStream_t stream) {
   // Raising the dynamic shared memory limit is a per-device, per-kernel setting; do it once.
   static std::mutex lock;
   static bool ready[64] = {};
@@ -818,7 +830,7 @@ int launch(const W3Params& p, const Plan& plan, bool pdl, cudaStream_t stream) {
   {
     std::lock_guard<std::mutex> guard(lock);
     if (!ready[device]) {
-      err = cudaFuncSetAttribute(w3_gemv_kernel<M, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
+      err = cudaFuncSetAttribute(w3_gemv_kernel<M, CORRECT, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
       if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(w3_gemv_kernel)");
       ready[device] = true;
     }
@@ -833,9 +845,15 @@ int launch(const W3Params& p, const Plan& plan, bool pdl, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = pdl && pdl_allowed() ? 1 : 0;
-  err = cudaLaunchKernelEx(&config, w3_gemv_kernel<M, CORRECT>, p);
+  err = cudaLaunchKernelEx(&config, w3_gemv_kernel<M, CORRECT, GATHER>, p);
   if (err != cudaSuccess) return cuda_fail(err, "w3_gemv_kernel launch");
   return FB_OK;
+}
+
+template <int M, bool CORRECT>
+int launch(const W3Params& p, const Plan& plan, bool pdl, cudaStream_t stream) {
+  if (M == 1 && p.perm) return launch_one<M, CORRECT, M == 1>(p, plan, pdl, stream);
+  return launch_one<M, CORRECT, false>(p, plan, pdl, stream);
 }
 
 // Scratch layout, identical for every problem size so that one scratch can serve calls of
@@ -860,9 +878,32 @@ extern "C" size_t fb_w3_gemv_scratch_bytes(int m, int out_features, int in_featu
 
 namespace {
 
+void bind_scratch(W3Params& p, void* scratch) {
+  unsigned char* base = static_cast<unsigned char*>(scratch);
+  p.status = reinterpret_cast<unsigned*>(base);
+  p.combine = reinterpret_cast<unsigned long long*>(base + kCombineOffset);
+  p.partials = reinterpret_cast<float*>(base + kPartialsOffset);
+}
+
+int dispatch(const W3Params& p, const Plan& plan, int m, bool correct, bool pdl, cudaStream_t s) {
+#define FB_DISPATCH(MM) \
+  case MM:              \
+    return correct ? launch<MM, true>(p, plan, pdl, s) : launch<MM, false>(p, plan, pdl, s);
+  switch (m) {
+    FB_DISPATCH(1)
+    FB_DISPATCH(2)
+    FB_DISPATCH(3)
+    FB_DISPATCH(4)
+  }
+#undef FB_DISPATCH
+  return fail(FB_ELIMIT, "fb_w3_gemv: unsupported M");
+}
+
+// Checks the arguments and lays the launch out.  With `keep` the launch is only kept there (x, out and scratch
+// come later).
 int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrices, int n_matrices, int scale_dtype,
               const int16_t* perm, int in_features, void* scratch, size_t scratch_bytes, unsigned flags,
-              fb_stream_t stream, int prologue, const void* prologue_arg, float eps, const fb_w3_push_t* push = nullptr) {
+              fb_stream_t stream, int prologue, const void* prologue_arg, float eps, const fb_w3_push_t* push = nullptr, W3Params* keep = nullptr, Plan* keep_plan = nullptr) {
   const int K = in_features;
   if (push) {
     if (m != 1 || n_matrices != 1 || (flags & FB_W3_GROUP_PARTIALS) || matrices[0].residual)
@@ -945,9 +986,11 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   }
   if (total > 65536) return fail(FB_ELIMIT, "fb_w3_gemv: %lld output rows in one launch, at most 65536", total);
   const size_t need = fb_w3_gemv_scratch_bytes(m, (int)total, K);
-  if (!scratch || scratch_bytes < need) return fail(FB_ESCRATCH, "fb_w3_gemv: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
-  if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemv: scratch must be 256-byte aligned");
-  if (overlaps(scratch, need, x, x_bytes)) return fail(FB_EALIAS, "fb_w3_gemv: scratch overlaps x");
+  if (!keep) {
+    if (!scratch || scratch_bytes < need) return fail(FB_ESCRATCH, "fb_w3_gemv: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
+    if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemv: scratch must be 256-byte aligned");
+    if (overlaps(scratch, need, x, x_bytes)) return fail(FB_EALIAS, "fb_w3_gemv: scratch overlaps x");
+  }
 
   const DeviceInfo* info = device_info();
   if (!info) return FB_ECUDA;
@@ -958,10 +1001,7 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   p.nRU = (int)(total / kUnitRows);
   p.act_dtype = act_dtype;
   p.scale_dtype = scale_dtype;
-  unsigned char* base = static_cast<unsigned char*>(scratch);
-  p.status = reinterpret_cast<unsigned*>(base);
-  p.combine = reinterpret_cast<unsigned long long*>(base + kCombineOffset);
-  p.partials = reinterpret_cast<float*>(base + kPartialsOffset);
+  if (scratch) bind_scratch(p, scratch);
   const Plan plan = make_plan(m, p.nKB, p.nRU, *info);
   p.S = plan.S;
   p.units_per_slice = p.nRU / plan.slices;
@@ -970,22 +1010,63 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   p.group_partials = group_partials ? 1 : 0;
   p.same_input = (flags & FB_W3_SAME_INPUT) ? 1 : 0;
   if (plan.smem > (size_t)info->max_smem_optin) return fail(FB_ELIMIT, "fb_w3_gemv: plan needs %zu bytes of shared memory", plan.smem);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool correct = (flags & FB_W3_DECODED_BF16) != 0;
-  const bool pdl = (flags & FB_W3_NO_PDL) == 0;
-#define FB_DISPATCH(MM) \
-  case MM:              \
-    return correct ? launch<MM, true>(p, plan, pdl, s) : launch<MM, false>(p, plan, pdl, s);
-  switch (m) {
-    FB_DISPATCH(1)
-    FB_DISPATCH(2)
-    FB_DISPATCH(3)
-    FB_DISPATCH(4)
+  if (keep) {
+    *keep = p;
+    *keep_plan = plan;
+    return FB_OK;
   }
-#undef FB_DISPATCH
-  return fail(FB_ELIMIT, "fb_w3_gemv: unsupported M");
+  return dispatch(p, plan, m, (flags & FB_W3_DECODED_BF16) != 0, (flags & FB_W3_NO_PDL) == 0, static_cast<cudaStream_t>(stream));
+}
+
+struct W3Prepared : Prepared {
+  W3Params p;
+  Plan plan;
+  int m;
+  bool correct;
+  size_t need;
+};
+
+int run_prepared(const Prepared* base, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags, cudaStream_t stream) {
+  const W3Prepared& self = *static_cast<const W3Prepared*>(base);
+  const size_t x_bytes = (size_t)self.m * self.p.K * 2, out_bytes = (size_t)self.m * self.p.O * 2;
+  if (!aligned(x, self.p.perm ? 2 : 16)) return fail(FB_EINVAL, "fb_w3_gemv: x must be 16-byte aligned");
+  if (!aligned(out, 2)) return fail(FB_EINVAL, "fb_w3_gemv: 16-bit tensors must be 2-byte aligned");
+  if (!scratch || scratch_bytes < self.need) return fail(FB_ESCRATCH, "fb_w3_gemv: scratch of %zu bytes needed, %zu given", self.need, scratch_bytes);
+  if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemv: scratch must be 256-byte aligned");
+  if (overlaps(out, out_bytes, x, x_bytes) || overlaps(scratch, self.need, x, x_bytes) || overlaps(scratch, self.need, out, out_bytes))
+    return fail(FB_EALIAS, "fb_w3_gemv: out overlaps an input, or scratch overlaps x or out");
+  if (flags & ~(FB_W3_NO_PDL | FB_W3_SAME_INPUT)) return fail(FB_EINVAL, "fb_w3_gemv: unknown flag bits 0x%x", flags);
+  W3Params p = self.p;
+  p.x = x;
+  p.mats[0].out = out;
+  bind_scratch(p, scratch);
+  p.same_input = (flags & FB_W3_SAME_INPUT) ? 1 : 0;
+  return dispatch(p, self.plan, self.m, self.correct, (flags & FB_W3_NO_PDL) == 0, stream);
 }
 }  // namespace
+
+extern "C" int fb_w3_prepare(int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype, const uint8_t* zeros, const int16_t* perm,
+                             int out_features, int in_features, unsigned flags, fb_prepared_t** out_launch) {
+  if (!out_launch) return fail(FB_EINVAL, "fb_w3_prepare: null result pointer");
+  if (flags & ~FB_W3_DECODED_BF16) return fail(FB_EINVAL, "fb_w3_prepare: flags 0x%x: only FB_W3_DECODED_BF16 is fixed here", flags);
+  // addresses that no tensor has stand in for x and out, which come with each run
+  fb_w3_matrix_t one = {planes, scales, zeros, reinterpret_cast<void*>(64), nullptr, out_features};
+  auto* made = new (std::nothrow) W3Prepared;
+  if (!made) return fail(FB_ELIMIT, "fb_w3_prepare: out of host memory");
+  const int rc = run_multi(reinterpret_cast<const void*>((uintptr_t)1 << 20), act_dtype, m, &one, 1, scale_dtype, perm, in_features, nullptr, 0, flags, nullptr, 0,
+                           nullptr, 0.f, nullptr, &made->p, &made->plan);
+  if (rc != FB_OK) {
+    delete made;
+    return rc;
+  }
+  made->run = run_prepared;
+  made->destroy = [](Prepared* self) { delete static_cast<W3Prepared*>(self); };
+  made->m = m;
+  made->correct = (flags & FB_W3_DECODED_BF16) != 0;
+  made->need = fb_w3_gemv_scratch_bytes(m, out_features, in_features);
+  *out_launch = reinterpret_cast<fb_prepared_t*>(static_cast<Prepared*>(made));
+  return FB_OK;
+}
 
 extern "C" int fb_w3_gemv_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrices, int n_matrices,
                                 int scale_dtype, const int16_t* perm, int in_features, void* scratch,

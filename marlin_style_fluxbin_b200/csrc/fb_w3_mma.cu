@@ -31,6 +31,7 @@
 #include <cudaTypedefs.h>
 
 #include <mutex>
+#include <new>
 #include <type_traits>
 
 #include "fb_common.cuh"
@@ -341,53 +342,63 @@ extern "C" size_t fb_w3_gemm_small_scratch_bytes(int m, int out_features, int in
   return kCombineOffset + (size_t)m * out_features * sizeof(unsigned long long);
 }
 
-extern "C" int fb_w3_gemm_small(const void* x, int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype,
-                                const uint8_t* zeros, const int16_t* perm, void* out, int out_features, int in_features,
-                                void* scratch, size_t scratch_bytes, fb_stream_t stream) {
-  const int O = out_features, K = in_features;
-  if (!x || !planes || !scales || !out) return fail(FB_EINVAL, "fb_w3_gemm_small: x, planes, scales and out must be non-null");
+namespace {
+
+struct MmaPrepared : Prepared {
+  MmaParams p;
+  int tiles;
+  size_t need;
+};
+
+// The arguments that do not change from call to call.
+int fill(MmaPrepared& made, int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype, const uint8_t* zeros,
+         const int16_t* perm, int O, int K) {
+  if (!planes || !scales) return fail(FB_EINVAL, "fb_w3_gemm_small: x, planes, scales and out must be non-null");
   if ((act_dtype != FB_F16 && act_dtype != FB_BF16) || (scale_dtype != FB_F16 && scale_dtype != FB_BF16))
     return fail(FB_EINVAL, "fb_w3_gemm_small: dtype tags must be FB_F16 or FB_BF16");
   if (m < 1 || m > kN) return fail(FB_ELIMIT, "fb_w3_gemm_small: M=%d outside 1..%d", m, kN);
   if (K < 128 || K % 128 || K / 128 > 255) return fail(FB_ELIMIT, "fb_w3_gemm_small: K=%d must be a multiple of 128 with at most 255 groups", K);
   if (O < 32 || O > 65536 || O % 32) return fail(FB_ELIMIT, "fb_w3_gemm_small: O=%d must be a multiple of 32 in 32..65536", O);
-  if (!aligned(planes, 16) || !aligned(scales, 2) || !aligned(out, 2) || !aligned(perm, 2))
+  if (!aligned(planes, 16) || !aligned(scales, 2) || !aligned(perm, 2))
     return fail(FB_EINVAL, "fb_w3_gemm_small: planes must be 16-byte aligned, 16-bit tensors 2-byte aligned");
-  if (!perm && !aligned(x, 16)) return fail(FB_EINVAL, "fb_w3_gemm_small: x must be 16-byte aligned");
   const int G = K / 128;
-  const size_t x_bytes = (size_t)m * K * 2, out_bytes = (size_t)m * O * 2;
-  if (overlaps(out, out_bytes, x, x_bytes) || overlaps(out, out_bytes, planes, (size_t)G * 3 * O * 16) ||
-      overlaps(out, out_bytes, scales, (size_t)G * O * 2))
-    return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input");
-  const size_t need = fb_w3_gemm_small_scratch_bytes(m, O, K);
-  if (!scratch || scratch_bytes < need) return fail(FB_ESCRATCH, "fb_w3_gemm_small: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
-  if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemm_small: scratch must be 256-byte aligned");
-  if (overlaps(scratch, need, out, out_bytes) || overlaps(scratch, need, x, x_bytes)) return fail(FB_EALIAS, "fb_w3_gemm_small: scratch overlaps x or out");
-
   const DeviceInfo* info = device_info();
   if (!info) return FB_ECUDA;
-  MmaParams p;
+  MmaParams& p = made.p;
   if (!plane_tensor_map(planes, O, G, kTileRows / 32, 3, &p.plane_map)) return FB_ECUDA;
-  p.x = x;
   p.scales = static_cast<const unsigned short*>(scales);
   p.zeros = zeros;
   p.perm = perm;
-  p.out = out;
-  p.status = reinterpret_cast<unsigned*>(scratch);
-  p.combine = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + kCombineOffset);
   p.M = m;
   p.O = O;
   p.K = K;
   p.G = G;
   p.act_dtype = act_dtype;
   p.scale_dtype = scale_dtype;
-  const int tiles = (O + kTileRows - 1) / kTileRows;
-  int splits = 2 * info->sm_count / tiles;
+  made.tiles = (O + kTileRows - 1) / kTileRows;
+  int splits = 2 * info->sm_count / made.tiles;
   if (splits < 1) splits = 1;
   if (splits > kMaxSplits) splits = kMaxSplits;
   if (splits > G) splits = G;
   p.groups_per_split = (G + splits - 1) / splits;
   p.splits = (G + p.groups_per_split - 1) / p.groups_per_split;
+  made.need = fb_w3_gemm_small_scratch_bytes(m, O, K);
+  return FB_OK;
+}
+
+int run_small(const Prepared* base, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags, cudaStream_t stream) {
+  const MmaPrepared& self = *static_cast<const MmaPrepared*>(base);
+  MmaParams p = self.p;
+  if (!aligned(out, 2) || !aligned(x, p.perm ? 2 : 16)) return fail(FB_EINVAL, "fb_w3_gemm_small: x must be 16-byte aligned, out 2-byte aligned");
+  const size_t x_bytes = (size_t)p.M * p.K * 2, out_bytes = (size_t)p.M * p.O * 2;
+  if (overlaps(out, out_bytes, x, x_bytes)) return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input");
+  if (!scratch || scratch_bytes < self.need) return fail(FB_ESCRATCH, "fb_w3_gemm_small: scratch of %zu bytes needed, %zu given", self.need, scratch_bytes);
+  if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemm_small: scratch must be 256-byte aligned");
+  if (overlaps(scratch, self.need, out, out_bytes) || overlaps(scratch, self.need, x, x_bytes)) return fail(FB_EALIAS, "fb_w3_gemm_small: scratch overlaps x or out");
+  p.x = x;
+  p.out = out;
+  p.status = reinterpret_cast<unsigned*>(scratch);
+  p.combine = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + kCombineOffset);
 
   const size_t smem = 2 * (size_t)kATile + 2 * kBTile + kPlaneStages * kPlaneTile + 128 + 16384;  // tiles, barriers, spread table
   static std::mutex lock;
@@ -404,16 +415,47 @@ extern "C" int fb_w3_gemm_small(const void* x, int act_dtype, int m, const uint8
     }
   }
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(tiles, p.splits);
+  config.gridDim = dim3(self.tiles, p.splits);
   config.blockDim = dim3(kThreads);
   config.dynamicSmemBytes = smem;
-  config.stream = static_cast<cudaStream_t>(stream);
+  config.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
-  config.numAttrs = pdl_allowed() ? 1 : 0;
-  cudaError_t err = act_dtype == FB_BF16 ? cudaLaunchKernelEx(&config, w3_mma_kernel<true>, p) : cudaLaunchKernelEx(&config, w3_mma_kernel<false>, p);
+  config.numAttrs = pdl_allowed() && !(flags & FB_W3_NO_PDL) ? 1 : 0;
+  cudaError_t err = p.act_dtype == FB_BF16 ? cudaLaunchKernelEx(&config, w3_mma_kernel<true>, p) : cudaLaunchKernelEx(&config, w3_mma_kernel<false>, p);
   if (err != cudaSuccess) return cuda_fail(err, "w3_mma_kernel launch");
   return FB_OK;
+}
+
+}  // namespace
+
+extern "C" int fb_w3_prepare_small(int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype, const uint8_t* zeros,
+                                   const int16_t* perm, int out_features, int in_features, fb_prepared_t** launch) {
+  if (!launch) return fail(FB_EINVAL, "fb_w3_prepare_small: null result pointer");
+  auto* made = new (std::nothrow) MmaPrepared;
+  if (!made) return fail(FB_ELIMIT, "fb_w3_prepare_small: out of host memory");
+  const int rc = fill(*made, act_dtype, m, planes, scales, scale_dtype, zeros, perm, out_features, in_features);
+  if (rc != FB_OK) {
+    delete made;
+    return rc;
+  }
+  made->run = run_small;
+  made->destroy = [](Prepared* self) { delete static_cast<MmaPrepared*>(self); };
+  *launch = reinterpret_cast<fb_prepared_t*>(static_cast<Prepared*>(made));
+  return FB_OK;
+}
+
+extern "C" int fb_w3_gemm_small(const void* x, int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype,
+                                const uint8_t* zeros, const int16_t* perm, void* out, int out_features, int in_features,
+                                void* scratch, size_t scratch_bytes, fb_stream_t stream) {
+  if (!x || !out) return fail(FB_EINVAL, "fb_w3_gemm_small: x, planes, scales and out must be non-null");
+  MmaPrepared made;
+  const int rc = fill(made, act_dtype, m, planes, scales, scale_dtype, zeros, perm, out_features, in_features);
+  if (rc != FB_OK) return rc;
+  const size_t out_bytes = (size_t)m * out_features * 2;
+  if (overlaps(out, out_bytes, planes, (size_t)in_features / 128 * 3 * out_features * 16) || overlaps(out, out_bytes, scales, (size_t)in_features / 128 * out_features * 2))
+    return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input");
+  return run_small(&made, x, out, scratch, scratch_bytes, 0, static_cast<cudaStream_t>(stream));
 }

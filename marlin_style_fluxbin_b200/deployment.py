@@ -10,6 +10,7 @@ otherwise) and the workspace shape contract, and all run the one sm_100a kernel
 """
 from __future__ import annotations
 
+import weakref
 from types import SimpleNamespace
 from typing import Mapping
 
@@ -297,19 +298,23 @@ class PackedHybridLinear(nn.Module):
         output = self._decode_output
         shaped = output.view(1, 1, self.out_features)
         expected = (1, 1, self.in_features)
-        in_features = self.in_features
+        index, buffers = output.get_device(), self._buffers
+        module = weakref.ref(self)  # no cycle: a dropped module gives its weights back at once
+        launch = _native.Launch("bb", dtype, tuple(layout[name] for name in ("codes", "rows", "columns", "sparse_codes", "sparse_rows", "sparse_columns",
+                                                                             "indices")), self.out_features, self.in_features)
 
         def apply(x):
             if torch.is_grad_enabled():
                 raise RuntimeError("prepared decode is inference only")
-            if tuple(x.shape) != expected or x.dtype != dtype or x.device != device or not x.is_contiguous():
+            if x.shape != expected or x.dtype != dtype or x.get_device() != index or not x.is_contiguous():
                 raise ValueError("prepared decode input shape/dtype/device/stride mismatch")
-            if self._decode_audit:
-                self.route_counts["packed_m1"] += 1
-                self.last_route = "packed_m1"
-            _native.bb_gemv(x.view(1, in_features), layout, output)
-            if self.bias is not None:
-                output.add_(self.bias)
+            me = module()
+            if me is not None and me._decode_audit:
+                me.route_counts["packed_m1"] += 1
+                me.last_route = "packed_m1"
+            launch(x, output)
+            if buffers["bias"] is not None:
+                output.add_(buffers["bias"])
             return shaped
 
         self._decode_binding = apply

@@ -119,26 +119,54 @@ def load_w3_lut_extension(row_tile: int, uniform_index_probe: bool = False):
                            finish=finish, m1_out=m1_out)
 
 
-# perm tensors that were checked to be the identity: the kernel then skips the gather.  Keyed by address, and an
-# entry holds only while the tensor it was made for lives unchanged (another one may get the address later).
+# Whether a perm tensor is the identity (the kernels then skip the gather).  A kernel compares it on the stream and
+# writes the answer to a word of pinned host memory, so that asking costs no wait: -1 until it has run.  Keyed by address,
+# and an entry holds only while the tensor it was made for lives unchanged (another one may get the address later).
 _IDENTITY_PERMS: dict[tuple[int, int], tuple] = {}
+_MAX_PERMS = 4096
+_perm_flags = None
 
 
-def _perm_or_none(perm: torch.Tensor):
-    """``None`` when ``perm`` is the identity (decided once per tensor, outside capture)."""
-    key = (perm.data_ptr(), perm.numel())
-    owner = perm if perm._base is None else perm._base
-    version = None if perm.is_inference() else perm._version
-    entry = _IDENTITY_PERMS.get(key)
-    if entry is not None and entry[0]() is owner and entry[1] == version:
-        return None if entry[2] else perm
-    if torch.cuda.is_current_stream_capturing():
-        return perm  # cannot inspect values now; the general gather path is always valid
-    known = bool(torch.equal(perm, torch.arange(perm.numel(), device=perm.device, dtype=perm.dtype)))
-    if len(_IDENTITY_PERMS) > 4096:
+def _perm_entry(perm: torch.Tensor):
+    """``(owner, version, slot)`` of a perm that was asked about, or None."""
+    entry = _IDENTITY_PERMS.get((perm.data_ptr(), perm.numel()))
+    if entry is None or entry[0]() is not (perm if perm._base is None else perm._base) or entry[1] != (None if perm.is_inference() else perm._version):
+        return None
+    return entry
+
+
+def _ask_perm(perm: torch.Tensor):
+    global _perm_flags
+    if _perm_flags is None:
+        pinned = torch.empty(_MAX_PERMS, dtype=torch.int32, pin_memory=True)
+        _perm_flags = (pinned, pinned.numpy())
+    if len(_IDENTITY_PERMS) >= _MAX_PERMS:
+        torch.cuda.synchronize(perm.device)  # no answer to a forgotten question may land in a slot that is used again
         _IDENTITY_PERMS.clear()
-    _IDENTITY_PERMS[key] = (weakref.ref(owner), version, known)
-    return None if known else perm
+    slot = len(_IDENTITY_PERMS)
+    key = (perm.data_ptr(), perm.numel())
+    if key in _IDENTITY_PERMS:
+        slot = _IDENTITY_PERMS[key][2]
+    _perm_flags[1][slot] = -1
+    with torch.cuda.device(perm.device):
+        _native.check(_native.library().fb_identity_order(perm.data_ptr(), perm.numel(), _perm_flags[0].data_ptr() + 4 * slot, _native.stream_handle(perm.device)))
+    entry = _IDENTITY_PERMS[key] = (weakref.ref(perm if perm._base is None else perm._base), None if perm.is_inference() else perm._version, slot)
+    return entry
+
+
+def _perm_or_none(perm: torch.Tensor, wait: bool = True):
+    """``None`` when ``perm`` is the identity.  ``perm`` itself, which is always valid, when it is not, or when that is not
+    known yet and must not (a capture) or need not (``wait``) be waited for."""
+    entry = _perm_entry(perm)
+    if entry is None:
+        if torch.cuda.is_current_stream_capturing():
+            return perm
+        entry = _ask_perm(perm)
+    known = int(_perm_flags[1][entry[2]])
+    if known < 0 and wait and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(perm.device).synchronize()
+        known = int(_perm_flags[1][entry[2]])
+    return None if known == 1 else perm
 
 
 def _check_native_args(x, planes, scales, perm, partial, splits) -> None:
@@ -177,8 +205,68 @@ def workspace_shape(out_features: int, in_features: int, groups_per_split: int =
     return -(-groups // groups_per_split), out_features
 
 
-def _layout_args(layout):
-    return layout["planes"], layout["scales"], layout.get("zeros"), _perm_or_none(layout["perm"])
+def _layout_args(layout, wait=True):
+    return layout["planes"], layout["scales"], layout.get("zeros"), _perm_or_none(layout["perm"], wait)
+
+
+class _LayoutRecord:
+    """A validated layout and the launches prepared for it.  Holds no tensor: it goes when the planes go."""
+
+    __slots__ = ("out_features", "in_features", "index", "_seen", "_perm_version", "launches", "keeper")
+
+    def __init__(self, layout):
+        self.out_features, self.in_features = validate_planar_w3(layout, check_values=False)
+        self._seen = tuple((name, weakref.ref(value), value.data_ptr()) for name, value in layout.items())
+        self._perm_version = self._version(layout["perm"])
+        self.index, self.launches = layout["planes"].get_device(), {}
+
+    @staticmethod
+    def _version(tensor):
+        return None if tensor.is_inference() else tensor._version
+
+    def describes(self, layout) -> bool:
+        if len(layout) != len(self._seen):
+            return False
+        for name, ref, address in self._seen:
+            value = layout.get(name)
+            if value is None or ref() is not value or value.data_ptr() != address:
+                return False
+        return self._version(layout["perm"]) == self._perm_version
+
+
+_RECORDS: dict[int, _LayoutRecord] = {}
+
+
+def _layout_record(layout) -> _LayoutRecord:
+    planes = layout.get("planes")
+    key = id(planes)
+    record = _RECORDS.get(key)
+    if record is None or not record.describes(layout):
+        record = _LayoutRecord(layout)
+        record.keeper = weakref.ref(planes, lambda _: _RECORDS.pop(key, None))
+        _RECORDS[key] = record
+    return record
+
+
+def _launch_layout(record, layout, x, out, kind, decoded) -> None:
+    key = (kind, x.shape[0], x.dtype, decoded)
+    launch = record.launches.get(key, 0)
+    if not launch or not (x.get_device() == record.index and x.is_contiguous() and out.is_contiguous()):
+        # a first call, odd operands, or a column order that cannot be looked at now: the plain entry points.  The second
+        # call prepares the launch (about 40 us), which pays from a few calls on.
+        prepare = launch is None and not torch.cuda.is_current_stream_capturing()
+        if launch == 0:
+            record.launches[key] = None
+        elif prepare:
+            record.launches[key] = _native.Launch(kind, x.dtype, _layout_args(layout), record.out_features, record.in_features,
+                                                  rows=x.shape[0], decoded=decoded, hold=False)
+        planes, scales, zeros, perm = _layout_args(layout, wait=False)
+        if kind == "small":
+            _native.w3_gemm_small(x, planes, scales, zeros, perm, out)
+        else:
+            _native.w3_gemv(x, planes, scales, zeros, perm, out, decoded_bf16=decoded)
+        return
+    launch(x, out)
 
 
 def inline_main(x, layout, workspace, *, row_tile: int, arithmetic: str = "structural") -> None:
@@ -219,7 +307,8 @@ def w3_lut_m1_out(x, layout, out, workspace, *, row_tile: int, groups_per_split:
         raise ValueError("out dtype must match x dtype")
     if arithmetic not in ARITHMETIC_MODES:
         raise ValueError(f"arithmetic must be one of {ARITHMETIC_MODES}")
-    out_features, in_features = validate_planar_w3(layout, check_values=False)
+    record = _layout_record(layout)
+    out_features, in_features = record.out_features, record.in_features
     if x.shape != (1, in_features) or out.shape != (1, out_features):
         raise ValueError("x/out shape mismatch")
     if workspace.shape != workspace_shape(out_features, in_features, groups_per_split) or workspace.dtype != torch.float32:
@@ -227,8 +316,7 @@ def w3_lut_m1_out(x, layout, out, workspace, *, row_tile: int, groups_per_split:
     if workspace.device != x.device or out.device != x.device:
         raise ValueError("x, out and workspace must share a device")
     load_w3_lut_extension(row_tile)
-    planes, scales, zeros, perm = _layout_args(layout)
-    _native.w3_gemv(x, planes, scales, zeros, perm, out, decoded_bf16=arithmetic == "decoded_bf16")
+    _launch_layout(record, layout, x, out, "w3", arithmetic == "decoded_bf16")
     return out
 
 
@@ -240,25 +328,21 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
     dtype, as the reference's dense fallback rounds them), ``"auto"`` picks ``"lut"`` up to M = 4
     (measured faster there on the Qwen3-8B shapes) and ``"mma"`` above.
     """
-    out_features, in_features = validate_planar_w3(layout, check_values=False)
-    if x.ndim != 2 or x.shape[1] != in_features or tuple(out.shape) != (x.shape[0], out_features):
+    record = _layout_record(layout)
+    rows = x.shape[0] if x.ndim else 0
+    if x.ndim != 2 or x.shape[1] != record.in_features or out.shape != (rows, record.out_features):
         raise ValueError("x/out shape mismatch")
     if out.dtype != x.dtype or out.device != x.device:
         raise ValueError("out must match x in dtype and device")
-    if kernel not in ("auto", "lut", "mma"):
-        raise ValueError("kernel must be auto, lut or mma")
-    rows = x.shape[0]
     if kernel == "auto":
         kernel = "lut" if rows <= 4 or arithmetic == "decoded_bf16" else "mma"
+    elif kernel not in ("lut", "mma"):
+        raise ValueError("kernel must be auto, lut or mma")
     if rows < 1 or rows > (4 if kernel == "lut" else 16):
         raise ValueError(f"the {kernel} kernel takes 1..{4 if kernel == 'lut' else 16} rows")
-    planes, scales, zeros, perm = _layout_args(layout)
-    if kernel == "mma":
-        if arithmetic != "structural":
-            raise ValueError("the tensor-core kernel has one arithmetic: weights rounded to the activation dtype")
-        _native.w3_gemm_small(x, planes, scales, zeros, perm, out)
-    else:
-        _native.w3_gemv(x, planes, scales, zeros, perm, out, decoded_bf16=arithmetic == "decoded_bf16")
+    if kernel == "mma" and arithmetic != "structural":
+        raise ValueError("the tensor-core kernel has one arithmetic: weights rounded to the activation dtype")
+    _launch_layout(record, layout, x, out, "small" if kernel == "mma" else "w3", arithmetic == "decoded_bf16")
     return out
 
 
@@ -396,19 +480,22 @@ class PackedW3Linear(nn.Module):
         output = self._decode_output
         shaped = output.view(1, 1, self.out_features)
         expected = (1, 1, self.in_features)
-        in_features = self.in_features
+        index, buffers = output.get_device(), self._buffers
+        module = weakref.ref(self)  # no cycle: a dropped module gives its weights back at once
+        launch = _native.Launch("w3", dtype, (planes, scales, zeros, perm), self.out_features, self.in_features, decoded=corrected)
 
         def apply(x: torch.Tensor) -> torch.Tensor:
             if torch.is_grad_enabled():
                 raise RuntimeError("prepared decode is inference only")
-            if tuple(x.shape) != expected or x.dtype != dtype or x.device != device or not x.is_contiguous():
+            if x.shape != expected or x.dtype != dtype or x.get_device() != index or not x.is_contiguous():
                 raise ValueError("prepared decode input shape/dtype/device/stride mismatch")
-            if self._decode_audit:
-                self.route_counts["packed_m1"] += 1
-                self.last_route = "packed_m1"
-            _native.w3_gemv(x.view(1, in_features), planes, scales, zeros, perm, output, decoded_bf16=corrected)
-            if self.bias is not None:
-                output.add_(self.bias)
+            me = module()
+            if me is not None and me._decode_audit:
+                me.route_counts["packed_m1"] += 1
+                me.last_route = "packed_m1"
+            launch(x, output)
+            if buffers["bias"] is not None:
+                output.add_(buffers["bias"])
             return shaped
 
         self._decode_binding = apply
