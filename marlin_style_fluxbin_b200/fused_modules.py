@@ -11,6 +11,8 @@ plain tensor operations, which is also what the patched functions compute in the
 """
 from __future__ import annotations
 
+import inspect
+import threading
 from contextlib import contextmanager
 
 import torch
@@ -69,12 +71,92 @@ def fused_apply_rotary_pos_emb(q, k, cos, sin, unsqueeze_dim=1):
     return _rope_algebra(q, k, cos, sin, unsqueeze_dim)
 
 
+# ---- one decode step on a static cache (StaticDecodeSession) ----
+# Between the Linears of a step lie some seventeen small launches per layer in the stock modules: norms and rotation,
+# two scatters into the cache and their index arithmetic, the expansion of the k/v heads, SDPA, gate and product.  While a
+# session announces the step it runs (position and cache known on the host), the attention module takes ONE launch
+# for everything between q/k/v and o_proj, and the MLP one between gate/up and down.
+_local = threading.local()
+
+
+class DecodeStep:
+    """What a session tells the modules about the step under way; ``position`` advances from step to step."""
+
+    def __init__(self, cache, scratch):
+        self.cache, self.scratch, self.position = cache, scratch, None
+
+    @contextmanager
+    def at(self, position: int):
+        self.position, previous, _local.step = position, getattr(_local, "step", None), self
+        try:
+            yield
+        finally:
+            _local.step = previous
+
+
+def _unobserved(*modules) -> bool:
+    """Nobody hooked the modules that a fused launch would skip."""
+    return not any(m._forward_hooks or m._forward_pre_hooks for m in modules)
+
+
+def _step_serves(step, attention, call) -> bool:
+    hidden, positions = call.get("hidden_states"), call.get("position_embeddings")
+    if call.get("past_key_values", call.get("past_key_value")) is not step.cache or positions is None:
+        return False
+    q_norm, k_norm = attention.q_norm, attention.k_norm
+    layer = step.cache.layers[attention.layer_idx]
+    keys, values = layer.keys, layer.values
+    dim = attention.head_dim
+    return (dim == 128 and hidden.numel() == hidden.shape[-1] and attention.config._attn_implementation == "sdpa"
+            and getattr(attention, "sliding_window", None) is None and not attention.training
+            and not call.get("output_attentions") and not call.get("kwargs", {}).get("output_attentions")
+            and positions[0].numel() == dim and _kernel_eligible(hidden, q_norm.weight, k_norm.weight, *positions, keys, values)
+            and q_norm.variance_epsilon == k_norm.variance_epsilon and keys.shape == values.shape and keys.shape[0] == 1 and keys.shape[-1] == dim
+            and step.position < keys.shape[2] and attention.config.num_attention_heads % keys.shape[1] == 0
+            and step.scratch.numel() >= _native.attn_scratch_bytes(attention.config.num_attention_heads) and _unobserved(q_norm, k_norm))
+
+
+def _fused_attention(original):
+    signature = inspect.signature(original)
+
+    def forward(self, *args, **kwargs):
+        step = getattr(_local, "step", None)
+        if step is not None:
+            call = signature.bind(self, *args, **kwargs).arguments
+            if _step_serves(step, self, call):
+                hidden, (cos, sin) = call["hidden_states"], call["position_embeddings"]
+                q, k, v = self.q_proj(hidden), self.k_proj(hidden), self.v_proj(hidden)
+                if _kernel_eligible(hidden, q, k, v):
+                    layer, out = step.cache.layers[self.layer_idx], torch.empty_like(q)
+                    _native.attn_decode_fused(q, k, v, self.q_norm.weight, self.k_norm.weight, cos, sin, layer.keys[0], layer.values[0], out,
+                                              step.position, self.q_norm.variance_epsilon, self.scaling, step.scratch)
+                    return self.o_proj(out), None
+        return original(self, *args, **kwargs)
+
+    return forward
+
+
+def _fused_mlp(original):
+    def forward(self, x):
+        if getattr(_local, "step", None) is None or self.config.hidden_act != "silu" or not _kernel_eligible(x) or not _unobserved(self.act_fn):
+            return original(self, x)
+        gate, up = self.gate_proj(x), self.up_proj(x)
+        if not _kernel_eligible(x, gate, up):
+            return original(self, x)
+        out = torch.empty_like(gate)
+        _native.silu_mul(gate, up, out)
+        return self.down_proj(out)
+
+    return forward
+
+
 @contextmanager
 def fused_qwen3_modules(*, rms_norm=True, rope=True):
     """Patch the HF Qwen3 RMSNorm class and rotary function in place; restore on exit or error.
 
     The patch is at class / module scope on purpose, so every arm of a comparison built
-    from ``transformers`` shares the same non-Linear path.
+    from ``transformers`` shares the same non-Linear path.  With both parts on, the decode steps of a
+    ``StaticDecodeSession`` also take the attention and the SwiGLU gate in one launch each.
     """
     from transformers.models.qwen3 import modeling_qwen3
 
@@ -87,9 +169,17 @@ def fused_qwen3_modules(*, rms_norm=True, rope=True):
         if rope:
             saved["rope"] = modeling_qwen3.apply_rotary_pos_emb
             modeling_qwen3.apply_rotary_pos_emb = fused_apply_rotary_pos_emb
+        if rms_norm and rope:
+            for name, wrap in (("Qwen3Attention", _fused_attention), ("Qwen3MLP", _fused_mlp)):
+                owner = getattr(modeling_qwen3, name)
+                saved[name] = owner.forward
+                owner.forward = wrap(owner.forward)
         yield applied
     finally:
         if "rms_norm" in saved:
             modeling_qwen3.Qwen3RMSNorm.forward = saved["rms_norm"]
         if "rope" in saved:
             modeling_qwen3.apply_rotary_pos_emb = saved["rope"]
+        for name in ("Qwen3Attention", "Qwen3MLP"):
+            if name in saved:
+                getattr(modeling_qwen3, name).forward = saved[name]

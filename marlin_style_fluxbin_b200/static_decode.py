@@ -13,12 +13,13 @@ length on the host) and the region clock shared with the dynamic-cache trace.
 """
 from __future__ import annotations
 
-from contextlib import contextmanager
+from contextlib import contextmanager, nullcontext
 
 import torch
 from transformers import StaticCache
 
 from . import _native
+from .fused_modules import DecodeStep
 from .full_model_trial import RegionClock, packed_modules
 
 _MODES = ("prepared_eager", "sequence_graph")
@@ -52,11 +53,16 @@ class _PromptKV:
             for target, source in ((layer.keys, keys), (layer.values, values)):
                 target.zero_()
                 target[:, :, :self.length].copy_(source)
+        self.count(self.length)
+
+    def count(self, length: int):
+        """The cache's own bookkeeping: ``length`` positions are filled (a fused step writes its rows without it)."""
+        for layer in self.cache.layers:
             counter = getattr(layer, "cumulative_length", None)  # absent, an int or a tensor, depending on the transformers version
             if isinstance(counter, torch.Tensor):
-                counter.fill_(self.length)
+                counter.fill_(length)
             elif counter is not None:
-                layer.cumulative_length = self.length
+                layer.cumulative_length = length
 
 
 class _StepInputs:
@@ -101,6 +107,9 @@ class StaticDecodeSession:
             self.prefill_logits = prefill.logits[:, -1, :].detach().clone()
             self.prompt_kv = _PromptKV(self.cache, self.prefix_length)
         self.graph = self.graph_outputs = self.capture_routes = None
+        self.step = None  # announced to the fused modules while a step runs on a GPU
+        if input_ids.device.type == "cuda":
+            self.step = DecodeStep(self.cache, torch.zeros(_native.attn_scratch_bytes(model.config.num_attention_heads), dtype=torch.uint8, device=input_ids.device))
 
     # ---- the decode loop and its bookkeeping ----
     @torch.inference_mode()
@@ -112,8 +121,10 @@ class StaticDecodeSession:
         """The whole continuation, eagerly; per step ``(logits [1,V], greedy token [1,1])``."""
         produced = []
         for index in range(len(self.inputs)):
-            row = self.model(past_key_values=self.cache, use_cache=True, logits_to_keep=1, **self.inputs.of(index)).logits[:, -1, :]
+            with self.step.at(self.prefix_length + index) if self.step is not None else nullcontext():
+                row = self.model(past_key_values=self.cache, use_cache=True, logits_to_keep=1, **self.inputs.of(index)).logits[:, -1, :]
             produced.append((row, row.argmax(-1, keepdim=True)))
+        self.prompt_kv.count(self.maximum_length)
         return produced
 
     def set_audit(self, enabled):
