@@ -204,10 +204,10 @@ int fb_tp_reduce(void* parts, int world, const void* residual, void* out, int n,
 
 /*
  * Small-batch form on the tensor cores: y[M,O] = x[M,K] . W^T for M = 1..16, same layout and
- * dtypes as fb_w3_gemv.  Every weight is dequantised once, T((code - zero) * scale) with T the
- * activation dtype, into a shared-memory operand tile and applied to all M rows by tcgen05.mma
- * (fp32 accumulation in tensor memory), so the time does not grow with M.  The K split is
- * combined as in fb_w3_gemv (repeat-exact).  Own scratch (zero-filled once, 256-byte aligned),
+ * dtypes as fb_w3_gemv.  The three planes of a group become register operands of the matrix
+ * instructions; sums are exact up to fp32 rounding, scales are applied in fp32 (weights are not
+ * rounded), and the time hardly grows with M.  A row's result does not depend on its neighbours
+ * and is the same on every call.  Own scratch (zero-filled once, 256-byte aligned),
  * not to be shared with the other kernels.  The reference has no packed path for M > 1
  * (csrc/w3_lut.cu:195); its dense fallback (w3_lut_deployment.py:343-359) is the oracle.
  */
@@ -215,6 +215,10 @@ size_t fb_w3_gemm_small_scratch_bytes(int m, int out_features, int in_features);
 int fb_w3_gemm_small(const void* x, int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype,
                      const uint8_t* zeros, const int16_t* perm, void* out, int out_features, int in_features,
                      void* scratch, size_t scratch_bytes, fb_stream_t stream);
+/* The same plus addend [M,O] of the activation dtype (NULL: none), added in fp32 before the one rounding. */
+int fb_w3_gemm_small_add(const void* x, int act_dtype, int m, const uint8_t* planes, const void* scales, int scale_dtype,
+                         const uint8_t* zeros, const int16_t* perm, const void* addend, void* out, int out_features, int in_features,
+                         void* scratch, size_t scratch_bytes, fb_stream_t stream);
 
 /*
  * out[o] = T( sum_s partials[s, o] ), rows summed in ascending order.

@@ -74,6 +74,8 @@ def library() -> ctypes.CDLL:
         lib.fb_w3_gemm_small.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                          ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
                                          ctypes.c_size_t, ctypes.c_void_p]
+        lib.fb_w3_gemm_small_add.restype = ctypes.c_int
+        lib.fb_w3_gemm_small_add.argtypes = lib.fb_w3_gemm_small.argtypes[:8] + [ctypes.c_void_p] + lib.fb_w3_gemm_small.argtypes[8:]
         lib.fb_w3_gemv_push.restype = ctypes.c_int
         lib.fb_w3_gemv_push.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_float,
                                         ctypes.POINTER(W3Matrix), ctypes.c_int, ctypes.c_int, ctypes.POINTER(W3Push), ctypes.c_void_p,
@@ -549,16 +551,17 @@ def w3_gemv_fused_input(x, transform: int, operand, eps: float, matrices, n_matr
                                                stream_handle(x.device)))
 
 
-def w3_gemm_small(x, planes, scales, zeros, perm, out, *, scratch=None) -> None:
-    """Tensor-core form for ``x`` of 1..16 rows: x [M,K], planes [G,3,O,16], scales [G,O], out [M,O]."""
+def w3_gemm_small(x, planes, scales, zeros, perm, out, *, addend=None, scratch=None) -> None:
+    """Tensor-core form for ``x`` of 1..16 rows: x [M,K], planes [G,3,O,16], scales [G,O], out [M,O]; ``addend`` [M,O] is added
+    before the result is rounded."""
     m, k = x.shape
     o = planes.shape[2]
     if scratch is None:
         scratch = scratch_for(x.device, library().fb_w3_gemm_small_scratch_bytes(m, o, k), "w3mma")
     with torch.cuda.device(x.device):
-        check(library().fb_w3_gemm_small(ptr(x), dtype_tag(x.dtype), m, ptr(planes), ptr(scales), dtype_tag(scales.dtype),
+        check(library().fb_w3_gemm_small_add(ptr(x), dtype_tag(x.dtype), m, ptr(planes), ptr(scales), dtype_tag(scales.dtype),
                                          ptr(zeros) if zeros is not None else None, ptr(perm) if perm is not None else None,
-                                         ptr(out), o, k, ptr(scratch), scratch.numel() * scratch.element_size(),
+                                         ptr(addend) if addend is not None else None, ptr(out), o, k, ptr(scratch), scratch.numel() * scratch.element_size(),
                                          stream_handle(x.device)))
 
 

@@ -21,7 +21,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
 # Per-file extras.  The GEMV kernels keep separate multiply and add, as the reference
 # builds its kernels (--fmad=false), so that products are rounded where it rounds them.
-EXTRA = {"fb_w3_gemv.cu": ["--fmad=false"], "fb_bb_gemv.cu": ["--fmad=false"]}
+EXTRA = {"fb_w3_gemv.cu": ["--fmad=false"], "fb_w3_rows.cu": ["--fmad=false"], "fb_bb_gemv.cu": ["--fmad=false"]}
 
 
 def _nvcc() -> str:

@@ -85,18 +85,18 @@ bool encoder_ready() {
 }
 }  // namespace
 
-bool plane_tensor_map(const uint8_t* planes, int O, int G, int box_units, int box_runs, CUtensorMap* out) {
+bool plane_tensor_map(const uint8_t* planes, int O, int G, int rows, int box_units, int box_runs, CUtensorMap* out) {
   std::lock_guard<std::mutex> guard(g_map_lock);
   if (!encoder_ready()) return false;
-  const MapKey key{planes, O, G, box_units * 256 + box_runs};
+  const MapKey key{planes, O, G, (rows << 16) + box_units * 256 + box_runs};
   auto found = g_maps.find(key);
   if (found != g_maps.end()) {
     *out = found->second;
     return true;
   }
-  const cuuint64_t dims[3] = {128, (cuuint64_t)(O / 32), (cuuint64_t)G * 3};
-  const cuuint64_t strides[2] = {512, (cuuint64_t)O * 16};  // bytes, dims 1 and 2
-  const cuuint32_t box[3] = {128, (cuuint32_t)box_units, (cuuint32_t)box_runs};
+  const cuuint64_t dims[3] = {(cuuint64_t)rows * 4, (cuuint64_t)(O / rows), (cuuint64_t)G * 3};
+  const cuuint64_t strides[2] = {(cuuint64_t)rows * 16, (cuuint64_t)O * 16};  // bytes, dims 1 and 2
+  const cuuint32_t box[3] = {(cuuint32_t)rows * 4, (cuuint32_t)box_units, (cuuint32_t)box_runs};
   const cuuint32_t step[3] = {1, 1, 1};
   CUtensorMap map;
   const CUresult rc = g_encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t*>(planes), dims, strides, box, step,
@@ -112,10 +112,10 @@ bool plane_tensor_map(const uint8_t* planes, int O, int G, int box_units, int bo
   return true;
 }
 
-bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, CUtensorMap* out) {
+bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, int rows, CUtensorMap* out) {
   std::lock_guard<std::mutex> guard(g_map_lock);
   if (!encoder_ready()) return false;
-  const MapKey key{base, O, G, 1 << 20 | elem_bytes};
+  const MapKey key{base, O, G, 1 << 24 | rows << 4 | elem_bytes};
   auto found = g_maps.find(key);
   if (found != g_maps.end()) {
     *out = found->second;
@@ -123,7 +123,7 @@ bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, CUtens
   }
   const cuuint64_t dims[2] = {(cuuint64_t)O, (cuuint64_t)G};
   const cuuint64_t strides[1] = {(cuuint64_t)O * elem_bytes};
-  const cuuint32_t box[2] = {32, 2};
+  const cuuint32_t box[2] = {(cuuint32_t)rows, 2};
   const cuuint32_t step[2] = {1, 1};
   CUtensorMap map;
   const CUresult rc = g_encode(&map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims,

@@ -28,14 +28,14 @@ const DeviceInfo* device_info();
 // environment variable FB_NO_PDL (read once); used to tell launch-overlap effects apart.
 bool pdl_allowed();
 
-// Tiled-copy descriptor of a W3 planes tensor [G,3,O,16] seen as uint32 [G*3][O/32][128] (a
-// 512-byte run per 32 rows, plane and group); one box is `box_runs` (group, plane) runs of
-// `box_units` 32-row units.  Encoding is pure host work; descriptors are cached per
+// Tiled-copy descriptor of a W3 planes tensor [G,3,O,16] seen as uint32 [G*3][O/rows][4*rows] (one run
+// of 16 * rows bytes per `rows` output rows, plane and group); one box is `box_runs` (group, plane) runs of
+// `box_units` row units.  Encoding is pure host work; descriptors are cached per
 // (address, O, G, box).  Returns false after recording the error.
-bool plane_tensor_map(const uint8_t* planes, int O, int G, int box_units, int box_runs, CUtensorMap* out);
+bool plane_tensor_map(const uint8_t* planes, int O, int G, int rows, int box_units, int box_runs, CUtensorMap* out);
 // Descriptor of a per-(group, row) tensor [G][O] of 1- or 2-byte elements (zero points, scales),
-// box = 32 rows x 2 groups; rows of the box beyond G read as zero.
-bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, CUtensorMap* out);
+// box = `rows` rows x 2 groups; rows of the box beyond G read as zero.
+bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, int rows, CUtensorMap* out);
 
 // Launch with the programmatic-dependent-launch attribute (unless switched off): the kernel's
 // prologue may overlap the tail of the previous kernel in the stream.

@@ -966,10 +966,10 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
         overlaps(in.out, out_bytes, in.scales, (size_t)G * O * 2))
       return fail(FB_EALIAS, "fb_w3_gemv: out overlaps an input");
     if (scratch && overlaps(scratch, scratch_bytes, in.out, out_bytes)) return fail(FB_EALIAS, "fb_w3_gemv: scratch overlaps out");
-    if (!plane_tensor_map(in.planes, O, G, 1, 6, &p.plane_maps[j])) return FB_ECUDA;
+    if (!plane_tensor_map(in.planes, O, G, kUnitRows, 1, 6, &p.plane_maps[j])) return FB_ECUDA;
     if (m == 1) {  // the M = 1 kernel stages scales and zero points with the planes
-      if (!group_row_tensor_map(in.scales, 2, O, G, &p.scale_maps[j])) return FB_ECUDA;
-      if (in.zeros && !group_row_tensor_map(in.zeros, 1, O, G, &p.zero_maps[j])) return FB_ECUDA;
+      if (!group_row_tensor_map(in.scales, 2, O, G, kUnitRows, &p.scale_maps[j])) return FB_ECUDA;
+      if (in.zeros && !group_row_tensor_map(in.zeros, 1, O, G, kUnitRows, &p.zero_maps[j])) return FB_ECUDA;
       if (!in.zeros) p.zero_maps[j] = p.scale_maps[j];
     } else {
       p.scale_maps[j] = p.plane_maps[j];

@@ -258,17 +258,16 @@ class DecodeEngine:
     # ------------------------------------------------------------------ prefill (many tokens)
     def _prompt_linear(self, x, layouts, dense, addend=None):
         """``x`` ``[T,K]`` times the stacked rows of ``layouts`` (``dense``: the same rows as one dense matrix, or None
-        on the packed arm), plus ``addend``.  The packed arm keeps up to 4 tokens packed; for more it forms the weight
+        on the packed arm), plus ``addend``.  The packed arm keeps up to 16 tokens packed; for more it forms the weight
         in chunks that stay in the L2 between the dequantising launch and the GEMM."""
         if dense is not None:
             return torch.mm(x, dense.t()) if addend is None else torch.addmm(addend, x, dense.t())
         t, k = x.shape
-        if t <= 4:
+        if t <= 16:
             parts = [torch.empty(t, lay["planes"].shape[2], device=self.device, dtype=self.dtype) for lay in layouts]
-            for lay, part in zip(layouts, parts):
-                _native.w3_gemv(x, lay["planes"], lay["scales"], lay["zeros"], None, part)
-            y = parts[0] if len(parts) == 1 else torch.cat(parts, dim=1)
-            return y if addend is None else y.add_(addend)
+            for lay, part in zip(layouts, parts):  # an addend comes with a single layout
+                _native.w3_gemm_small(x, lay["planes"], lay["scales"], lay["zeros"], None, part, addend=addend)
+            return parts[0] if len(parts) == 1 else torch.cat(parts, dim=1)
         rows = sum(lay["planes"].shape[2] for lay in layouts)
         if len(layouts) > 1 or rows * k * 2 <= DENSE_CHUNK_BYTES:
             weight = self._dense_rows(layouts)
@@ -288,7 +287,7 @@ class DecodeEngine:
         """``silu(x gate^T) * (x up^T)`` ``[T, inter]``; the packed arm takes matching rows of gate and up together."""
         t, k = x.shape
         act = torch.empty(t, self.inter, device=self.device, dtype=self.dtype)
-        if layer.dense is not None or t <= 4:
+        if layer.dense is not None or t <= 16:
             _native.silu_mul_rows(self._prompt_linear(x, (layer.gate, layer.up), None if layer.dense is None else layer.dense["gate_up"]), act)
             return act
         step = _chunk_rows(2 * self.inter, k) // 2

@@ -324,9 +324,9 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
     """Small-batch form (``x`` is ``[M,K]``, M = 1..16) of ``w3_lut_m1_out``; no reference counterpart.
 
     ``kernel``: ``"lut"`` is the table-lookup kernel (M <= 4, cost grows with M), ``"mma"`` the
-    tensor-core kernel (M <= 16, cost independent of M; weights are rounded to the activation
-    dtype, as the reference's dense fallback rounds them), ``"auto"`` picks ``"lut"`` up to M = 4
-    (measured faster there on the Qwen3-8B shapes) and ``"mma"`` above.
+    tensor-core kernel (M <= 16, cost hardly grows with M; weights are not rounded).  ``"auto"`` picks
+    ``"lut"`` for one row (4096 x 4096: 3.8 us against 5.5) and for the dequantised-weight arithmetic, which
+    only that kernel has, and ``"mma"`` from two rows on (two rows: 5.5 us against 5.9, four: 5.6 against 10.1).
     """
     record = _layout_record(layout)
     rows = x.shape[0] if x.ndim else 0
@@ -335,28 +335,26 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
     if out.dtype != x.dtype or out.device != x.device:
         raise ValueError("out must match x in dtype and device")
     if kernel == "auto":
-        kernel = "lut" if rows <= 4 or arithmetic == "decoded_bf16" else "mma"
+        kernel = "lut" if rows == 1 or arithmetic == "decoded_bf16" else "mma"
     elif kernel not in ("lut", "mma"):
         raise ValueError("kernel must be auto, lut or mma")
     if rows < 1 or rows > (4 if kernel == "lut" else 16):
         raise ValueError(f"the {kernel} kernel takes 1..{4 if kernel == 'lut' else 16} rows")
     if kernel == "mma" and arithmetic != "structural":
-        raise ValueError("the tensor-core kernel has one arithmetic: weights rounded to the activation dtype")
+        raise ValueError("the tensor-core kernel has one arithmetic: weights that are not rounded")
     _launch_layout(record, layout, x, out, "small" if kernel == "mma" else "w3", arithmetic == "decoded_bf16")
     return out
 
 
 def dense_linear(x, layout, bias=None):
-    """``x`` ``[T,K]`` (16-bit, CUDA) times the dequantised weight, without the table kernels' row limit: up to 16 rows
-    without a bias stay packed (the tensor-core kernel rounds the weights as a dense weight would be rounded), the rest goes
-    through dense chunks of the weight in group-sorted column order, with the activations gathered into that order."""
+    """``x`` ``[T,K]`` (16-bit, CUDA) times the dequantised weight, without the packed kernels' row limit: up to 16 rows
+    without a bias stay packed (the tensor-core kernel, whose weights are not rounded at all), the rest goes through dense chunks of the weight in group-sorted column order, with the activations gathered into that order."""
     planes, scales, zeros, perm = _layout_args(layout)
     rows, (out_features, in_features) = x.shape[0], (planes.shape[2], x.shape[1])
     y = torch.empty(rows, out_features, device=x.device, dtype=x.dtype)
     x = x.contiguous()
-    # the tensor-core kernel rounds a scale to x's dtype first, so bf16 rows with fp16 scales would lose bits there; a bias
-    # added to its rounded output would round twice
-    if rows <= 16 and bias is None and out_features % 32 == 0 and x.data_ptr() % 16 == 0 and x.dtype in (scales.dtype, torch.float16):
+    # a bias added to the packed kernel's rounded output would round twice
+    if rows <= 16 and bias is None and out_features % 32 == 0 and x.data_ptr() % 16 == 0:
         _native.w3_gemm_small(x, planes, scales, zeros, perm, y)
         return y
     if perm is not None:
