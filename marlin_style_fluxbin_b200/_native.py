@@ -21,6 +21,7 @@ FB_W3_GROUP_PARTIALS = 4
 FB_W3_SAME_INPUT = 8
 
 _lib = None
+_calls = None
 
 
 class W3Matrix(ctypes.Structure):
@@ -38,6 +39,18 @@ class W3Push(ctypes.Structure):
 
 class NativeError(RuntimeError):
     """A call into the CUDA library was rejected (message from ``fb_last_error``)."""
+
+
+def calls():
+    """The extension module behind eager calls on prepared launches (``csrc/python/fb_calls.cpp``)."""
+    global _calls
+    if _calls is None:
+        try:
+            from . import _fb_calls
+        except ImportError as exc:
+            raise RuntimeError("_fb_calls.so is not built; run `python -m marlin_style_fluxbin_b200.build`") from exc
+        _calls = _fb_calls
+    return _calls
 
 
 def library() -> ctypes.CDLL:
@@ -284,7 +297,7 @@ class Launch:
     Holds the tensors whose addresses it keeps, unless told not to (``hold``).  ``kind``: ``"w3"`` (M = 1..4, table kernel), ``"small"`` (M = 1..16,
     tensor cores) or ``"bb"`` (two-base)."""
 
-    __slots__ = ("kind", "rows", "_handle", "_tensors", "_index", "_follows", "_need", "_width", "_run", "_release")
+    __slots__ = ("call", "_handle", "_tensors", "_release")
 
     def __init__(self, kind, act_dtype, tensors, out_features, in_features, rows=1, decoded=False, hold=True):
         lib = library()
@@ -294,52 +307,41 @@ class Launch:
             if kind == "bb":
                 codes, *rest = tensors
                 code = lib.fb_bb_prepare(tag, codes.data_ptr(), int(codes.ndim == 4), *(t.data_ptr() for t in rest), out_features, in_features, ctypes.byref(handle))
-                self._need = bb_scratch_bytes(out_features, in_features, False)
+                need, families = bb_scratch_bytes(out_features, in_features, False), ("bb",)
             else:
                 planes, scales, zeros, perm = tensors
                 args = (tag, rows, planes.data_ptr(), scales.data_ptr(), dtype_tag(scales.dtype), _addr(zeros), _addr(perm), out_features, in_features)
                 if kind == "w3":
                     code = lib.fb_w3_prepare(*args, FB_W3_DECODED_BF16 if decoded else 0, ctypes.byref(handle))
-                    self._need = w3_scratch_bytes(rows, out_features, in_features)
+                    need, families = w3_scratch_bytes(rows, out_features, in_features), _W3_SLOTS if rows == 1 else _W3_SLOTS[:1]
                 else:
                     code = lib.fb_w3_prepare_small(*args, ctypes.byref(handle))
-                    self._need = int(lib.fb_w3_gemm_small_scratch_bytes(rows, out_features, in_features))
+                    need, families = int(lib.fb_w3_gemm_small_scratch_bytes(rows, out_features, in_features)), ("w3mma",)
         if code:
             raise NativeError(lib.fb_last_error().decode())
-        self.kind, self.rows, self._handle, self._tensors = kind, rows, handle.value, tensors if hold else None
-        self._index = device.index if device.index is not None else torch.cuda.current_device()
-        self._follows = kind == "w3" and rows == 1
-        self._width, self._run, self._release = in_features, lib.fb_prepared_run, lib.fb_prepared_release
+        self._handle, self._tensors, self._release = handle.value, tensors if hold else None, lib.fb_prepared_release
+        # a plain launch of one row may follow another on the same activations: see _w3_slot
+        index = device.index if device.index is not None else torch.cuda.current_device()
+        self.call = calls().Call(ctypes.cast(lib.fb_prepared_run, ctypes.c_void_p).value, handle.value, rows, in_features, out_features, index, act_dtype,
+                                 FB_W3_NO_PDL if _NO_PDL else 0, 0 if _NO_PDL or _NO_SAME_INPUT else FB_W3_SAME_INPUT, int(kind == "w3" and rows == 1),
+                                 need, families, _scratch, _same_input, _scratch_on, torch.cuda.is_current_stream_capturing, _refused)
 
     def __del__(self):
         if getattr(self, "_release", None) is not None:  # absent when the launch was refused
             self._release(self._handle)
 
     def __call__(self, x, out) -> None:
-        """``x`` and ``out`` as the plain entry point takes them, contiguous on the launch's device (the caller checks)."""
-        index = self._index
-        stream = _raw_stream(index)
-        x_ptr = x.data_ptr()
-        flags = FB_W3_NO_PDL if _NO_PDL else 0
-        family = "bb" if self.kind == "bb" else ("w3mma" if self.kind == "small" else "w3")
-        if self._follows:
-            key, here = (index, stream), (x_ptr, (1, self._width), x.dtype)
-            slot = _w3_slot(key, here)
-            if slot:
-                family, flags = _W3_SLOTS[slot], FB_W3_SAME_INPUT
-        buf = _scratch.get((index, stream, family))
-        if buf is None or buf.numel() < self._need:
-            buf = scratch_for(x.device, self._need, family)
-        if _current_device() == index:
-            code = self._run(self._handle, x_ptr, out.data_ptr(), buf.data_ptr(), buf.numel(), flags, stream)
-        else:
-            with torch.cuda.device(index):
-                code = self._run(self._handle, x_ptr, out.data_ptr(), buf.data_ptr(), buf.numel(), flags, stream)
-        _same_input.clear()
-        if code:
-            raise NativeError(library().fb_last_error().decode() or f"native call failed with code {code}")
-        if self._follows and not _NO_PDL:
-            _same_input[key] = (here, slot + 1)
+        """``x`` and ``out`` as the plain entry point takes them, contiguous on the launch's device (the caller checks;
+        ``call.fits`` checks by itself)."""
+        self.call.run(x, out)
+
+
+def _scratch_on(index: int, nbytes: int, family: str) -> torch.Tensor:
+    return scratch_for(torch.device("cuda", index), nbytes, family)
+
+
+def _refused(code: int) -> None:
+    raise NativeError(library().fb_last_error().decode() or f"native call failed with code {code}")
 
 
 def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_partials=False,

@@ -1,6 +1,7 @@
-"""Ahead-of-time build of the CUDA library (``libfluxbin_b200.so``) with nvcc for sm_100a.
+"""Ahead-of-time build of the CUDA library (``libfluxbin_b200.so``) with nvcc for sm_100a, and of the extension
+module behind eager calls (``_fb_calls.so``) with the host compiler against torch's C++ interface.
 
-The library is built in-tree, next to this file, so that it travels with the source tree.
+Both are built in-tree, next to this file, so that they travel with the source tree.
 ``python -m marlin_style_fluxbin_b200.build`` rebuilds it; ``build()`` is incremental.
 """
 from __future__ import annotations
@@ -15,6 +16,7 @@ from pathlib import Path
 PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libfluxbin_b200.so"
+CALLS = PACKAGE / "_fb_calls.so"
 STAMP = PACKAGE / "csrc" / ".build_stamp"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -37,16 +39,33 @@ def sources() -> list[Path]:
 
 def _fingerprint() -> str:
     digest = hashlib.sha256()
-    for path in sorted(sources() + list(CSRC.glob("*.cuh")) + [PACKAGE.parent / "include" / "fluxbin_b200.h", Path(__file__)]):
+    for path in sorted(sources() + list(CSRC.glob("*.cuh")) + list(CSRC.glob("python/*.cpp")) + [PACKAGE.parent / "include" / "fluxbin_b200.h", Path(__file__)]):
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
     return digest.hexdigest()
 
 
+def _build_calls(nvcc: str) -> str:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    libraries = Path(torch.__file__).resolve().parent / "lib"
+    headers = [*include_paths(), sysconfig.get_paths()["include"], str(Path(nvcc).resolve().parent.parent / "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(flag for path in headers for flag in ("-isystem", path)), str(CSRC / "python" / "fb_calls.cpp"), "-o", str(CALLS),
+           f"-L{libraries}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    done = subprocess.run(cmd, capture_output=True, text=True)
+    if done.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on fb_calls.cpp:\n{done.stdout}{done.stderr}")
+    return f"$ {' '.join(cmd)}\n{done.stdout}{done.stderr}"
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` for sm_100a (and the host-only ``*.cpp``) and link the shared library."""
+    """Compile every ``csrc/*.cu`` for sm_100a (and the host-only ``*.cpp``), link the shared library and build the extension."""
     fingerprint = _fingerprint()
-    if not force and LIBRARY.exists() and STAMP.exists() and STAMP.read_text() == fingerprint:
+    if not force and LIBRARY.exists() and CALLS.exists() and STAMP.exists() and STAMP.read_text() == fingerprint:
         return LIBRARY
     nvcc = _nvcc()
     objects = []
@@ -63,6 +82,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     done = subprocess.run(cmd, capture_output=True, text=True)
     if done.returncode != 0:
         raise RuntimeError(f"link failed:\n{done.stdout}{done.stderr}")
+    logs.append(_build_calls(nvcc))
     (CSRC / "ptxas_report.txt").write_text("\n".join(logs))
     STAMP.write_text(fingerprint)
     if verbose:

@@ -297,27 +297,10 @@ class PackedHybridLinear(nn.Module):
         self._decode_output = torch.empty((1, self.out_features), device=device, dtype=dtype)
         output = self._decode_output
         shaped = output.view(1, 1, self.out_features)
-        expected = (1, 1, self.in_features)
-        index, buffers = output.get_device(), self._buffers
-        module = weakref.ref(self)  # no cycle: a dropped module gives its weights back at once
         launch = _native.Launch("bb", dtype, tuple(layout[name] for name in ("codes", "rows", "columns", "sparse_codes", "sparse_rows", "sparse_columns",
                                                                              "indices")), self.out_features, self.in_features)
-
-        def apply(x):
-            if torch.is_grad_enabled():
-                raise RuntimeError("prepared decode is inference only")
-            if x.shape != expected or x.dtype != dtype or x.get_device() != index or not x.is_contiguous():
-                raise ValueError("prepared decode input shape/dtype/device/stride mismatch")
-            me = module()
-            if me is not None and me._decode_audit:
-                me.route_counts["packed_m1"] += 1
-                me.last_route = "packed_m1"
-            launch(x, output)
-            if buffers["bias"] is not None:
-                output.add_(buffers["bias"])
-            return shaped
-
-        self._decode_binding = apply
+        # a weak reference to the module, so no cycle: a dropped module gives its weights back at once
+        self._decode_binding = _native.calls().Bound(launch.call, launch, output, shaped, weakref.ref(self), self._buffers)
 
     def forward(self, x):
         if self._decode_binding is not None:
