@@ -221,6 +221,16 @@ int fb_w3_gemm_small_add(const void* x, int act_dtype, int m, const uint8_t* pla
                          void* scratch, size_t scratch_bytes, fb_stream_t stream);
 
 /*
+ * Many rows: mats[j].out[t, o] = x[t, :] . W_j[o, :] (+ mats[j].residual[t, o]) for t < tokens, any
+ * number of them; up to four matrices of one K over the same x.  Weights are formed as in
+ * fb_w3_dequant, in tensor memory, and applied by tcgen05.mma with fp32 accumulation; one rounding
+ * after the addition.  Rows of out and residual are out_stride elements apart.  x must be 16-byte
+ * aligned, in group-sorted column order (fb_gather_columns).  scratch: 256 bytes (the status word).
+ */
+int fb_w3_gemm(const void* x, int act_dtype, int tokens, const fb_w3_matrix_t* mats, int n_mats, int scale_dtype, int in_features,
+               int out_stride, void* scratch, size_t scratch_bytes, fb_stream_t stream);
+
+/*
  * out[o] = T( sum_s partials[s, o] ), rows summed in ascending order.
  * partials fp32 [splits, O]; out f16|bf16 [O].
  * Replaces the reference's finish (csrc/w3_lut.cu:275-296, kernel :142-150).

@@ -89,6 +89,9 @@ def library() -> ctypes.CDLL:
                                          ctypes.c_size_t, ctypes.c_void_p]
         lib.fb_w3_gemm_small_add.restype = ctypes.c_int
         lib.fb_w3_gemm_small_add.argtypes = lib.fb_w3_gemm_small.argtypes[:8] + [ctypes.c_void_p] + lib.fb_w3_gemm_small.argtypes[8:]
+        lib.fb_w3_gemm.restype = ctypes.c_int
+        lib.fb_w3_gemm.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.POINTER(W3Matrix)] + [ctypes.c_int] * 4 + [
+            ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
         lib.fb_w3_gemv_push.restype = ctypes.c_int
         lib.fb_w3_gemv_push.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_float,
                                         ctypes.POINTER(W3Matrix), ctypes.c_int, ctypes.c_int, ctypes.POINTER(W3Push), ctypes.c_void_p,
@@ -638,6 +641,22 @@ def embed_row(embedding, token, out) -> None:
     vocab, k = embedding.shape
     with torch.cuda.device(out.device):
         check(library().fb_embed_row(ptr(embedding), ptr(token), ptr(out), vocab, k, stream_handle(out.device)))
+
+
+def w3_gemm(x, layouts, out, addend=None) -> None:
+    """Many rows: ``out`` ``[T, sum of O]`` = ``x`` ``[T,K]`` times the stacked rows of one to four layouts, plus ``addend``
+    (as ``out``); ``x`` in group-sorted column order."""
+    matrices, begin, step = (W3Matrix * len(layouts))(), 0, out.element_size()
+    for matrix, layout in zip(matrices, layouts):
+        rows = layout["planes"].shape[2]
+        matrix.planes, matrix.scales, matrix.zeros = layout["planes"].data_ptr(), layout["scales"].data_ptr(), _addr(layout.get("zeros"))
+        matrix.out, matrix.residual = out.data_ptr() + begin * step, None if addend is None else addend.data_ptr() + begin * step
+        matrix.out_features = rows
+        begin += rows
+    scratch = scratch_for(x.device, 256, "w3mma")
+    with torch.cuda.device(x.device):
+        check(library().fb_w3_gemm(ptr(x), dtype_tag(x.dtype), x.shape[0], matrices, len(layouts), dtype_tag(layouts[0]["scales"].dtype), x.shape[1], out.stride(0),
+                                   ptr(scratch), scratch.numel(), stream_handle(x.device)))
 
 
 def w3_dequant(entries, out_dtype, *, row_begin: int = 0, row_count: int = 0) -> None:

@@ -112,6 +112,19 @@ bool plane_tensor_map(const uint8_t* planes, int O, int G, int rows, int box_uni
   return true;
 }
 
+bool activation_tensor_map(const void* base, int T, int K, int rows, CUtensorMap* out) {
+  std::lock_guard<std::mutex> guard(g_map_lock);
+  if (!encoder_ready()) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)T};
+  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)rows};
+  const cuuint32_t step[2] = {1, 1};
+  const CUresult rc = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (rc != CUDA_SUCCESS) fail(FB_ECUDA, "cuTensorMapEncodeTiled failed with code %d for activations [%d,%d]", (int)rc, T, K);
+  return rc == CUDA_SUCCESS;
+}
+
 bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, int rows, CUtensorMap* out) {
   std::lock_guard<std::mutex> guard(g_map_lock);
   if (!encoder_ready()) return false;

@@ -37,6 +37,10 @@ bool plane_tensor_map(const uint8_t* planes, int O, int G, int rows, int box_uni
 // box = `rows` rows x 2 groups; rows of the box beyond G read as zero.
 bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, int rows, CUtensorMap* out);
 
+// Descriptor of 16-bit activations [T][K], box = `rows` rows x 64 inputs with a 128-byte swizzle; rows beyond T
+// read as zero.  Not cached: activations come and go.
+bool activation_tensor_map(const void* base, int T, int K, int rows, CUtensorMap* out);
+
 // Launch with the programmatic-dependent-launch attribute (unless switched off): the kernel's
 // prologue may overlap the tail of the previous kernel in the stream.
 template <class Kernel, class... Args>

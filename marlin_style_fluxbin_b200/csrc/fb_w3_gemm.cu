@@ -1,0 +1,460 @@
+// GPTQ W3 group-128 planar weights times many activation rows (prompts, the dense fallback): y[T,O] = x[T,K] . W^T.
+//
+// One persistent kernel instead of chunks that were dequantised into L2 and read back by a library GEMM, two
+// or three launches each.  A CTA owns 128 output rows of up to 256 tokens at a time; roles are warps:
+//
+//   warp 0         TMA: activations of a group, 128-byte swizzle, ring of three stages of 256 tokens or more of fewer
+//   warp 2         TMA: plane tiles (three planes of 128 rows of a group), ring of four
+//   warps 4..19    four warpgroups take turns on groups: a thread dequantises ITS row of the group and puts the 16-bit
+//                  weights into tensor memory (tcgen05.st), where the MMA takes its A operand from: shared
+//                  memory, which the B operand and its copies already load to two thirds, never sees them
+//   warp 1         tcgen05.mma, 128 x tokens x 16
+//   warps 20..27   epilogue: accumulator -> outputs
+//
+// Tensor memory: the accumulator (256 columns) and four operand slots of a group (64 columns each).  Two slots
+// and two accumulators of 192 columns, which let the epilogue overlap the next tile, ran 10 % slower: the way
+// from a finished MMA over the refilled slot to the next one is longer than an MMA.  A weight takes one of
+// eight values per (row, group), scale * (code - zero) rounded in the scale's dtype and then in the
+// activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes.
+//
+// What bounds it: up to about 100 tokens a tile the integer instructions of the look-ups (some 800 clocks per
+// 128 x 128 weights), at 256 the MMA (1300 TFLOP/s where the tiles fill the SMs).  us on a B200, weights cold, chunks
+// -> this, without the launches' host time: 12288 x 4096 at 64 / 512 / 1024 tokens 40 / 62 / 95 -> 22 / 49 / 90,
+// 24576 x 4096 at 512 119 -> 88, 4096 x 12288 at 512 / 1024 71 / 98 -> 54 / 78.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <mutex>
+
+#include "fb_common.cuh"
+
+namespace {
+
+using namespace fb;
+
+constexpr int kRows = 128;
+constexpr int kMaxTokens = 256;  // of a tile
+constexpr int kDequant = 4;      // warpgroups that dequantise
+constexpr int kEpilogue = 2;     // warpgroups that write outputs
+constexpr int kThreads = 128 * (1 + kDequant + kEpilogue);
+constexpr int kBBytes = 192 * 1024;  // ring of activation stages, a group each: three of 256 tokens, more of fewer
+constexpr int kMaxBStages = 8;
+constexpr int kPlaneStages = 4;  // even: a stage always serves the same warpgroup (a wait by parity must not fall two phases behind)
+constexpr int kPlaneStage = 3 * kRows * 16;
+constexpr int kASlots = 4;             // weights of a group, 64 columns
+constexpr int kAColumn = kMaxTokens;  // behind the accumulator
+constexpr int kMaxMats = 4;
+constexpr int kBars = 2 * kMaxBStages + 2 * kPlaneStages + 2 * kASlots + 2;
+constexpr size_t kSmem = kBBytes + kPlaneStages * kPlaneStage + kBars * 8 + 16;
+
+struct GemmMatrix {
+  CUtensorMap plane_map;  // planes as uint32 [G*3][O/32][128], box 3 x 4 x 128
+  const unsigned short* scales;
+  const uint8_t* zeros;
+  unsigned short* out;
+  const unsigned short* addend;
+  int O, tile_begin;  // first row tile
+};
+
+struct GemmParams {
+  alignas(64) GemmMatrix mats[kMaxMats];
+  CUtensorMap x_map;  // [T][K], box = tokens of a tile x 64
+  unsigned* status;
+  int n, T, G, ldo;
+  int tokens, token_tiles, tiles, b_stages;
+  int act_dtype, scale_dtype;
+};
+
+__device__ __forceinline__ void tcgen_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tcgen_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool elected() {
+  uint32_t yes;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+  return yes != 0;
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// 32 columns of this warp's 32 lanes
+__device__ __forceinline__ void tmem_store32(uint32_t at, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
+      "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(at),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+      "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
+      "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t at, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(at));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned short bits16(float v, int dtype) {
+  return dtype == FB_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+}
+
+// scale * c and scale * (c + 1), rounded in the scale's dtype and then in the activations'
+__device__ __forceinline__ uint32_t two_values(float scale, float c, int scale_dtype, int act_dtype) {
+  float2 v = make_float2(scale * c, scale * (c + 1.f));
+  if (scale_dtype == FB_BF16)
+    v = __bfloat1622float2(__floats2bfloat162_rn(v.x, v.y));
+  else
+    v = __half22float2(__floats2half2_rn(v.x, v.y));
+  uint32_t bits;
+  if (act_dtype == FB_BF16)
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(bits) : "f"(v.y), "f"(v.x));
+  else
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(bits) : "f"(v.y), "f"(v.x));
+  return bits;
+}
+
+// Bytes picked by a selector whose nibbles are below eight (__byte_perm would mask it first).
+__device__ __forceinline__ uint32_t pick(uint32_t a, uint32_t b, uint32_t selector) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(selector));
+  return d;
+}
+// (a & m) | (b & ~m)
+__device__ __forceinline__ uint32_t blend(uint32_t a, uint32_t b, uint32_t m) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(m));
+  return d;
+}
+
+// 32 codes of a row (one word per plane, the high one inverted) -> 16 operand registers, inputs in order.  low, high: bytes
+// of the values of the eight codes.
+__device__ __forceinline__ void look_up(uint32_t p0, uint32_t p1, uint32_t p2, const uint32_t (&low)[2], const uint32_t (&high)[2], uint32_t* to) {
+  uint32_t codes[4];  // nibble n of codes[s]: the code of input 4 n + s
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const uint32_t a = p0 >> s, b = s == 0 ? p1 << 1 : p1 >> (s - 1), c = s < 2 ? p2 << (2 - s) : p2 >> (s - 2);
+    const uint32_t two = blend(a, b, 0x11111111u) & 0x33333333u;
+    asm("lop3.b32 %0, %1, %2, %3, 0xF4;" : "=r"(codes[s]) : "r"(two), "r"(0x44444444u), "r"(c));  // two | (0x4444... & ~c)
+  }
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t x[4][2];  // [s]: inputs 16 half + s, + 4 and + 8, + 12
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const uint32_t sel = half ? codes[s] >> 16 : codes[s];
+      const uint32_t l = pick(low[0], low[1], sel), h = pick(high[0], high[1], sel);
+      x[s][0] = pick(l, h, 0x5140u), x[s][1] = pick(l, h, 0x7362u);
+    }
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      uint32_t* const eight = to + 8 * half + 4 * b;
+      eight[0] = pick(x[0][b], x[1][b], 0x5410u), eight[1] = pick(x[2][b], x[3][b], 0x5410u);
+      eight[2] = pick(x[0][b], x[1][b], 0x7632u), eight[3] = pick(x[2][b], x[3][b], 0x7632u);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_constant__ GemmParams p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char* const planes_s = smem + kBBytes;
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(planes_s + kPlaneStages * kPlaneStage);
+  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kMaxBStages;
+  const uint32_t p_full = b_empty + 8 * kMaxBStages, p_empty = p_full + 8 * kPlaneStages;
+  const uint32_t a_full = p_empty + 8 * kPlaneStages, a_empty = a_full + 8 * kASlots;
+  const uint32_t d_full = a_empty + 8 * kASlots, d_empty = d_full + 8;
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars);
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+
+  if (tid < kBars) {
+    const int at = tid - 2 * kMaxBStages;
+    const bool by_group = (at >= kPlaneStages && at < 2 * kPlaneStages + kASlots);  // p_empty, a_full: a dequantising warpgroup
+    mbar_init(b_full + 8 * tid, tid == kBars - 1 ? 128 * kEpilogue : by_group ? 128 : 1);
+    mbar_init_fence();
+  }
+  if (warp == 3) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen_before();
+  __syncthreads();
+  tcgen_after();
+  const uint32_t tmem = *tmem_slot;
+  const int G = p.G;
+  bool dead = false;
+
+  auto matrix_of = [&](int row_tile) {
+    int j = 0;
+    while (j + 1 < p.n && row_tile >= p.mats[j + 1].tile_begin) ++j;
+    return j;
+  };
+
+  // What lies in x, the addends and the outputs belongs to the launches ahead; the weights do not.
+  if (warp != 2) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  if (warp == 0) {
+    if (lane == 0) {
+      unsigned stage = 0, phase = 0;
+      bool first = true;  // round of the ring
+      for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x) {
+        const int token0 = (tile % p.token_tiles) * p.tokens;
+        for (int g = 0; g < G; ++g) {
+          if (!first && !mbar_wait_bounded(b_empty + 8 * stage, phase ^ 1u)) {
+            dead = true;
+            break;
+          }
+          mbar_expect_tx(b_full + 8 * stage, (uint32_t)p.tokens * 256u);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                             smem_u32(smem) + (uint32_t)((2 * stage + h) * p.tokens * 128)),
+                         "l"(&p.x_map), "r"(g * 128 + h * 64), "r"(token0), "r"(b_full + 8 * stage)
+                         : "memory");
+          if (++stage == (unsigned)p.b_stages) stage = 0, phase ^= 1u, first = false;
+        }
+      }
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      unsigned step = 0;
+      for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x) {
+        const int row_tile = tile / p.token_tiles, j = matrix_of(row_tile);
+        const int unit = (row_tile - p.mats[j].tile_begin) * (kRows / 32);
+        for (int g = 0; g < G; ++g, ++step) {
+          const unsigned stage = step % kPlaneStages, use = step / kPlaneStages;
+          if (use && !mbar_wait_bounded(p_empty + 8 * stage, (use - 1) & 1)) {
+            dead = true;
+            break;
+          }
+          mbar_expect_tx(p_full + 8 * stage, (uint32_t)kPlaneStage);
+          asm volatile(
+              "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                  smem_u32(planes_s + stage * kPlaneStage)),
+              "l"(&p.mats[j].plane_map), "r"(0), "r"(unit), "r"(3 * g), "r"(p_full + 8 * stage)
+              : "memory");
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // the whole warp walks the loop and one elected lane issues: operands known to be the same in all lanes go to the
+    // tensor core's instructions as they are (issued from a lane's own branch, four of them took 480 clocks)
+    // D fp32, A and B in the activation dtype, both K-major
+    const uint32_t format = p.act_dtype == FB_BF16 ? 1u : 0u;
+    const uint32_t idesc = (1u << 4) | (format << 7) | (format << 10) | ((uint32_t)(p.tokens >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+    // K-major, 128-byte swizzle: 8-row groups 1024 bytes apart; 16 inputs are 32 bytes of a row
+    const uint64_t b_desc0 = (uint64_t)((smem_u32(smem) >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+    unsigned step = 0, stage = 0, stage_phase = 0, it = 0;
+    for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x, ++it) {
+      if (it && !__all_sync(0xffffffffu, mbar_wait_bounded(d_empty, (it - 1) & 1))) {
+        dead = true;
+        break;
+      }
+      for (int g = 0; g < G; ++g, ++step) {
+        const unsigned slot = step % kASlots, use = step / kASlots;
+        const bool there = mbar_wait_bounded(b_full + 8 * stage, stage_phase) && mbar_wait_bounded(a_full + 8 * slot, use & 1);
+        if (!__all_sync(0xffffffffu, there)) {
+          dead = true;
+          break;
+        }
+        tcgen_after();
+        const uint64_t b_desc = b_desc0 + stage * (p.tokens * 16);
+        const uint32_t a = tmem + kAColumn + slot * 64;
+        const uint32_t a_done = a_empty + 8 * slot, b_done = b_empty + 8 * stage;
+        if (elected()) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            asm volatile(
+                "{\n\t"
+                ".reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+                "}\n" ::"r"(tmem),
+                "r"(a + 8 * i), "l"(b_desc + (i >> 2) * (p.tokens * 8) + 2 * (i & 3)), "r"(idesc), "r"(g + i > 0 ? 1u : 0u)
+                : "memory");
+          commit(a_done);
+          commit(b_done);
+          if (g + 1 == G) commit(d_full);
+        }
+        __syncwarp();
+        if (++stage == (unsigned)p.b_stages) stage = 0, stage_phase ^= 1u;
+      }
+    }
+  } else if (warp >= 4 && warp < 4 + 4 * kDequant) {
+    const int group_of = (warp - 4) >> 2, row_in_tile = tid & 127;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    unsigned count = 0;  // groups of this CTA so far
+    for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x) {
+      const int row_tile = tile / p.token_tiles, j = matrix_of(row_tile);
+      const GemmMatrix& m = p.mats[j];
+      const int row = (row_tile - m.tile_begin) * kRows + row_in_tile;
+      // scale and zero point are requested one group of this warpgroup ahead; rows past O have weight zero
+      uint32_t scale_next = 0, zero_next = 4;
+      auto fetch = [&](int g) {
+        scale_next = 0, zero_next = 4;
+        if (row < m.O && g < G) {
+          asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(scale_next) : "l"(m.scales + (size_t)g * m.O + row));
+          if (m.zeros) asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(zero_next) : "l"(m.zeros + (size_t)g * m.O + row));
+        }
+      };
+      int g = (int)((group_of - count) % kDequant);  // the warpgroups take turns, across tiles too
+      fetch(g);
+      for (; g < G; g += kDequant) {
+        const unsigned at = count + g, stage = at % kPlaneStages;
+        const float scale = bits_to_float((unsigned short)scale_next, p.scale_dtype);
+        const float zero = (float)zero_next;
+        fetch(g + kDequant);
+        uint32_t low[2], high[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t a = two_values(scale, (float)(4 * q) - zero, p.scale_dtype, p.act_dtype), b = two_values(scale, (float)(4 * q + 2) - zero, p.scale_dtype, p.act_dtype);
+          low[q] = __byte_perm(a, b, 0x6420), high[q] = __byte_perm(a, b, 0x7531);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full + 8 * stage, (at / kPlaneStages) & 1))) {
+          dead = true;
+          break;
+        }
+        const uint4* const from = reinterpret_cast<const uint4*>(planes_s + stage * kPlaneStage) + row_in_tile;
+        const uint4 w0 = from[0], w1 = from[kRows], w2 = from[2 * kRows];
+        arrive(p_empty + 8 * stage);
+        const unsigned slot = at % kASlots, use = at / kASlots;
+        bool late = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t v[32];
+          look_up(h ? w0.z : w0.x, h ? w1.z : w1.x, h ? w2.z : w2.x, low, high, v);
+          look_up(h ? w0.w : w0.y, h ? w1.w : w1.y, h ? w2.w : w2.y, low, high, v + 16);
+          if (h == 0) {
+            late = use && !__all_sync(0xffffffffu, mbar_wait_bounded(a_empty + 8 * slot, (use - 1) & 1));
+            if (late) break;
+            tcgen_after();
+          }
+          tmem_store32(tmem + lanes + kAColumn + slot * 64 + h * 32, v);
+        }
+        if (late) {
+          dead = true;
+          break;
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tcgen_before();
+        arrive(a_full + 8 * slot);
+      }
+      count += G;
+    }
+  } else if (warp >= 4 + 4 * kDequant) {
+    const int row_in_tile = tid & 127, part = (warp - 4 - 4 * kDequant) >> 2;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    unsigned it = 0;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
+      const int row_tile = tile / p.token_tiles, j = matrix_of(row_tile);
+      const GemmMatrix& m = p.mats[j];
+      const int row = (row_tile - m.tile_begin) * kRows + row_in_tile, token0 = (tile - row_tile * p.token_tiles) * p.tokens;
+      const int tokens = min(p.tokens, p.T - token0);
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(d_full, it & 1))) {
+        dead = true;
+        break;
+      }
+      tcgen_after();
+      for (int c = 16 * part; c < tokens; c += 16 * kEpilogue) {
+        uint32_t v[16];
+        __syncwarp();
+        tmem_load16(tmem + lanes + c, v);
+        if (row < m.O) {
+          const size_t at = (size_t)(token0 + c) * p.ldo + row;
+          unsigned short* to = m.out + at;
+          const unsigned short* add = m.addend + at;
+#pragma unroll
+          for (int i = 0; i < 16; ++i, to += p.ldo, add += p.ldo) {
+            if (c + i < tokens) {
+              float y = __uint_as_float(v[i]);
+              if (m.addend) y += bits_to_float(*add, p.act_dtype);
+              *to = bits16(y, p.act_dtype);
+            }
+          }
+        }
+      }
+      __syncwarp();
+      tcgen_before();
+      arrive(d_empty);
+    }
+  }
+  if (dead) atomicExch(p.status, 3u);
+  __syncwarp();
+  tcgen_before();
+  __syncthreads();
+  tcgen_after();
+  if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// Tokens of a tile: a group of a tile measures about 330 + 1.75 tokens ns (16 to 256 tokens, K 4096 and 12288), in rounds of
+// one tile per SM; of the splits that fit, the cheapest.
+int token_tile(int T, int row_tiles, int sms) {
+  int best = 0;
+  long long best_cost = 0;
+  const int fewest = (T + kMaxTokens - 1) / kMaxTokens;
+  for (int n = fewest; n <= fewest + 12; ++n) {
+    const int tokens = ((T + n - 1) / n + 15) / 16 * 16;
+    const long long tiles = (long long)row_tiles * ((T + tokens - 1) / tokens), cost = (tiles + sms - 1) / sms * (190 + tokens);
+    if (!best || cost < best_cost) best = tokens, best_cost = cost;
+  }
+  return best;
+}
+
+}  // namespace
+
+extern "C" int fb_w3_gemm(const void* x, int act_dtype, int tokens, const fb_w3_matrix_t* mats, int n_mats, int scale_dtype, int in_features, int out_stride,
+                          void* scratch, size_t scratch_bytes, fb_stream_t stream) {
+  if (!x || !mats) return fail(FB_EINVAL, "fb_w3_gemm: null pointer");
+  if (n_mats < 1 || n_mats > kMaxMats) return fail(FB_ELIMIT, "fb_w3_gemm: %d matrices outside 1..%d", n_mats, kMaxMats);
+  if ((act_dtype != FB_F16 && act_dtype != FB_BF16) || (scale_dtype != FB_F16 && scale_dtype != FB_BF16))
+    return fail(FB_EINVAL, "fb_w3_gemm: dtype tags must be FB_F16 or FB_BF16");
+  if (tokens < 1 || in_features < 128 || in_features % 128 || in_features / 128 > 255)
+    return fail(FB_ELIMIT, "fb_w3_gemm: T=%d, K=%d: K must be a multiple of 128 with at most 255 groups", tokens, in_features);
+  if (!aligned(x, 16)) return fail(FB_EINVAL, "fb_w3_gemm: x must be 16-byte aligned");
+  if (!scratch || scratch_bytes < 256 || !aligned(scratch, 4)) return fail(FB_ESCRATCH, "fb_w3_gemm: scratch of 256 bytes needed, %zu given", scratch_bytes);
+  const DeviceInfo* info = device_info();
+  if (!info) return FB_ECUDA;
+  if (kSmem > (size_t)info->max_smem_optin) return fail(FB_ELIMIT, "fb_w3_gemm: needs %zu bytes of shared memory", kSmem);
+  GemmParams p;
+  p.n = n_mats, p.T = tokens, p.G = in_features / 128, p.ldo = out_stride;
+  p.act_dtype = act_dtype, p.scale_dtype = scale_dtype;
+  p.status = static_cast<unsigned*>(scratch);
+  int row_tiles = 0;
+  for (int j = 0; j < n_mats; ++j) {
+    const fb_w3_matrix_t& in = mats[j];
+    if (!in.planes || !in.scales || !in.out) return fail(FB_EINVAL, "fb_w3_gemm: planes, scales and out must be non-null");
+    if (in.out_features < 32 || in.out_features > 65536 || in.out_features % 32) return fail(FB_ELIMIT, "fb_w3_gemm: O=%d must be a multiple of 32 in 32..65536", in.out_features);
+    if (out_stride < in.out_features) return fail(FB_EINVAL, "fb_w3_gemm: rows of out are %d apart, %d long", out_stride, in.out_features);
+    if (!aligned(in.planes, 16) || !aligned(in.scales, 2) || !aligned(in.out, 2) || !aligned(in.residual, 2))
+      return fail(FB_EINVAL, "fb_w3_gemm: planes must be 16-byte aligned, 16-bit tensors 2-byte aligned");
+    const size_t out_bytes = ((size_t)(tokens - 1) * out_stride + in.out_features) * 2;
+    if (overlaps(in.out, out_bytes, x, (size_t)tokens * in_features * 2)) return fail(FB_EALIAS, "fb_w3_gemm: out overlaps x");
+    GemmMatrix& m = p.mats[j];
+    if (!plane_tensor_map(in.planes, in.out_features, p.G, 32, kRows / 32, 3, &m.plane_map)) return FB_ECUDA;
+    m.scales = static_cast<const unsigned short*>(in.scales), m.zeros = in.zeros;
+    m.out = static_cast<unsigned short*>(in.out), m.addend = static_cast<const unsigned short*>(in.residual);
+    m.O = in.out_features, m.tile_begin = row_tiles;
+    row_tiles += (in.out_features + kRows - 1) / kRows;
+  }
+  p.tokens = token_tile(tokens, row_tiles, info->sm_count);
+  p.token_tiles = (tokens + p.tokens - 1) / p.tokens;
+  p.tiles = row_tiles * p.token_tiles;
+  p.b_stages = kBBytes / (p.tokens * 256);
+  if (p.b_stages > kMaxBStages) p.b_stages = kMaxBStages;
+  if (!activation_tensor_map(x, tokens, in_features, p.tokens, &p.x_map)) return FB_ECUDA;
+
+  static std::mutex lock;
+  static bool ready[64] = {};
+  int device = 0;
+  if (cudaError_t err = cudaGetDevice(&device); err != cudaSuccess) return cuda_fail(err, "cudaGetDevice");
+  if (device < 0 || device >= 64) return fail(FB_ELIMIT, "device ordinal %d outside 0..63", device);
+  {
+    std::lock_guard<std::mutex> guard(lock);
+    if (!ready[device]) {
+      if (cudaError_t err = cudaFuncSetAttribute(w3_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem); err != cudaSuccess)
+        return cuda_fail(err, "cudaFuncSetAttribute(w3_gemm_kernel)");
+      ready[device] = true;
+    }
+  }
+  const int grid = p.tiles < info->sm_count ? p.tiles : info->sm_count;
+  return launch_pdl(w3_gemm_kernel, dim3(grid), dim3(kThreads), kSmem, static_cast<cudaStream_t>(stream), "w3_gemm_kernel launch", p);
+}

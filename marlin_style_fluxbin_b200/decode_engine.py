@@ -27,7 +27,7 @@ from torch.nn import functional as F
 
 from . import _native
 from .gptq_deployment import restore_planar_w3
-from .w3_lut_deployment import DENSE_CHUNK_BYTES
+from .w3_lut_deployment import DENSE_CHUNK_BYTES, fused_gemm_pays
 
 
 @dataclass(frozen=True)
@@ -258,8 +258,9 @@ class DecodeEngine:
     # ------------------------------------------------------------------ prefill (many tokens)
     def _prompt_linear(self, x, layouts, dense, addend=None):
         """``x`` ``[T,K]`` times the stacked rows of ``layouts`` (``dense``: the same rows as one dense matrix, or None
-        on the packed arm), plus ``addend``.  The packed arm keeps up to 16 tokens packed; for more it forms the weight
-        in chunks that stay in the L2 between the dequantising launch and the GEMM."""
+        on the packed arm), plus ``addend``.  The packed arm keeps up to 16 tokens packed; up to a thousand go through the
+        kernel that dequantises into tensor memory; beyond, and for narrow matrices, the weight is formed in chunks
+        that stay in the L2 between the dequantising launch and the GEMM."""
         if dense is not None:
             return torch.mm(x, dense.t()) if addend is None else torch.addmm(addend, x, dense.t())
         t, k = x.shape
@@ -269,6 +270,10 @@ class DecodeEngine:
                 _native.w3_gemm_small(x, lay["planes"], lay["scales"], lay["zeros"], None, part, addend=addend)
             return parts[0] if len(parts) == 1 else torch.cat(parts, dim=1)
         rows = sum(lay["planes"].shape[2] for lay in layouts)
+        if fused_gemm_pays(t, rows):
+            y = torch.empty(t, rows, device=self.device, dtype=self.dtype)
+            _native.w3_gemm(x, layouts, y, addend)
+            return y
         if len(layouts) > 1 or rows * k * 2 <= DENSE_CHUNK_BYTES:
             weight = self._dense_rows(layouts)
             return torch.mm(x, weight.t()) if addend is None else torch.addmm(addend, x, weight.t())
@@ -287,7 +292,7 @@ class DecodeEngine:
         """``silu(x gate^T) * (x up^T)`` ``[T, inter]``; the packed arm takes matching rows of gate and up together."""
         t, k = x.shape
         act = torch.empty(t, self.inter, device=self.device, dtype=self.dtype)
-        if layer.dense is not None or t <= 16:
+        if layer.dense is not None or t <= 16 or fused_gemm_pays(t, 2 * self.inter):
             _native.silu_mul_rows(self._prompt_linear(x, (layer.gate, layer.up), None if layer.dense is None else layer.dense["gate_up"]), act)
             return act
         step = _chunk_rows(2 * self.inter, k) // 2

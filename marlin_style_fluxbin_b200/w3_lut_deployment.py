@@ -25,6 +25,13 @@ from .gptq_deployment import FIELDS, OPTIONAL_FIELDS, restore_planar_w3, validat
 # chunk out of the L2 (126 MB), and the next chunk overwrites it there before it is written back.
 DENSE_CHUNK_BYTES = 52 << 20
 
+
+def fused_gemm_pays(rows: int, out_features: int) -> bool:
+    """Whether ``rows`` activation rows go through the kernel that dequantises into tensor memory rather than through dense
+    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy (1024 x 4096: 24 us against 14, at
+    4096 x 4096 they meet); beyond a thousand rows the chunks, dequantised once for all of them, catch up."""
+    return rows <= 1024 and out_features > 2048 and out_features % 32 == 0
+
 ROW_TILES = (256, 512, 1024)
 EXPERIMENTAL_ROW_TILES = ROW_TILES + (2048,)
 ARITHMETIC_MODES = ("structural", "decoded_bf16")
@@ -344,7 +351,9 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
 
 def dense_linear(x, layout, bias=None):
     """``x`` ``[T,K]`` (16-bit, CUDA) times the dequantised weight, without the packed kernels' row limit: up to 16 rows
-    without a bias stay packed (the tensor-core kernel, whose weights are not rounded at all), the rest goes through dense chunks of the weight in group-sorted column order, with the activations gathered into that order."""
+    without a bias stay packed (the tensor-core kernel, whose weights are not rounded at all), the rest, its
+    activations gathered into group-sorted column order, goes through the kernel that dequantises into tensor memory or
+    through dense chunks of the weight."""
     planes, scales, zeros, perm = _layout_args(layout)
     rows, (out_features, in_features) = x.shape[0], (planes.shape[2], x.shape[1])
     y = torch.empty(rows, out_features, device=x.device, dtype=x.dtype)
@@ -357,6 +366,9 @@ def dense_linear(x, layout, bias=None):
         ordered = torch.empty_like(x)
         _native.gather_columns(x, perm, ordered)
         x = ordered
+    if fused_gemm_pays(rows, out_features) and x.data_ptr() % 16 == 0:
+        _native.w3_gemm(x, (layout,), y, None if bias is None else bias.to(x.dtype).expand(rows, out_features).contiguous())
+        return y
     chunks = -(-out_features * in_features * 2 // DENSE_CHUNK_BYTES)
     step = -(-(-(-out_features // chunks)) // 64) * 64
     weight = torch.empty(min(step, out_features), in_features, device=x.device, dtype=x.dtype)
