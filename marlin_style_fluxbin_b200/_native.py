@@ -6,6 +6,7 @@ used for the launch.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os as _os
 from pathlib import Path
@@ -196,12 +197,12 @@ def dtype_tag(dtype: torch.dtype) -> int:
 
 
 def ptr(tensor):
-    return None if tensor is None else ctypes.c_void_p(tensor.data_ptr())
+    return None if tensor is None else tensor.data_ptr()
 
 
-def stream_handle(device) -> ctypes.c_void_p:
+def stream_handle(device) -> int:
     index = device.index
-    return ctypes.c_void_p(_raw_stream(_current_device() if index is None else index))
+    return _raw_stream(_current_device() if index is None else index)
 
 
 def query(key: str) -> int:
@@ -235,8 +236,8 @@ def _family_bytes(family: str) -> int:
 def scratch_for(device: torch.device, nbytes: int, family: str = "w3") -> torch.Tensor:
     """Zero-filled scratch per (device, stream, kernel family).  Families lay their control words
     out differently, and each kernel relies on finding its own words zero, so they never share."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream, family)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (index, _raw_stream(index), family)
     buf = _scratch.get(key)
     if buf is None or buf.numel() < nbytes:
         if torch.cuda.is_current_stream_capturing():
@@ -272,6 +273,15 @@ def check_status(device: torch.device | None = None) -> None:
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 _current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_HERE = contextlib.nullcontext()
+
+
+def _on(device):
+    """The device as current device; nothing is done, and nothing looked up, when it is that already."""
+    index = device if isinstance(device, int) else device.index
+    return _HERE if index is not None and index == _current_device() else torch.cuda.device(device)
+
+
 _W3_SLOTS = ("w3", "w3#1", "w3#2")
 _NO_PDL, _NO_SAME_INPUT = bool(_os.environ.get("FB_NO_PDL")), bool(_os.environ.get("FB_NO_SAME_INPUT"))
 
@@ -306,7 +316,7 @@ class Launch:
         lib = library()
         handle, device = ctypes.c_void_p(), tensors[0].device
         tag = dtype_tag(act_dtype)
-        with torch.cuda.device(device):
+        with _on(device):
             if kind == "bb":
                 codes, *rest = tensors
                 code = lib.fb_bb_prepare(tag, codes.data_ptr(), int(codes.ndim == 4), *(t.data_ptr() for t in rest), out_features, in_features, ctypes.byref(handle))
@@ -364,7 +374,7 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
         scratch = scratch_for(x.device, w3_scratch_bytes(m, o, k), _W3_SLOTS[slot])
     flags = (FB_W3_DECODED_BF16 if decoded_bf16 else 0) | (0 if pdl else FB_W3_NO_PDL) | (
         FB_W3_GROUP_PARTIALS if group_partials else 0) | (FB_W3_SAME_INPUT if slot else 0)
-    with torch.cuda.device(index):
+    with _on(index):
         check(library().fb_w3_gemv(
             x.data_ptr(), dtype_tag(x.dtype), m, planes.data_ptr(), scales.data_ptr(), dtype_tag(scales.dtype),
             _addr(zeros), _addr(perm), out.data_ptr(), o, k, scratch.data_ptr(), scratch.numel() * scratch.element_size(),
@@ -376,7 +386,7 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
 def w3_finish(partials, out) -> None:
     """out[0, o] = sum over rows of partials[:, o] (ascending), cast to out's dtype."""
     splits, o = partials.shape
-    with torch.cuda.device(out.device):
+    with _on(out.device):
         check(library().fb_w3_finish(ptr(partials), splits, o, ptr(out), dtype_tag(out.dtype),
                                      stream_handle(out.device)))
 
@@ -394,7 +404,7 @@ def w3_gemv_static(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, p
     m, k = x.shape
     o = planes.shape[2]
     flags = (FB_W3_DECODED_BF16 if decoded_bf16 else 0) | (0 if pdl else FB_W3_NO_PDL)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemv_static(
             ptr(x), dtype_tag(x.dtype), m, ptr(planes), ptr(scales), dtype_tag(scales.dtype),
             ptr(zeros), ptr(perm), ptr(out), o, k, flags, stream_handle(x.device)))
@@ -403,7 +413,7 @@ def w3_gemv_static(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, p
 def rmsnorm(x, weight, out, eps: float) -> None:
     """``out = weight * dtype(x * rsqrt(mean(x^2) + eps))`` over the last dimension of ``x``."""
     dim = x.shape[-1]
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_rmsnorm(ptr(x), ptr(weight), ptr(out), x.numel() // dim, dim, float(eps),
                                    dtype_tag(x.dtype), stream_handle(x.device)))
 
@@ -411,7 +421,7 @@ def rmsnorm(x, weight, out, eps: float) -> None:
 def rope_qk(q, k, cos, sin, q_out, k_out) -> None:
     """Rotary embedding of one position: ``q [Hq,D]``, ``k [Hk,D]`` (any leading unit dims), ``cos/sin [D]``."""
     dim = q.shape[-1]
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(library().fb_rope_qk(ptr(q), ptr(k), ptr(cos), ptr(sin), ptr(q_out), ptr(k_out),
                                    q.numel() // dim, k.numel() // dim, dim, dtype_tag(q.dtype), stream_handle(q.device)))
 
@@ -427,7 +437,7 @@ def bb_gemv(x, layout, out, *, pdl=True, scratch=None) -> None:
     k = groups * 128
     if scratch is None:
         scratch = scratch_for(x.device, bb_scratch_bytes(o, k, False), "bb")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_bb_gemv(
             ptr(x), dtype_tag(x.dtype), ptr(codes), int(codes.ndim == 4), ptr(layout["rows"]), ptr(layout["columns"]),
             ptr(layout["sparse_codes"]), ptr(layout["sparse_rows"]), ptr(layout["sparse_columns"]), ptr(layout["indices"]),
@@ -442,7 +452,7 @@ def bb_global_gemv(x, codes, row_scales, col_scales, salient_idx, salient, out, 
     if scratch is None:
         scratch = scratch_for(x.device, bb_scratch_bytes(o, k, True), "bb")
     n_sal = 0 if salient_idx is None else salient_idx.numel()
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_bb_global_gemv(
             ptr(x), dtype_tag(x.dtype), ptr(codes), ptr(row_scales), ptr(col_scales), ptr(salient_idx), ptr(salient),
             n_sal, ptr(out), o, k, ptr(scratch), scratch.numel() * scratch.element_size(), 0 if pdl else FB_W3_NO_PDL,
@@ -470,7 +480,7 @@ def w3_gemv_multi(x, matrices, n_matrices, total_out, scale_dtype, perm, *, deco
     if scratch is None:
         scratch = scratch_for(x.device, w3_scratch_bytes(m, total_out, k))
     flags = (FB_W3_DECODED_BF16 if decoded_bf16 else 0) | (0 if pdl else FB_W3_NO_PDL)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemv_multi(ptr(x), dtype_tag(x.dtype), m, matrices, n_matrices, dtype_tag(scale_dtype),
                                          ptr(perm), k, ptr(scratch), scratch.numel() * scratch.element_size(), flags,
                                          stream_handle(x.device)))
@@ -479,7 +489,7 @@ def w3_gemv_multi(x, matrices, n_matrices, total_out, scale_dtype, perm, *, deco
 def qknorm_rope_cache(q, k, v, q_weight, k_weight, cos, sin, q_out, k_cache, v_cache, position: int, eps: float) -> None:
     """Per-head RMSNorm of q/k, rotary embedding, and the KV-cache write of one token (see the header)."""
     dim = q_weight.numel()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(library().fb_qknorm_rope_cache(ptr(q), ptr(k), ptr(v), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(q_out),
                                              ptr(k_cache), ptr(v_cache), q.numel() // dim, k.numel() // dim, dim, int(position),
                                              k_cache.shape[-2], float(eps), dtype_tag(q.dtype), stream_handle(q.device)))
@@ -492,7 +502,7 @@ def attn_scratch_bytes(q_heads: int) -> int:
 def attn_decode(q, k_cache, v_cache, out, length: int, scale: float, scratch) -> None:
     """Single-query attention over cache positions ``0..length-1``; ``scratch``: zeroed uint8 buffer of ``attn_scratch_bytes``."""
     dim = k_cache.shape[-1]
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(library().fb_attn_decode(ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), q.numel() // dim, k_cache.shape[-3], dim,
                                        int(length), k_cache.shape[-2], float(scale), dtype_tag(q.dtype), ptr(scratch),
                                        scratch.numel(), stream_handle(q.device)))
@@ -503,7 +513,7 @@ def attn_decode_fused(q, k, v, q_weight, k_weight, cos, sin, k_cache, v_cache, o
     """``qknorm_rope_cache`` + ``attn_decode`` in one launch: raw q/k/v rows of the token at ``position``;
     writes cache row ``position`` and attends over positions ``0..position``."""
     dim = k_cache.shape[-1]
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(library().fb_attn_decode_fused(ptr(q), ptr(k), ptr(v), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(k_cache),
                                              ptr(v_cache), ptr(out), q.numel() // dim, k_cache.shape[-3], dim, int(position),
                                              k_cache.shape[-2], float(eps), float(scale), dtype_tag(q.dtype), ptr(scratch),
@@ -515,7 +525,7 @@ def attn_decode_partial(q, k, v, q_weight, k_weight, cos, sin, k_cache, v_cache,
     """``attn_decode_fused`` without its last step: every CTA leaves its share (output, max, sum) in ``partials``
     (uint8, ``attn_scratch_bytes`` long) for ``w3_gemv_attn_merge``.  Returns the number of splits per head."""
     dim = k_cache.shape[-1]
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(library().fb_attn_decode_partial(ptr(q), ptr(k), ptr(v), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(k_cache),
                                                ptr(v_cache), q.numel() // dim, k_cache.shape[-3], dim, int(position), k_cache.shape[-2],
                                                float(eps), float(scale), dtype_tag(q.dtype), ptr(partials), partials.numel(),
@@ -529,14 +539,14 @@ def w3_gemv_attn_merge(partials, splits: int, act_dtype, in_features: int, matri
     (``attn_decode_partial``); the pieces are merged while the tables are built."""
     if scratch is None:
         scratch = scratch_for(partials.device, w3_scratch_bytes(1, total_out, in_features))
-    with torch.cuda.device(partials.device):
+    with _on(partials.device):
         check(library().fb_w3_gemv_attn_merge(ptr(partials), int(splits), dtype_tag(act_dtype), matrices, n_matrices, dtype_tag(scale_dtype),
                                               int(in_features), ptr(scratch), scratch.numel() * scratch.element_size(),
                                               FB_W3_DECODED_BF16 if decoded_bf16 else 0, stream_handle(partials.device)))
 
 
 def silu_mul(gate, up, out) -> None:
-    with torch.cuda.device(gate.device):
+    with _on(gate.device):
         check(library().fb_silu_mul(ptr(gate), ptr(up), ptr(out), gate.numel(), dtype_tag(gate.dtype), stream_handle(gate.device)))
 
 
@@ -549,7 +559,7 @@ def w3_gemv_fused_input(x, transform: int, operand, eps: float, matrices, n_matr
     k = x.shape[-1]
     if scratch is None:
         scratch = scratch_for(x.device, w3_scratch_bytes(1, total_out, k))
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemv_fused_input(ptr(x), dtype_tag(x.dtype), transform, ptr(operand), float(eps), matrices, n_matrices,
                                                dtype_tag(scale_dtype), k, ptr(scratch), scratch.numel() * scratch.element_size(),
                                                (0 if pdl else FB_W3_NO_PDL) | (FB_W3_DECODED_BF16 if decoded_bf16 else 0),
@@ -563,7 +573,7 @@ def w3_gemm_small(x, planes, scales, zeros, perm, out, *, addend=None, scratch=N
     o = planes.shape[2]
     if scratch is None:
         scratch = scratch_for(x.device, library().fb_w3_gemm_small_scratch_bytes(m, o, k), "w3mma")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemm_small_add(ptr(x), dtype_tag(x.dtype), m, ptr(planes), ptr(scales), dtype_tag(scales.dtype),
                                          ptr(zeros) if zeros is not None else None, ptr(perm) if perm is not None else None,
                                          ptr(addend) if addend is not None else None, ptr(out), o, k, ptr(scratch), scratch.numel() * scratch.element_size(),
@@ -584,7 +594,7 @@ def w3_gemv_push(x, transform: int, operand, eps: float, matrix, k: int, scale_d
     """Row-split Linear of a tensor-parallel rank: results go to every rank's exchange buffer (see the header).
     With ``W3_INPUT_ATTN_PIECES`` ``x`` is the pieces buffer of ``attn_decode_partial``, ``eps`` the splits per head and
     ``act_dtype`` the activation dtype."""
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemv_push(ptr(x), dtype_tag(x.dtype if act_dtype is None else act_dtype), transform, ptr(operand), float(eps), matrix, dtype_tag(scale_dtype), k,
                                         ctypes.byref(push), ptr(scratch), scratch.numel() * scratch.element_size(),
                                         (0 if pdl else FB_W3_NO_PDL) | (FB_W3_DECODED_BF16 if decoded_bf16 else 0),
@@ -596,7 +606,7 @@ def tp_reduce(parts_ptr: int, world: int, residual, out, status_ptr: int, wait_n
 
     ``wait_ns`` bounds the poll (0 = the library default of ten seconds); on expiry the status word
     becomes 4 and the kernel returns."""
-    with torch.cuda.device(out.device):
+    with _on(out.device):
         check(library().fb_tp_reduce(ctypes.c_void_p(parts_ptr), world, ptr(residual), ptr(out), out.numel(), dtype_tag(out.dtype),
                                      ctypes.c_void_p(status_ptr), int(wait_ns), stream_handle(out.device)))
 
@@ -611,7 +621,7 @@ def lm_head_argmax(x, norm_weight, eps: float, weight, best, *, logits=None, for
     ``best`` (int64 ``[1]``); optionally the 16-bit logits, and the embedding row of the next token
     (``forced_next`` int64 ``[1]`` on the device, else the choice) copied into ``next_hidden``."""
     vocab, k = weight.shape
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_lm_head_argmax(ptr(x), ptr(norm_weight), float(eps), ptr(weight), vocab, k, dtype_tag(x.dtype), ptr(logits),
                                           ptr(best), ptr(forced_next), ptr(embedding), ptr(next_hidden), ptr(scratch),
                                           scratch.numel() * scratch.element_size(), stream_handle(x.device)))
@@ -621,7 +631,7 @@ def lm_head_shard(x, norm_weight, eps: float, weight_shard, row_base: int, keys:
     """The LM head over one rank's rows of the vocabulary (``weight_shard [V/p, K]``, a contiguous row range starting at
     ``row_base``): the shard's best key goes to slot ``rank`` of every rank's key array; follow with ``tp_argmax``."""
     rows, k = weight_shard.shape
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_lm_head_shard(ptr(x), ptr(norm_weight), float(eps), ptr(weight_shard), rows, int(row_base), k, dtype_tag(x.dtype),
                                          ptr(logits_shard), ctypes.byref(keys), int(rank), ptr(scratch), scratch.numel() * scratch.element_size(),
                                          stream_handle(x.device)))
@@ -631,7 +641,7 @@ def tp_argmax(keys_ptr: int, world: int, best, status_ptr: int, *, forced_next=N
     """Receiving half of ``lm_head_shard``: the largest of the ``world`` delivered keys becomes ``best`` (int64 ``[1]``); optionally
     the embedding row of ``forced_next`` (or of the choice) is copied into ``next_hidden``.  Bounded poll, status 6 on expiry."""
     vocab, k = embedding.shape if embedding is not None else (0, 0)
-    with torch.cuda.device(best.device):
+    with _on(best.device):
         check(library().fb_tp_argmax(ctypes.c_void_p(keys_ptr), world, ptr(best), ptr(forced_next), ptr(embedding), ptr(next_hidden), vocab, k,
                                      ctypes.c_void_p(status_ptr), int(wait_ns), stream_handle(best.device)))
 
@@ -639,7 +649,7 @@ def tp_argmax(keys_ptr: int, world: int, best, status_ptr: int, *, forced_next=N
 def embed_row(embedding, token, out) -> None:
     """``out[0, :] = embedding[token[0], :]`` for a token id held on the device (int64 ``[1]``)."""
     vocab, k = embedding.shape
-    with torch.cuda.device(out.device):
+    with _on(out.device):
         check(library().fb_embed_row(ptr(embedding), ptr(token), ptr(out), vocab, k, stream_handle(out.device)))
 
 
@@ -654,7 +664,7 @@ def w3_gemm(x, layouts, out, addend=None) -> None:
         matrix.out_features = rows
         begin += rows
     scratch = scratch_for(x.device, 256, "w3mma")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_w3_gemm(ptr(x), dtype_tag(x.dtype), x.shape[0], matrices, len(layouts), dtype_tag(layouts[0]["scales"].dtype), x.shape[1], out.stride(0),
                                    ptr(scratch), scratch.numel(), stream_handle(x.device)))
 
@@ -665,20 +675,20 @@ def w3_dequant(entries, out_dtype, *, row_begin: int = 0, row_count: int = 0) ->
     matrices = w3_matrix_list([(layout["planes"], layout["scales"], layout.get("zeros"), out, None) for layout, out in entries])
     layout = entries[0][0]
     device = layout["planes"].device
-    with torch.cuda.device(device):
+    with _on(device):
         check(library().fb_w3_dequant(matrices, len(entries), row_begin, row_count, dtype_tag(layout["scales"].dtype), layout["planes"].shape[0] * 128,
                                       dtype_tag(out_dtype), stream_handle(device)))
 
 
 def gather_columns(x, perm, out) -> None:
     """``out[t, k] = x[t, perm[k]]`` for contiguous 16-bit ``x`` ``[T,K]``."""
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(library().fb_gather_columns(ptr(x), ptr(perm), ptr(out), x.shape[0], x.shape[1], stream_handle(x.device)))
 
 
 def qknorm_rope_prompt(qkv, q_weight, k_weight, cos, sin, q_out, k_cache, v_cache, eps: float) -> None:
     """q/k RMSNorm, rotary embedding and cache rows of a prompt: ``qkv`` ``[T, (q_heads + 2 kv_heads) * 128]``, ``q_out`` ``[q_heads, T, 128]``."""
-    with torch.cuda.device(qkv.device):
+    with _on(qkv.device):
         check(library().fb_qknorm_rope_prompt(ptr(qkv), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(q_out), ptr(k_cache), ptr(v_cache),
                                               qkv.shape[0], q_out.shape[0], k_cache.shape[-3], q_out.shape[-1], k_cache.shape[-2], float(eps),
                                               dtype_tag(qkv.dtype), stream_handle(qkv.device)))
@@ -686,5 +696,5 @@ def qknorm_rope_prompt(qkv, q_weight, k_weight, cos, sin, q_out, k_cache, v_cach
 
 def silu_mul_rows(gate_up, out) -> None:
     """``out[t, i] = silu(gate_up[t, i]) * gate_up[t, width + i]``; ``out`` may be a column slice of a wider buffer."""
-    with torch.cuda.device(out.device):
+    with _on(out.device):
         check(library().fb_silu_mul_rows(ptr(gate_up), ptr(out), out.shape[0], out.shape[1], out.stride(0), dtype_tag(out.dtype), stream_handle(out.device)))

@@ -349,6 +349,16 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
       const GemmMatrix& m = p.mats[j];
       const int row = (row_tile - m.tile_begin) * kRows + row_in_tile, token0 = (tile - row_tile * p.token_tiles) * p.tokens;
       const int tokens = min(p.tokens, p.T - token0);
+      // addends are requested 16 tokens ahead, the first ones while the tile still accumulates
+      unsigned short next[16];
+      auto fetch = [&](int c) {
+        if (!m.addend || row >= m.O) return;
+        const unsigned short* from = m.addend + (size_t)(token0 + c) * p.ldo + row;
+#pragma unroll
+        for (int i = 0; i < 16; ++i, from += p.ldo)
+          if (c + i < tokens) next[i] = *from;
+      };
+      fetch(16 * part);
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(d_full, it & 1))) {
         dead = true;
         break;
@@ -358,18 +368,16 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
         uint32_t v[16];
         __syncwarp();
         tmem_load16(tmem + lanes + c, v);
-        if (row < m.O) {
-          const size_t at = (size_t)(token0 + c) * p.ldo + row;
-          unsigned short* to = m.out + at;
-          const unsigned short* add = m.addend + at;
+        if (m.addend) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i, to += p.ldo, add += p.ldo) {
-            if (c + i < tokens) {
-              float y = __uint_as_float(v[i]);
-              if (m.addend) y += bits_to_float(*add, p.act_dtype);
-              *to = bits16(y, p.act_dtype);
-            }
-          }
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + bits_to_float(next[i], p.act_dtype));
+          fetch(c + 16 * kEpilogue);
+        }
+        if (row < m.O) {
+          unsigned short* to = m.out + (size_t)(token0 + c) * p.ldo + row;
+#pragma unroll
+          for (int i = 0; i < 16; ++i, to += p.ldo)
+            if (c + i < tokens) *to = bits16(__uint_as_float(v[i]), p.act_dtype);
         }
       }
       __syncwarp();
