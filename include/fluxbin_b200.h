@@ -397,7 +397,7 @@ int fb_tp_argmax(void* keys, int world, int64_t* best, const int64_t* forced_nex
  *   the layout's (group-sorted) order: T_out(T_scale(scale * (code - zero))).
  * fb_gather_columns: out[t, k] = x[t, perm[k]], the activations that go with that order.
  * fb_qknorm_rope_prompt: rows of qkv [tokens, q_heads + 2 kv_heads, 128] -> per-head RMSNorm of q and k,
- *   rotary embedding with cos / sin [tokens, 128]; q to q_out [q_heads, tokens, 128], k and v to
+ *   rotary embedding with cos / sin [tokens, 128]; q to q_out [tokens, q_heads, 128], k and v to
  *   positions 0 .. tokens - 1 of the caches [kv_heads, max_positions, 128].
  * fb_identity_order: writes 1 to *flag (pinned host memory that the device can reach) if perm[k] == k for all k, else 0.
  * fb_silu_mul_rows: out[t, i] = T(silu(gate_up[t, i])) * gate_up[t, width + i]; out rows out_stride apart.

@@ -687,10 +687,10 @@ def gather_columns(x, perm, out) -> None:
 
 
 def qknorm_rope_prompt(qkv, q_weight, k_weight, cos, sin, q_out, k_cache, v_cache, eps: float) -> None:
-    """q/k RMSNorm, rotary embedding and cache rows of a prompt: ``qkv`` ``[T, (q_heads + 2 kv_heads) * 128]``, ``q_out`` ``[q_heads, T, 128]``."""
+    """q/k RMSNorm, rotary embedding and cache rows of a prompt: ``qkv`` ``[T, (q_heads + 2 kv_heads) * 128]``, ``q_out`` ``[T, q_heads, 128]``."""
     with _on(qkv.device):
         check(library().fb_qknorm_rope_prompt(ptr(qkv), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(q_out), ptr(k_cache), ptr(v_cache),
-                                              qkv.shape[0], q_out.shape[0], k_cache.shape[-3], q_out.shape[-1], k_cache.shape[-2], float(eps),
+                                              qkv.shape[0], q_out.shape[1], k_cache.shape[-3], q_out.shape[-1], k_cache.shape[-2], float(eps),
                                               dtype_tag(qkv.dtype), stream_handle(qkv.device)))
 
 

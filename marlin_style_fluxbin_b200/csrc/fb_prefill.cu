@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) gather_columns_kernel(const unsigned shor
 }
 
 // A warp per (token, head), head_dim 128: a lane holds dims 2 l, 2 l + 1 and their partners + 64.  q heads
-// go to q_out [q_heads, T, 128], k heads (normed, rotated) and v heads (as they are) to the cache rows.
+// go to q_out [T, q_heads, 128], k heads (normed, rotated) and v heads (as they are) to the cache rows.
 __global__ void __launch_bounds__(256) qknorm_rope_prompt_kernel(const unsigned short* __restrict__ qkv, const unsigned short* __restrict__ q_weight,
                                                                  const unsigned short* __restrict__ k_weight, const unsigned short* __restrict__ cosv,
                                                                  const unsigned short* __restrict__ sinv, unsigned short* __restrict__ q_out,
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_prompt_kernel(const unsigned 
   }
   const bool is_q = head < q_heads;
   const unsigned short* const weight = is_q ? q_weight : k_weight;
-  unsigned short* const dst = is_q ? q_out + ((size_t)head * tokens + t) * D : k_cache + ((size_t)(head - q_heads) * max_positions + t) * D;
+  unsigned short* const dst = is_q ? q_out + ((size_t)t * q_heads + head) * D : k_cache + ((size_t)(head - q_heads) * max_positions + t) * D;
   auto two = [&](uint32_t w, float (&f)[2]) { f[0] = bits_to_float((unsigned short)(w & 0xffffu), dtype), f[1] = bits_to_float((unsigned short)(w >> 16), dtype); };
   auto load2 = [&](const unsigned short* from, float (&f)[2]) { two(*reinterpret_cast<const uint32_t*>(from), f); };
   float lo[2], hi[2], wl[2], wh[2], cl[2], ch[2], sl[2], sh[2];

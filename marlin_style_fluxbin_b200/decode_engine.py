@@ -315,7 +315,7 @@ class DecodeEngine:
             raise ValueError("prompt does not fit the KV cache")
         h = self.embedding[tokens]
         xn = torch.empty_like(h)
-        q_rot = torch.empty(self.q_heads, t, s.head_dim, device=self.device, dtype=self.dtype)
+        q_rot = torch.empty(t, self.q_heads, s.head_dim, device=self.device, dtype=self.dtype)
         alone = self.tp_size == 1
         for index, layer in enumerate(self.layers):
             dense = layer.dense or {}
@@ -323,7 +323,8 @@ class DecodeEngine:
             qkv = self._prompt_linear(xn, (layer.q, layer.k, layer.v), dense.get("qkv"))
             nat.qknorm_rope_prompt(qkv, layer.q_norm, layer.k_norm, self.cos, self.sin, q_rot, self.k_cache[index], self.v_cache[index], s.eps)
             k, v = self.k_cache[index, :, :t], self.v_cache[index, :, :t]
-            attn = F.scaled_dot_product_attention(q_rot.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), is_causal=True, enable_gqa=True)
+            # token-major queries: the output then comes token-major too, and needs no copy for the projection
+            attn = F.scaled_dot_product_attention(q_rot.transpose(0, 1).unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), is_causal=True, enable_gqa=True)
             x = attn[0].transpose(0, 1).reshape(t, -1)
             if alone:
                 h = self._prompt_linear(x, (layer.o,), dense.get("o"), addend=h)
