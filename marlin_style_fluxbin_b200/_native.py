@@ -22,7 +22,10 @@ FB_W3_GROUP_PARTIALS = 4
 FB_W3_SAME_INPUT = 8
 
 _lib = None
-_calls = None
+try:
+    from . import _fb_calls as _calls
+except ImportError:  # not built: calls() says so
+    _calls = None
 
 
 class W3Matrix(ctypes.Structure):
@@ -44,13 +47,8 @@ class NativeError(RuntimeError):
 
 def calls():
     """The extension module behind eager calls on prepared launches (``csrc/python/fb_calls.cpp``)."""
-    global _calls
     if _calls is None:
-        try:
-            from . import _fb_calls
-        except ImportError as exc:
-            raise RuntimeError("_fb_calls.so is not built; run `python -m marlin_style_fluxbin_b200.build`") from exc
-        _calls = _fb_calls
+        raise RuntimeError("_fb_calls.so is not built; run `python -m marlin_style_fluxbin_b200.build`")
     return _calls
 
 
