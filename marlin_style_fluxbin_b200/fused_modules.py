@@ -18,6 +18,7 @@ from contextlib import contextmanager
 import torch
 
 from . import _native
+from .w3_lut_deployment import PackedW3Linear
 
 
 def rms_norm_reference(hidden_states, weight, eps):
@@ -75,7 +76,8 @@ def fused_apply_rotary_pos_emb(q, k, cos, sin, unsqueeze_dim=1):
 # Between the Linears of a step lie some seventeen small launches per layer in the stock modules: norms and rotation,
 # two scatters into the cache and their index arithmetic, the expansion of the k/v heads, SDPA, gate and product.  While a
 # session announces the step it runs (position and cache known on the host), the attention module takes ONE launch
-# for everything between q/k/v and o_proj, and the MLP one between gate/up and down.
+# for everything between q/k/v and o_proj, and the MLP one between gate/up and down.  Bound W3 projections o_proj and
+# down_proj also add the residual in their launch: two of thirteen launches of a layer, 4 % of a step.
 _local = threading.local()
 
 
@@ -116,36 +118,78 @@ def _step_serves(step, attention, call) -> bool:
             and step.scratch.numel() >= _native.attn_scratch_bytes(attention.config.num_attention_heads) and _unobserved(q_norm, k_norm))
 
 
+def _attention_heads(step, attention, call):
+    """What o_proj takes, in one launch behind q/k/v; None where that launch does not serve."""
+    if not _step_serves(step, attention, call):
+        return None
+    hidden, (cos, sin) = call["hidden_states"], call["position_embeddings"]
+    q, k, v = attention.q_proj(hidden), attention.k_proj(hidden), attention.v_proj(hidden)
+    if not _kernel_eligible(hidden, q, k, v):
+        return None
+    layer, out = step.cache.layers[attention.layer_idx], torch.empty_like(q)
+    _native.attn_decode_fused(q, k, v, attention.q_norm.weight, attention.k_norm.weight, cos, sin, layer.keys[0], layer.values[0], out,
+                              step.position, attention.q_norm.variance_epsilon, attention.scaling, step.scratch)
+    return out
+
+
+def _gated(mlp, x):
+    """What down_proj takes, in one launch behind gate/up; None where that launch does not serve."""
+    if mlp.config.hidden_act != "silu" or not _kernel_eligible(x) or not _unobserved(mlp.act_fn):
+        return None
+    gate, up = mlp.gate_proj(x), mlp.up_proj(x)
+    if not _kernel_eligible(x, gate, up):
+        return None
+    out = torch.empty_like(gate)
+    _native.silu_mul(gate, up, out)
+    return out
+
+
 def _fused_attention(original):
     signature = inspect.signature(original)
 
     def forward(self, *args, **kwargs):
         step = getattr(_local, "step", None)
-        if step is not None:
-            call = signature.bind(self, *args, **kwargs).arguments
-            if _step_serves(step, self, call):
-                hidden, (cos, sin) = call["hidden_states"], call["position_embeddings"]
-                q, k, v = self.q_proj(hidden), self.k_proj(hidden), self.v_proj(hidden)
-                if _kernel_eligible(hidden, q, k, v):
-                    layer, out = step.cache.layers[self.layer_idx], torch.empty_like(q)
-                    _native.attn_decode_fused(q, k, v, self.q_norm.weight, self.k_norm.weight, cos, sin, layer.keys[0], layer.values[0], out,
-                                              step.position, self.q_norm.variance_epsilon, self.scaling, step.scratch)
-                    return self.o_proj(out), None
-        return original(self, *args, **kwargs)
+        heads = None if step is None else _attention_heads(step, self, signature.bind(self, *args, **kwargs).arguments)
+        return original(self, *args, **kwargs) if heads is None else (self.o_proj(heads), None)
 
     return forward
 
 
 def _fused_mlp(original):
     def forward(self, x):
-        if getattr(_local, "step", None) is None or self.config.hidden_act != "silu" or not _kernel_eligible(x) or not _unobserved(self.act_fn):
-            return original(self, x)
-        gate, up = self.gate_proj(x), self.up_proj(x)
-        if not _kernel_eligible(x, gate, up):
-            return original(self, x)
-        out = torch.empty_like(gate)
-        _native.silu_mul(gate, up, out)
-        return self.down_proj(out)
+        act = None if getattr(_local, "step", None) is None else _gated(self, x)
+        return original(self, x) if act is None else self.down_proj(act)
+
+    return forward
+
+
+def _joins(projection, wrapped) -> bool:
+    """Whether a projection can take the residual addition that follows it into its launch."""
+    return isinstance(projection, PackedW3Linear) and projection._decode_binding is not None and projection.bias is None and _unobserved(projection, wrapped)
+
+
+def _fused_layer(original):
+    signature = inspect.signature(original)
+
+    def forward(self, *args, **kwargs):
+        step, attention, mlp = getattr(_local, "step", None), self.self_attn, self.mlp
+        if step is None or not _joins(attention.o_proj, attention) or not _joins(mlp.down_proj, mlp):
+            return original(self, *args, **kwargs)
+        call = dict(signature.bind(self, *args, **kwargs).arguments)
+        residual = call["hidden_states"]
+        # both halves have to serve before anything is launched
+        if not _step_serves(step, attention, call) or mlp.config.hidden_act != "silu" or not _kernel_eligible(residual) or not _unobserved(mlp.act_fn):
+            return original(self, *args, **kwargs)
+        call["hidden_states"] = self.input_layernorm(residual)
+        heads = _attention_heads(step, attention, call)
+        if heads is None or not attention.o_proj.adds_residual(heads):
+            return original(self, *args, **kwargs)
+        middle = attention.o_proj.add_to(residual, heads)
+        normed = self.post_attention_layernorm(middle)
+        act = _gated(mlp, normed)
+        if act is None or not mlp.down_proj.adds_residual(act):
+            return middle + mlp(normed)
+        return mlp.down_proj.add_to(middle, act)
 
     return forward
 
@@ -170,7 +214,7 @@ def fused_qwen3_modules(*, rms_norm=True, rope=True):
             saved["rope"] = modeling_qwen3.apply_rotary_pos_emb
             modeling_qwen3.apply_rotary_pos_emb = fused_apply_rotary_pos_emb
         if rms_norm and rope:
-            for name, wrap in (("Qwen3Attention", _fused_attention), ("Qwen3MLP", _fused_mlp)):
+            for name, wrap in (("Qwen3Attention", _fused_attention), ("Qwen3MLP", _fused_mlp), ("Qwen3DecoderLayer", _fused_layer)):
                 owner = getattr(modeling_qwen3, name)
                 saved[name] = owner.forward
                 owner.forward = wrap(owner.forward)
@@ -180,6 +224,6 @@ def fused_qwen3_modules(*, rms_norm=True, rope=True):
             modeling_qwen3.Qwen3RMSNorm.forward = saved["rms_norm"]
         if "rope" in saved:
             modeling_qwen3.apply_rotary_pos_emb = saved["rope"]
-        for name in ("Qwen3Attention", "Qwen3MLP"):
+        for name in ("Qwen3Attention", "Qwen3MLP", "Qwen3DecoderLayer"):
             if name in saved:
                 getattr(modeling_qwen3, name).forward = saved[name]

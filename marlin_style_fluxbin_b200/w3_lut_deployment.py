@@ -489,6 +489,22 @@ class PackedW3Linear(nn.Module):
         # a weak reference to the module, so no cycle: a dropped module gives its weights back at once
         self._decode_binding = _native.calls().Bound(launch.call, launch, output, shaped, weakref.ref(self), self._buffers)
 
+    def adds_residual(self, x: torch.Tensor) -> bool:
+        """Whether ``add_to`` can stand for a call of this bound module and an addition."""
+        return (self._decode_binding is not None and self.bias is None and self._decode_output.dtype == x.dtype and x.is_cuda and x.is_contiguous()
+                and x.numel() == self.in_features and x.get_device() == self._decode_output.get_device())
+
+    def add_to(self, residual: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
+        """``residual + self(x)`` for one token in one launch, the sum rounded once."""
+        if self._decode_audit:
+            self.route_counts["packed_m1"] += 1
+            self.last_route = "packed_m1"
+        planes, scales, zeros, perm = _layout_args(self.layout(), wait=False)
+        out = torch.empty_like(residual)
+        _native.w3_gemv_multi(x.view(1, self.in_features), _native.w3_matrix_list([(planes, scales, zeros, out, residual)]), 1, self.out_features, scales.dtype,
+                              perm, decoded_bf16=self.arithmetic == "decoded_bf16")
+        return out
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self._decode_binding is not None:
             return self._decode_binding(x)
