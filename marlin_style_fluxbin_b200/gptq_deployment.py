@@ -332,7 +332,8 @@ def restore_planar_w3(layout: Mapping[str, torch.Tensor], *, dtype: torch.dtype 
     rounding, as a GPTQ module loaded in that dtype computes it) and then cast to ``dtype``.
     """
     out_features, in_features = validate_planar_w3(layout)
-    if layout["planes"].is_cuda and dtype in (torch.float16, torch.bfloat16):
+    # the kernel's bounds: 65536 rows, planes on a 16-byte boundary
+    if layout["planes"].is_cuda and dtype in (torch.float16, torch.bfloat16) and out_features <= 65536 and layout["planes"].data_ptr() % 16 == 0:
         from . import _native
 
         ordered = torch.empty(out_features, in_features, device=layout["planes"].device, dtype=dtype)
