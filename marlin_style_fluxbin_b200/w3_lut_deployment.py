@@ -11,6 +11,7 @@ own tiling, reduces its K split internally and leaves a caller's workspace untou
 """
 from __future__ import annotations
 
+import threading
 import weakref
 from types import SimpleNamespace
 
@@ -129,36 +130,54 @@ def load_w3_lut_extension(row_tile: int, uniform_index_probe: bool = False):
 # Whether a perm tensor is the identity (the kernels then skip the gather).  A kernel compares it on the stream and
 # writes the answer to a word of pinned host memory, so that asking costs no wait: -1 until it has run.  Keyed by address,
 # and an entry holds only while the tensor it was made for lives unchanged (another one may get the address later).
+# Every question has a word of its own: an older one, about a tensor that was there before or about values since
+# overwritten, may still be queued on some stream of some device, and its answer must not pass for the newer one's.
 _IDENTITY_PERMS: dict[tuple[int, int], tuple] = {}
 _MAX_PERMS = 4096
-_perm_flags = None
+_perm_lock = threading.Lock()
+_perm_blocks: list = []  # blocks of words: the last gives them out, those before it are full and still wait for answers
+_perm_given = 0          # words of the last block
 
 
 def _perm_entry(perm: torch.Tensor):
-    """``(owner, version, slot)`` of a perm that was asked about, or None."""
+    """``(owner, version, words, index)`` of a perm that was asked about, or None."""
     entry = _IDENTITY_PERMS.get((perm.data_ptr(), perm.numel()))
     if entry is None or entry[0]() is not (perm if perm._base is None else perm._base) or entry[1] != (None if perm.is_inference() else perm._version):
         return None
     return entry
 
 
+def _answer_word():
+    """A word that no question has had, under the lock: ``(words, index)``."""
+    global _perm_given
+    if not _perm_blocks or _perm_given == _MAX_PERMS:
+        # a full block whose answers are all there can go; entries keep the one they read
+        _perm_blocks[:] = [words for words in _perm_blocks if int(words.min()) < 0]
+        _perm_blocks.append(torch.full((_MAX_PERMS,), -1, dtype=torch.int32, pin_memory=torch.cuda.is_available()).numpy())
+        _perm_given = 0
+        for key in [key for key, entry in _IDENTITY_PERMS.items() if entry[0]() is None]:
+            del _IDENTITY_PERMS[key]
+        if len(_IDENTITY_PERMS) >= _MAX_PERMS:
+            _IDENTITY_PERMS.clear()
+    _perm_given += 1
+    return _perm_blocks[-1], _perm_given - 1
+
+
 def _ask_perm(perm: torch.Tensor):
-    global _perm_flags
-    if _perm_flags is None:
-        pinned = torch.empty(_MAX_PERMS, dtype=torch.int32, pin_memory=True)
-        _perm_flags = (pinned, pinned.numpy())
-    if len(_IDENTITY_PERMS) >= _MAX_PERMS:
-        torch.cuda.synchronize(perm.device)  # no answer to a forgotten question may land in a slot that is used again
-        _IDENTITY_PERMS.clear()
-    slot = len(_IDENTITY_PERMS)
-    key = (perm.data_ptr(), perm.numel())
-    if key in _IDENTITY_PERMS:
-        slot = _IDENTITY_PERMS[key][2]
-    _perm_flags[1][slot] = -1
-    with torch.cuda.device(perm.device):
-        _native.check(_native.library().fb_identity_order(perm.data_ptr(), perm.numel(), _perm_flags[0].data_ptr() + 4 * slot, _native.stream_handle(perm.device)))
-    entry = _IDENTITY_PERMS[key] = (weakref.ref(perm if perm._base is None else perm._base), None if perm.is_inference() else perm._version, slot)
-    return entry
+    with _perm_lock:
+        entry = _perm_entry(perm)  # another thread may have asked meanwhile
+        if entry is not None:
+            return entry
+        words, index = _answer_word()
+        try:
+            with torch.cuda.device(perm.device):
+                _native.check(_native.library().fb_identity_order(perm.data_ptr(), perm.numel(), words.ctypes.data + 4 * index, _native.stream_handle(perm.device)))
+        except BaseException:
+            words[index] = 0  # nothing will answer
+            raise
+        entry = (weakref.ref(perm if perm._base is None else perm._base), None if perm.is_inference() else perm._version, words, index)
+        _IDENTITY_PERMS[(perm.data_ptr(), perm.numel())] = entry
+        return entry
 
 
 def _perm_or_none(perm: torch.Tensor, wait: bool = True):
@@ -169,10 +188,11 @@ def _perm_or_none(perm: torch.Tensor, wait: bool = True):
         if torch.cuda.is_current_stream_capturing():
             return perm
         entry = _ask_perm(perm)
-    known = int(_perm_flags[1][entry[2]])
+    words, index = entry[2:]
+    known = int(words[index])
     if known < 0 and wait and not torch.cuda.is_current_stream_capturing():
         torch.cuda.current_stream(perm.device).synchronize()
-        known = int(_perm_flags[1][entry[2]])
+        known = int(words[index])
     return None if known == 1 else perm
 
 
