@@ -139,6 +139,9 @@ class DecodeEngine:
         s, p = shape, tp_size
         self.q_heads, self.kv_heads = s.q_heads // p, s.kv_heads // p
         self.inter = s.intermediate // p
+        # what the kernels of the prompt path take; every other prompt runs as plain tensor operations
+        self._prompt_kernels = (self.device.type == "cuda" and dtype in (torch.float16, torch.bfloat16) and s.head_dim == 128
+                                and max(self.q_heads * s.head_dim, self.inter, s.hidden) <= 65536)
         gen = torch.Generator(device=self.device).manual_seed(seed)  # same stream of draws on every rank
         normal = lambda *size: (torch.randn(*size, device=self.device, generator=gen) * 0.02).to(dtype)  # noqa: E731
         self.embedding = normal(s.vocab, s.hidden)
@@ -197,6 +200,8 @@ class DecodeEngine:
 
     def _dense_rows(self, layouts, begin=0, count=0, into=None):
         """Rows ``begin .. begin + count`` (0: all) of each layout, dequantised, one below the other."""
+        if not self._prompt_kernels:
+            return torch.cat([restore_planar_w3(lay, dtype=self.dtype) for lay in layouts], 0)
         heights = [count or lay["planes"].shape[2] - begin for lay in layouts]
         dense = torch.empty(sum(heights), layouts[0]["planes"].shape[0] * 128, device=self.device, dtype=self.dtype) if into is None else into
         entries, at = [], 0
@@ -303,17 +308,43 @@ class DecodeEngine:
             _native.silu_mul_rows(torch.mm(x, part.t()), act[:, begin:begin + count])
         return act
 
+    def _tensor_prefill(self, h):
+        """``prefill`` as plain tensor operations on dequantised weights: any device, dtype and head width."""
+        s, t = self.shape, h.shape[0]
+        cos, sin = self.cos[:t].unsqueeze(0), self.sin[:t].unsqueeze(0)
+        rotate = lambda x: torch.cat((-x[..., s.head_dim // 2:], x[..., :s.head_dim // 2]), dim=-1)  # noqa: E731
+        norm = lambda x, w: (w * (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + s.eps)).to(self.dtype))  # noqa: E731
+        for index, layer in enumerate(self.layers):
+            dense = layer.dense if layer.dense is not None else self._dense(layer)
+            q, k, v = F.linear(norm(h, layer.ln1), dense["qkv"]).split((self.q_heads * s.head_dim, self.kv_heads * s.head_dim, self.kv_heads * s.head_dim), dim=-1)
+            q = norm(q.reshape(t, self.q_heads, s.head_dim), layer.q_norm).transpose(0, 1)
+            k = norm(k.reshape(t, self.kv_heads, s.head_dim), layer.k_norm).transpose(0, 1)
+            q, k = (x * cos + rotate(x) * sin for x in (q, k))
+            v = v.reshape(t, self.kv_heads, s.head_dim).transpose(0, 1)
+            self.k_cache[index, :, :t], self.v_cache[index, :, :t] = k, v
+            attn = F.scaled_dot_product_attention(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), is_causal=True, enable_gqa=True)
+            y = F.linear(attn[0].transpose(0, 1).reshape(t, -1), dense["o"])
+            self._allreduce(y)
+            h = h + y
+            gate, up = F.linear(norm(h, layer.ln2), dense["gate_up"]).split(self.inter, dim=-1)
+            y = F.linear(F.silu(gate) * up, dense["down"])
+            self._allreduce(y)
+            h = h + y
+        return F.linear(norm(h[-1:], self.final_norm), self.lm_head)
+
     @torch.inference_mode()
     def prefill(self, input_ids: torch.Tensor) -> torch.Tensor:
-        """Run the prompt through dense (dequantised) weights, fill the KV cache for positions ``0..T-1`` and
-        return the logits of the last position.  GEMMs and attention are library calls; dequantisation and
-        the element-wise steps between them are one launch each."""
+        """Run the prompt, fill the KV cache for positions ``0..T-1`` and return the logits of the last position.
+        The dense arm multiplies by its 16-bit weights, the packed arm takes one of the three routes of ``_prompt_linear``; the
+        element-wise steps are one launch each, attention and LM head library calls."""
         s, nat = self.shape, _native
         tokens = input_ids.reshape(-1).to(self.device)
         t = tokens.numel()
         if not 1 <= t < self.max_positions:
             raise ValueError("prompt does not fit the KV cache")
         h = self.embedding[tokens]
+        if not self._prompt_kernels:
+            return self._tensor_prefill(h)
         xn = torch.empty_like(h)
         q_rot = torch.empty(t, self.q_heads, s.head_dim, device=self.device, dtype=self.dtype)
         alone = self.tp_size == 1
