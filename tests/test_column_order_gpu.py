@@ -23,6 +23,7 @@ def test_a_late_answer_is_not_taken_for_the_next_question(replaced):
     x = torch.randn(1, k, device="cuda", generator=gen).bfloat16()
     want, first, second, third = (torch.empty(1, o, device="cuda", dtype=torch.bfloat16) for _ in range(4))
     _native.w3_gemv(x, layout["planes"], layout["scales"], None, shuffled, want)
+    w3._perm_or_none(shuffled)  # the first question allocates
     torch.cuda.synchronize()
     torch.cuda._sleep(100_000_000)  # some 50 ms
     w3._perm_or_none(layout["perm"], wait=False)
