@@ -264,10 +264,17 @@ def _layout_record(layout) -> _LayoutRecord:
 
 
 def _launch_layout(record, layout, x, out, kind, decoded) -> None:
+    if x.get_device() != record.index:
+        raise ValueError("x, out and the layout must share a device")
+    if not (x.is_contiguous() and out.is_contiguous()):  # the kernels know rows that lie side by side only
+        packed = torch.empty(out.shape, device=out.device, dtype=out.dtype)
+        _launch_layout(record, layout, x.contiguous(), packed, kind, decoded)
+        out.copy_(packed)
+        return
     key = (kind, x.shape[0], x.dtype, decoded)
     launch = record.launches.get(key, 0)
-    if not launch or not (x.get_device() == record.index and x.is_contiguous() and out.is_contiguous()):
-        # a first call, odd operands, or a column order that cannot be looked at now: the plain entry points.  The second
+    if not launch:
+        # a first call, or a column order that cannot be looked at now: the plain entry points.  The second
         # call prepares the launch (about 40 us), which pays from a few calls on.
         prepare = launch is None and not torch.cuda.is_current_stream_capturing()
         if launch == 0:
