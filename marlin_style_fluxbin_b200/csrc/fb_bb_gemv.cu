@@ -454,7 +454,8 @@ struct BBPrepared : Prepared {
 
 int run_prepared(const Prepared* base, const void* x, void* out, void* scratch, size_t scratch_bytes, unsigned flags, cudaStream_t stream) {
   BBParams p = static_cast<const BBPrepared*>(base)->p;
-  if (overlaps(out, (size_t)p.O * 2, x, (size_t)p.K * 2)) return fail(FB_EALIAS, "fb_bb_gemv: out overlaps an input");
+  if (overlaps(out, (size_t)p.O * 2, x, (size_t)p.K * 2) || overlaps(out, (size_t)p.O * 2, p.codes, (size_t)p.G * p.O * 32))
+    return fail(FB_EALIAS, "fb_bb_gemv: out overlaps an input");
   if (!aligned(x, 16)) return fail(FB_EINVAL, "fb_bb_gemv: x must be 16-byte aligned");
   if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_gemv: unknown flag bits 0x%x", flags);
   p.x = x;

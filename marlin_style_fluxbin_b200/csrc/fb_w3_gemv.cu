@@ -1035,6 +1035,8 @@ int run_prepared(const Prepared* base, const void* x, void* out, void* scratch, 
   if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemv: scratch must be 256-byte aligned");
   if (overlaps(out, out_bytes, x, x_bytes) || overlaps(scratch, self.need, x, x_bytes) || overlaps(scratch, self.need, out, out_bytes))
     return fail(FB_EALIAS, "fb_w3_gemv: out overlaps an input, or scratch overlaps x or out");
+  if (overlaps(out, out_bytes, self.p.mats[0].planes, (size_t)self.p.G * 3 * self.p.O * 16) || overlaps(out, out_bytes, self.p.mats[0].scales, (size_t)self.p.G * self.p.O * 2))
+    return fail(FB_EALIAS, "fb_w3_gemv: out overlaps an input");
   if (flags & ~(FB_W3_NO_PDL | FB_W3_SAME_INPUT)) return fail(FB_EINVAL, "fb_w3_gemv: unknown flag bits 0x%x", flags);
   W3Params p = self.p;
   p.x = x;

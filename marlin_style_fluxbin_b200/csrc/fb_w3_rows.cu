@@ -577,6 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
 
 struct RowsPrepared : Prepared {
   RowsParams p;
+  const uint8_t* planes;
   int rows, splits, slices;  // rows of the call; a launch takes 16, or 8
 };
 
@@ -686,6 +687,7 @@ int fill(RowsPrepared& made, int act_dtype, int m, const uint8_t* planes, const 
   p.scale_map = p.zero_map = p.plane_map;
   if (!p.direct && !group_row_tensor_map(scales, 2, O, G, kUnitRows, &p.scale_map)) return FB_ECUDA;
   if (!p.direct && zeros && !group_row_tensor_map(zeros, 1, O, G, kUnitRows, &p.zero_map)) return FB_ECUDA;
+  made.planes = planes;
   made.rows = m;
   return FB_OK;
 }
@@ -701,6 +703,8 @@ int run_add(const Prepared* base, const void* x, void* out, const void* addend, 
   if (!aligned(scratch, 256)) return fail(FB_EINVAL, "fb_w3_gemm_small: scratch must be 256-byte aligned");
   if (overlaps(out, out_bytes, x, x_bytes) || overlaps(scratch, kScratchBytes, out, out_bytes) || overlaps(scratch, kScratchBytes, x, x_bytes))
     return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input, or scratch overlaps x or out");
+  if (overlaps(out, out_bytes, self.planes, (size_t)p.G * 3 * p.O * 16) || overlaps(out, out_bytes, p.scales, (size_t)p.G * p.O * 2))
+    return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input");
   p.status = reinterpret_cast<unsigned*>(scratch);
   p.out_aligned = aligned(out, 8) ? 1 : 0;
   const bool pdl = (flags & FB_W3_NO_PDL) == 0;
@@ -777,8 +781,6 @@ extern "C" int fb_w3_gemm_small_add(const void* x, int act_dtype, int m, const u
   if (rc != FB_OK) return rc;
   const size_t out_bytes = (size_t)m * out_features * 2;
   if (addend && overlaps(out, out_bytes, addend, out_bytes)) return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps the addend");
-  if (overlaps(out, out_bytes, planes, (size_t)in_features / 128 * 3 * out_features * 16) || overlaps(out, out_bytes, scales, (size_t)in_features / 128 * out_features * 2))
-    return fail(FB_EALIAS, "fb_w3_gemm_small: out overlaps an input");
   RowsPrepared made;
   rc = fill(made, act_dtype, m, planes, scales, scale_dtype, zeros, perm, out_features, in_features);
   return rc != FB_OK ? rc : run_add(&made, x, out, addend, scratch, scratch_bytes, 0u, static_cast<cudaStream_t>(stream));

@@ -49,3 +49,33 @@ def test_repeated_calls_on_a_layout(rows, kernel, arithmetic, perm):
     del layout
     gc.collect()
     assert key not in w3._RECORDS  # nothing outlives the planes
+
+
+@pytest.mark.parametrize("rows,kernel", ((1, "lut"), (2, "mma")))
+@pytest.mark.parametrize("name", ("planes", "scales"))
+def test_an_output_inside_the_weights_is_refused_every_time(rows, kernel, name):
+    from marlin_style_fluxbin_b200 import _native, w3_lut_deployment as w3
+
+    layout = _layout(96, 640, 3, False)
+    before = {key: value.clone() for key, value in layout.items()}
+    x = torch.zeros(rows, 640, device="cuda", dtype=torch.bfloat16)
+    out = layout[name].view(torch.bfloat16).view(-1)[:rows * 96].view(rows, 96)
+    for _ in range(4):
+        with pytest.raises(_native.NativeError, match="overlaps"):
+            w3.w3_lut_gemv_out(x, layout, out, kernel=kernel)
+    assert all(torch.equal(layout[key], before[key]) for key in layout)
+
+
+def test_an_output_inside_two_base_codes_is_refused():
+    from marlin_style_fluxbin_b200 import _native
+    from marlin_style_fluxbin_b200.deployment import PackedHybridLinear
+    from test_deployment import make_payload
+
+    module = PackedHybridLinear(make_payload(64, 2)).cuda()
+    lay = module.layout()
+    launch = _native.Launch("bb", torch.bfloat16, tuple(lay[n] for n in ("codes", "rows", "columns", "sparse_codes", "sparse_rows", "sparse_columns", "indices")),
+                            64, 256)
+    before = module.codes.clone()
+    with pytest.raises(_native.NativeError, match="overlaps"):
+        launch(torch.zeros(1, 256, device="cuda", dtype=torch.bfloat16), module.codes.view(torch.bfloat16).view(-1)[:64].view(1, 64))
+    assert torch.equal(module.codes, before)
