@@ -248,8 +248,8 @@ int fb_w3_finish(const float* partials, int splits, int out_features, void* out,
  * s_b the same over the group's 8 refined columns; fp32 within a group; the groups (at most 255)
  * are combined by 64-bit fixed-point integer adds (steps of 2^-26, order-independent, so
  * repeat-exact; a group's term that is not finite or is 8192 or more in magnitude gives NaN).
- * Any O in 1..65536; scratch zero-filled once and 256-byte aligned, not shared with other
- * kernels, sized by fb_bb_gemv_scratch_bytes(O, K, 0).
+ * Any O in 1..65536; x and codes 16-byte aligned; scratch zero-filled once and 256-byte aligned, not
+ * shared with other kernels, sized by fb_bb_gemv_scratch_bytes(O, K, 0).
  * Replaces the reference's m1_out of the v5 kernels (csrc/m1_v5.cu:132-195); all the
  * reference's kernel names map to this one entry point.
  */
@@ -262,7 +262,8 @@ int fb_bb_gemv(const void* x, int act_dtype, const uint8_t* codes, int planar, c
 /*
  * Two-base GEMV with matrix-wide scales:  W = sum_b diag(r_b) B_b diag(c_b) + dense residual
  * columns.  codes uint8 [G,O,2,16] planar sign bits; row_scales f16 [2,O]; col_scales f16 [2,K];
- * salient_idx int32 [n] input columns; salient bf16 [O,n] added weights on those columns.
+ * salient_idx int32 [n] input columns; salient bf16 [O,n] added weights on those columns.  x, codes and
+ * col_scales 16-byte aligned.
  * Scratch sized by fb_bb_gemv_scratch_bytes(O, K, 1).  The two-base part follows the
  * reference's global materialiser (evaluation.py:59-95) with one scale per row and per column.
  */

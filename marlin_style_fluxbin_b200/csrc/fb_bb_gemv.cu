@@ -468,7 +468,7 @@ int check_common(const char* who, const void* x, int act_dtype, const uint8_t* c
   if (act_dtype != FB_F16 && act_dtype != FB_BF16) return fail(FB_EINVAL, "%s: activation dtype must be FB_F16 or FB_BF16", who);
   if (K < 128 || K % 128 || K / 128 > 255) return fail(FB_ELIMIT, "%s: K=%d must be a multiple of 128 with at most 255 groups", who, K);
   if (O < 1 || O > 65536) return fail(FB_ELIMIT, "%s: O=%d outside 1..65536", who, O);
-  if (!aligned(codes, 16)) return fail(FB_EINVAL, "%s: codes must be 16-byte aligned", who);
+  if (!aligned(codes, 16) || !aligned(x, 16)) return fail(FB_EINVAL, "%s: x and codes must be 16-byte aligned", who);
   if (overlaps(out, (size_t)O * 2, x, (size_t)K * 2) || overlaps(out, (size_t)O * 2, codes, (size_t)(K / 128) * O * 32))
     return fail(FB_EALIAS, "%s: out overlaps an input", who);
   return FB_OK;
@@ -536,6 +536,7 @@ extern "C" int fb_bb_global_gemv(const void* x, int act_dtype, const uint8_t* co
   int rc = check_common("fb_bb_global_gemv", x, act_dtype, codes, out, out_features, in_features);
   if (rc) return rc;
   if (!row_scales || !col_scales) return fail(FB_EINVAL, "fb_bb_global_gemv: scales must be non-null");
+  if (!aligned(col_scales, 16)) return fail(FB_EINVAL, "fb_bb_global_gemv: column scales must be 16-byte aligned");
   if (n_salient < 0 || n_salient > 256 || (n_salient > 0 && (!salient_idx || !salient)))
     return fail(FB_EINVAL, "fb_bb_global_gemv: salient columns: 0..256 with index and value tensors");
   if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_global_gemv: unknown flag bits 0x%x", flags);
