@@ -241,7 +241,9 @@ extern "C" int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, cons
   if (bad_dtype(dtype)) return fail(FB_EINVAL, "fb_qknorm_rope_prompt: dtype must be FB_F16 or FB_BF16");
   if (head_dim != 128) return fail(FB_ELIMIT, "fb_qknorm_rope_prompt: head_dim must be 128");
   if (q_heads < 1 || kv_heads < 1 || tokens < 1 || tokens > max_positions) return fail(FB_ELIMIT, "fb_qknorm_rope_prompt: %d tokens, cache of %d positions", tokens, max_positions);
-  if (!aligned(qkv, 4) || !aligned(q_out, 4) || !aligned(k_cache, 4) || !aligned(v_cache, 4)) return fail(FB_EINVAL, "fb_qknorm_rope_prompt: tensors must be 4-byte aligned");
+  if (!aligned(qkv, 4) || !aligned(q_weight, 4) || !aligned(k_weight, 4) || !aligned(cosv, 4) || !aligned(sinv, 4) || !aligned(q_out, 4) || !aligned(k_cache, 4) ||
+      !aligned(v_cache, 4))
+    return fail(FB_EINVAL, "fb_qknorm_rope_prompt: tensors must be 4-byte aligned");
   const long long warps = (long long)tokens * (q_heads + 2 * kv_heads);
   if (warps > 0x7fffffff) return fail(FB_ELIMIT, "fb_qknorm_rope_prompt: too many tokens");
   qknorm_rope_prompt_kernel<<<(int)((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(u16(qkv), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), u16(q_out), u16(k_cache),

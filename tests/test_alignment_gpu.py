@@ -30,3 +30,16 @@ def test_two_base_activations_and_column_scales():
     _native.bb_gemv(x, module.layout(), _off(out))  # an output may lie anywhere
     _native.bb_global_gemv(x, codes, rows, columns, None, None, out)
     torch.cuda.synchronize()
+
+
+def test_prompt_norm_and_rotation():
+    from marlin_style_fluxbin_b200 import _native
+
+    new = lambda *size: torch.ones(*size, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    plain = {"qkv": new(3, 4 * 128), "q_weight": new(128), "k_weight": new(128), "cos": new(3, 128), "sin": new(3, 128), "q_out": new(3, 2, 128),
+             "k_cache": new(1, 8, 128), "v_cache": new(1, 8, 128)}
+    for name in plain:
+        with pytest.raises(_native.NativeError, match="aligned"):
+            _native.qknorm_rope_prompt(**{**plain, name: _off(plain[name])}, eps=1e-6)
+    _native.qknorm_rope_prompt(**plain, eps=1e-6)
+    torch.cuda.synchronize()
