@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
     for (int d = 4; d >= 1; d >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, d)), all_sum += __shfl_xor_sync(0xffffffffu, all_sum, d);
     const float rest = all_sum - all_top;
     const bool wild = !(all_sum < 1.1529215e18f);  // 2^60 and beyond, infinities, NaN
-    const bool ours = wild || (rest > 0.f && rest < all_top * 4.8828125e-4f);
+    // a rest of zero may be one that the sum's rounding swallowed
+    const bool ours = wild || rest < all_top * 4.8828125e-4f;
     bool lost = false;
     if (live && (lane & 7) == 0) outliers[g * M + m].k = -1;
     if (__any_sync(0xffffffffu, ours)) {  // rare

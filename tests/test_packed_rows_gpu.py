@@ -67,3 +67,27 @@ def test_packed_rows(o, k, m, dtype, options):
         alone = torch.empty(1, o, device="cuda", dtype=dtype)
         _native.w3_gemm_small(x[row:row + 1].contiguous(), planes, scales, zeros, perm, alone, addend=None if addend is None else addend[row:row + 1].contiguous())
         assert torch.equal(alone[0].nan_to_num(), out[row].nan_to_num())
+
+
+@pytest.mark.parametrize("top", (3e4, 3e9, 1e17, 1e30))
+@pytest.mark.parametrize("m", (1, 4, 16))
+def test_one_activation_above_all_others_of_its_group(m, top):
+    """An output whose code is zero there sees the others alone, with the error that THEY give rise to: fp32 sums of three groups
+    (the bound of the test above over the products that occur), one rounding, and nothing from the large one."""
+    from marlin_style_fluxbin_b200 import _native
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    o, k = 64, 384
+    planes = torch.randint(0, 256, (3, 3, o, 16), device="cuda", generator=gen, dtype=torch.uint8)
+    planes[0, :, :16, 77 // 8] &= 0xFF ^ 1 << 77 % 8  # code 4, the zero point, for sixteen outputs
+    planes[1, :, :16, 72 // 8] &= 0xFF ^ 1 << 72 % 8
+    scales = (torch.rand(3, o, device="cuda", generator=gen) * 0.015 + 0.005).half()
+    x = torch.randn(m, k, device="cuda", generator=gen).bfloat16()
+    x[:, 77], x[:, 128:256] = top, 0.0
+    x[:, 200] = -top  # alone in its group
+    out = torch.full((m, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    _native.w3_gemm_small(x, planes, scales, None, None, out)
+    weight = _weight(planes, scales, None)
+    want, size = x.double() @ weight.t(), x.double().abs() @ weight.abs().t()
+    assert bool((size[:, :16] < 1e3).all())
+    assert bool(((out.double() - want).abs() <= (11 + 3 + 32) * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 2.0 ** -24).all())
