@@ -205,10 +205,11 @@ int fb_tp_reduce(void* parts, int world, const void* residual, void* out, int n,
 /*
  * Small-batch form on the tensor cores: y[M,O] = x[M,K] . W^T for M = 1..16, same layout and
  * dtypes as fb_w3_gemv.  The three planes of a group become register operands of the matrix
- * instructions; sums are exact up to fp32 rounding, scales are applied in fp32 (weights are not
- * rounded), and the time hardly grows with M.  A row's result does not depend on its neighbours
- * and is the same on every call.  Own scratch (zero-filled once, 256-byte aligned),
- * not to be shared with the other kernels.  The reference has no packed path for M > 1
+ * instructions; a group's sum carries the fp32 rounding of its largest possible products (7 * scale * |x|),
+ * scales are applied in fp32 (weights are not rounded), and the time hardly grows with M.  A row's result
+ * does not depend on its neighbours and is the same on every call.  An infinite or NaN activation reaches the
+ * outputs whose code is not the zero point; two of them in one group of a row make all of that row's outputs
+ * NaN.  Own scratch (zero-filled once, 256-byte aligned), not to be shared with the other kernels.  The reference has no packed path for M > 1
  * (csrc/w3_lut.cu:195); its dense fallback (w3_lut_deployment.py:343-359) is the oracle.
  */
 size_t fb_w3_gemm_small_scratch_bytes(int m, int out_features, int in_features);

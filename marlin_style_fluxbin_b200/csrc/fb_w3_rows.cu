@@ -19,7 +19,8 @@
 //    [2^14, 2^15), every bit of a bf16 down to 2^-21 of it survives (fp16: 2^-18), what is smaller is
 //    rounded to 2^-39 of it, below the fp32 rounding of the sums.  An activation that dwarfs the rest of its
 //    group (above 2^11 times their sum) or is not finite stays out of the MMA and is added in fp32 where
-//    its signed code is not zero (one per group and row; a second non-finite one makes the group's sums NaN).
+//    its signed code is not zero (one per group and row; a second one that is not finite makes the group's sums
+//    NaN).  Finite activations of any size stay finite as long as the products with the weights do.
 //  * Scales are applied per group in fp32: weights are never rounded.
 //  * A cluster owns a slice of the output rows, its CTAs split K between them (four pairs of groups each
 //    where there are enough: the activations of a CTA are converted once and stay in shared memory).  The
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
   // sums of the cluster's CTAs | barriers ----
   const int quarter = 8 * M;  // sums of eight rows: [activation row][8]
   unsigned char* const operands = smem + kWarps * kStages * kSlotBytes;
-  float* const stat = reinterpret_cast<float*>(operands + 2 * p.npairs * M * kOperandBytes);  // [group][row], rows padded to 8 NT
+  float* const stat = reinterpret_cast<float*>(operands + 2 * p.npairs * M * kOperandBytes);  // [group][row]: 2^(ex - 5); rows padded to 8 NT
   Outlier* const outliers = reinterpret_cast<Outlier*>(stat + 2 * p.npairs * 8 * NT);
   float* const part = reinterpret_cast<float*>(outliers + 2 * p.npairs * M);  // slot (unit + warp): four quarters
   float* const inbox = part + (p.batch + kWarps - 1) * 4 * quarter;          // [quarter of this CTA][sender][quarter]
@@ -313,16 +314,16 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
     locate(i, g, m);
     const bool live = i < items_x;
     // statistics over the eight threads of a (group, row)
-    float top = 0.f, sum = 0.f;
+    float top = 0.f, sum = 0.f;  // the sum in units of 2^8: 128 finite values do not overflow it
 #pragma unroll
-    for (int j = 0; j < 16; ++j) top = fmaxf(top, fabsf(v[j])), sum += fabsf(v[j]);
+    for (int j = 0; j < 16; ++j) top = fmaxf(top, fabsf(v[j])), sum = fmaf(fabsf(v[j]), 0.00390625f, sum);
     float all_top = top, all_sum = sum;
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, d)), all_sum += __shfl_xor_sync(0xffffffffu, all_sum, d);
-    const float rest = all_sum - all_top;
-    const bool wild = !(all_sum < 1.1529215e18f);  // 2^60 and beyond, infinities, NaN
-    // a rest of zero may be one that the sum's rounding swallowed
-    const bool ours = wild || rest < all_top * 4.8828125e-4f;
+    const float rest = all_sum - all_top * 0.00390625f;
+    const bool wild = !(all_sum <= 3.4028235e38f);  // infinities, NaN
+    // 2^-11 of the largest; a rest of zero may be one that the sum's rounding swallowed
+    const bool ours = wild || rest < all_top * 1.9073486e-6f;
     bool lost = false;
     if (live && (lane & 7) == 0) outliers[g * M + m].k = -1;
     if (__any_sync(0xffffffffu, ours)) {  // rare
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
       top = 0.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const bool out = ours && (wild ? !(fabsf(v[j]) < 1.1529215e18f) : fabsf(v[j]) == all_top);
+        const bool out = ours && (wild ? !(fabsf(v[j]) <= 3.4028235e38f) : fabsf(v[j]) == all_top);
         if (out) {
           ++large;
           if (live) outliers[g * M + m].k = k_in_group + (j & 7) + (j >> 3) * 16, outliers[g * M + m].x = v[j], any_out = 1;
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
       for (int d = 4; d >= 1; d >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, d)), large += __shfl_xor_sync(0xffffffffu, large, d);
       lost = large > 1;
     }
-    const int ex = max(-112, min(112, (int)(__float_as_uint(all_top) >> 23) - 127));
+    const int ex = max(-112, (int)(__float_as_uint(all_top) >> 23) - 127);
     if (live) {
       const float one = __uint_as_float((uint32_t)(141 - ex) << 23);  // 2^(14 - ex)
       uint32_t word[8];
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (uint32_t)(j * M * 64)), "r"(word[4 * j]), "r"(word[4 * j + 1]), "r"(word[4 * j + 2]),
                      "r"(word[4 * j + 3])
                      : "memory");
-      if ((lane & 7) == 0) stat[g * 8 * NT + m] = lost ? __int_as_float(0x7fc00000) : __uint_as_float((uint32_t)(127 + ex) << 23);
+      if ((lane & 7) == 0) stat[g * 8 * NT + m] = lost ? __int_as_float(0x7fc00000) : __uint_as_float((uint32_t)(122 + ex) << 23);
     }
   }
   const bool has_outliers = __syncthreads_or(any_out) != 0;
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
   uint32_t sa = ring_u32, bar = bars_u32, phase = 0;  // the slot at hand
   bool dead = false;
   float acc[kTiles][NT][4];
-  // fp32 terms of the activations kept out of the MMA (rare): those of group g of the task at `sa`, in units of 2^-5
+  // fp32 terms of the activations kept out of the MMA (rare): those of group g of the task at `sa`
   auto add_outliers = [&](int pair, int g) {
     for (int m = 0; m < M; ++m) {
       const Outlier o = outliers[(2 * pair + g) * M + m];
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
           const int bit = o.k & 31, zero = (int)lds8(sa + (uint32_t)(kSlotZeros + g * kUnitRows) + row);
           const int code = (int)((lds32(at) >> bit) & 1u) + 2 * (int)((lds32(at + kTiles * kRun) >> bit) & 1u) + 4 - 4 * (int)((lds32(at + 2 * kTiles * kRun) >> bit) & 1u) - zero;
           const uint32_t bits = lds16(sa + (uint32_t)(kSlotPlanes + g * 2 * kUnitRows) + row * 2u);
-          const float term = code != 0 ? (float)code * o.x * bits_to_float((unsigned short)bits, p.scale_dtype) * 32.f : 0.f;
+          const float term = code != 0 ? (float)code * bits_to_float((unsigned short)bits, p.scale_dtype) * o.x : 0.f;
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -468,7 +469,8 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
             }
           }
         }
-        // in units of 1/32 of the result: scale * 2^ex * sum
+        // scale * 2^(ex - 5) * sum of the operands' products, the power of two first: a product on the way is as large as the
+        // result, not as the sum of unscaled activations, which fp32 need not hold
         float sc[kTiles][2];
 #pragma unroll
         for (int tile = 0; tile < kTiles; ++tile)
@@ -481,9 +483,9 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
         for (int nt = 0; nt < NT; ++nt) {
           const float2 st = *reinterpret_cast<const float2*>(&stat[gl * 8 * NT + nt * 8 + 2 * tig]);
 #pragma unroll
-          for (int tile = 0; tile < kTiles; ++tile)
+          for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[tile][nt][q] = fmaf(sc[tile][q >> 1], d[tile][nt][q] * ((q & 1) ? st.y : st.x), acc[tile][nt][q]);
+            for (int tile = 0; tile < kTiles; ++tile) acc[tile][nt][q] = fmaf(sc[tile][q >> 1] * ((q & 1) ? st.y : st.x), d[tile][nt][q], acc[tile][nt][q]);
         }
       }
       if (has_outliers) add_outliers(pair, 0), add_outliers(pair, 1);
@@ -549,8 +551,8 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
           const float4 o = *from;
           v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
         }
-        const float unscale = arrived ? 0.03125f : __int_as_float(0x7fc00000);
-        float r[4] = {v.x * unscale, v.y * unscale, v.z * unscale, v.w * unscale};
+        float r[4] = {v.x, v.y, v.z, v.w};
+        if (!arrived) r[0] = r[1] = r[2] = r[3] = __int_as_float(0x7fc00000);
         const int at = (lane >> 1) * p.O + (unit0 + first) * kUnitRows + i * 8 + (lane & 1) * 4;
         if (p.addend)
           for (int q = 0; q < 4; ++q) r[q] += load_act(p.addend, p.act_dtype, at + q);

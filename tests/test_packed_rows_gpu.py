@@ -91,3 +91,25 @@ def test_one_activation_above_all_others_of_its_group(m, top):
     want, size = x.double() @ weight.t(), x.double().abs() @ weight.abs().t()
     assert bool((size[:, :16] < 1e3).all())
     assert bool(((out.double() - want).abs() <= (11 + 3 + 32) * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 2.0 ** -24).all())
+
+
+@pytest.mark.parametrize("values", ((1e19, -3e19), (2.0 ** 127, 2.0 ** 126, 1e38), (-3.3895313892515355e38,), (-3.3895313892515355e38, -3.3895313892515355e38)))
+@pytest.mark.parametrize("m", (1, 3, 16))
+def test_finite_activations_up_to_the_largest(m, values):
+    """Finite in, finite out: products with weights below one fit fp32 (the type's lowest value, as masks hold it, among them).  Several
+    large ones share a group's scale, so what their own code hides is rounded with them: the bound of ``test_packed_rows``."""
+    from marlin_style_fluxbin_b200 import _native
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    o, k = 64, 384
+    planes = torch.randint(0, 256, (3, 3, o, 16), device="cuda", generator=gen, dtype=torch.uint8)
+    scales = (torch.rand(3, o, device="cuda", generator=gen) * 0.015 + 0.005).half()
+    x = torch.randn(m, k, device="cuda", generator=gen).bfloat16()
+    for at, value in zip((131, 140, 250), values):
+        x[m - 1, at] = value
+    out = torch.full((m, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    _native.w3_gemm_small(x, planes, scales, None, None, out)
+    weight = _weight(planes, scales, None)
+    want, size = x.double() @ weight.t(), x.double().abs() @ (7 * scales.double()).t().repeat_interleave(128, dim=1).t()
+    assert bool(torch.isfinite(out).all())
+    assert bool(((out.double() - want).abs() <= (11 + 3 + 32) * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 2.0 ** -24).all())
