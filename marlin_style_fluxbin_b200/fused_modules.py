@@ -16,6 +16,7 @@ import threading
 from contextlib import contextmanager
 
 import torch
+from torch.nn.modules import module as module_base
 
 from . import _native
 from .w3_lut_deployment import PackedW3Linear
@@ -81,6 +82,18 @@ def fused_apply_rotary_pos_emb(q, k, cos, sin, unsqueeze_dim=1):
 _local = threading.local()
 
 
+def _qwen3():
+    from transformers.models.qwen3 import modeling_qwen3
+
+    return modeling_qwen3
+
+
+def _activations():
+    from transformers.activations import ACT2FN
+
+    return ACT2FN
+
+
 class DecodeStep:
     """What a session tells the modules about the step under way; ``position`` advances from step to step."""
 
@@ -96,9 +109,12 @@ class DecodeStep:
             _local.step = previous
 
 
-def _unobserved(*modules) -> bool:
-    """Nobody hooked the modules that a fused launch would skip."""
-    return not any(m._forward_hooks or m._forward_pre_hooks for m in modules)
+def _runs(module, *classes) -> bool:
+    """Whether calling ``module`` runs the forward of one of these classes and nothing else, so that a fused launch may stand
+    for it: no class or instance of its own making, no hooks on it or on every module, no compiled call."""
+    return (any(getattr(type(module), "forward", None) is owner.forward for owner in classes) and "forward" not in module.__dict__
+            and getattr(module, "_compiled_call_impl", None) is None
+            and not (module._forward_hooks or module._forward_pre_hooks or module_base._global_forward_hooks or module_base._global_forward_pre_hooks))
 
 
 def _step_serves(step, attention, call) -> bool:
@@ -106,6 +122,8 @@ def _step_serves(step, attention, call) -> bool:
     if call.get("past_key_values", call.get("past_key_value")) is not step.cache or positions is None:
         return False
     q_norm, k_norm = attention.q_norm, attention.k_norm
+    if not _runs(q_norm, _qwen3().Qwen3RMSNorm) or not _runs(k_norm, _qwen3().Qwen3RMSNorm):
+        return False
     layer = step.cache.layers[attention.layer_idx]
     keys, values = layer.keys, layer.values
     dim = attention.head_dim
@@ -115,7 +133,7 @@ def _step_serves(step, attention, call) -> bool:
             and positions[0].numel() == dim and _kernel_eligible(hidden, q_norm.weight, k_norm.weight, *positions, keys, values)
             and q_norm.variance_epsilon == k_norm.variance_epsilon and keys.shape == values.shape and keys.shape[0] == 1 and keys.shape[-1] == dim
             and step.position < keys.shape[2] and attention.config.num_attention_heads % keys.shape[1] == 0
-            and step.scratch.numel() >= _native.attn_scratch_bytes(attention.config.num_attention_heads) and _unobserved(q_norm, k_norm))
+            and step.scratch.numel() >= _native.attn_scratch_bytes(attention.config.num_attention_heads))
 
 
 def _attention_heads(step, attention, call):
@@ -132,9 +150,13 @@ def _attention_heads(step, attention, call):
     return out
 
 
+def _gates(mlp) -> bool:
+    return _runs(mlp.act_fn, torch.nn.SiLU, type(_activations()["silu"]))
+
+
 def _gated(mlp, x):
     """What down_proj takes, in one launch behind gate/up; None where that launch does not serve."""
-    if mlp.config.hidden_act != "silu" or not _kernel_eligible(x) or not _unobserved(mlp.act_fn):
+    if not _gates(mlp) or not _kernel_eligible(x):
         return None
     gate, up = mlp.gate_proj(x), mlp.up_proj(x)
     if not _kernel_eligible(x, gate, up):
@@ -163,9 +185,9 @@ def _fused_mlp(original):
     return forward
 
 
-def _joins(projection, wrapped) -> bool:
+def _joins(projection) -> bool:
     """Whether a projection can take the residual addition that follows it into its launch."""
-    return isinstance(projection, PackedW3Linear) and projection._decode_binding is not None and projection.bias is None and _unobserved(projection, wrapped)
+    return _runs(projection, PackedW3Linear) and projection._decode_binding is not None and projection.bias is None
 
 
 def _fused_layer(original):
@@ -173,12 +195,12 @@ def _fused_layer(original):
 
     def forward(self, *args, **kwargs):
         step, attention, mlp = getattr(_local, "step", None), self.self_attn, self.mlp
-        if step is None or not _joins(attention.o_proj, attention) or not _joins(mlp.down_proj, mlp):
+        if step is None or not (_runs(attention, _qwen3().Qwen3Attention) and _runs(mlp, _qwen3().Qwen3MLP) and _joins(attention.o_proj) and _joins(mlp.down_proj)):
             return original(self, *args, **kwargs)
         call = dict(signature.bind(self, *args, **kwargs).arguments)
         residual = call["hidden_states"]
         # both halves have to serve before anything is launched
-        if not _step_serves(step, attention, call) or mlp.config.hidden_act != "silu" or not _kernel_eligible(residual) or not _unobserved(mlp.act_fn):
+        if not _step_serves(step, attention, call) or not _gates(mlp) or not _kernel_eligible(residual):
             return original(self, *args, **kwargs)
         call["hidden_states"] = self.input_layernorm(residual)
         heads = _attention_heads(step, attention, call)

@@ -51,3 +51,42 @@ def test_steps_with_packed_projections(dtype, shuffled, monkeypatch):
             assert len(joined) == 2 * 4  # an observed MLP is called, not passed over
     gap = (fused["logits"].float() - stock["logits"].float()).square().mean().sqrt() / stock["logits"].float().square().mean().sqrt()
     assert float(gap) < 0.02
+
+
+@pytest.mark.parametrize("change", ("attention", "mlp", "projection"))
+def test_exchanged_parts_are_called(change):
+    """A layer whose attention, MLP or projection has a forward of its own is not run past it; logits as by the stock layer."""
+    from transformers import Qwen3Config, Qwen3ForCausalLM
+
+    from marlin_style_fluxbin_b200.fused_modules import fused_qwen3_modules
+    from marlin_style_fluxbin_b200.qwen3 import QWEN3_LINEAR_MODULES
+    from marlin_style_fluxbin_b200.static_decode import StaticDecodeSession, prepared_linears
+    from marlin_style_fluxbin_b200.w3_lut_deployment import PackedW3Linear
+
+    torch.manual_seed(5)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    config = Qwen3Config(vocab_size=96, hidden_size=256, intermediate_size=384, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=2, head_dim=128)
+    config._attn_implementation = "sdpa"
+    model = Qwen3ForCausalLM(config).eval().cuda().bfloat16()
+    block = model.model.layers[0]
+    for name in QWEN3_LINEAR_MODULES:
+        old = block.get_submodule(name)
+        o, k = old.out_features, old.in_features
+        layout = {"planes": torch.randint(0, 256, (k // 128, 3, o, 16), device="cuda", generator=gen, dtype=torch.uint8),
+                  "scales": (torch.rand(k // 128, o, device="cuda", generator=gen) * 0.015 + 0.005).bfloat16(),
+                  "perm": torch.arange(k, device="cuda").to(torch.int16)}
+        parent, attribute = name.rsplit(".", 1)
+        setattr(block.get_submodule(parent), attribute, PackedW3Linear(layout, fallback="dense", row_tile=256))
+    part = {"attention": block.self_attn, "mlp": block.mlp, "projection": block.mlp.down_proj}[change]
+
+    def tripled(self, *args, **kwargs):
+        out = super(part.__class__, self).forward(*args, **kwargs)
+        return (out[0] * 3, *out[1:]) if isinstance(out, tuple) else out * 3
+
+    part.__class__ = type("Own", (type(part),), {"forward": tripled})
+    session = StaticDecodeSession(model, torch.randint(0, 96, (1, 7), device="cuda", generator=gen), torch.randint(0, 96, (1, 3), device="cuda", generator=gen))
+    with prepared_linears(model, torch.bfloat16):
+        stock = session.audit()["logits"].float()
+        with fused_qwen3_modules():
+            fused = session.audit()["logits"].float()
+    assert float((fused - stock).square().mean().sqrt() / stock.square().mean().sqrt()) < 0.02
