@@ -238,6 +238,9 @@ def fused_qwen3_modules(*, rms_norm=True, rope=True):
         if rms_norm and rope:
             for name, wrap in (("Qwen3Attention", _fused_attention), ("Qwen3MLP", _fused_mlp), ("Qwen3DecoderLayer", _fused_layer)):
                 owner = getattr(modeling_qwen3, name)
+                # layers of some transformers versions return a tuple; the fused one returns the hidden states alone
+                if wrap is _fused_layer and inspect.signature(owner.forward).return_annotation not in (torch.Tensor, "torch.Tensor"):
+                    continue
                 saved[name] = owner.forward
                 owner.forward = wrap(owner.forward)
         yield applied

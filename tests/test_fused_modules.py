@@ -131,3 +131,19 @@ def test_patched_tiny_model_decode_on_gpu_matches_stock():
         with fused_qwen3_modules():
             fused = model(input_ids=torch.tensor([[5]], device="cuda"), past_key_values=copy.deepcopy(cache), use_cache=True).logits
     assert float((fused.float() - stock.float()).abs().max()) <= 0.02 * float(stock.float().abs().max())
+
+
+def test_layers_that_return_a_tuple_are_left_alone(monkeypatch):
+    from transformers.models.qwen3 import modeling_qwen3
+
+    stock = modeling_qwen3.Qwen3DecoderLayer.forward
+    with fused_qwen3_modules():
+        assert modeling_qwen3.Qwen3DecoderLayer.forward is not stock
+
+    def forward(self, hidden_states, **kwargs) -> tuple[torch.Tensor, ...]:
+        return (stock(self, hidden_states, **kwargs),)
+
+    monkeypatch.setattr(modeling_qwen3.Qwen3DecoderLayer, "forward", forward)
+    with fused_qwen3_modules():
+        assert modeling_qwen3.Qwen3DecoderLayer.forward is forward
+    assert modeling_qwen3.Qwen3DecoderLayer.forward is forward
