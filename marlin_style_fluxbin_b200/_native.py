@@ -280,6 +280,16 @@ def _on(device):
     return _HERE if index is not None and index == _current_device() else torch.cuda.device(device)
 
 
+def plain_tensors(*tensors) -> bool:
+    """Whether a launch with raw addresses can stand for tensor operations on these: none of a subclass or with a forward-mode
+    tangent, no transform at work (vmap, jvp) and nothing that records operations (tracing, dispatch modes)."""
+    if torch._C._len_torch_dispatch_stack() or torch._C._get_tracing_state() is not None or torch._C._functorch.maybe_current_level() is not None:
+        return False
+    dual = torch.autograd.forward_ad
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and (dual._current_level < 0 or dual.unpack_dual(t).tangent is None)
+               for t in tensors if t is not None)
+
+
 _W3_SLOTS = ("w3", "w3#1", "w3#2")
 _NO_PDL, _NO_SAME_INPUT = bool(_os.environ.get("FB_NO_PDL")), bool(_os.environ.get("FB_NO_SAME_INPUT"))
 

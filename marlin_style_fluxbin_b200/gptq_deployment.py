@@ -325,6 +325,12 @@ def _signed_codes(layout: Mapping[str, torch.Tensor]) -> torch.Tensor:
     return grouped - (ZERO if zeros is None else zeros.to(torch.int16).unsqueeze(1))
 
 
+def _raw(layout) -> bool:
+    from . import _native
+
+    return _native.plain_tensors(*layout.values()) and layout["planes"].data_ptr() % 16 == 0
+
+
 def restore_planar_w3(layout: Mapping[str, torch.Tensor], *, dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """Dequantise to a dense ``[O,K]`` weight.
 
@@ -333,7 +339,7 @@ def restore_planar_w3(layout: Mapping[str, torch.Tensor], *, dtype: torch.dtype 
     """
     out_features, in_features = validate_planar_w3(layout)
     # the kernel's bounds: 65536 rows, planes on a 16-byte boundary
-    if layout["planes"].is_cuda and dtype in (torch.float16, torch.bfloat16) and out_features <= 65536 and layout["planes"].data_ptr() % 16 == 0:
+    if layout["planes"].is_cuda and dtype in (torch.float16, torch.bfloat16) and out_features <= 65536 and _raw(layout):
         from . import _native
 
         ordered = torch.empty(out_features, in_features, device=layout["planes"].device, dtype=dtype)

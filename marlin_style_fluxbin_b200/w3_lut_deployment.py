@@ -516,6 +516,13 @@ class PackedW3Linear(nn.Module):
         # a weak reference to the module, so no cycle: a dropped module gives its weights back at once
         self._decode_binding = _native.calls().Bound(launch.call, launch, output, shaped, weakref.ref(self), self._buffers)
 
+    def _launches(self, x, rows) -> bool:
+        """Whether the dense fallback may go through the kernels; what they do not take, and what tensor operations refuse
+        (a bias of another dtype), is left to tensor operations."""
+        return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.device == self.planes.device and rows > 0
+                and (self.bias is None or (self.bias.dtype == x.dtype and self.bias.device == x.device and self.bias.shape == (self.out_features,)))
+                and _native.plain_tensors(x, self.bias, *self.layout().values()) and self.planes.data_ptr() % 16 == 0 and self.perm.data_ptr() % 16 == 0)
+
     def adds_residual(self, x: torch.Tensor) -> bool:
         """Whether ``add_to`` can stand for a call of this bound module and an addition."""
         return (self._decode_binding is not None and self.bias is None and self._decode_output.dtype == x.dtype and x.is_cuda and x.is_contiguous()
@@ -546,7 +553,7 @@ class PackedW3Linear(nn.Module):
                 raise ValueError("unsupported input; enable explicit dense fallback if needed")
             self.last_route = "dense_fallback"
             self.route_counts["dense_fallback"] += 1
-            if not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16) or x.device != self.planes.device or rows == 0:
+            if not self._launches(x, rows):
                 return F.linear(x, restore_planar_w3(layout, dtype=x.dtype), self.bias)
             self._require_valid_values(layout)
             return dense_linear(x.reshape(rows, self.in_features), layout, self.bias).reshape(*x.shape[:-1], self.out_features)
