@@ -22,10 +22,21 @@ FB_W3_GROUP_PARTIALS = 4
 FB_W3_SAME_INPUT = 8
 
 _lib = None
-try:
-    from . import _fb_calls as _calls
-except ImportError:  # not built: calls() says so
-    _calls = None
+
+
+def _load_calls():
+    """``(module, None)``, or ``(None, why)``: not built, or built against another torch (whose objects it would misread)."""
+    try:
+        from . import _fb_calls as module
+    except ImportError as error:
+        return None, error
+    built = getattr(module, "torch_version", "of an unknown version")
+    if built != torch.__version__:
+        return None, ImportError(f"{module.__file__} was built against torch {built}, this is {torch.__version__}")
+    return module, None
+
+
+_calls, _calls_error = _load_calls()
 
 
 class W3Matrix(ctypes.Structure):
@@ -48,7 +59,7 @@ class NativeError(RuntimeError):
 def calls():
     """The extension module behind eager calls on prepared launches (``csrc/python/fb_calls.cpp``)."""
     if _calls is None:
-        raise RuntimeError("_fb_calls.so is not built; run `python -m marlin_style_fluxbin_b200.build`")
+        raise RuntimeError(f"the extension module of the eager calls cannot be used ({_calls_error}); run `python -m marlin_style_fluxbin_b200.build`") from _calls_error
     return _calls
 
 

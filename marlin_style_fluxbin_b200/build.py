@@ -1,5 +1,5 @@
 """Ahead-of-time build of the CUDA library (``libfluxbin_b200.so``) with nvcc for sm_100a, and of the extension
-module behind eager calls (``_fb_calls.so``) with the host compiler against torch's C++ interface.
+module behind eager calls (``_fb_calls``, tagged with Python's ABI) with the host compiler against torch's C++ interface.
 
 Both are built in-tree, next to this file, so that they travel with the source tree.
 ``python -m marlin_style_fluxbin_b200.build`` rebuilds it; ``build()`` is incremental.
@@ -11,12 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libfluxbin_b200.so"
-CALLS = PACKAGE / "_fb_calls.so"
+CALLS = PACKAGE / f"_fb_calls{sysconfig.get_config_var('EXT_SUFFIX')}"
 STAMP = PACKAGE / "csrc" / ".build_stamp"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -38,7 +39,10 @@ def sources() -> list[Path]:
 
 
 def _fingerprint() -> str:
-    digest = hashlib.sha256()
+    import torch
+
+    # the extension module reads tensor objects as this torch lays them out
+    digest = hashlib.sha256(f"{torch.__version__} {torch._C._GLIBCXX_USE_CXX11_ABI} {CALLS.name}".encode())
     for path in sorted(sources() + list(CSRC.glob("*.cuh")) + list(CSRC.glob("python/*.cpp")) + [PACKAGE.parent / "include" / "fluxbin_b200.h", Path(__file__)]):
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
@@ -46,14 +50,12 @@ def _fingerprint() -> str:
 
 
 def _build_calls(nvcc: str) -> str:
-    import sysconfig
-
     import torch
     from torch.utils.cpp_extension import include_paths
 
     libraries = Path(torch.__file__).resolve().parent / "lib"
     headers = [*include_paths(), sysconfig.get_paths()["include"], str(Path(nvcc).resolve().parent.parent / "include")]
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f'-DFB_TORCH_VERSION="{torch.__version__}"', f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *(flag for path in headers for flag in ("-isystem", path)), str(CSRC / "python" / "fb_calls.cpp"), "-o", str(CALLS),
            f"-L{libraries}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     done = subprocess.run(cmd, capture_output=True, text=True)

@@ -330,7 +330,7 @@ PyMODINIT_FUNC PyInit__fb_calls(void) {
   name_last = PyUnicode_InternFromString("last_route"), name_add = PyUnicode_InternFromString("add_");
   PyObject* module = PyModule_Create(&module_def);
   if (!module) return nullptr;
-  if (PyModule_AddObjectRef(module, "Call", reinterpret_cast<PyObject*>(&call_type)) < 0 || PyModule_AddObjectRef(module, "Bound", reinterpret_cast<PyObject*>(&bound_type)) < 0) {
+  if (PyModule_AddStringConstant(module, "torch_version", FB_TORCH_VERSION) < 0 || PyModule_AddObjectRef(module, "Call", reinterpret_cast<PyObject*>(&call_type)) < 0 || PyModule_AddObjectRef(module, "Bound", reinterpret_cast<PyObject*>(&bound_type)) < 0) {
     Py_DECREF(module);
     return nullptr;
   }
