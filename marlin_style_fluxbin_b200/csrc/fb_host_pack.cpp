@@ -6,8 +6,16 @@
 // eight input positions make one byte of each plane: the code's three bits are spread to bytes 0, 1 and 2 of a
 // 32-bit lane by one multiplication, shifted to the position's bit and or-ed.  The compiler vectorises these
 // loops over the columns (in the widest form the CPU has).  The layout wants the 16 bytes of a row together, so
-// 16 x 16 byte blocks are transposed with unpack instructions.  Groups are dealt to threads.
+// 16 x 16 byte blocks are transposed, with unpack instructions on x86; other hosts (the Arm ones of some B200 systems, or
+// FB_PORTABLE) take the plain loops.  Groups are dealt to threads.
+#if defined(__x86_64__) && !defined(FB_PORTABLE)
 #include <emmintrin.h>
+#define FB_X86 1
+#define FB_CLONES __attribute__((target_clones("arch=skylake-avx512", "avx2", "default")))
+#else
+#define FB_X86 0
+#define FB_CLONES
+#endif
 #include <stdint.h>
 #include <string.h>
 
@@ -27,6 +35,7 @@ constexpr int kColumns = 64;
 
 // 16 rows of 16 bytes (row stride `stride`) -> 16 columns, written as 16 contiguous rows of 16 bytes.
 inline void transpose16(const uint8_t* from, size_t stride, uint8_t* to) {
+#if FB_X86
   __m128i a[16], b[16];
   for (int i = 0; i < 16; ++i) a[i] = _mm_loadu_si128(reinterpret_cast<const __m128i*>(from + i * stride));
   for (int round = 0; round < 4; ++round) {  // a perfect shuffle of the 256 bytes, four times, is the transpose
@@ -37,10 +46,14 @@ inline void transpose16(const uint8_t* from, size_t stride, uint8_t* to) {
     memcpy(a, b, sizeof(a));
   }
   for (int i = 0; i < 16; ++i) _mm_storeu_si128(reinterpret_cast<__m128i*>(to + 16 * i), a[i]);
+#else
+  for (int i = 0; i < 16; ++i)
+    for (int j = 0; j < 16; ++j) to[16 * j + i] = from[i * stride + j];
+#endif
 }
 
 // Plane bytes of group g for columns [o0, o0 + n): n <= kColumns.
-__attribute__((target_clones("arch=skylake-avx512", "avx2", "default"))) void pack_block(const uint32_t* words, const int64_t* order, int O, int o0, int n, uint8_t (*bytes)[16][kColumns]) {
+FB_CLONES void pack_block(const uint32_t* words, const int64_t* order, int O, int o0, int n, uint8_t (*bytes)[16][kColumns]) {
   for (int c = 0; c < 16; ++c) {
     uint32_t acc[kColumns] = {};
     for (int j = 0; j < 8; ++j) {
