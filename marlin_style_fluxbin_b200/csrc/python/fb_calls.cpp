@@ -291,8 +291,15 @@ PyObject* bound_copy(PyObject* object, PyObject*) { return Py_NewRef(object); } 
 PyMethodDef bound_methods[] = {{"__copy__", bound_copy, METH_NOARGS, nullptr}, {"__deepcopy__", bound_copy, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyTypeObject bound_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// holds(layout, seen): seen = ((name, weak reference, address[, version]), ...); whether the layout is exactly these tensors, where
-// they were, and in the stated version (None: an inference tensor, which has none)
+bool shaped_as(const at::Tensor& t, PyObject* sizes, PyObject* dtype) {
+  if (t.dim() != PyTuple_GET_SIZE(sizes) || t.scalar_type() != reinterpret_cast<THPDtype*>(dtype)->scalar_type || !t.is_contiguous()) return false;
+  for (int64_t i = 0; i < t.dim(); ++i)
+    if (t.size(i) != PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i))) return false;
+  return true;
+}
+
+// holds(layout, seen): seen = ((name, weak reference, address, sizes, dtype[, version]), ...); whether the layout is exactly these
+// tensors, where and as they were, contiguous, and in the stated version (None: an inference tensor, which has none)
 PyObject* holds(PyObject*, PyObject* const* args, Py_ssize_t count) {
   return guarded([&]() -> PyObject* {
     if (count != 2 || !PyTuple_Check(args[1])) return PyErr_SetString(PyExc_TypeError, "expected a layout and a tuple"), nullptr;
@@ -304,8 +311,9 @@ PyObject* holds(PyObject*, PyObject* const* args, Py_ssize_t count) {
       if (!value || PyWeakref_GetObject(PyTuple_GET_ITEM(entry, 1)) != value || !THPVariable_Check(value)) Py_RETURN_FALSE;
       const at::Tensor& tensor = THPVariable_Unpack(value);
       if (reinterpret_cast<uintptr_t>(tensor.const_data_ptr()) != PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(entry, 2))) Py_RETURN_FALSE;
-      if (PyTuple_GET_SIZE(entry) > 3) {
-        PyObject* version = PyTuple_GET_ITEM(entry, 3);
+      if (!shaped_as(tensor, PyTuple_GET_ITEM(entry, 3), PyTuple_GET_ITEM(entry, 4))) Py_RETURN_FALSE;
+      if (PyTuple_GET_SIZE(entry) > 5) {
+        PyObject* version = PyTuple_GET_ITEM(entry, 5);
         if (tensor.is_inference() != (version == Py_None) || (version != Py_None && static_cast<long long>(tensor._version()) != PyLong_AsLongLong(version))) Py_RETURN_FALSE;
       }
     }

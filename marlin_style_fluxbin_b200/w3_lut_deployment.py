@@ -243,9 +243,10 @@ class _LayoutRecord:
 
     def __init__(self, layout):
         self.out_features, self.in_features = validate_planar_w3(layout, check_values=False)
-        # the perm with its version: a launch knows whether it was the identity
-        self.seen = tuple((name, weakref.ref(value), value.data_ptr()) + ((None if value.is_inference() else value._version,) if name == "perm" else ())
-                          for name, value in layout.items())
+        # what the checks looked at, so that they hold only while it does; the perm with its version: a launch knows whether it
+        # was the identity
+        self.seen = tuple((name, weakref.ref(value), value.data_ptr(), tuple(value.shape), value.dtype)
+                          + ((None if value.is_inference() else value._version,) if name == "perm" else ()) for name, value in layout.items())
         self.index, self.launches, self.recent = layout["planes"].get_device(), {}, None
 
 
