@@ -474,11 +474,17 @@ class PackedW3Linear(nn.Module):
         return {name: getattr(self, name) for name in self._fields}
 
     def _require_valid_values(self, layout) -> None:
-        """The value checks of ``validate_planar_w3`` (they synchronise), once per state of the buffers."""
-        stamp = None if any(t.is_inference() for t in layout.values()) else tuple((t.data_ptr(), t._version) for t in layout.values())
-        if stamp is None or stamp != self._valid_values:
+        """The value checks of ``validate_planar_w3`` (they synchronise), once per state of the buffers: these very tensors, where
+        they were, not written to since (inference tensors do not tell, and are checked every time)."""
+        seen = self._valid_values
+        if seen is None or len(seen) != len(layout) or any(owner() is not t or address != t.data_ptr() or version != t._version
+                                                           for (owner, address, version), t in zip(seen, layout.values())):
             validate_planar_w3(layout)
-            self._valid_values = stamp
+            known = not any(t.is_inference() for t in layout.values())
+            self._valid_values = tuple((weakref.ref(t), t.data_ptr(), t._version) for t in layout.values()) if known else None
+
+    def __getstate__(self):
+        return {**self.__dict__, "_valid_values": None}  # weak references, to the buffers of this module
 
     def clear_prepared_decode(self) -> None:
         self._decode_binding = None

@@ -1,4 +1,8 @@
 """What the packed calls remember of a layout holds only while the tensors are as they were checked."""
+import copy
+import io
+
+import numpy as np
 import pytest
 import torch
 
@@ -32,3 +36,26 @@ def test_another_dtype_at_the_same_place_is_checked_again():
     layout["scales"].data = layout["scales"].data.view(torch.bfloat16)
     again = w3._layout_record(layout)
     assert again is not record and again.seen[1][4] == torch.bfloat16
+
+
+def test_values_at_a_known_address_are_checked_again():
+    """Buffers exchanged for others over the same memory: address and version are those that were checked."""
+    module = w3.PackedW3Linear(_layout(), fallback="dense", row_tile=256)
+    values = np.full((2, 64), 3, dtype=np.uint8)
+    module.zeros = torch.from_numpy(values)
+    module._require_valid_values(module.layout())
+    values[:] = 9
+    module.zeros = torch.from_numpy(values)
+    with pytest.raises(ValueError, match="zero points"):
+        module._require_valid_values(module.layout())
+
+
+def test_checked_modules_are_copied_and_saved():
+    module = w3.PackedW3Linear(_layout(), fallback="dense", row_tile=256)
+    module._require_valid_values(module.layout())
+    twin = copy.deepcopy(module)
+    assert torch.equal(twin.planes, module.planes)
+    file = io.BytesIO()
+    torch.save(module, file)
+    file.seek(0)
+    assert torch.equal(torch.load(file, weights_only=False).planes, module.planes)
