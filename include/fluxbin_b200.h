@@ -417,7 +417,7 @@ int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int width, int ou
  * Checkpoint preparation on the host (plain host memory, no CUDA call): the reference's converter
  * (gptq_deployment.py:25-205) without tensors of single codes.
  * fb_host_w3_order: stable order of the input columns by group; FB_ELIMIT if the group indexes do not span
- *   0 .. K/128 - 1, FB_EINVAL if a group does not hold exactly 128 columns.
+ *   0 .. K/128 - 1 or K is above 32767, FB_EINVAL if a group does not hold exactly 128 columns.
  * fb_host_w3_planes: qweight [3K/32, O] and that order -> planes [K/128, 3, O, 16] (high plane inverted), on at most
  *   `threads` threads.
  * fb_host_w3_zeros: qzeros [G, 3O/32] -> zero points [G, O], (code + plus) & 7; bit z of *seen: z occurs.

@@ -6,6 +6,7 @@
 #include <cudaTypedefs.h>
 
 #include <mutex>
+#include <new>
 #include <unordered_map>
 
 #include "fb_common.cuh"
@@ -70,6 +71,15 @@ std::mutex g_map_lock;
 std::unordered_map<MapKey, CUtensorMap, MapHash> g_maps;
 PFN_cuTensorMapEncodeTiled g_encode = nullptr;
 
+// Caller holds g_map_lock.  Without memory the descriptor is not kept, and encoded again next time.
+void keep(const MapKey& key, const CUtensorMap& map) {
+  try {
+    if (g_maps.size() >= 16384) g_maps.clear();
+    g_maps.emplace(key, map);
+  } catch (const std::bad_alloc&) {
+  }
+}
+
 // Caller holds g_map_lock.
 bool encoder_ready() {
   if (g_encode) return true;
@@ -106,8 +116,7 @@ bool plane_tensor_map(const uint8_t* planes, int O, int G, int rows, int box_uni
     fail(FB_ECUDA, "cuTensorMapEncodeTiled failed with code %d for planes [%d,3,%d,16]", (int)rc, G, O);
     return false;
   }
-  if (g_maps.size() >= 16384) g_maps.clear();
-  g_maps.emplace(key, map);
+  keep(key, map);
   *out = map;
   return true;
 }
@@ -146,8 +155,7 @@ bool group_row_tensor_map(const void* base, int elem_bytes, int O, int G, int ro
     fail(FB_ECUDA, "cuTensorMapEncodeTiled failed with code %d for a [%d,%d] tensor of %d-byte elements", (int)rc, G, O, elem_bytes);
     return false;
   }
-  if (g_maps.size() >= 16384) g_maps.clear();
-  g_maps.emplace(key, map);
+  keep(key, map);
   *out = map;
   return true;
 }

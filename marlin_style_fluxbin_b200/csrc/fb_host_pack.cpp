@@ -102,8 +102,9 @@ void pack_groups(const uint32_t* words, const int64_t* order, int O, uint8_t* pl
 
 extern "C" int fb_host_w3_order(const int32_t* g_idx, int in_features, int64_t* order) {
   if (!g_idx || !order || in_features < 128 || in_features % 128) return fb::fail(FB_EINVAL, "fb_host_w3_order: bad argument");
+  if (in_features > 32767) return fb::fail(FB_ELIMIT, "fb_host_w3_order: K=%d: columns must be numbered by int16", in_features);
   const int G = in_features / 128;
-  std::vector<int> next(G);
+  int next[255];
   for (int g = 0; g < G; ++g) next[g] = 128 * g;
   bool low = false, high = false, uneven = false;
   for (int k = 0; k < in_features; ++k) {

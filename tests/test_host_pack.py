@@ -20,3 +20,15 @@ def test_native_conversion_equals_the_tensor_form(o, k, desc_act):
     assert torch.equal(layout["planes"], planes_from_sorted_codes(unpack_gptq_w3_qweight(raw["qweight"])[by_group]))
     assert torch.equal(layout["zeros"], unpack_gptq_w3_qzeros(raw["qzeros"], qzero_format=1))
     assert torch.equal(layout["perm"].long(), by_group)
+
+
+def test_column_orders_beyond_int16_are_refused():
+    from marlin_style_fluxbin_b200 import _native
+
+    if not _native.LIBRARY.exists():
+        pytest.skip("not built")
+    groups, order = (torch.arange(65536) // 128).to(torch.int32), torch.zeros(65536, dtype=torch.int64)
+    assert _native.library().fb_host_w3_order(groups.data_ptr(), 65536, order.data_ptr()) == -2  # FB_ELIMIT
+    assert not bool(order.any())
+    assert _native.library().fb_host_w3_order(groups.data_ptr(), 32640, order.data_ptr()) == 0
+    assert torch.equal(order[:32640], torch.arange(32640))
