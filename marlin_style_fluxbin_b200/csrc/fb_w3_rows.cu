@@ -539,7 +539,10 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
                      : "memory");
       }
     }
-    const bool arrived = mbar_wait_bounded(inbox_bar, inbox_phase);
+    // Longer than a CTA of the cluster is held up by copies that do not land (one limit, then it sends NaN): none may leave
+    // while another still stores into its shared memory.
+    bool arrived = false;
+    for (int limit = 0; limit < 3 && !arrived; ++limit) arrived = mbar_wait_bounded(inbox_bar, inbox_phase);
     inbox_phase ^= 1u;
     if (!arrived) atomicExch(p.status, 1u);
     for (int i = warp * splits + rank; i < 4 * units; i += kWarps * splits) {
