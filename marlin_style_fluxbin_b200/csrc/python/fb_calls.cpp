@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
+#include <cstring>
 
 namespace {
 
@@ -291,15 +292,30 @@ PyObject* bound_copy(PyObject* object, PyObject*) { return Py_NewRef(object); } 
 PyMethodDef bound_methods[] = {{"__copy__", bound_copy, METH_NOARGS, nullptr}, {"__deepcopy__", bound_copy, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyTypeObject bound_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-bool shaped_as(const at::Tensor& t, PyObject* sizes, PyObject* dtype) {
-  if (t.dim() != PyTuple_GET_SIZE(sizes) || t.scalar_type() != reinterpret_cast<THPDtype*>(dtype)->scalar_type || !t.is_contiguous()) return false;
-  for (int64_t i = 0; i < t.dim(); ++i)
-    if (t.size(i) != PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i))) return false;
-  return true;
+// What a check saw of a tensor: compared byte by byte, it costs a call next to nothing.
+struct Stamp {
+  int64_t address = 0, sizes[4] = {}, dim = 0, dtype = 0, tracked = 0, version = 0;  // version -1: an inference tensor, which has none
+
+  Stamp(const at::Tensor& t, bool with_version) {
+    address = static_cast<int64_t>(reinterpret_cast<uintptr_t>(t.const_data_ptr()));
+    dim = t.is_contiguous() && t.dim() <= 4 ? t.dim() : -1;
+    for (int64_t i = 0; i < dim; ++i) sizes[i] = t.size(i);
+    dtype = static_cast<int64_t>(t.scalar_type());
+    tracked = with_version;
+    if (with_version) version = t.is_inference() ? -1 : static_cast<int64_t>(t._version());
+  }
+};
+
+// stamp(tensor, whether its version counts) -> bytes
+PyObject* stamp(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 2 || !THPVariable_Check(args[0])) return PyErr_SetString(PyExc_TypeError, "expected a tensor and a truth value"), nullptr;
+    const Stamp seen(THPVariable_Unpack(args[0]), args[1] == Py_True);
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(&seen), sizeof seen);
+  });
 }
 
-// holds(layout, seen): seen = ((name, weak reference, address, sizes, dtype[, version]), ...); whether the layout is exactly these
-// tensors, where and as they were, contiguous, and in the stated version (None: an inference tensor, which has none)
+// holds(layout, seen): seen = ((name, weak reference, stamp), ...); whether the layout is exactly these tensors, as they were
 PyObject* holds(PyObject*, PyObject* const* args, Py_ssize_t count) {
   return guarded([&]() -> PyObject* {
     if (count != 2 || !PyTuple_Check(args[1])) return PyErr_SetString(PyExc_TypeError, "expected a layout and a tuple"), nullptr;
@@ -309,19 +325,16 @@ PyObject* holds(PyObject*, PyObject* const* args, Py_ssize_t count) {
       PyObject* value = PyDict_GetItemWithError(args[0], PyTuple_GET_ITEM(entry, 0));
       if (!value && PyErr_Occurred()) return nullptr;
       if (!value || PyWeakref_GetObject(PyTuple_GET_ITEM(entry, 1)) != value || !THPVariable_Check(value)) Py_RETURN_FALSE;
-      const at::Tensor& tensor = THPVariable_Unpack(value);
-      if (reinterpret_cast<uintptr_t>(tensor.const_data_ptr()) != PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(entry, 2))) Py_RETURN_FALSE;
-      if (!shaped_as(tensor, PyTuple_GET_ITEM(entry, 3), PyTuple_GET_ITEM(entry, 4))) Py_RETURN_FALSE;
-      if (PyTuple_GET_SIZE(entry) > 5) {
-        PyObject* version = PyTuple_GET_ITEM(entry, 5);
-        if (tensor.is_inference() != (version == Py_None) || (version != Py_None && static_cast<long long>(tensor._version()) != PyLong_AsLongLong(version))) Py_RETURN_FALSE;
-      }
+      const char* const then = PyBytes_AS_STRING(PyTuple_GET_ITEM(entry, 2));
+      const Stamp now(THPVariable_Unpack(value), reinterpret_cast<const Stamp*>(then)->tracked != 0);
+      if (memcmp(&now, then, sizeof now)) Py_RETURN_FALSE;
     }
     Py_RETURN_TRUE;
   });
 }
 
-PyMethodDef module_methods[] = {{"holds", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(holds)), METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef module_methods[] = {{"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},
+                                {"holds", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(holds)), METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fb_calls", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

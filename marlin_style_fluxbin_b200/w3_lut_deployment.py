@@ -148,19 +148,21 @@ def _perm_entry(perm: torch.Tensor):
 
 
 def _answer_word():
-    """A word that no question has had, under the lock: ``(words, index)``."""
+    """A word that no question has had, under the lock: ``(words, index, address)``."""
     global _perm_given
     if not _perm_blocks or _perm_given == _MAX_PERMS:
         # a full block whose answers are all there can go; entries keep the one they read
-        _perm_blocks[:] = [words for words in _perm_blocks if int(words.min()) < 0]
-        _perm_blocks.append(torch.full((_MAX_PERMS,), -1, dtype=torch.int32, pin_memory=torch.cuda.is_available()).numpy())
+        _perm_blocks[:] = [block for block in _perm_blocks if int(block[0].min()) < 0]
+        words = torch.full((_MAX_PERMS,), -1, dtype=torch.int32, pin_memory=torch.cuda.is_available())
+        _perm_blocks.append((words.numpy(), words.data_ptr()))
         _perm_given = 0
         for key in [key for key, entry in _IDENTITY_PERMS.items() if entry[0]() is None]:
             del _IDENTITY_PERMS[key]
         if len(_IDENTITY_PERMS) >= _MAX_PERMS:
             _IDENTITY_PERMS.clear()
+    words, address = _perm_blocks[-1]
     _perm_given += 1
-    return _perm_blocks[-1], _perm_given - 1
+    return words, _perm_given - 1, address + 4 * (_perm_given - 1)
 
 
 def _ask_perm(perm: torch.Tensor):
@@ -168,10 +170,10 @@ def _ask_perm(perm: torch.Tensor):
         entry = _perm_entry(perm)  # another thread may have asked meanwhile
         if entry is not None:
             return entry
-        words, index = _answer_word()
+        words, index, address = _answer_word()
         try:
             with torch.cuda.device(perm.device):
-                _native.check(_native.library().fb_identity_order(perm.data_ptr(), perm.numel(), words.ctypes.data + 4 * index, _native.stream_handle(perm.device)))
+                _native.check(_native.library().fb_identity_order(perm.data_ptr(), perm.numel(), address, _native.stream_handle(perm.device)))
         except BaseException:
             words[index] = 0  # nothing will answer
             raise
@@ -245,8 +247,7 @@ class _LayoutRecord:
         self.out_features, self.in_features = validate_planar_w3(layout, check_values=False)
         # what the checks looked at, so that they hold only while it does; the perm with its version: a launch knows whether it
         # was the identity
-        self.seen = tuple((name, weakref.ref(value), value.data_ptr(), tuple(value.shape), value.dtype)
-                          + ((None if value.is_inference() else value._version,) if name == "perm" else ()) for name, value in layout.items())
+        self.seen = tuple((name, weakref.ref(value), _native.calls().stamp(value, name == "perm")) for name, value in layout.items())
         self.index, self.launches, self.recent = layout["planes"].get_device(), {}, None
 
 
