@@ -37,7 +37,7 @@ struct Call {
   PyObject* shape;       // (1, in_features)
   PyObject* families;    // scratch families: the one, or the three that rotate
   PyObject* scratch;     // dict (index, stream, family) -> tensor
-  PyObject* ahead;       // dict (index, stream) -> ((address, shape, dtype), launches in a row)
+  PyObject* ahead;       // dict (index, stream) -> ((address, shape, dtype), launches in a row, ((output's begin, end), ...) of these)
   PyObject* scratch_for; // (device index, bytes, family) -> tensor
   PyObject* capturing;   // () -> bool
   PyObject* failed;      // raises the error of a refused launch
@@ -56,6 +56,17 @@ PyObject* scratch_at(Call* self, PyObject* index, PyObject* stream, PyObject* fa
   return found;
 }
 
+// Whether an output overlaps one of those of the launches ahead; -1 after an error.
+int overlaps_any(PyObject* outputs, uintptr_t begin, uintptr_t end) {
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(outputs); ++i) {
+    PyObject* const other = PyTuple_GET_ITEM(outputs, i);
+    const uintptr_t from = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(other, 0)), to = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(other, 1));
+    if (PyErr_Occurred()) return -1;
+    if (begin < to && from < end) return 1;
+  }
+  return 0;
+}
+
 bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
   const c10::cuda::OptionalCUDAGuard guard(c10::cuda::current_device() == self->index ? c10::optional<c10::DeviceIndex>() : c10::optional<c10::DeviceIndex>(self->index));
   void* const stream = c10::cuda::getCurrentCUDAStream(self->index).stream();
@@ -63,7 +74,8 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
   void* const out_ptr = out.data_ptr();
   PyObject* index = PyLong_FromLong(self->index);
   PyObject* stream_key = PyLong_FromUnsignedLongLong(reinterpret_cast<uintptr_t>(stream));
-  PyObject *pair = nullptr, *here = nullptr, *buffer = nullptr;
+  PyObject *pair = nullptr, *here = nullptr, *buffer = nullptr, *outputs = nullptr;
+  const uintptr_t out_begin = reinterpret_cast<uintptr_t>(out_ptr), out_end = out_begin + static_cast<uintptr_t>(2 * self->rows * self->out_features);
   long slot = 0;
   bool ok = index && stream_key;
   if (ok && self->follows) {
@@ -77,8 +89,10 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
         const long in_a_row = PyLong_AsLong(PyTuple_GET_ITEM(entry, 1));
         if (in_a_row < PyTuple_GET_SIZE(self->families)) {
           const int same = PyObject_RichCompareBool(PyTuple_GET_ITEM(entry, 0), here, Py_EQ);
-          ok = same >= 0;
-          if (same == 1) slot = in_a_row;
+          // launches that overlap may not write to one place: the older one could be the last to do so
+          const int taken = same == 1 ? overlaps_any(PyTuple_GET_ITEM(entry, 2), out_begin, out_end) : 0;
+          ok = same >= 0 && taken >= 0;
+          if (same == 1 && taken == 0) slot = in_a_row, outputs = Py_NewRef(PyTuple_GET_ITEM(entry, 2));
         }
       }
       ok = ok && !PyErr_Occurred();
@@ -123,12 +137,14 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
       ok = false;
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "native call failed");
     } else if (self->follows && self->follow_flags) {
-      PyObject* entry = Py_BuildValue("(Ol)", here, slot + 1);
+      PyObject* mine = Py_BuildValue("((KK))", static_cast<unsigned long long>(out_begin), static_cast<unsigned long long>(out_end));
+      PyObject* all = mine && slot ? PySequence_Concat(outputs, mine) : Py_XNewRef(mine);
+      PyObject* entry = all ? Py_BuildValue("(OlO)", here, slot + 1, all) : nullptr;
       ok = entry && PyDict_SetItem(self->ahead, pair, entry) == 0;
-      Py_XDECREF(entry);
+      Py_XDECREF(entry), Py_XDECREF(all), Py_XDECREF(mine);
     }
   }
-  Py_XDECREF(buffer), Py_XDECREF(here), Py_XDECREF(pair), Py_XDECREF(stream_key), Py_XDECREF(index);
+  Py_XDECREF(outputs), Py_XDECREF(buffer), Py_XDECREF(here), Py_XDECREF(pair), Py_XDECREF(stream_key), Py_XDECREF(index);
   return ok;
 }
 
