@@ -67,6 +67,11 @@ int overlaps_any(PyObject* outputs, uintptr_t begin, uintptr_t end) {
   return 0;
 }
 
+// Launches under way, and how many there have been, under the GIL (a launch gives it up): one may follow the launch ahead, and be
+// remembered as that, only if no other thread's came between the look at `ahead` and the note in it.
+long under_way = 0;
+unsigned long long turns = 0;
+
 bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
   const c10::cuda::OptionalCUDAGuard guard(c10::cuda::current_device() == self->index ? c10::optional<c10::DeviceIndex>() : c10::optional<c10::DeviceIndex>(self->index));
   void* const stream = c10::cuda::getCurrentCUDAStream(self->index).stream();
@@ -84,7 +89,7 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
     here = address ? PyTuple_Pack(3, address, self->shape, self->dtype_object) : nullptr;
     Py_XDECREF(address);
     ok = pair && here;
-    if (ok && self->follow_flags) {
+    if (ok && self->follow_flags && under_way == 0) {
       if (PyObject* entry = PyDict_GetItemWithError(self->ahead, pair)) {
         const long in_a_row = PyLong_AsLong(PyTuple_GET_ITEM(entry, 1));
         if (in_a_row < PyTuple_GET_SIZE(self->families)) {
@@ -128,15 +133,18 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
     const size_t bytes = memory.nbytes();
     const unsigned flags = self->flags | (slot ? self->follow_flags : 0u);
     int code = 0;
+    const unsigned long long turn = ++turns;
+    ++under_way;
     Py_BEGIN_ALLOW_THREADS;
     code = self->run(self->handle, x_ptr, out_ptr, address, bytes, flags, stream);
     Py_END_ALLOW_THREADS;
+    const bool alone = --under_way == 0 && turn == turns;
     PyDict_Clear(self->ahead);
     if (code != 0) {
       Py_XDECREF(PyObject_CallFunction(self->failed, "i", code));
       ok = false;
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "native call failed");
-    } else if (self->follows && self->follow_flags) {
+    } else if (self->follows && self->follow_flags && alone) {
       PyObject* mine = Py_BuildValue("((KK))", static_cast<unsigned long long>(out_begin), static_cast<unsigned long long>(out_end));
       PyObject* all = mine && slot ? PySequence_Concat(outputs, mine) : Py_XNewRef(mine);
       PyObject* entry = all ? Py_BuildValue("(OlO)", here, slot + 1, all) : nullptr;
@@ -349,7 +357,17 @@ PyObject* holds(PyObject*, PyObject* const* args, Py_ssize_t count) {
   });
 }
 
-PyMethodDef module_methods[] = {{"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},
+// begin() -> (whether no launch is under way, turn); end(turn) -> whether none came in between: the same for a launch by ctypes
+PyObject* begin(PyObject*, PyObject*) {
+  const bool alone = under_way++ == 0;
+  return Py_BuildValue("(NK)", PyBool_FromLong(alone), ++turns);
+}
+PyObject* end(PyObject*, PyObject* turn) {
+  --under_way;
+  return PyBool_FromLong(under_way == 0 && PyLong_AsUnsignedLongLong(turn) == turns);
+}
+
+PyMethodDef module_methods[] = {{"begin", begin, METH_NOARGS, nullptr}, {"end", end, METH_O, nullptr}, {"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},
                                 {"holds", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(holds)), METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fb_calls", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
