@@ -186,8 +186,8 @@ def library() -> ctypes.CDLL:
     return _lib
 
 
-# The last call into the library per (device, stream), when it was a plain W3 GEMV launch: its activation
-# buffer, how many launches in a row have read it, and where these write.  Any other library call forgets it (see ``w3_gemv``).
+# The last call into the library per (device, stream), when it was a plain W3 GEMV launch: the row of launches on one
+# activation buffer that it ends (a ``Row`` of the extension), and how many these are.  Any other library call forgets it (see ``w3_gemv``).
 _same_input: dict = {}
 
 
@@ -305,22 +305,22 @@ _W3_SLOTS = ("w3", "w3#1", "w3#2")
 _NO_PDL, _NO_SAME_INPUT = bool(_os.environ.get("FB_NO_PDL")), bool(_os.environ.get("FB_NO_SAME_INPUT"))
 
 
-def _w3_slot(key, here, span) -> tuple:
+def _w3_slot(key, ahead, here) -> int:
     """Which of the three scratches the next plain W3 launch on ``key`` = (device, stream) uses; above 0 it follows a
-    launch on the same activations and need not wait for it.  Second: where the launches in that row write.
+    launch on the same activations and need not wait for it.
 
     Consecutive Linears on the SAME activations (k_proj and v_proj behind q_proj, up_proj behind gate_proj): the launch
     ahead is a W3 GEMV that read this very buffer, so the buffer was complete before that launch began and this one need
     not wait for it (FB_W3_SAME_INPUT).  Such launches may overlap, so each takes its own scratch (three rotate; a fourth
-    launch in a row waits again), and none may write (``span``: begin and end of the output) where another does.  Any other call into the library in between, a scratch chosen by the caller, or several
-    rows switch this off, and so do another thread's launch meanwhile and a capture on a stream whose next scratch no warm-up call has allocated."""
-    ahead = _same_input.get(key)
-    if ahead is None or ahead[1] >= 3 or ahead[0] != here or any(span[0] < end and begin < span[1] for begin, end in ahead[2]) or _NO_SAME_INPUT or _NO_PDL:
-        return 0, ()
-    slot = ahead[1]
-    if (*key, _W3_SLOTS[slot]) not in _scratch and torch.cuda.is_current_stream_capturing():
-        return 0, ()
-    return slot, ahead[2]
+    launch in a row waits again), and none may write where another does.  Any other call into the library in between,
+    another thread's launch meanwhile, a scratch chosen by the caller, or several rows switch this off, and so does a
+    capture on a stream whose next scratch no warm-up call has allocated."""
+    if ahead is None or _NO_SAME_INPUT or _NO_PDL:
+        return 0
+    slot = calls().place(ahead, *here)
+    if slot and (*key, _W3_SLOTS[slot]) not in _scratch and torch.cuda.is_current_stream_capturing():
+        return 0
+    return slot
 
 
 class Launch:
@@ -386,12 +386,13 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
     pdl = pdl and not _NO_PDL
     index = x.get_device()
     stream = _raw_stream(index)
-    key, here, span = (index, stream), (x.data_ptr(), (m, k), x.dtype), (out.data_ptr(), out.data_ptr() + 2 * m * o)
+    key, here = (index, stream), (x.data_ptr(), k, x.dtype, out.data_ptr(), out.data_ptr() + 2 * m * o)
     own_scratch = scratch is None
     follows = own_scratch and pdl and m == 1 and not group_partials
     alone, turn = calls().begin()
     try:
-        slot, outputs = _w3_slot(key, here, span) if follows and alone else (0, ())
+        ahead = _same_input.get(key)
+        slot = _w3_slot(key, ahead, here) if follows and alone else 0
         if own_scratch:
             scratch = scratch_for(x.device, w3_scratch_bytes(m, o, k), _W3_SLOTS[slot])
         flags = (FB_W3_DECODED_BF16 if decoded_bf16 else 0) | (0 if pdl else FB_W3_NO_PDL) | (
@@ -404,7 +405,7 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
     finally:
         clean = calls().end(turn)
     if follows and clean:
-        _same_input[key] = (here, slot + 1, (*outputs, span))
+        _same_input[key] = calls().row(ahead, slot, *here)
 
 
 def w3_finish(partials, out) -> None:

@@ -34,10 +34,9 @@ struct Call {
   bool follows;                  // a launch that may follow another on the same activations, or be followed
   size_t need;
   PyObject* dtype_object;
-  PyObject* shape;       // (1, in_features)
   PyObject* families;    // scratch families: the one, or the three that rotate
   PyObject* scratch;     // dict (index, stream, family) -> tensor
-  PyObject* ahead;       // dict (index, stream) -> ((address, shape, dtype), launches in a row, ((output's begin, end), ...) of these)
+  PyObject* ahead;       // dict (index, stream) -> (Row, launches in it)
   PyObject* scratch_for; // (device index, bytes, family) -> tensor
   PyObject* capturing;   // () -> bool
   PyObject* failed;      // raises the error of a refused launch
@@ -56,16 +55,36 @@ PyObject* scratch_at(Call* self, PyObject* index, PyObject* stream, PyObject* fa
   return found;
 }
 
-// Whether an output overlaps one of those of the launches ahead; -1 after an error.
-int overlaps_any(PyObject* outputs, uintptr_t begin, uintptr_t end) {
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(outputs); ++i) {
-    PyObject* const other = PyTuple_GET_ITEM(outputs, i);
-    const uintptr_t from = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(other, 0)), to = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(other, 1));
-    if (PyErr_Occurred()) return -1;
-    if (begin < to && from < end) return 1;
+constexpr int kMostInARow = 3;
+
+// Launches one after the other on the same activations: which, and where each of them writes.  Kept as bytes: a call on a
+// prepared launch compares and makes one, and as Python objects that took 0.3 us.
+struct Row {
+  uint64_t x = 0, k = 0, dtype = 0, launches = 0, outputs[kMostInARow][2] = {};
+
+  // Which place a launch takes in the row; 0: it does not belong to it.  Launches of a row overlap and may not write to one place:
+  // the older one could be the last to do so.
+  long place(uint64_t x_, uint64_t k_, c10::ScalarType dtype_, uint64_t begin, uint64_t end) const {
+    if (launches >= kMostInARow || x != x_ || k != k_ || dtype != static_cast<uint64_t>(dtype_)) return 0;
+    for (uint64_t i = 0; i < launches; ++i)
+      if (begin < outputs[i][1] && outputs[i][0] < end) return 0;
+    return static_cast<long>(launches);
   }
-  return 0;
-}
+  // ... and the row with it; place 0 begins one.
+  Row with(long place, uint64_t x_, uint64_t k_, c10::ScalarType dtype_, uint64_t begin, uint64_t end) const {
+    Row row = place ? *this : Row();
+    row.x = x_, row.k = k_, row.dtype = static_cast<uint64_t>(dtype_);
+    row.outputs[row.launches][0] = begin, row.outputs[row.launches][1] = end, ++row.launches;
+    return row;
+  }
+  // of an entry of `ahead` (null, or None: an empty one)
+  static Row of(PyObject* entry) {
+    Row row;
+    if (entry && entry != Py_None) memcpy(&row, PyBytes_AS_STRING(PyTuple_GET_ITEM(entry, 0)), sizeof row);
+    return row;
+  }
+  PyObject* entry() const { return Py_BuildValue("(y#l)", reinterpret_cast<const char*>(this), static_cast<Py_ssize_t>(sizeof *this), static_cast<long>(launches)); }
+};
 
 // Launches under way, and how many there have been, under the GIL (a launch gives it up): one may follow the launch ahead, and be
 // remembered as that, only if no other thread's came between the look at `ahead` and the note in it.
@@ -79,28 +98,18 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
   void* const out_ptr = out.data_ptr();
   PyObject* index = PyLong_FromLong(self->index);
   PyObject* stream_key = PyLong_FromUnsignedLongLong(reinterpret_cast<uintptr_t>(stream));
-  PyObject *pair = nullptr, *here = nullptr, *buffer = nullptr, *outputs = nullptr;
-  const uintptr_t out_begin = reinterpret_cast<uintptr_t>(out_ptr), out_end = out_begin + static_cast<uintptr_t>(2 * self->rows * self->out_features);
+  PyObject *pair = nullptr, *buffer = nullptr;
+  const uint64_t x_at = reinterpret_cast<uintptr_t>(x_ptr), out_begin = reinterpret_cast<uintptr_t>(out_ptr), out_end = out_begin + 2 * self->rows * self->out_features;
+  Row row;
   long slot = 0;
   bool ok = index && stream_key;
   if (ok && self->follows) {
     pair = key_of(index, stream_key, nullptr);
-    PyObject* address = PyLong_FromUnsignedLongLong(reinterpret_cast<uintptr_t>(x_ptr));
-    here = address ? PyTuple_Pack(3, address, self->shape, self->dtype_object) : nullptr;
-    Py_XDECREF(address);
-    ok = pair && here;
+    ok = pair != nullptr;
     if (ok && self->follow_flags && under_way == 0) {
-      if (PyObject* entry = PyDict_GetItemWithError(self->ahead, pair)) {
-        const long in_a_row = PyLong_AsLong(PyTuple_GET_ITEM(entry, 1));
-        if (in_a_row < PyTuple_GET_SIZE(self->families)) {
-          const int same = PyObject_RichCompareBool(PyTuple_GET_ITEM(entry, 0), here, Py_EQ);
-          // launches that overlap may not write to one place: the older one could be the last to do so
-          const int taken = same == 1 ? overlaps_any(PyTuple_GET_ITEM(entry, 2), out_begin, out_end) : 0;
-          ok = same >= 0 && taken >= 0;
-          if (same == 1 && taken == 0) slot = in_a_row, outputs = Py_NewRef(PyTuple_GET_ITEM(entry, 2));
-        }
-      }
-      ok = ok && !PyErr_Occurred();
+      row = Row::of(PyDict_GetItemWithError(self->ahead, pair));
+      ok = !PyErr_Occurred();
+      slot = row.place(x_at, self->in_features, self->dtype, out_begin, out_end);
     }
   }
   if (ok) {
@@ -145,14 +154,12 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
       ok = false;
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "native call failed");
     } else if (self->follows && self->follow_flags && alone) {
-      PyObject* mine = Py_BuildValue("((KK))", static_cast<unsigned long long>(out_begin), static_cast<unsigned long long>(out_end));
-      PyObject* all = mine && slot ? PySequence_Concat(outputs, mine) : Py_XNewRef(mine);
-      PyObject* entry = all ? Py_BuildValue("(OlO)", here, slot + 1, all) : nullptr;
+      PyObject* entry = row.with(slot, x_at, self->in_features, self->dtype, out_begin, out_end).entry();
       ok = entry && PyDict_SetItem(self->ahead, pair, entry) == 0;
-      Py_XDECREF(entry), Py_XDECREF(all), Py_XDECREF(mine);
+      Py_XDECREF(entry);
     }
   }
-  Py_XDECREF(outputs), Py_XDECREF(buffer), Py_XDECREF(here), Py_XDECREF(pair), Py_XDECREF(stream_key), Py_XDECREF(index);
+  Py_XDECREF(buffer), Py_XDECREF(pair), Py_XDECREF(stream_key), Py_XDECREF(index);
   return ok;
 }
 
@@ -214,13 +221,12 @@ int call_init(PyObject* object, PyObject* args, PyObject*) {
   self->rows = rows, self->in_features = in_features, self->out_features = out_features;
   self->need = static_cast<size_t>(need), self->follows = follows != 0;
   self->dtype = reinterpret_cast<THPDtype*>(self->dtype_object)->scalar_type;
-  self->shape = Py_BuildValue("(iL)", 1, in_features);
-  return self->shape ? 0 : -1;
+  return self->follows && PyTuple_GET_SIZE(self->families) != kMostInARow ? (PyErr_SetString(PyExc_ValueError, "a launch that follows takes three scratches"), -1) : 0;
 }
 
 void call_dealloc(PyObject* object) {
   auto* self = reinterpret_cast<Call*>(object);
-  for (PyObject* held : {self->dtype_object, self->shape, self->families, self->scratch, self->ahead, self->scratch_for, self->capturing, self->failed}) Py_XDECREF(held);
+  for (PyObject* held : {self->dtype_object, self->families, self->scratch, self->ahead, self->scratch_for, self->capturing, self->failed}) Py_XDECREF(held);
   Py_TYPE(object)->tp_free(object);
 }
 
@@ -367,7 +373,22 @@ PyObject* end(PyObject*, PyObject* turn) {
   return PyBool_FromLong(under_way == 0 && PyLong_AsUnsignedLongLong(turn) == turns);
 }
 
-PyMethodDef module_methods[] = {{"begin", begin, METH_NOARGS, nullptr}, {"end", end, METH_O, nullptr}, {"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},
+// place(entry, x address, K, dtype, output's begin, end) and row(entry, place, the same): for a launch by ctypes
+PyObject* place(PyObject*, PyObject* args) {
+  PyObject *entry, *dtype;
+  unsigned long long x, k, begin, end;
+  if (!PyArg_ParseTuple(args, "OKKOKK", &entry, &x, &k, &dtype, &begin, &end)) return nullptr;
+  return PyLong_FromLong(Row::of(entry).place(x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, begin, end));
+}
+PyObject* row_with(PyObject*, PyObject* args) {
+  PyObject *entry, *dtype;
+  long at;
+  unsigned long long x, k, begin, end;
+  if (!PyArg_ParseTuple(args, "OlKKOKK", &entry, &at, &x, &k, &dtype, &begin, &end)) return nullptr;
+  return Row::of(entry).with(at, x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, begin, end).entry();
+}
+
+PyMethodDef module_methods[] = {{"place", place, METH_VARARGS, nullptr}, {"row", row_with, METH_VARARGS, nullptr}, {"begin", begin, METH_NOARGS, nullptr}, {"end", end, METH_O, nullptr}, {"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},
                                 {"holds", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(holds)), METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fb_calls", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
