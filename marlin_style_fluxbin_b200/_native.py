@@ -386,7 +386,7 @@ def w3_gemv(x, planes, scales, zeros, perm, out, *, decoded_bf16=False, group_pa
     pdl = pdl and not _NO_PDL
     index = x.get_device()
     stream = _raw_stream(index)
-    key, here = (index, stream), (x.data_ptr(), k, x.dtype, out.data_ptr(), out.data_ptr() + 2 * m * o)
+    key, here = (index, stream), (x.data_ptr(), k, x.dtype, torch.cuda.is_current_stream_capturing(), out.data_ptr(), out.data_ptr() + 2 * m * o)
     own_scratch = scratch is None
     follows = own_scratch and pdl and m == 1 and not group_partials
     alone, turn = calls().begin()

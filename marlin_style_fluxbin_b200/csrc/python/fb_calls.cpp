@@ -12,6 +12,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -57,23 +58,24 @@ PyObject* scratch_at(Call* self, PyObject* index, PyObject* stream, PyObject* fa
 
 constexpr int kMostInARow = 3;
 
-// Launches one after the other on the same activations: which, and where each of them writes.  Kept as bytes: a call on a
+// Launches one after the other on the same activations: which, and where each of them writes; all captured or all eager,
+// since one kind is not ahead of the other.  Kept as bytes: a call on a
 // prepared launch compares and makes one, and as Python objects that took 0.3 us.
 struct Row {
-  uint64_t x = 0, k = 0, dtype = 0, launches = 0, outputs[kMostInARow][2] = {};
+  uint64_t x = 0, k = 0, dtype = 0, captured = 0, launches = 0, outputs[kMostInARow][2] = {};
 
   // Which place a launch takes in the row; 0: it does not belong to it.  Launches of a row overlap and may not write to one place:
   // the older one could be the last to do so.
-  long place(uint64_t x_, uint64_t k_, c10::ScalarType dtype_, uint64_t begin, uint64_t end) const {
-    if (launches >= kMostInARow || x != x_ || k != k_ || dtype != static_cast<uint64_t>(dtype_)) return 0;
+  long place(uint64_t x_, uint64_t k_, c10::ScalarType dtype_, bool captured_, uint64_t begin, uint64_t end) const {
+    if (launches >= kMostInARow || x != x_ || k != k_ || dtype != static_cast<uint64_t>(dtype_) || captured != captured_) return 0;
     for (uint64_t i = 0; i < launches; ++i)
       if (begin < outputs[i][1] && outputs[i][0] < end) return 0;
     return static_cast<long>(launches);
   }
   // ... and the row with it; place 0 begins one.
-  Row with(long place, uint64_t x_, uint64_t k_, c10::ScalarType dtype_, uint64_t begin, uint64_t end) const {
+  Row with(long place, uint64_t x_, uint64_t k_, c10::ScalarType dtype_, bool captured_, uint64_t begin, uint64_t end) const {
     Row row = place ? *this : Row();
-    row.x = x_, row.k = k_, row.dtype = static_cast<uint64_t>(dtype_);
+    row.x = x_, row.k = k_, row.dtype = static_cast<uint64_t>(dtype_), row.captured = captured_;
     row.outputs[row.launches][0] = begin, row.outputs[row.launches][1] = end, ++row.launches;
     return row;
   }
@@ -83,7 +85,12 @@ struct Row {
     if (entry && entry != Py_None) memcpy(&row, PyBytes_AS_STRING(PyTuple_GET_ITEM(entry, 0)), sizeof row);
     return row;
   }
-  PyObject* entry() const { return Py_BuildValue("(y#l)", reinterpret_cast<const char*>(this), static_cast<Py_ssize_t>(sizeof *this), static_cast<long>(launches)); }
+  PyObject* entry() const {
+    PyObject *bytes = PyBytes_FromStringAndSize(reinterpret_cast<const char*>(this), sizeof *this), *count = PyLong_FromLong(static_cast<long>(launches));
+    PyObject* made = bytes && count ? PyTuple_Pack(2, bytes, count) : nullptr;
+    Py_XDECREF(count), Py_XDECREF(bytes);
+    return made;
+  }
 };
 
 // Launches under way, and how many there have been, under the GIL (a launch gives it up): one may follow the launch ahead, and be
@@ -101,15 +108,17 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
   PyObject *pair = nullptr, *buffer = nullptr;
   const uint64_t x_at = reinterpret_cast<uintptr_t>(x_ptr), out_begin = reinterpret_cast<uintptr_t>(out_ptr), out_end = out_begin + 2 * self->rows * self->out_features;
   Row row;
+  bool captured = false;
   long slot = 0;
   bool ok = index && stream_key;
   if (ok && self->follows) {
+    captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     pair = key_of(index, stream_key, nullptr);
     ok = pair != nullptr;
     if (ok && self->follow_flags && under_way == 0) {
       row = Row::of(PyDict_GetItemWithError(self->ahead, pair));
       ok = !PyErr_Occurred();
-      slot = row.place(x_at, self->in_features, self->dtype, out_begin, out_end);
+      slot = row.place(x_at, self->in_features, self->dtype, captured, out_begin, out_end);
     }
   }
   if (ok) {
@@ -154,7 +163,7 @@ bool run_call(Call* self, const at::Tensor& x, const at::Tensor& out) {
       ok = false;
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "native call failed");
     } else if (self->follows && self->follow_flags && alone) {
-      PyObject* entry = row.with(slot, x_at, self->in_features, self->dtype, out_begin, out_end).entry();
+      PyObject* entry = row.with(slot, x_at, self->in_features, self->dtype, captured, out_begin, out_end).entry();
       ok = entry && PyDict_SetItem(self->ahead, pair, entry) == 0;
       Py_XDECREF(entry);
     }
@@ -373,19 +382,21 @@ PyObject* end(PyObject*, PyObject* turn) {
   return PyBool_FromLong(under_way == 0 && PyLong_AsUnsignedLongLong(turn) == turns);
 }
 
-// place(entry, x address, K, dtype, output's begin, end) and row(entry, place, the same): for a launch by ctypes
+// place(entry, x address, K, dtype, captured, output's begin, end) and row(entry, place, the same): for a launch by ctypes
 PyObject* place(PyObject*, PyObject* args) {
   PyObject *entry, *dtype;
   unsigned long long x, k, begin, end;
-  if (!PyArg_ParseTuple(args, "OKKOKK", &entry, &x, &k, &dtype, &begin, &end)) return nullptr;
-  return PyLong_FromLong(Row::of(entry).place(x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, begin, end));
+  int captured;
+  if (!PyArg_ParseTuple(args, "OKKOpKK", &entry, &x, &k, &dtype, &captured, &begin, &end)) return nullptr;
+  return PyLong_FromLong(Row::of(entry).place(x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, captured != 0, begin, end));
 }
 PyObject* row_with(PyObject*, PyObject* args) {
   PyObject *entry, *dtype;
   long at;
   unsigned long long x, k, begin, end;
-  if (!PyArg_ParseTuple(args, "OlKKOKK", &entry, &at, &x, &k, &dtype, &begin, &end)) return nullptr;
-  return Row::of(entry).with(at, x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, begin, end).entry();
+  int captured;
+  if (!PyArg_ParseTuple(args, "OlKKOpKK", &entry, &at, &x, &k, &dtype, &captured, &begin, &end)) return nullptr;
+  return Row::of(entry).with(at, x, k, reinterpret_cast<THPDtype*>(dtype)->scalar_type, captured != 0, begin, end).entry();
 }
 
 PyMethodDef module_methods[] = {{"place", place, METH_VARARGS, nullptr}, {"row", row_with, METH_VARARGS, nullptr}, {"begin", begin, METH_NOARGS, nullptr}, {"end", end, METH_O, nullptr}, {"stamp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stamp)), METH_FASTCALL, nullptr},

@@ -83,3 +83,21 @@ def test_a_launch_during_another_threads_launch_waits():
     scratches, flags = zip(*recorded.seen)
     assert [bool(f) for f in flags] == [False, True, False, False, True]
     assert scratches[2] != scratches[1] and scratches[4] != scratches[3]
+
+
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+def test_a_capture_and_eager_launches_do_not_follow_one_another():
+    recorded = _Recorded()
+    x = torch.zeros(1, 640, device="cuda", dtype=torch.bfloat16)
+    outs = [torch.empty(1, 96, device="cuda", dtype=torch.bfloat16) for _ in range(6)]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        recorded.call.run(x, outs[0])
+        recorded.call.run(x, outs[1])
+        stream.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            recorded.call.run(x, outs[2])  # nothing is ahead of it in the graph
+            recorded.call.run(x, outs[3])
+        recorded.call.run(x, outs[4])  # the captured ones have not run
+        recorded.call.run(x, outs[5])
+    assert [bool(flags) for _, flags in recorded.seen] == [False, True] * 3
