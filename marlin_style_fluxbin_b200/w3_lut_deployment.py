@@ -407,8 +407,10 @@ def dense_linear(x, layout, bias=None):
         target = y[:, begin:begin + count]
         if bias is None:
             torch.mm(x, weight[:count].t(), out=target)
-        else:
-            torch.addmm(bias[begin:begin + count], x, weight[:count].t(), out=target)
+        elif count == out_features:
+            torch.addmm(bias, x, weight.t(), out=y)
+        else:  # into columns of a wider output the library rounds the product before it adds (error 2.3e-3 against 1.7e-3)
+            target.copy_(F.linear(x, weight[:count], bias[begin:begin + count]))
     return y
 
 
