@@ -19,6 +19,7 @@ def _near(got, want):
     return float((got.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())
 
 
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning", "ignore::DeprecationWarning")
 @pytest.mark.parametrize("rows", (5, 20))
 def test_transforms_see_the_product(rows):
     module, x = _module(), torch.randn(2, rows, 256, device="cuda").bfloat16()

@@ -2,9 +2,13 @@
 import pytest
 import torch
 
+from marlin_style_fluxbin_b200 import _native
 from marlin_style_fluxbin_b200.gptq_deployment import (
     convert_gptq_w3_to_planar, planes_from_sorted_codes, unpack_gptq_w3_qweight, unpack_gptq_w3_qzeros,
 )
+
+# without the library the tensor form would be compared with itself
+pytestmark = pytest.mark.skipif(not _native.LIBRARY.exists(), reason="not built")
 
 
 @pytest.mark.parametrize("o,k,desc_act", ((32, 128, False), (96, 640, True), (160, 256, True), (2048, 1024, True)))
@@ -23,10 +27,6 @@ def test_native_conversion_equals_the_tensor_form(o, k, desc_act):
 
 
 def test_column_orders_beyond_int16_are_refused():
-    from marlin_style_fluxbin_b200 import _native
-
-    if not _native.LIBRARY.exists():
-        pytest.skip("not built")
     groups, order = (torch.arange(65536) // 128).to(torch.int32), torch.zeros(65536, dtype=torch.int64)
     assert _native.library().fb_host_w3_order(groups.data_ptr(), 65536, order.data_ptr()) == -2  # FB_ELIMIT
     assert not bool(order.any())
