@@ -267,8 +267,8 @@ def status_word(device: torch.device | None = None) -> int:
 
 def check_status(device: torch.device | None = None) -> None:
     """Synchronise and raise if a bounded device-side wait expired in any kernel that used a scratch
-    handed out by ``scratch_for`` (status word 1: W3 GEMV staging, 3: tensor-core kernel); the scratch
-    is re-zeroed, the results of the calls since the last check are invalid."""
+    handed out by ``scratch_for`` (status word 1: a staging copy of the one-row, several-row or two-base
+    kernel, or a sum that did not cross its cluster, 3: many-row kernel); the scratch is re-zeroed, the results of the calls since the last check are invalid."""
     torch.cuda.synchronize(device)
     bad = {}
     for key, buf in _scratch.items():

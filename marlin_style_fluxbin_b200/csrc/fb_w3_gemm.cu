@@ -18,9 +18,12 @@
 // activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes.
 //
 // What bounds it: up to about 100 tokens a tile the integer instructions of the look-ups (some 800 clocks per
-// 128 x 128 weights), at 256 the MMA (1300 TFLOP/s where the tiles fill the SMs).  us on a B200, weights cold, chunks
-// -> this, without the launches' host time: 12288 x 4096 at 64 / 512 / 1024 tokens 40 / 62 / 95 -> 22 / 49 / 90,
-// 24576 x 4096 at 512 119 -> 88, 4096 x 12288 at 512 / 1024 71 / 98 -> 54 / 78.
+// 128 x 128 weights), at 256 the MMA (1370 TFLOP/s where the tiles fill the SMs).  us on a B200, weights cold, in a graph, chunks
+// -> this: 12288 x 4096 at 64 / 512 / 1024 tokens 39 / 63 / 92 -> 19 / 46 / 81, 24576 x 4096 at 512 126 -> 82,
+// 4096 x 12288 at 512 / 1024 72 / 96 -> 54 / 75.
+//
+// A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
+// the CTA ends; it leaves with the status word set and the tensor memory freed.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 

@@ -6,8 +6,8 @@
 // tcgen05.mma needs its operand in shared memory: expanding the weights into it took 3300 instructions and
 // as many shared-memory wavefronts per 128 x 128 tile.  This one takes no trip through shared memory.
 // us on a B200, cold weights (before: tcgen05 form from five rows on, tables below), at 4 / 16 rows:
-// 1024 x 4096 3.8 / 4.6 (8.3 / 10.5), 4096 x 4096 5.6 / 7.1 (10.1 / 11.4), 12288 x 4096 11.1 / 13.4 (22.4 / 22.5),
-// 4096 x 12288 11.5 / 14.5 (24.7 / 22.5).
+// 1024 x 4096 3.6 / 4.3 (8.3 / 10.5), 4096 x 4096 5.5 / 6.8 (10.1 / 11.4), 12288 x 4096 11.0 / 13.4 (22.4 / 22.5),
+// 4096 x 12288 11.5 / 14.4 (24.7 / 22.5).
 //
 //  * The three planes of a group become operands of mma.sync.m16n8k16 in registers, without a table.  Two
 //    bit-selects per word interleave them into 3-bit fields; a field inside the ten mantissa bits of an

@@ -29,8 +29,10 @@ DENSE_CHUNK_BYTES = 52 << 20
 
 def fused_gemm_pays(rows: int, out_features: int) -> bool:
     """Whether ``rows`` activation rows go through the kernel that dequantises into tensor memory rather than through dense
-    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy (1024 x 4096: 24 us against 14, at
-    4096 x 4096 they meet); beyond a thousand rows the chunks, dequantised once for all of them, catch up."""
+    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy: 512 rows, in a graph, weights cold,
+    1024 x 4096 19 us against 14; with the L2 flushed 2048 x 4096 25 / 26, 2048 x 12288 53 / 46, 3072 x 12288 57 / 71, 4096 x 4096
+    29 / 32.  Beyond a thousand rows the chunks, dequantised once for all of them, catch up: 2048 rows of 12288 x 1024 70 / 60, of
+    12288 x 4096 164 / 175."""
     return rows <= 1024 and out_features > 2048 and out_features % 32 == 0
 
 ROW_TILES = (256, 512, 1024)
@@ -349,8 +351,8 @@ def w3_lut_gemv_out(x, layout, out, *, arithmetic: str = "structural", kernel: s
 
     ``kernel``: ``"lut"`` is the table-lookup kernel (M <= 4, cost grows with M), ``"mma"`` the
     tensor-core kernel (M <= 16, cost hardly grows with M; weights are not rounded).  ``"auto"`` picks
-    ``"lut"`` for one row (4096 x 4096: 3.8 us against 5.5) and for the dequantised-weight arithmetic, which
-    only that kernel has, and ``"mma"`` from two rows on (two rows: 5.5 us against 5.9, four: 5.6 against 10.1).
+    ``"lut"`` for one row (4096 x 4096: 3.8 us against 5.1) and for the dequantised-weight arithmetic, which
+    only that kernel has, and ``"mma"`` from two rows on (two rows: 5.1 us against 5.6, four: 5.3 against 9.3).
     """
     record = _layout_record(layout)
     recent = record.recent
@@ -539,7 +541,7 @@ class PackedW3Linear(nn.Module):
                 and x.numel() == self.in_features and x.get_device() == self._decode_output.get_device())
 
     def add_to(self, residual: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
-        """``residual + self(x)`` for one token in one launch, the sum rounded once."""
+        """``residual + self(x)`` for one token in one launch, with the roundings of the two steps."""
         if self._decode_audit:
             self.route_counts["packed_m1"] += 1
             self.last_route = "packed_m1"
