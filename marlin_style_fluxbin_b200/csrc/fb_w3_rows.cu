@@ -328,11 +328,15 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
     if (live && (lane & 7) == 0) outliers[g * M + m].k = -1;
     if (__any_sync(0xffffffffu, ours)) {  // rare
       __syncwarp();
-      int large = 0;
+      int large = 0, nonzero = 0;  // one value by itself needs no separate sum: nothing is rounded beside it
+#pragma unroll
+      for (int j = 0; j < 16; ++j) nonzero += v[j] != 0.f;
+#pragma unroll
+      for (int d = 4; d >= 1; d >>= 1) nonzero += __shfl_xor_sync(0xffffffffu, nonzero, d);
       top = 0.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const bool out = ours && (wild ? !(fabsf(v[j]) <= 3.4028235e38f) : fabsf(v[j]) == all_top);
+        const bool out = ours && (wild || nonzero > 1) && (wild ? !(fabsf(v[j]) <= 3.4028235e38f) : fabsf(v[j]) == all_top);
         if (out) {
           ++large;
           if (live) outliers[g * M + m].k = k_in_group + (j & 7) + (j >> 3) * 16, outliers[g * M + m].x = v[j], any_out = 1;
