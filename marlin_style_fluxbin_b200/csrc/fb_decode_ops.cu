@@ -361,6 +361,282 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_kernel(const unsi
   if (!CLUSTER && lane == 0) tickets[head] = 0u;
 }
 
+// Long caches, grouped-query heads: a CTA serves TWO query heads of a k/v head, so that a cache row crosses the L2 half as
+// often (the first kernel reads each once per query head: 67 MB of L2 traffic at 4096 positions of the 8B shape), and eight lanes share a
+// position, sixteen dims each: three shuffle steps for a score instead of five, rows unpacked once for both heads, products
+// two at a time (packed fp32).  Four positions per lane are in flight; the next keys are requested as soon as the scores are
+// formed, the next values after the sums.  What bounds it: the round trips of the four batches of a CTA.
+// us of a launch, rows cold (32 query heads over 8; 4 over 2), first kernel -> this: 641 positions 4.40 -> 3.84; 3.64 -> 3.02,
+// 1200 5.27 -> 5.02; 4.10 -> 4.25, 2048 8.70 -> 5.89; 7.04 -> 4.87, 4096 14.1 -> 8.6; 11.7 -> 7.8.  Up to 640 positions the first kernel
+// has a single round, whose chains are shorter (512: 3.48).
+// FUSED, PARTIAL and the merge over the splits as there; without PARTIAL the splits form a cluster.
+constexpr int kLongHeads = 2, kLongBatch = 4, kLongFrom = 640;
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+template <int ACT>
+__device__ __forceinline__ uint64_t widen2(uint32_t two) {  // two 16-bit values
+  if (ACT == FB_BF16) return pack2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u));
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+  return pack2(f.x, f.y);
+}
+
+template <bool FUSED, bool PARTIAL, int ACT>
+__global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const unsigned short* __restrict__ q, unsigned short* __restrict__ k_cache,
+                                                                    unsigned short* __restrict__ v_cache, unsigned short* __restrict__ out,
+                                                                    float* __restrict__ scratch, int q_heads, int kv_heads, int length,
+                                                                    int max_positions, float scale, const NewToken nt) {
+  constexpr int D = 128;
+  const int split = blockIdx.y, splits = gridDim.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = q_heads / kv_heads, pairs = (group + kLongHeads - 1) / kLongHeads, kvh = blockIdx.x / pairs;
+  const int head0 = kvh * group + kLongHeads * (blockIdx.x - kvh * pairs);
+  const int heads = min(kLongHeads, (kvh + 1) * group - head0);  // an odd group leaves the last CTA one
+  // lane = (position of four, eighth of the dims: eight from 8 part and eight from 64 + 8 part)
+  const int of = lane >> 3, part = lane & 7;
+  const unsigned short* kbase = k_cache + (size_t)kvh * max_positions * D + part * 8;
+  const unsigned short* vbase = v_cache + (size_t)kvh * max_positions * D + part * 8;
+  const int chunk = (length + splits - 1) / splits;
+  const int p0 = split * chunk, p1 = min(length, p0 + chunk);
+  const int newest = length - 1;
+  if (!PARTIAL) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  __shared__ __align__(16) unsigned short sm_new[kLongHeads + 2][D];  // rotated q of the heads, rotated k, v of the new token
+  constexpr int kStep = kAttnWarps * 4;                               // positions of a step of the CTA
+  uint4 kr[kLongBatch][2], vr[kLongBatch][2];
+  auto fetch = [&](const unsigned short* rows, int first, uint4 (&to)[kLongBatch][2]) {  // first: this lane's first position
+#pragma unroll
+    for (int j = 0; j < kLongBatch; ++j) {
+      const int pos = min(first + j * kStep, p1 - 1);
+      to[j][0] = to[j][1] = make_uint4(0u, 0u, 0u, 0u);
+      if (first < p1 && !(FUSED && pos == newest)) {
+        to[j][0] = *reinterpret_cast<const uint4*>(rows + (size_t)pos * D);
+        to[j][1] = *reinterpret_cast<const uint4*>(rows + (size_t)pos * D + 64);
+      }
+    }
+  };
+  const int mine = p0 + warp * 4 + of;
+  HeadConstants hc = {};
+  if (FUSED) {  // constants and rows of earlier positions ahead of the wait, ordered as in the kernel above
+    if (warp <= kLongHeads) hc = load_head_constants(warp < kLongHeads ? nt.q_weight : nt.k_weight, nt.cosv, nt.sinv, ACT, lane);
+    fetch(kbase, mine, kr);
+    fetch(vbase, mine, vr);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (FUSED) {
+    if (warp < kLongHeads)
+      norm_rope_head(nt.q + (size_t)(head0 + min(warp, heads - 1)) * D, hc, nt.eps, ACT, lane, sm_new[warp]);
+    else if (warp == kLongHeads)
+      norm_rope_head(nt.k + (size_t)kvh * D, hc, nt.eps, ACT, lane, sm_new[kLongHeads]);
+    else if (warp == kLongHeads + 1)
+      *reinterpret_cast<uint2*>(&sm_new[kLongHeads + 1][lane * 4]) = *reinterpret_cast<const uint2*>(nt.v + (size_t)kvh * D + lane * 4);
+  } else {
+    fetch(kbase, mine, kr);
+    fetch(vbase, mine, vr);
+    if (warp < kLongHeads) *reinterpret_cast<uint2*>(&sm_new[warp][lane * 4]) = *reinterpret_cast<const uint2*>(q + (size_t)(head0 + min(warp, heads - 1)) * D + lane * 4);
+  }
+  __syncthreads();
+  if (FUSED && head0 == kvh * group && split == splits - 1 && warp < 2) {  // the cache row of the new token
+    unsigned short* row = (warp == 0 ? k_cache : v_cache) + ((size_t)kvh * max_positions + newest) * D;
+    *reinterpret_cast<uint2*>(row + lane * 4) = *reinterpret_cast<const uint2*>(&sm_new[kLongHeads + warp][lane * 4]);
+  }
+  uint64_t qv[kLongHeads][8], acc[kLongHeads][8];
+  float m[kLongHeads], l[kLongHeads];
+  const uint64_t scale2 = pack2(scale, scale);
+#pragma unroll
+  for (int h = 0; h < kLongHeads; ++h) {
+    m[h] = -INFINITY, l[h] = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(&sm_new[h][half * 64 + part * 8]);
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) qv[h][half * 4 + i] = mul2(widen2<ACT>(w[i]), scale2), acc[h][half * 4 + i] = 0ull;
+    }
+  }
+  // all warps take as many batches; lanes without a position in one add nothing
+  for (int base = p0; base < p1; base += kStep * kLongBatch) {
+    const int first = base + warp * 4 + of, next = first + kStep * kLongBatch;
+    if (FUSED) {
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j)
+        if (first + j * kStep == newest) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            kr[j][half] = *reinterpret_cast<const uint4*>(&sm_new[kLongHeads][half * 64 + part * 8]);
+            vr[j][half] = *reinterpret_cast<const uint4*>(&sm_new[kLongHeads + 1][half * 64 + part * 8]);
+          }
+        }
+    }
+    float s[kLongBatch][kLongHeads];
+#pragma unroll
+    for (int j = 0; j < kLongBatch; ++j) {
+      if (base + j * kStep >= p1) {  // no lane has this position of the last batch
+        s[j][0] = s[j][1] = 0.f;
+        continue;
+      }
+      uint64_t dot[kLongHeads] = {};
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t w[4] = {kr[j][half].x, kr[j][half].y, kr[j][half].z, kr[j][half].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t key = widen2<ACT>(w[i]);
+#pragma unroll
+          for (int h = 0; h < kLongHeads; ++h) dot[h] = fma2(key, qv[h][half * 4 + i], dot[h]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < kLongHeads; ++h) {
+        float lo, hi;
+        unpack2(dot[h], lo, hi);
+        s[j][h] = lo + hi;
+      }
+    }
+    fetch(kbase, next, kr);
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1)
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j)
+#pragma unroll
+        for (int h = 0; h < kLongHeads; ++h) s[j][h] += __shfl_xor_sync(0xffffffffu, s[j][h], d);
+#pragma unroll
+    for (int h = 0; h < kLongHeads; ++h) {
+      float top = m[h];
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j)
+        if (first + j * kStep < p1) top = fmaxf(top, s[j][h]);
+      const float safe = top == -INFINITY ? 0.f : top;  // a lane group without a position so far
+      const float correction = __expf(m[h] - safe);
+      l[h] *= correction;
+      const uint64_t c2 = pack2(correction, correction);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[h][i] = mul2(acc[h][i], c2);
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j) {
+        s[j][h] = first + j * kStep < p1 ? __expf(s[j][h] - safe) : 0.f;
+        l[h] += s[j][h];
+      }
+      m[h] = top;
+    }
+#pragma unroll
+    for (int j = 0; j < kLongBatch; ++j) {
+      if (base + j * kStep >= p1) continue;
+      uint64_t p2[kLongHeads];
+#pragma unroll
+      for (int h = 0; h < kLongHeads; ++h) p2[h] = pack2(s[j][h], s[j][h]);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t w[4] = {vr[j][half].x, vr[j][half].y, vr[j][half].z, vr[j][half].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t value = widen2<ACT>(w[i]);
+#pragma unroll
+          for (int h = 0; h < kLongHeads; ++h) acc[h][half * 4 + i] = fma2(value, p2[h], acc[h][half * 4 + i]);
+        }
+      }
+    }
+    fetch(vbase, next, vr);
+  }
+  // the four positions of a warp, then the warps, then the splits
+  __shared__ float sm_m[kLongHeads][kAttnWarps], sm_l[kLongHeads][kAttnWarps];
+  __shared__ __align__(16) float sm_acc[kLongHeads][kAttnWarps][D];
+#pragma unroll
+  for (int h = 0; h < kLongHeads; ++h) {
+    float top = fmaxf(m[h], __shfl_xor_sync(0xffffffffu, m[h], 8));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+    const float f = m[h] == -INFINITY ? 0.f : __expf(m[h] - top);
+    float sum = l[h] * f;
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    float o[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      unpack2(acc[h][i], o[2 * i], o[2 * i + 1]);
+#pragma unroll
+      for (int e = 2 * i; e < 2 * i + 2; ++e) {
+        o[e] *= f;
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8);
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16);
+      }
+    }
+    if (lane == 0) sm_m[h][warp] = top, sm_l[h][warp] = sum;
+    if (of == 0) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          *reinterpret_cast<float4*>(&sm_acc[h][warp][half * 64 + part * 8 + i * 4]) = make_float4(o[half * 8 + i * 4], o[half * 8 + i * 4 + 1], o[half * 8 + i * 4 + 2], o[half * 8 + i * 4 + 3]);
+    }
+  }
+  __syncthreads();
+  __shared__ __align__(16) float cl_part[PARTIAL ? 1 : kLongHeads][PARTIAL ? 1 : 8][kAttnSlot];
+  if (!PARTIAL) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // all CTAs of the cluster have started
+  if (warp < heads) {
+    float gm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) gm = fmaxf(gm, sm_m[warp][w]);
+    float total = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) {
+      const float f = sm_m[warp][w] == -INFINITY ? 0.f : __expf(sm_m[warp][w] - gm);
+      total = fmaf(sm_l[warp][w], f, total);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = fmaf(sm_acc[warp][w][lane * 4 + i], f, o[i]);
+    }
+    if (PARTIAL) {
+      float* slot = scratch + ((size_t)(head0 + warp) * kAttnMaxSplits + split) * kAttnSlot;
+      *reinterpret_cast<float4*>(slot + lane * 4) = make_float4(o[0], o[1], o[2], o[3]);
+      if (lane == 0) *reinterpret_cast<float2*>(slot + 128) = make_float2(gm, total);
+    } else {
+      uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : split][0])), "r"(0));
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote + lane * 16), "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]) : "memory");
+      if (lane == 0) {
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + 512), "f"(gm) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + 516), "f"(total) : "memory");
+      }
+    }
+  }
+  if (PARTIAL) return;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (split != 0 || warp >= heads) return;
+  float gm = -INFINITY;
+#pragma unroll
+  for (int sp = 0; sp < 8; ++sp)
+    if (sp < splits) gm = fmaxf(gm, cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : sp][128]);
+  float total = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int sp = 0; sp < 8; ++sp) {
+    if (sp >= splits) break;
+    const float* piece = cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : sp];
+    const float f = piece[128] == -INFINITY ? 0.f : __expf(piece[128] - gm);
+    total = fmaf(piece[129], f, total);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = fmaf(piece[lane * 4 + i], f, o[i]);
+  }
+  const float inv = 1.f / total;
+  uint2 packed;
+  packed.x = (uint32_t)to_bits(o[0] * inv, ACT) | ((uint32_t)to_bits(o[1] * inv, ACT) << 16);
+  packed.y = (uint32_t)to_bits(o[2] * inv, ACT) | ((uint32_t)to_bits(o[3] * inv, ACT) << 16);
+  *reinterpret_cast<uint2*>(out + (size_t)(head0 + warp) * D + lane * 4) = packed;
+}
+
 __global__ void silu_mul_kernel(const unsigned short* __restrict__ gate, const unsigned short* __restrict__ up,
                                 unsigned short* __restrict__ out, int n, int dtype) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -463,6 +739,38 @@ int launch_attention(Kernel kernel, Kernel cluster_kernel, dim3 grid, cudaStream
   return FB_OK;
 }
 
+// Two heads to share, and more positions than one round of the other kernel takes; rows are read 16 bytes at a time.
+inline bool long_cache(int length, int q_heads, int kv_heads, const void* k_cache, const void* v_cache) {
+  return length > kLongFrom && q_heads >= 2 * kv_heads && aligned(k_cache, 16) && aligned(v_cache, 16);
+}
+
+template <bool FUSED, bool PARTIAL>
+int launch_long(cudaStream_t stream, const char* what, const unsigned short* q, unsigned short* k_cache, unsigned short* v_cache, unsigned short* out, float* scratch,
+                int q_heads, int kv_heads, int length, int max_positions, float scale, int dtype, const NewToken& nt) {
+  const int group = q_heads / kv_heads, pairs = (group + kLongHeads - 1) / kLongHeads;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(kv_heads * pairs, attention_splits(length));
+  config.blockDim = dim3(kAttnWarps * 32);
+  config.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (pdl_allowed()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (!PARTIAL) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+    attr[n++].val.clusterDim.y = config.gridDim.y;
+  }
+  config.attrs = attr;
+  config.numAttrs = n;
+  const cudaError_t err = dtype == FB_BF16
+      ? cudaLaunchKernelEx(&config, attn_long_kernel<FUSED, PARTIAL, FB_BF16>, q, k_cache, v_cache, out, scratch, q_heads, kv_heads, length, max_positions, scale, nt)
+      : cudaLaunchKernelEx(&config, attn_long_kernel<FUSED, PARTIAL, FB_F16>, q, k_cache, v_cache, out, scratch, q_heads, kv_heads, length, max_positions, scale, nt);
+  return err == cudaSuccess ? FB_OK : cuda_fail(err, what);
+}
+
 inline const unsigned short* u16(const void* p) { return static_cast<const unsigned short*>(p); }
 inline unsigned short* u16(void* p) { return static_cast<unsigned short*>(p); }
 
@@ -501,6 +809,9 @@ extern "C" int fb_attn_decode(const void* q, const void* k_cache, const void* v_
   const int splits = attention_splits(length);
   float* partial = static_cast<float*>(scratch);
   unsigned* tickets = reinterpret_cast<unsigned*>(partial + (size_t)q_heads * kAttnMaxSplits * kAttnSlot);
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
+    return launch_long<false, false>(static_cast<cudaStream_t>(stream), "attn_decode launch", u16(q), const_cast<unsigned short*>(u16(k_cache)), const_cast<unsigned short*>(u16(v_cache)),
+                                     u16(out), partial, q_heads, kv_heads, length, max_positions, scale, dtype, NewToken{});
   return launch_attention(attn_decode_kernel<false, false>, attn_decode_kernel<false, true>, dim3(q_heads, splits), static_cast<cudaStream_t>(stream), "attn_decode launch",
                     u16(q), const_cast<unsigned short*>(u16(k_cache)), const_cast<unsigned short*>(u16(v_cache)), u16(out), partial, tickets,
                     q_heads, kv_heads, length, max_positions, scale, dtype, NewToken{});
@@ -524,6 +835,9 @@ extern "C" int fb_attn_decode_fused(const void* q, const void* k, const void* v,
   float* partial = static_cast<float*>(scratch);
   unsigned* tickets = reinterpret_cast<unsigned*>(partial + (size_t)q_heads * kAttnMaxSplits * kAttnSlot);
   const NewToken nt = {u16(q), u16(k), u16(v), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), eps};
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
+    return launch_long<true, false>(static_cast<cudaStream_t>(stream), "attn_decode_fused launch", nullptr, u16(k_cache), u16(v_cache), u16(out), partial, q_heads, kv_heads,
+                                    length, max_positions, scale, dtype, nt);
   return launch_attention(attn_decode_kernel<true, false>, attn_decode_kernel<true, true>, dim3(q_heads, splits), static_cast<cudaStream_t>(stream), "attn_decode_fused launch",
                     static_cast<const unsigned short*>(nullptr), u16(k_cache), u16(v_cache), u16(out), partial, tickets, q_heads, kv_heads, length,
                     max_positions, scale, dtype, nt);
@@ -546,6 +860,9 @@ extern "C" int fb_attn_decode_partial(const void* q, const void* k, const void* 
   if (!partials || partial_bytes < need || !aligned(partials, 16)) return fail(FB_ESCRATCH, "fb_attn_decode_partial: 16-byte aligned buffer of %zu bytes needed", need);
   const int length = position + 1;
   const NewToken nt = {u16(q), u16(k), u16(v), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), eps};
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
+    return launch_long<true, true>(static_cast<cudaStream_t>(stream), "attn_decode_partial launch", nullptr, u16(k_cache), u16(v_cache), nullptr, static_cast<float*>(partials), q_heads,
+                                   kv_heads, length, max_positions, scale, dtype, nt);
   return launch_pdl(attn_decode_kernel<true, false, true>, dim3(q_heads, attention_splits(length)), dim3(kAttnWarps * 32), 0,
                     static_cast<cudaStream_t>(stream), "attn_decode_partial launch", static_cast<const unsigned short*>(nullptr), u16(k_cache),
                     u16(v_cache), static_cast<unsigned short*>(nullptr), static_cast<float*>(partials), static_cast<unsigned*>(nullptr), q_heads,

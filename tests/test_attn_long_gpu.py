@@ -1,0 +1,51 @@
+"""Attention over long caches (two query heads a CTA) at the edges of its rounds, against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,length,dtype", (
+    (4, 2, 640, torch.bfloat16),    # the last length of the other kernel
+    (4, 2, 641, torch.bfloat16),    # the first of this one: the last split is one row short of the others
+    (32, 8, 1024, torch.bfloat16),  # whole rounds
+    (10, 2, 1033, torch.float16),   # an odd group: a CTA with one head; one row in a second round
+    (5, 1, 3333, torch.bfloat16),
+    (64, 8, 777, torch.float16),
+    (8, 8, 1000, torch.bfloat16),   # nothing to share: the other kernel
+))
+def test_long_cache(q_heads, kv_heads, length, dtype):
+    from marlin_style_fluxbin_b200 import _native as nat
+
+    gen = torch.Generator(device="cuda").manual_seed(q_heads + length)
+    normal = lambda *size: torch.randn(*size, device="cuda", generator=gen).to(dtype)  # noqa: E731
+    q, k, v = normal(1, q_heads * 128), normal(1, kv_heads * 128), normal(1, kv_heads * 128)
+    caches = [normal(kv_heads, length + 3, 128) for _ in range(2)]
+    weights = [(1 + 0.1 * normal(128).float()).to(dtype) for _ in range(2)]
+    angle = torch.rand(64, device="cuda", generator=gen).repeat(2) * 6
+    cos, sin, scale = angle.cos().to(dtype), angle.sin().to(dtype), 128 ** -0.5
+    scratch = torch.zeros(nat.attn_scratch_bytes(q_heads), dtype=torch.uint8, device="cuda")
+    rotated = torch.empty(q_heads, 128, device="cuda", dtype=dtype)
+    filled = [cache.clone() for cache in caches]
+    nat.qknorm_rope_cache(q, k, v, *weights, cos, sin, rotated, *filled, length - 1, 1e-6)
+    two = torch.empty(1, q_heads * 128, device="cuda", dtype=dtype)
+    nat.attn_decode(rotated, *filled, two, length, scale, scratch)
+    keys, values = (cache[:, :length].double() for cache in filled)
+    scores = rotated.double().view(kv_heads, -1, 128) @ keys.transpose(1, 2) * scale
+    share = scores.softmax(-1)
+    want = share @ values
+    # fp32: scores good to 128 x 2^-24 of their magnitudes, exponentials to as much again and 2^-21, sums of `length` terms; one rounding
+    slack = 2.0 ** -24 * (2 * 128 * float((rotated.double().abs().view(kv_heads, -1, 128) @ keys.abs().transpose(1, 2)).max()) * scale + length + 8)
+    bound = slack * (share @ values.abs()) + 2.0 ** (-8 if dtype == torch.bfloat16 else -11) * want.abs() + 2.0 ** -24
+    assert bool(((two.double().view_as(want) - want).abs() <= bound).all())
+    one = torch.empty_like(two)
+    again = [cache.clone() for cache in caches]
+    nat.attn_decode_fused(q, k, v, *weights, cos, sin, *again, one, length - 1, 1e-6, scale, scratch)
+    assert torch.equal(one, two) and all(torch.equal(a, b) for a, b in zip(again, filled))
+    # the pieces left for the o projection, merged here
+    again = [cache.clone() for cache in caches]
+    splits = nat.attn_decode_partial(q, k, v, *weights, cos, sin, *again, length - 1, 1e-6, scale, scratch)
+    pieces = scratch[: q_heads * 16 * 132 * 4].view(torch.float32).view(q_heads, 16, 132)[:, :splits].double()
+    factor = (pieces[..., 128] - pieces[..., 128].amax(1, keepdim=True)).exp()
+    merged = (pieces[..., :128] * factor[..., None]).sum(1) / (pieces[..., 129] * factor).sum(1, keepdim=True)
+    assert bool(((merged.view_as(want) - want).abs() <= bound).all()) and all(torch.equal(a, b) for a, b in zip(again, filled))
