@@ -3,7 +3,7 @@
 // One persistent kernel instead of chunks that were dequantised into L2 and read back by a library GEMM, two
 // or three launches each.  A CTA owns 128 output rows of up to 256 tokens at a time; roles are warps:
 //
-//   warp 0         TMA: activations of a group, 128-byte swizzle, ring of three stages of 256 tokens or more of fewer
+//   warp 0         TMA: activations of a group, 128-byte swizzle, ring of three stages of 256 tokens, four of fewer
 //   warp 2         TMA: plane tiles (three planes of 128 rows of a group), ring of four
 //   warps 4..19    four warpgroups take turns on groups: a thread dequantises ITS row of the group and puts the 16-bit
 //                  weights into tensor memory (tcgen05.st), where the MMA takes its A operand from: shared
@@ -21,6 +21,10 @@
 // 128 x 128 weights), at 256 the MMA (1370 TFLOP/s where the tiles fill the SMs).  us on a B200, weights cold, in a graph, chunks
 // -> this: 12288 x 4096 at 64 / 512 / 1024 tokens 39 / 63 / 92 -> 19 / 46 / 81, 24576 x 4096 at 512 126 -> 82,
 // 4096 x 12288 at 512 / 1024 72 / 96 -> 54 / 75.
+//
+// The MMA warp's own course over a group (two barriers, eight instructions, commits) takes 500 to 600 clocks and is what a
+// group of few tokens waits for.  It looks at both barriers with one instruction, and where the activations' ring has as many stages as there
+// are operand slots (up to 192 tokens) one commit releases both: 512 tokens of 12288 x 4096 47.6 -> 45.6 us, 100 of 25600 x 5120 46.9 -> 45.8.
 //
 // A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
 // the CTA ends; it leaves with the status word set and the tensor memory freed.
@@ -40,11 +44,12 @@ constexpr int kMaxTokens = 256;  // of a tile
 constexpr int kDequant = 4;      // warpgroups that dequantise
 constexpr int kEpilogue = 2;     // warpgroups that write outputs
 constexpr int kThreads = 128 * (1 + kDequant + kEpilogue);
-constexpr int kBBytes = 192 * 1024;  // ring of activation stages, a group each: three of 256 tokens, more of fewer
-constexpr int kMaxBStages = 8;
+constexpr int kBBytes = 192 * 1024;  // ring of activation stages, a group each: three of 256 tokens, four of 192 or fewer
+constexpr int kMaxBStages = 4;  // as many as operand slots
 constexpr int kPlaneStages = 4;  // even: a stage always serves the same warpgroup (a wait by parity must not fall two phases behind)
 constexpr int kPlaneStage = 3 * kRows * 16;
 constexpr int kASlots = 4;             // weights of a group, 64 columns
+static_assert(kMaxBStages == kASlots, "a full ring goes round with the operand slots");
 constexpr int kAColumn = kMaxTokens;  // behind the accumulator
 constexpr int kMaxMats = 4;
 constexpr int kBars = 2 * kMaxBStages + 2 * kPlaneStages + 2 * kASlots + 2;
@@ -184,6 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
   tcgen_after();
   const uint32_t tmem = *tmem_slot;
   const int G = p.G;
+  const bool paired = p.b_stages == kASlots;
   bool dead = false;
 
   auto matrix_of = [&](int row_tile) {
@@ -202,7 +208,8 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
       for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x) {
         const int token0 = (tile % p.token_tiles) * p.tokens;
         for (int g = 0; g < G; ++g) {
-          if (!first && !mbar_wait_bounded(b_empty + 8 * stage, phase ^ 1u)) {
+          // with as many stages as operand slots the MMA's one commit of a group releases both
+          if (!first && !mbar_wait_bounded((paired ? a_empty : b_empty) + 8 * stage, phase ^ 1u)) {
             dead = true;
             break;
           }
@@ -254,8 +261,9 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
       }
       for (int g = 0; g < G; ++g, ++step) {
         const unsigned slot = step % kASlots, use = step / kASlots;
-        const bool there = mbar_wait_bounded(b_full + 8 * stage, stage_phase) && mbar_wait_bounded(a_full + 8 * slot, use & 1);
-        if (!__all_sync(0xffffffffu, there)) {
+        // half of the lanes look at either barrier
+        const uint32_t full = lane & 1 ? a_full + 8 * slot : b_full + 8 * stage, parity = lane & 1 ? use & 1 : stage_phase;
+        if (!__all_sync(0xffffffffu, mbar_try_wait(full, parity)) && !__all_sync(0xffffffffu, mbar_wait_bounded(full, parity))) {
           dead = true;
           break;
         }
@@ -275,7 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
                 "r"(a + 8 * i), "l"(b_desc + (i >> 2) * (p.tokens * 8) + 2 * (i & 3)), "r"(idesc), "r"(g + i > 0 ? 1u : 0u)
                 : "memory");
           commit(a_done);
-          commit(b_done);
+          if (!paired) commit(b_done);
           if (g + 1 == G) commit(d_full);
         }
         __syncwarp();
