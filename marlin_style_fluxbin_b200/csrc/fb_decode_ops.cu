@@ -364,13 +364,14 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_kernel(const unsi
 // Long caches, grouped-query heads: a CTA serves TWO query heads of a k/v head, so that a cache row crosses the L2 half as
 // often (the first kernel reads each once per query head: 67 MB of L2 traffic at 4096 positions of the 8B shape), and eight lanes share a
 // position, sixteen dims each: three shuffle steps for a score instead of five, rows unpacked once for both heads, products
-// two at a time (packed fp32).  Four positions per lane are in flight; the next keys are requested as soon as the scores are
-// formed, the next values after the sums.  What bounds it: the round trips of the four batches of a CTA.
-// us of a launch, rows cold (32 query heads over 8; 4 over 2), first kernel -> this: 641 positions 4.40 -> 3.84; 3.64 -> 3.02,
-// 1200 5.27 -> 5.02; 4.10 -> 4.25, 2048 8.70 -> 5.89; 7.04 -> 4.87, 4096 14.1 -> 8.6; 11.7 -> 7.8.  Up to 640 positions the first kernel
+// two at a time (packed fp32).  Rows come by asynchronous copies, three batches of 128 positions (192 KB) under way.  What
+// bounds it: a batch's instructions (unpacking, packed products) on two warps a scheduler; a test that skips the empty positions of the
+// last batch breaks them up and cost 0.8 us at 4096, rows in registers instead of shared memory 0.5 us, sixteen warps 0.6 us.
+// us of a launch, rows cold (32 query heads over 8; 4 over 2), first kernel -> this: 641 positions 4.40 -> 3.74; 3.64 -> 3.02,
+// 1200 5.27 -> 4.81, 2048 8.70 -> 5.63, 4096 14.1 -> 8.1; 11.7 -> 6.3.  Up to 640 positions the first kernel
 // has a single round, whose chains are shorter (512: 3.48).
 // FUSED, PARTIAL and the merge over the splits as there; without PARTIAL the splits form a cluster.
-constexpr int kLongHeads = 2, kLongBatch = 4, kLongFrom = 640;
+constexpr int kLongHeads = 2, kLongBatch = 4, kLongStages = 3, kLongFrom = 640;
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   uint64_t r;
@@ -416,24 +417,35 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
   if (!PARTIAL) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   __shared__ __align__(16) unsigned short sm_new[kLongHeads + 2][D];  // rotated q of the heads, rotated k, v of the new token
   constexpr int kStep = kAttnWarps * 4;                               // positions of a step of the CTA
-  uint4 kr[kLongBatch][2], vr[kLongBatch][2];
-  auto fetch = [&](const unsigned short* rows, int first, uint4 (&to)[kLongBatch][2]) {  // first: this lane's first position
+  // A thread copies what it reads itself, so its own copies are all it waits for: [stage][position][16 bytes of k, k, v, v][thread]
+  extern __shared__ __align__(16) unsigned char ring[];
+  const uint32_t my_ring = smem_u32(ring) + threadIdx.x * 16;
+  constexpr int kPiece = kAttnWarps * 32 * 16, kStage = kLongBatch * 4 * kPiece;
+  auto request = [&](int first, int stage) {  // first: this lane's first position; rows that are not there (yet) are zeros
 #pragma unroll
     for (int j = 0; j < kLongBatch; ++j) {
-      const int pos = min(first + j * kStep, p1 - 1);
-      to[j][0] = to[j][1] = make_uint4(0u, 0u, 0u, 0u);
-      if (first < p1 && !(FUSED && pos == newest)) {
-        to[j][0] = *reinterpret_cast<const uint4*>(rows + (size_t)pos * D);
-        to[j][1] = *reinterpret_cast<const uint4*>(rows + (size_t)pos * D + 64);
-      }
+      const int pos = first + j * kStep;
+      const bool there = pos < p1 && !(FUSED && pos == newest);
+      const size_t at = there ? (size_t)pos * D : 0;
+      const int bytes = there ? 16 : 0;
+      const uint32_t to = my_ring + (uint32_t)(stage * kStage + j * 4 * kPiece);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(kbase + at), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + kPiece), "l"(kbase + at + 64), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + 2 * kPiece), "l"(vbase + at), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + 3 * kPiece), "l"(vbase + at + 64), "r"(bytes) : "memory");
     }
   };
-  const int mine = p0 + warp * 4 + of;
+  auto request_all = [&]() {  // the first rounds, a group each
+#pragma unroll
+    for (int n = 0; n < kLongStages; ++n) {
+      if (p0 + n * kStep * kLongBatch < p1) request(p0 + warp * 4 + of + n * kStep * kLongBatch, n);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  };
   HeadConstants hc = {};
   if (FUSED) {  // constants and rows of earlier positions ahead of the wait, ordered as in the kernel above
     if (warp <= kLongHeads) hc = load_head_constants(warp < kLongHeads ? nt.q_weight : nt.k_weight, nt.cosv, nt.sinv, ACT, lane);
-    fetch(kbase, mine, kr);
-    fetch(vbase, mine, vr);
+    request_all();
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -445,8 +457,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
     else if (warp == kLongHeads + 1)
       *reinterpret_cast<uint2*>(&sm_new[kLongHeads + 1][lane * 4]) = *reinterpret_cast<const uint2*>(nt.v + (size_t)kvh * D + lane * 4);
   } else {
-    fetch(kbase, mine, kr);
-    fetch(vbase, mine, vr);
+    request_all();
     if (warp < kLongHeads) *reinterpret_cast<uint2*>(&sm_new[warp][lane * 4]) = *reinterpret_cast<const uint2*>(q + (size_t)(head0 + min(warp, heads - 1)) * D + lane * 4);
   }
   __syncthreads();
@@ -469,30 +480,23 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
     }
   }
   // all warps take as many batches; lanes without a position in one add nothing
+  int stage = 0;
   for (int base = p0; base < p1; base += kStep * kLongBatch) {
-    const int first = base + warp * 4 + of, next = first + kStep * kLongBatch;
-    if (FUSED) {
-#pragma unroll
-      for (int j = 0; j < kLongBatch; ++j)
-        if (first + j * kStep == newest) {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            kr[j][half] = *reinterpret_cast<const uint4*>(&sm_new[kLongHeads][half * 64 + part * 8]);
-            vr[j][half] = *reinterpret_cast<const uint4*>(&sm_new[kLongHeads + 1][half * 64 + part * 8]);
-          }
-        }
-    }
+    const int first = base + warp * 4 + of;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLongStages - 1) : "memory");
+    const unsigned char* const from = ring + threadIdx.x * 16 + stage * kStage;
+    auto row = [&](int j, int piece) {  // pieces 0, 1: key; 2, 3: value
+      if (FUSED && first + j * kStep == newest) return *reinterpret_cast<const uint4*>(&sm_new[kLongHeads + (piece >> 1)][(piece & 1) * 64 + part * 8]);
+      return *reinterpret_cast<const uint4*>(from + (j * 4 + piece) * kPiece);
+    };
     float s[kLongBatch][kLongHeads];
 #pragma unroll
     for (int j = 0; j < kLongBatch; ++j) {
-      if (base + j * kStep >= p1) {  // no lane has this position of the last batch
-        s[j][0] = s[j][1] = 0.f;
-        continue;
-      }
       uint64_t dot[kLongHeads] = {};
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const uint32_t w[4] = {kr[j][half].x, kr[j][half].y, kr[j][half].z, kr[j][half].w};
+        const uint4 raw = row(j, half);
+        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint64_t key = widen2<ACT>(w[i]);
@@ -507,7 +511,6 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
         s[j][h] = lo + hi;
       }
     }
-    fetch(kbase, next, kr);
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1)
 #pragma unroll
@@ -535,13 +538,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
     }
 #pragma unroll
     for (int j = 0; j < kLongBatch; ++j) {
-      if (base + j * kStep >= p1) continue;
       uint64_t p2[kLongHeads];
 #pragma unroll
       for (int h = 0; h < kLongHeads; ++h) p2[h] = pack2(s[j][h], s[j][h]);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const uint32_t w[4] = {vr[j][half].x, vr[j][half].y, vr[j][half].z, vr[j][half].w};
+        const uint4 raw = row(j, 2 + half);
+        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint64_t value = widen2<ACT>(w[i]);
@@ -550,7 +553,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
         }
       }
     }
-    fetch(vbase, next, vr);
+    if (base + kLongStages * kStep * kLongBatch < p1) request(first + kLongStages * kStep * kLongBatch, stage);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    stage = stage + 1 == kLongStages ? 0 : stage + 1;
   }
   // the four positions of a warp, then the warps, then the splits
   __shared__ float sm_m[kLongHeads][kAttnWarps], sm_l[kLongHeads][kAttnWarps];
@@ -751,7 +756,22 @@ int launch_long(cudaStream_t stream, const char* what, const unsigned short* q, 
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(kv_heads * pairs, attention_splits(length));
   config.blockDim = dim3(kAttnWarps * 32);
+  config.dynamicSmemBytes = kLongStages * kLongBatch * 4 * kAttnWarps * 32 * 16;
   config.stream = stream;
+  static std::mutex lock;
+  static bool ready[64] = {};
+  int device = 0;
+  if (const cudaError_t got = cudaGetDevice(&device); got != cudaSuccess) return cuda_fail(got, "cudaGetDevice");
+  if (device < 0 || device >= 64) return fail(FB_ELIMIT, "device ordinal %d outside 0..63", device);
+  {
+    std::lock_guard<std::mutex> guard(lock);
+    if (!ready[device]) {
+      for (const void* kernel : {reinterpret_cast<const void*>(attn_long_kernel<FUSED, PARTIAL, FB_BF16>), reinterpret_cast<const void*>(attn_long_kernel<FUSED, PARTIAL, FB_F16>)})
+        if (const cudaError_t got = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)config.dynamicSmemBytes); got != cudaSuccess)
+          return cuda_fail(got, "cudaFuncSetAttribute(attn_long_kernel)");
+      ready[device] = true;
+    }
+  }
   cudaLaunchAttribute attr[2];
   int n = 0;
   if (pdl_allowed()) {
