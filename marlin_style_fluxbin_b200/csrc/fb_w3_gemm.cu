@@ -17,14 +17,13 @@
 // eight values per (row, group), scale * (code - zero) rounded in the scale's dtype and then in the
 // activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes.
 //
-// What bounds it: up to about 100 tokens a tile the integer instructions of the look-ups (some 800 clocks per
-// 128 x 128 weights), at 256 the MMA (1370 TFLOP/s where the tiles fill the SMs).  us on a B200, weights cold, in a graph, chunks
-// -> this: 12288 x 4096 at 64 / 512 / 1024 tokens 39 / 63 / 92 -> 19 / 46 / 81, 24576 x 4096 at 512 126 -> 82,
-// 4096 x 12288 at 512 / 1024 72 / 96 -> 54 / 75.
-//
-// The MMA warp's own course over a group (two barriers, eight instructions, commits) takes 500 to 600 clocks and is what a
-// group of few tokens waits for.  It looks at both barriers with one instruction, and where the activations' ring has as many stages as there
-// are operand slots (up to 192 tokens) one commit releases both: 512 tokens of 12288 x 4096 47.6 -> 45.6 us, 100 of 25600 x 5120 46.9 -> 45.8.
+// What bounds it: up to about 200 tokens a tile the look-ups (59 integer instructions for 32 weights of a row, 472 clocks per 128 x 128
+// weights on pipes of half rate) and, side by side with them, the MMA warp's own course over a group (two barriers, eight instructions,
+// commits: 450 to 500 clocks); at 256 the MMA.  Either alone changes nothing while the other stays: with 70 instructions and a branch around
+// the issue both took 600.  The MMA warp looks at both barriers with one instruction, its instructions are predicated on the elected lane
+// (operands stay in uniform registers), and where the activations' ring has as many stages as there are operand slots (up to 192 tokens) one
+// commit releases both.  us on a B200, weights cold, in a graph, before these three -> now: 12288 x 4096 at 64 / 112 / 333 / 512 tokens 20.0 / 22.3 /
+// 41.0 / 48.1 -> 19.5 / 21.0 / 38.2 / 43.5, 4096 x 12288 at 512 55.0 -> 49.7; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 63.
 //
 // A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
 // the CTA ends; it leaves with the status word set and the tensor memory freed.
@@ -136,29 +135,25 @@ __device__ __forceinline__ uint32_t blend(uint32_t a, uint32_t b, uint32_t m) {
 }
 
 // 32 codes of a row (one word per plane, the high one inverted) -> 16 operand registers, inputs in order.  low, high: bytes
-// of the values of the eight codes.
+// of the values of the eight codes.  Neighbouring inputs share a byte of the selector words, so that what two look-ups
+// pick is interleaved once and is in order then.
 __device__ __forceinline__ void look_up(uint32_t p0, uint32_t p1, uint32_t p2, const uint32_t (&low)[2], const uint32_t (&high)[2], uint32_t* to) {
-  uint32_t codes[4];  // nibble n of codes[s]: the code of input 4 n + s
+  // low two bits of the codes of inputs 0 2 4 6 of every byte, of 1 3 5 7, and from these of (0, 2 | 1, 3) and (4, 6 | 5, 7)
+  const uint32_t even = blend(p0, p1 << 1, 0x55555555u), odd = blend(p0 >> 1, p1, 0x55555555u);
+  const uint32_t first = blend(even, odd << 4, 0x0f0f0f0fu), last = blend(even >> 4, odd, 0x0f0f0f0fu);
+  const uint32_t two[4] = {first, first >> 2, last, last >> 2};
+  // bits 2 and 6: high bits of inputs 2 s and 2 s + 1
+  const uint32_t top[4] = {blend(p2 << 2, p2 << 5, 0x0f0f0f0fu), blend(p2, p2 << 3, 0x0f0f0f0fu), blend(p2 >> 2, p2 << 1, 0x0f0f0f0fu), blend(p2 >> 4, p2 >> 1, 0x0f0f0f0fu)};
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
-    const uint32_t a = p0 >> s, b = s == 0 ? p1 << 1 : p1 >> (s - 1), c = s < 2 ? p2 << (2 - s) : p2 >> (s - 2);
-    const uint32_t two = blend(a, b, 0x11111111u) & 0x33333333u;
-    asm("lop3.b32 %0, %1, %2, %3, 0xF4;" : "=r"(codes[s]) : "r"(two), "r"(0x44444444u), "r"(c));  // two | (0x4444... & ~c)
-  }
+    const uint32_t bits = two[s] & 0x33333333u;
+    uint32_t codes;  // byte m: the codes of inputs 8 m + 2 s and 8 m + 2 s + 1
+    asm("lop3.b32 %0, %1, %2, %3, 0xF4;" : "=r"(codes) : "r"(bits), "r"(0x44444444u), "r"(top[s]));  // bits | (0x4444... & ~top)
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    uint32_t x[4][2];  // [s]: inputs 16 half + s, + 4 and + 8, + 12
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const uint32_t sel = half ? codes[s] >> 16 : codes[s];
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t sel = half ? codes >> 16 : codes;
       const uint32_t l = pick(low[0], low[1], sel), h = pick(high[0], high[1], sel);
-      x[s][0] = pick(l, h, 0x5140u), x[s][1] = pick(l, h, 0x7362u);
-    }
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      uint32_t* const eight = to + 8 * half + 4 * b;
-      eight[0] = pick(x[0][b], x[1][b], 0x5410u), eight[1] = pick(x[2][b], x[3][b], 0x5410u);
-      eight[2] = pick(x[0][b], x[1][b], 0x7632u), eight[3] = pick(x[2][b], x[3][b], 0x7632u);
+      to[8 * half + s] = pick(l, h, 0x5140u), to[8 * half + 4 + s] = pick(l, h, 0x7362u);
     }
   }
 }
@@ -187,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
   tcgen_before();
   __syncthreads();
   tcgen_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const int G = p.G;
   const bool paired = p.b_stages == kASlots;
   bool dead = false;
@@ -271,17 +266,20 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
         const uint64_t b_desc = b_desc0 + stage * (p.tokens * 16);
         const uint32_t a = tmem + kAColumn + slot * 64;
         const uint32_t a_done = a_empty + 8 * slot, b_done = b_empty + 8 * stage;
-        if (elected()) {
+        // the elected lane's predicate sits on the instruction, not on a branch around it: operands stay uniform
+        const uint32_t elect = elected() ? 1u : 0u, later = g > 0 ? 1u : 0u;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            asm volatile(
-                "{\n\t"
-                ".reg .pred p;\n\t"
-                "setp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-                "}\n" ::"r"(tmem),
-                "r"(a + 8 * i), "l"(b_desc + (i >> 2) * (p.tokens * 8) + 2 * (i & 3)), "r"(idesc), "r"(g + i > 0 ? 1u : 0u)
-                : "memory");
+        for (int i = 0; i < 8; ++i)
+          asm volatile(
+              "{\n\t"
+              ".reg .pred e, p;\n\t"
+              "setp.ne.b32 e, %5, 0;\n\t"
+              "setp.ne.b32 p, %4, 0;\n\t"
+              "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+              "}\n" ::"r"(tmem),
+              "r"(a + 8 * i), "l"(b_desc + (i >> 2) * (p.tokens * 8) + 2 * (i & 3)), "r"(idesc), "r"(i ? 1u : later), "r"(elect)
+              : "memory");
+        if (elect) {
           commit(a_done);
           if (!paired) commit(b_done);
           if (g + 1 == G) commit(d_full);
