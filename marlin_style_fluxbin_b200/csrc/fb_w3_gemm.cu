@@ -256,12 +256,14 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
       }
       for (int g = 0; g < G; ++g, ++step) {
         const unsigned slot = step % kASlots, use = step / kASlots;
-        // half of the lanes look at either barrier
+        // half of the lanes look at either barrier; a vote tells them that both have completed but orders no memory
+        // between them, the __syncwarp does: the elected lane may then build on what the barrier of the others released
         const uint32_t full = lane & 1 ? a_full + 8 * slot : b_full + 8 * stage, parity = lane & 1 ? use & 1 : stage_phase;
         if (!__all_sync(0xffffffffu, mbar_try_wait(full, parity)) && !__all_sync(0xffffffffu, mbar_wait_bounded(full, parity))) {
           dead = true;
           break;
         }
+        __syncwarp();
         tcgen_after();
         const uint64_t b_desc = b_desc0 + stage * (p.tokens * 16);
         const uint32_t a = tmem + kAColumn + slot * 64;

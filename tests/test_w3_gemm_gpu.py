@@ -11,6 +11,10 @@ pytestmark = pytest.mark.gpu
     ((256, 64, 64), 1152, 257, torch.bfloat16, torch.float16, True),  # stacked matrices, two token tiles, the second short
     ((8192,), 384, 600, torch.bfloat16, torch.bfloat16, False),       # more tiles than SMs: accumulator and rings change hands
     ((4096,), 4096, 333, torch.bfloat16, torch.float16, False),
+    # tiles of 256 tokens, three stages beside four operand slots: the MMA's two barriers are of different rounds; SMs with several tiles
+    ((12288, 12288), 1152, 500, torch.bfloat16, torch.float16, False),
+    ((12288,), 1152, 250, torch.bfloat16, torch.float16, True),       # one such tile of an SM, ragged
+    ((12288,), 1152, 192, torch.float16, torch.bfloat16, False),      # the largest tile whose rings go round together
 ))
 def test_many_rows(widths, k, t, dtype, scale_dtype, add):
     from marlin_style_fluxbin_b200 import _native
