@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
       for (int j = 0; j < kLongBatch; ++j)
 #pragma unroll
         for (int h = 0; h < kLongHeads; ++h) s[j][h] += __shfl_xor_sync(0xffffffffu, s[j][h], d);
+    uint64_t c2[kLongHeads];
 #pragma unroll
     for (int h = 0; h < kLongHeads; ++h) {
       float top = m[h];
@@ -525,33 +526,39 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
         if (first + j * kStep < p1) top = fmaxf(top, s[j][h]);
       const float safe = top == -INFINITY ? 0.f : top;  // a lane group without a position so far
       const float correction = __expf(m[h] - safe);
-      l[h] *= correction;
-      const uint64_t c2 = pack2(correction, correction);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[h][i] = mul2(acc[h][i], c2);
+      float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < kLongBatch; ++j) {
         s[j][h] = first + j * kStep < p1 ? __expf(s[j][h] - safe) : 0.f;
-        l[h] += s[j][h];
+        sum += s[j][h];
       }
+      l[h] = fmaf(l[h], correction, sum);
+      c2[h] = pack2(correction, correction);
       m[h] = top;
     }
+    // a batch's products are summed by themselves, and meet the sums so far in one multiply-add with one rounding: rescaled
+    // first and added to one by one they were 4 % (4096 positions) to 10 % (8000) further from fp64 than in the kernel above
 #pragma unroll
-    for (int j = 0; j < kLongBatch; ++j) {
-      uint64_t p2[kLongHeads];
+    for (int half = 0; half < 2; ++half) {
+      uint64_t pv[kLongHeads][4];
 #pragma unroll
-      for (int h = 0; h < kLongHeads; ++h) p2[h] = pack2(s[j][h], s[j][h]);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      for (int j = 0; j < kLongBatch; ++j) {
         const uint4 raw = row(j, 2 + half);
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+        uint64_t p2[kLongHeads];
+#pragma unroll
+        for (int h = 0; h < kLongHeads; ++h) p2[h] = pack2(s[j][h], s[j][h]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint64_t value = widen2<ACT>(w[i]);
 #pragma unroll
-          for (int h = 0; h < kLongHeads; ++h) acc[h][half * 4 + i] = fma2(value, p2[h], acc[h][half * 4 + i]);
+          for (int h = 0; h < kLongHeads; ++h) pv[h][i] = j ? fma2(value, p2[h], pv[h][i]) : mul2(value, p2[h]);
         }
       }
+#pragma unroll
+      for (int h = 0; h < kLongHeads; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[h][half * 4 + i] = fma2(acc[h][half * 4 + i], c2[h], pv[h][i]);
     }
     if (base + kLongStages * kStep * kLongBatch < p1) request(first + kLongStages * kStep * kLongBatch, stage);
     asm volatile("cp.async.commit_group;" ::: "memory");

@@ -49,3 +49,28 @@ def test_long_cache(q_heads, kv_heads, length, dtype):
     factor = (pieces[..., 128] - pieces[..., 128].amax(1, keepdim=True)).exp()
     merged = (pieces[..., :128] * factor[..., None]).sum(1) / (pieces[..., 129] * factor).sum(1, keepdim=True)
     assert bool(((merged.view_as(want) - want).abs() <= bound).all()) and all(torch.equal(a, b) for a, b in zip(again, filled))
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+def test_batches_are_summed_before_they_meet_the_sums(dtype):
+    """Equal scores; in the first 32 positions of every split's 256 values of `large`, zeros up to 128, ones from there.  A lane adds
+    four ones to its `large`: one by one they fall below half a unit of its last place and are lost, together they are kept.  All sums
+    kept that way are whole multiples of the units they meet, so that a split's output is exact."""
+    from marlin_style_fluxbin_b200 import _native as nat
+
+    q_heads, kv_heads, length = 4, 2, 2048
+    large = 2.0 ** 24 if dtype == torch.bfloat16 else 2.0 ** 14
+    one = large * 2.0 ** -24
+    values = torch.zeros(8, 256, device="cuda", dtype=torch.float64)
+    values[:, :32], values[:, 128:] = large, one
+    v_cache = values.reshape(1, length, 1).expand(kv_heads, length, 128).to(dtype).contiguous()
+    assert torch.equal(v_cache[0, :, 0].double(), values.reshape(-1))  # 16 bits hold them
+    k_cache = torch.zeros_like(v_cache)
+    zeros = lambda n: torch.zeros(1, n, device="cuda", dtype=dtype)  # noqa: E731
+    ones = torch.ones(128, device="cuda", dtype=dtype)
+    scratch = torch.zeros(nat.attn_scratch_bytes(q_heads), dtype=torch.uint8, device="cuda")
+    splits = nat.attn_decode_partial(zeros(q_heads * 128), zeros(kv_heads * 128), v_cache[:, -1].reshape(1, -1).contiguous(), ones, ones, ones, ones,
+                                     k_cache, v_cache, length - 1, 1e-6, 128 ** -0.5, scratch)
+    pieces = scratch[: q_heads * 16 * 132 * 4].view(torch.float32).view(q_heads, 16, 132)[:, :splits]
+    assert splits == 8 and bool((pieces[..., 129] == 256).all())
+    assert bool((pieces[..., :128].double() == 32 * large + 128 * one).all())
