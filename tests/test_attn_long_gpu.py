@@ -53,16 +53,15 @@ def test_long_cache(q_heads, kv_heads, length, dtype):
 
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
 def test_batches_are_summed_before_they_meet_the_sums(dtype):
-    """Equal scores; in the first 32 positions of every split's 256 values of `large`, zeros up to 128, ones from there.  A lane adds
-    four ones to its `large`: one by one they fall below half a unit of its last place and are lost, together they are kept.  All sums
-    kept that way are whole multiples of the units they meet, so that a split's output is exact."""
+    """Equal scores; a split's 256 positions hold one `large` value, and 2^-24 of it in the four positions that the same lane takes in its
+    next batch.  One by one these are half a unit of the last place of `large` and lost to the rounding; together they are kept, and
+    nothing else of the sums rounds."""
     from marlin_style_fluxbin_b200 import _native as nat
 
     q_heads, kv_heads, length = 4, 2, 2048
-    large = 2.0 ** 24 if dtype == torch.bfloat16 else 2.0 ** 14
-    one = large * 2.0 ** -24
+    large = 2.0 ** 14
     values = torch.zeros(8, 256, device="cuda", dtype=torch.float64)
-    values[:, :32], values[:, 128:] = large, one
+    values[:, 0], values[:, 128::32] = large, large * 2.0 ** -24
     v_cache = values.reshape(1, length, 1).expand(kv_heads, length, 128).to(dtype).contiguous()
     assert torch.equal(v_cache[0, :, 0].double(), values.reshape(-1))  # 16 bits hold them
     k_cache = torch.zeros_like(v_cache)
@@ -73,4 +72,4 @@ def test_batches_are_summed_before_they_meet_the_sums(dtype):
                                      k_cache, v_cache, length - 1, 1e-6, 128 ** -0.5, scratch)
     pieces = scratch[: q_heads * 16 * 132 * 4].view(torch.float32).view(q_heads, 16, 132)[:, :splits]
     assert splits == 8 and bool((pieces[..., 129] == 256).all())
-    assert bool((pieces[..., :128].double() == 32 * large + 128 * one).all())
+    assert bool((pieces[..., :128].double() == large * (1 + 2.0 ** -22)).all())
