@@ -370,8 +370,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_kernel(const unsi
 // us of a launch, rows cold (32 query heads over 8; 4 over 2), first kernel -> this: 641 positions 4.40 -> 3.74; 3.64 -> 3.02,
 // 1200 5.27 -> 4.81, 2048 8.70 -> 5.63, 4096 14.1 -> 8.1; 11.7 -> 6.3.  Up to 640 positions the first kernel
 // has a single round, whose chains are shorter (512: 3.48).
-// FUSED, PARTIAL and the merge over the splits as there; without PARTIAL the splits form a cluster.
+// FUSED and the merge over the splits as there.
 constexpr int kLongHeads = 2, kLongBatch = 4, kLongStages = 3, kLongFrom = 640;
+constexpr int kLongSmem = kLongStages * kLongBatch * 4 * kAttnWarps * 32 * 16;
+// What becomes of the splits of a head: left for the consumer; merged through a cluster; merged by whichever CTA is the last to leave its piece.
+enum LongMerge { kPieces, kCluster, kLast };
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   uint64_t r;
@@ -396,7 +399,7 @@ __device__ __forceinline__ uint64_t widen2(uint32_t two) {  // two 16-bit values
   return pack2(f.x, f.y);
 }
 
-template <bool FUSED, bool PARTIAL, int ACT>
+template <bool FUSED, LongMerge MERGE, int ACT>
 __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const unsigned short* __restrict__ q, unsigned short* __restrict__ k_cache,
                                                                     unsigned short* __restrict__ v_cache, unsigned short* __restrict__ out,
                                                                     float* __restrict__ scratch, int q_heads, int kv_heads, int length,
@@ -414,7 +417,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
   const int chunk = (length + splits - 1) / splits;
   const int p0 = split * chunk, p1 = min(length, p0 + chunk);
   const int newest = length - 1;
-  if (!PARTIAL) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  if (MERGE == kCluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   __shared__ __align__(16) unsigned short sm_new[kLongHeads + 2][D];  // rotated q of the heads, rotated k, v of the new token
   constexpr int kStep = kAttnWarps * 4;                               // positions of a step of the CTA
   // A thread copies what it reads itself, so its own copies are all it waits for: [stage][position][16 bytes of k, k, v, v][thread]
@@ -596,8 +599,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
     }
   }
   __syncthreads();
-  __shared__ __align__(16) float cl_part[PARTIAL ? 1 : kLongHeads][PARTIAL ? 1 : 8][kAttnSlot];
-  if (!PARTIAL) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // all CTAs of the cluster have started
+  __shared__ __align__(16) float cl_part[MERGE == kCluster ? kLongHeads : 1][MERGE == kCluster ? 8 : 1][kAttnSlot];
+  if (MERGE == kCluster) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // all CTAs of the cluster have started
+  const float* const slots = scratch + (size_t)(head0 + warp) * kAttnMaxSplits * kAttnSlot;  // of this warp's head
   if (warp < heads) {
     float gm = -INFINITY;
 #pragma unroll
@@ -610,37 +614,66 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) attn_long_kernel(const uns
 #pragma unroll
       for (int i = 0; i < 4; ++i) o[i] = fmaf(sm_acc[warp][w][lane * 4 + i], f, o[i]);
     }
-    if (PARTIAL) {
-      float* slot = scratch + ((size_t)(head0 + warp) * kAttnMaxSplits + split) * kAttnSlot;
-      *reinterpret_cast<float4*>(slot + lane * 4) = make_float4(o[0], o[1], o[2], o[3]);
-      if (lane == 0) *reinterpret_cast<float2*>(slot + 128) = make_float2(gm, total);
-    } else {
+    if (MERGE == kCluster) {
       uint32_t remote;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : split][0])), "r"(0));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&cl_part[MERGE == kCluster ? warp : 0][MERGE == kCluster ? split : 0][0])), "r"(0));
       asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote + lane * 16), "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]) : "memory");
       if (lane == 0) {
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + 512), "f"(gm) : "memory");
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + 516), "f"(total) : "memory");
       }
+    } else {
+      float* const slot = const_cast<float*>(slots) + split * kAttnSlot;
+      *reinterpret_cast<float4*>(slot + lane * 4) = make_float4(o[0], o[1], o[2], o[3]);
+      if (lane == 0) *reinterpret_cast<float2*>(slot + 128) = make_float2(gm, total);
     }
   }
-  if (PARTIAL) return;
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (split != 0 || warp >= heads) return;
+  if (MERGE == kPieces) return;
+  if (MERGE == kCluster) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (split != 0 || warp >= heads) return;
+  } else {  // barrier, ticket (release, and acquire by the last) and barrier order every piece before the merge of the CTA with the last ticket
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned* const ticket = reinterpret_cast<unsigned*>(scratch + (size_t)q_heads * kAttnMaxSplits * kAttnSlot) + head0;
+      unsigned before;
+      asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(ticket) : "memory");
+      last = before == (unsigned)splits - 1u;
+      if (last) *ticket = 0u;  // zero for the next launch
+    }
+    __syncthreads();
+    if (!last || warp >= heads) return;
+  }
+  // splits in ascending order, as fb_w3_gemv_attn_merge takes them: the results are the same bits in all three forms
+  float4 piece_of[8];
+  float2 ml[8];  // (max, sum)
+#pragma unroll
+  for (int sp = 0; sp < 8; ++sp) {
+    piece_of[sp] = make_float4(0.f, 0.f, 0.f, 0.f), ml[sp] = make_float2(-INFINITY, 0.f);
+    if (sp >= splits) continue;
+    if (MERGE == kCluster) {
+      const float* const piece = cl_part[MERGE == kCluster ? warp : 0][MERGE == kCluster ? sp : 0];
+      piece_of[sp] = *reinterpret_cast<const float4*>(piece + lane * 4), ml[sp] = *reinterpret_cast<const float2*>(piece + 128);
+    } else {
+      const float* const piece = slots + sp * kAttnSlot;
+      piece_of[sp] = __ldcg(reinterpret_cast<const float4*>(piece + lane * 4)), ml[sp] = __ldcg(reinterpret_cast<const float2*>(piece + 128));
+    }
+  }
   float gm = -INFINITY;
 #pragma unroll
-  for (int sp = 0; sp < 8; ++sp)
-    if (sp < splits) gm = fmaxf(gm, cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : sp][128]);
+  for (int sp = 0; sp < 8; ++sp) gm = fmaxf(gm, ml[sp].x);
   float total = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int sp = 0; sp < 8; ++sp) {
     if (sp >= splits) break;
-    const float* piece = cl_part[PARTIAL ? 0 : warp][PARTIAL ? 0 : sp];
-    const float f = piece[128] == -INFINITY ? 0.f : __expf(piece[128] - gm);
-    total = fmaf(piece[129], f, total);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = fmaf(piece[lane * 4 + i], f, o[i]);
+    const float f = ml[sp].x == -INFINITY ? 0.f : __expf(ml[sp].x - gm);
+    total = fmaf(ml[sp].y, f, total);
+    o[0] = fmaf(piece_of[sp].x, f, o[0]);
+    o[1] = fmaf(piece_of[sp].y, f, o[1]);
+    o[2] = fmaf(piece_of[sp].z, f, o[2]);
+    o[3] = fmaf(piece_of[sp].w, f, o[3]);
   }
   const float inv = 1.f / total;
   uint2 packed;
@@ -751,51 +784,100 @@ int launch_attention(Kernel kernel, Kernel cluster_kernel, dim3 grid, cudaStream
   return FB_OK;
 }
 
-// Two heads to share, and more positions than one round of the other kernel takes; rows are read 16 bytes at a time.
-inline bool long_cache(int length, int q_heads, int kv_heads, const void* k_cache, const void* v_cache) {
-  return length > kLongFrom && q_heads >= 2 * kv_heads && aligned(k_cache, 16) && aligned(v_cache, 16);
+// Two heads to share, and more positions than one round of the first kernel takes; rows are read 16 bytes at a time.  Where the CTAs need
+// more rounds than the first kernel's, two of which fit an SM (half or a third of them have one head: 30 heads over 10, 36 over 4 or 12),
+// only from 2048 positions on: a decode layer with the first kernel over one with this, 641 / 1280 / 1536 / 2048 positions 0.95 to 0.98 / 0.95 to 0.97 /
+// 0.99 to 1.01 / 1.04 to 1.06; where they need as many, 1.02 to 1.09 at 641 positions already (32 heads over 8 17.8 us for 19.4, 64 over 8 25.0
+// for 27.0).  The rule is the same for all forms of the call: their results are the same bits.
+inline bool long_cache(int length, int q_heads, int kv_heads, const void* k_cache, const void* v_cache, int sms) {
+  if (length <= kLongFrom || q_heads < 2 * kv_heads || !aligned(k_cache, 16) || !aligned(v_cache, 16)) return false;
+  const int columns = kv_heads * ((q_heads / kv_heads + kLongHeads - 1) / kLongHeads);
+  return (8 * columns + sms - 1) / sms <= (8 * q_heads + 2 * sms - 1) / (2 * sms) || length >= 2048;
 }
 
-template <bool FUSED, bool PARTIAL>
-int launch_long(cudaStream_t stream, const char* what, const unsigned short* q, unsigned short* k_cache, unsigned short* v_cache, unsigned short* out, float* scratch,
-                int q_heads, int kv_heads, int length, int max_positions, float scale, int dtype, const NewToken& nt) {
-  const int group = q_heads / kv_heads, pairs = (group + kLongHeads - 1) / kLongHeads;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(kv_heads * pairs, attention_splits(length));
-  config.blockDim = dim3(kAttnWarps * 32);
-  config.dynamicSmemBytes = kLongStages * kLongBatch * 4 * kAttnWarps * 32 * 16;
-  config.stream = stream;
+// Shared memory beyond 48 KB is granted per kernel and device, once.  clusters: how many of eight CTAs run at a time.
+template <bool FUSED, LongMerge MERGE>
+int long_ready(int* clusters = nullptr) {
   static std::mutex lock;
   static bool ready[64] = {};
+  static int known[64] = {};
   int device = 0;
   if (const cudaError_t got = cudaGetDevice(&device); got != cudaSuccess) return cuda_fail(got, "cudaGetDevice");
   if (device < 0 || device >= 64) return fail(FB_ELIMIT, "device ordinal %d outside 0..63", device);
-  {
-    std::lock_guard<std::mutex> guard(lock);
-    if (!ready[device]) {
-      for (const void* kernel : {reinterpret_cast<const void*>(attn_long_kernel<FUSED, PARTIAL, FB_BF16>), reinterpret_cast<const void*>(attn_long_kernel<FUSED, PARTIAL, FB_F16>)})
-        if (const cudaError_t got = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)config.dynamicSmemBytes); got != cudaSuccess)
-          return cuda_fail(got, "cudaFuncSetAttribute(attn_long_kernel)");
-      ready[device] = true;
+  std::lock_guard<std::mutex> guard(lock);
+  if (!ready[device]) {
+    for (const void* kernel : {reinterpret_cast<const void*>(attn_long_kernel<FUSED, MERGE, FB_BF16>), reinterpret_cast<const void*>(attn_long_kernel<FUSED, MERGE, FB_F16>)})
+      if (const cudaError_t got = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem); got != cudaSuccess)
+        return cuda_fail(got, "cudaFuncSetAttribute(attn_long_kernel)");
+    if (MERGE == kCluster) {
+      cudaLaunchAttribute eight[1];
+      eight[0].id = cudaLaunchAttributeClusterDimension;
+      eight[0].val.clusterDim.x = eight[0].val.clusterDim.z = 1;
+      eight[0].val.clusterDim.y = 8;
+      cudaLaunchConfig_t config = {};
+      config.gridDim = dim3(1, 8);
+      config.blockDim = dim3(kAttnWarps * 32);
+      config.dynamicSmemBytes = kLongSmem;
+      config.attrs = eight;
+      config.numAttrs = 1;
+      if (const cudaError_t got = cudaOccupancyMaxActiveClusters(&known[device], attn_long_kernel<FUSED, MERGE, FB_BF16>, &config); got != cudaSuccess)
+        return cuda_fail(got, "cudaOccupancyMaxActiveClusters(attn_long_kernel)");
     }
+    ready[device] = true;
   }
+  if (clusters) *clusters = known[device];
+  return FB_OK;
+}
+
+struct LongCall {
+  cudaStream_t stream;
+  const char* what;
+  const unsigned short* q;
+  unsigned short *k_cache, *v_cache, *out;
+  float* scratch;
+  int q_heads, kv_heads, length, max_positions, dtype;
+  float scale;
+  NewToken nt;
+  int columns() const { return kv_heads * ((q_heads / kv_heads + kLongHeads - 1) / kLongHeads); }  // CTAs of a split
+};
+
+template <bool FUSED, LongMerge MERGE>
+int launch_long(const LongCall& c) {
+  if (const int code = long_ready<FUSED, MERGE>(); code != FB_OK) return code;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(c.columns(), attention_splits(c.length));
+  config.blockDim = dim3(kAttnWarps * 32);
+  config.dynamicSmemBytes = kLongSmem;
+  config.stream = c.stream;
   cudaLaunchAttribute attr[2];
   int n = 0;
   if (pdl_allowed()) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (!PARTIAL) {
+  if (MERGE == kCluster) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
     attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
     attr[n++].val.clusterDim.y = config.gridDim.y;
   }
   config.attrs = attr;
   config.numAttrs = n;
-  const cudaError_t err = dtype == FB_BF16
-      ? cudaLaunchKernelEx(&config, attn_long_kernel<FUSED, PARTIAL, FB_BF16>, q, k_cache, v_cache, out, scratch, q_heads, kv_heads, length, max_positions, scale, nt)
-      : cudaLaunchKernelEx(&config, attn_long_kernel<FUSED, PARTIAL, FB_F16>, q, k_cache, v_cache, out, scratch, q_heads, kv_heads, length, max_positions, scale, nt);
-  return err == cudaSuccess ? FB_OK : cuda_fail(err, what);
+  const cudaError_t err = cudaLaunchKernelEx(&config, c.dtype == FB_BF16 ? attn_long_kernel<FUSED, MERGE, FB_BF16> : attn_long_kernel<FUSED, MERGE, FB_F16>,
+                                             c.q, c.k_cache, c.v_cache, c.out, c.scratch, c.q_heads, c.kv_heads, c.length, c.max_positions, c.scale, c.nt);
+  return err == cudaSuccess ? FB_OK : cuda_fail(err, c.what);
+}
+
+// A cluster takes eight whole SMs of one group of SMs, and a B200 runs 15 at a time: 16 clusters (32 heads over 8) would go round twice,
+// although their 128 CTAs have room on 148 SMs.  Where CTAs by themselves need two thirds of the clusters' rounds or fewer, the splits meet in
+// scratch memory instead, merged by the CTA that is the last to leave its piece.  q/k/v GEMV, attention and o GEMV in a graph, rows cold, first
+// kernel / clusters / scratch, 641, 1280 and 4096 positions: 32 heads over 8 14.3, 15.7, 29.0 / 15.1, 17.1, 22.3 / 12.9, 14.2, 18.6 us; 64 over 8 (three rounds of
+// clusters, two of CTAs) 21.9, 24.5, 44.1 / 20.1, 23.6, 30.8 / 18.8, 21.7, 30.8.  With as many rounds of either, clusters: 40 over 8 16.5, 18.5, 24.0 against 18.7, 21.6, 30.2.
+template <bool FUSED>
+int launch_long_whole(const LongCall& c, int sms) {
+  int clusters = 0;
+  if (const int code = long_ready<FUSED, kCluster>(&clusters); code != FB_OK) return code;
+  const int rounds = clusters < 1 ? c.columns() : (c.columns() + clusters - 1) / clusters, alone = (8 * c.columns() + sms - 1) / sms;
+  return 2 * rounds < 3 * alone ? launch_long<FUSED, kCluster>(c) : launch_long<FUSED, kLast>(c);
 }
 
 inline const unsigned short* u16(const void* p) { return static_cast<const unsigned short*>(p); }
@@ -836,9 +918,11 @@ extern "C" int fb_attn_decode(const void* q, const void* k_cache, const void* v_
   const int splits = attention_splits(length);
   float* partial = static_cast<float*>(scratch);
   unsigned* tickets = reinterpret_cast<unsigned*>(partial + (size_t)q_heads * kAttnMaxSplits * kAttnSlot);
-  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
-    return launch_long<false, false>(static_cast<cudaStream_t>(stream), "attn_decode launch", u16(q), const_cast<unsigned short*>(u16(k_cache)), const_cast<unsigned short*>(u16(v_cache)),
-                                     u16(out), partial, q_heads, kv_heads, length, max_positions, scale, dtype, NewToken{});
+  const DeviceInfo* const info = device_info();
+  if (!info) return FB_ECUDA;
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache, info->sm_count))
+    return launch_long_whole<false>({static_cast<cudaStream_t>(stream), "attn_decode launch", u16(q), const_cast<unsigned short*>(u16(k_cache)), const_cast<unsigned short*>(u16(v_cache)),
+                                     u16(out), partial, q_heads, kv_heads, length, max_positions, dtype, scale, NewToken{}}, info->sm_count);
   return launch_attention(attn_decode_kernel<false, false>, attn_decode_kernel<false, true>, dim3(q_heads, splits), static_cast<cudaStream_t>(stream), "attn_decode launch",
                     u16(q), const_cast<unsigned short*>(u16(k_cache)), const_cast<unsigned short*>(u16(v_cache)), u16(out), partial, tickets,
                     q_heads, kv_heads, length, max_positions, scale, dtype, NewToken{});
@@ -862,9 +946,11 @@ extern "C" int fb_attn_decode_fused(const void* q, const void* k, const void* v,
   float* partial = static_cast<float*>(scratch);
   unsigned* tickets = reinterpret_cast<unsigned*>(partial + (size_t)q_heads * kAttnMaxSplits * kAttnSlot);
   const NewToken nt = {u16(q), u16(k), u16(v), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), eps};
-  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
-    return launch_long<true, false>(static_cast<cudaStream_t>(stream), "attn_decode_fused launch", nullptr, u16(k_cache), u16(v_cache), u16(out), partial, q_heads, kv_heads,
-                                    length, max_positions, scale, dtype, nt);
+  const DeviceInfo* const info = device_info();
+  if (!info) return FB_ECUDA;
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache, info->sm_count))
+    return launch_long_whole<true>({static_cast<cudaStream_t>(stream), "attn_decode_fused launch", nullptr, u16(k_cache), u16(v_cache), u16(out), partial, q_heads, kv_heads,
+                                    length, max_positions, dtype, scale, nt}, info->sm_count);
   return launch_attention(attn_decode_kernel<true, false>, attn_decode_kernel<true, true>, dim3(q_heads, splits), static_cast<cudaStream_t>(stream), "attn_decode_fused launch",
                     static_cast<const unsigned short*>(nullptr), u16(k_cache), u16(v_cache), u16(out), partial, tickets, q_heads, kv_heads, length,
                     max_positions, scale, dtype, nt);
@@ -887,9 +973,11 @@ extern "C" int fb_attn_decode_partial(const void* q, const void* k, const void* 
   if (!partials || partial_bytes < need || !aligned(partials, 16)) return fail(FB_ESCRATCH, "fb_attn_decode_partial: 16-byte aligned buffer of %zu bytes needed", need);
   const int length = position + 1;
   const NewToken nt = {u16(q), u16(k), u16(v), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), eps};
-  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache))
-    return launch_long<true, true>(static_cast<cudaStream_t>(stream), "attn_decode_partial launch", nullptr, u16(k_cache), u16(v_cache), nullptr, static_cast<float*>(partials), q_heads,
-                                   kv_heads, length, max_positions, scale, dtype, nt);
+  const DeviceInfo* const info = device_info();
+  if (!info) return FB_ECUDA;
+  if (long_cache(length, q_heads, kv_heads, k_cache, v_cache, info->sm_count))
+    return launch_long<true, kPieces>({static_cast<cudaStream_t>(stream), "attn_decode_partial launch", nullptr, u16(k_cache), u16(v_cache), nullptr, static_cast<float*>(partials), q_heads,
+                                       kv_heads, length, max_positions, dtype, scale, nt});
   return launch_pdl(attn_decode_kernel<true, false, true>, dim3(q_heads, attention_splits(length)), dim3(kAttnWarps * 32), 0,
                     static_cast<cudaStream_t>(stream), "attn_decode_partial launch", static_cast<const unsigned short*>(nullptr), u16(k_cache),
                     u16(v_cache), static_cast<unsigned short*>(nullptr), static_cast<float*>(partials), static_cast<unsigned*>(nullptr), q_heads,
