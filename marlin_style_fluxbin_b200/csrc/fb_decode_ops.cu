@@ -365,8 +365,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_kernel(const unsi
 // often (the first kernel reads each once per query head: 67 MB of L2 traffic at 4096 positions of the 8B shape), and eight lanes share a
 // position, sixteen dims each: three shuffle steps for a score instead of five, rows unpacked once for both heads, products
 // two at a time (packed fp32).  Rows come by asynchronous copies, three batches of 128 positions (192 KB) under way.  What
-// bounds it: a batch's instructions (unpacking, packed products) on two warps a scheduler; a test that skips the empty positions of the
-// last batch breaks them up and cost 0.8 us at 4096, rows in registers instead of shared memory 0.5 us, sixteen warps 0.6 us.
+// bounds it: at 4096 positions neither memory nor issue, but a chain (copies, scores, exponentials, products, merges) with two warps a scheduler to hide
+// its latencies: the instructions are 2.9 of 8.1 us of issue slots (active in 43 %), the rows 2.6 us of the copy peak.  A test that skips the
+// empty positions of the last batch breaks the chain up and cost 0.8 us at 4096, rows in registers instead of shared memory 0.5 us, sixteen warps 0.6 us.
 // us of a launch, rows cold (32 query heads over 8; 4 over 2), first kernel -> this: 641 positions 4.40 -> 3.74; 3.64 -> 3.02,
 // 1200 5.27 -> 4.81, 2048 8.70 -> 5.63, 4096 14.1 -> 8.1; 11.7 -> 6.3.  Up to 640 positions the first kernel
 // has a single round, whose chains are shorter (512: 3.48).

@@ -3,7 +3,7 @@
 // One persistent kernel instead of chunks that were dequantised into L2 and read back by a library GEMM, two
 // or three launches each.  A CTA owns 128 output rows of up to 256 tokens at a time; roles are warps:
 //
-//   warp 0         TMA: activations of a group, 128-byte swizzle, ring of three stages of 256 tokens, four of fewer
+//   warp 0         TMA: activations of a group, 128-byte swizzle, ring of four stages of up to 192 tokens, three of more
 //   warp 2         TMA: plane tiles (three planes of 128 rows of a group), ring of four
 //   warps 4..19    four warpgroups take turns on groups: a thread dequantises ITS row of the group and puts the 16-bit
 //                  weights into tensor memory (tcgen05.st), where the MMA takes its A operand from: shared
@@ -17,13 +17,14 @@
 // eight values per (row, group), scale * (code - zero) rounded in the scale's dtype and then in the
 // activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes.
 //
-// What bounds it: up to about 200 tokens a tile the look-ups (59 integer instructions for 32 weights of a row, 472 clocks per 128 x 128
-// weights on pipes of half rate) and, side by side with them, the MMA warp's own course over a group (two barriers, eight instructions,
-// commits: 450 to 500 clocks); at 256 the MMA.  Either alone changes nothing while the other stays: with 70 instructions and a branch around
-// the issue both took 600.  The MMA warp looks at both barriers with one instruction, its instructions are predicated on the elected lane
+// What bounds it: at 256 tokens a tile the MMA (tensor pipe 86 % active).  Up to 128 tokens a group takes 0.43 us, 840 clocks of 1965 MHz, whatever the
+// tokens (12288 rows, 32 groups less 8), and no unit is near its limit (issue 48 % active, tensor pipe 25 % at 64 tokens, 41 % at 112): counted, the
+// look-ups are 472 of these clocks (59 integer instructions for 32 weights of a row, on pipes of half rate) and, side by side with them, the MMA
+// warp's own course over a group 450 to 500 (two barriers, eight instructions, commits); the rest goes into handing slots over between the two.
+// Either part alone changes nothing while the other stays: with 70 instructions and a branch around the issue both took 600.  The MMA warp looks at both barriers with one instruction, its instructions are predicated on the elected lane
 // (operands stay in uniform registers), and where the activations' ring has as many stages as there are operand slots (up to 192 tokens) one
-// commit releases both.  us on a B200, weights cold, in a graph, before these three -> now: 12288 x 4096 at 64 / 112 / 333 / 512 tokens 20.0 / 22.3 /
-// 41.0 / 48.1 -> 19.5 / 21.0 / 38.2 / 43.5, 4096 x 12288 at 512 55.0 -> 49.7; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 63.
+// commit releases both.  us on a B200, weights cold, in a graph, before these three -> now: 12288 x 4096 at 64 / 112 / 333 / 512 tokens 18.9 / 21.3 /
+// 38.7 / 45.6 -> 18.8 / 19.9 / 36.0 / 42.4, 4096 x 12288 at 512 52.4 -> 47.8; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 64.
 //
 // A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
 // the CTA ends; it leaves with the status word set and the tensor memory freed.
@@ -43,7 +44,7 @@ constexpr int kMaxTokens = 256;  // of a tile
 constexpr int kDequant = 4;      // warpgroups that dequantise
 constexpr int kEpilogue = 2;     // warpgroups that write outputs
 constexpr int kThreads = 128 * (1 + kDequant + kEpilogue);
-constexpr int kBBytes = 192 * 1024;  // ring of activation stages, a group each: three of 256 tokens, four of 192 or fewer
+constexpr int kBBytes = 192 * 1024;  // ring of activation stages, a group each: four of up to 192 tokens, three of more
 constexpr int kMaxBStages = 4;  // as many as operand slots
 constexpr int kPlaneStages = 4;  // even: a stage always serves the same warpgroup (a wait by parity must not fall two phases behind)
 constexpr int kPlaneStage = 3 * kRows * 16;
@@ -404,8 +405,9 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
   if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// Tokens of a tile: a group of a tile measures about 330 + 1.75 tokens ns (16 to 256 tokens, K 4096 and 12288), in rounds of
-// one tile per SM; of the splits that fit, the cheapest.
+// Tokens of a tile: the tiles go round the SMs, and a round costs 190 + tokens.  One round of 12288 x 4096 measures 18.5 us at 48 tokens, 20.4 at
+// 128, 24.8 at 208 and 27.9 at 256, so that the line is too steep for small tiles; what it picks, of the splits that fit, is all the same within 3 %
+// of the best tile for eight shapes from 3072 x 1024 to 25600 x 5120 at 40 to 1024 tokens (333 of 12288 x 4096: 112 tokens 37.1 us, 128 37.0, 96 50.7).
 int token_tile(int T, int row_tiles, int sms) {
   int best = 0;
   long long best_cost = 0;

@@ -29,10 +29,10 @@ DENSE_CHUNK_BYTES = 52 << 20
 
 def fused_gemm_pays(rows: int, out_features: int) -> bool:
     """Whether ``rows`` activation rows go through the kernel that dequantises into tensor memory rather than through dense
-    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy: 512 rows, in a graph, weights cold,
-    1024 x 4096 19 us against 14; with the L2 flushed 2048 x 4096 25 / 26, 2048 x 12288 53 / 46, 3072 x 12288 57 / 71, 4096 x 4096
-    29 / 32.  Beyond a thousand rows the chunks, dequantised once for all of them, catch up: 2048 rows of 12288 x 1024 70 / 60, of
-    12288 x 4096 164 / 175."""
+    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy.  us in a graph, weights cold, this / chunks, 512 rows:
+    1024 x 4096 18.6 / 12.7, 2048 x 4096 19.5 / 17.4, 2048 x 12288 47.4 / 36.4, 3072 x 4096 20.3 / 20.0, 3072 x 12288 47.5 / 57.0, 4096 x 4096
+    21.2 / 23.9; 64 rows: 3072 x 4096 17.7 / 15.5, 4096 x 4096 20.2 / 18.4, 3072 x 12288 44.6 / 51.9, 12288 x 4096 19.2 / 39.3.  Beyond a thousand
+    rows the chunks, dequantised once for all of them, catch up: 2048 rows of 12288 x 1024 59 / 50, of 12288 x 4096 157 / 160."""
     return rows <= 1024 and out_features > 2048 and out_features % 32 == 0
 
 ROW_TILES = (256, 512, 1024)
