@@ -16,10 +16,20 @@
 //  * group mode (the reference's hybrid g128-s8 payload, deployment.py:23-27, kernel
 //    csrc/m1_v5.cu:27-104): fp32 row scales per (group,row,base), fp32 column scales per
 //    (group,input,base), plus a two-base refinement on 8 selected columns per group (two more
-//    tables).  Codes may be planar [G,O,2,16] or interleaved [G,O,32].
+//    tables).  Codes may be planar [G,O,2,16] or interleaved [G,O,32]; interleaved words are unshuffled in
+//    registers (16 instructions a word) and looked up like planar ones.
 //  * global mode (matrix-wide fp16 scales r_b[O], c_b[K], planar codes, and `n_sal` dense bf16
-//    residual columns): the per-base sums are kept separate through the K split and the row
-//    scales and the residual are applied once, by whoever reduces a row.
+//    residual columns): both groups of a unit share one sum per base; row scales are applied, and the residual
+//    columns dealt, per contribution.
+//
+// What bounds it: the launch chain and, per unit, latencies; a unit carries two thirds of a W3 unit's bytes.  Whatever is
+// constant is therefore requested before it is needed: column scales and indices at once, ahead of the codes (behind them they
+// arrived after the activations: 5.04 us against 4.39 for 4096 x 4096 with scales per group), a row's scales and residual one
+// unit ahead of their use (requested where they were used, every unit of a warp waited for HBM once more).  A unit
+// costs about 250 instructions (419 before, with the share of a CTA computed by 64-bit divisions, ring slots by a modulo).
+// us on a B200, weights cold, in a graph, before -> now: matrix-wide scales 1024x4096 3.27 -> 2.78, 4096x4096 5.16 -> 3.81,
+// 12288x4096 8.83 -> 7.31, 4096x12288 8.37 -> 6.98; scales per group, planar 4.00 -> 2.82, 6.25 -> 4.39, 9.92 -> 7.62,
+// 9.97 -> 7.62, interleaved 4.35 -> 3.09, 8.50 -> 5.30, 16.5 -> 10.1, 16.5 -> 10.1.
 #include <mutex>
 #include <new>
 
@@ -33,7 +43,6 @@ constexpr int kUnitRows = 32;
 constexpr int kGroupBytes = kUnitRows * 32;  // 1 KB of codes per unit and group
 constexpr int kWarps = 8;
 constexpr int kCtasPerSm = 2;
-constexpr int kMaxSlots = 4;                // staged units per warp: at most 4 KB in flight per warp
 constexpr int kGroupLutBytes = 32768;       // 256 entries x 32 tables x 4 B
 constexpr int kGroupSparseBytes = 2048;     // 2 tables x 256 entries
 
@@ -55,15 +64,20 @@ struct BBParams {
   unsigned* status;
   int O, K, G, nKB, nRU;
   int act_dtype, interleaved, global_mode, n_sal;
-  int slots, ctas_per_kb;
+  int sal_pairs;                // the residual values of two groups lie in one aligned 32-bit word
+  int slots;                    // staged units per warp
+  int units_few, units_extra;   // row units of a slice; slices that have one more
 };
 
-// one base's eight sign bits out of sixteen interleaved bits (reference csrc/lut8.cuh:10-15)
-__device__ __forceinline__ uint32_t compact_even(uint32_t word) {
-  word &= 0x5555u;
-  word = (word | (word >> 1)) & 0x3333u;
-  word = (word | (word >> 2)) & 0x0f0fu;
-  return (word | (word >> 4)) & 0xffu;
+// Two words of eight sign bits per base, interleaved bit by bit, become [base 0: two bytes][base 1: two bytes]: the four
+// steps of a perfect unshuffle.
+__device__ __forceinline__ uint32_t unshuffle(uint32_t w) {
+  uint32_t t;
+  t = (w ^ (w >> 1)) & 0x22222222u, w ^= t ^ (t << 1);
+  t = (w ^ (w >> 2)) & 0x0c0c0c0cu, w ^= t ^ (t << 2);
+  t = (w ^ (w >> 4)) & 0x00f000f0u, w ^= t ^ (t << 4);
+  t = (w ^ (w >> 8)) & 0x0000ff00u, w ^= t ^ (t << 8);
+  return w;
 }
 
 // acc + {table entry at a0, table entry at a1}, each OFFSET bytes further: one packed add
@@ -80,92 +94,240 @@ __device__ __forceinline__ uint64_t add2_lds(uint64_t acc, uint32_t a0, uint32_t
       : "l"(acc), "r"(a0), "r"(a1), "n"(OFFSET));
   return r;
 }
+__device__ __forceinline__ void halves(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ float sum2(uint64_t v) {
   float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  halves(v, lo, hi);
   return lo + hi;
 }
+__device__ __forceinline__ uint32_t ldg16(const void* at) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(v) : "l"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t ldg32(const void* at) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(at));
+  return v;
+}
+__device__ __forceinline__ float ldgf(const float* at) { return __uint_as_float(ldg32(at)); }
+__device__ __forceinline__ float2 ldgf2(const float* at) {
+  float2 v;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(at));
+  return v;
+}
+__device__ __forceinline__ float half_bits(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 
 template <bool INTERLEAVED, bool GLOBAL, int GPB>
 __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const BBParams p) {
-  constexpr int kBlockGroups = GPB;
   constexpr int kUnitBytes = GPB * kGroupBytes;  // staged per unit
-  constexpr int kLutBytes = GPB * kGroupLutBytes, kSparseLutBytes = GPB * kGroupSparseBytes;
+  constexpr int kLutBytes = GPB * kGroupLutBytes, kSparseLutBytes = GLOBAL ? 0 : GPB * kGroupSparseBytes;
   extern __shared__ __align__(1024) unsigned char smem[];
   // the warp index through a shuffle, so that the compiler knows it is the same in all lanes (uniform registers)
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int S = p.slots;
   unsigned char* const lut = smem;
   float* const sparse_lut = reinterpret_cast<float*>(smem + kLutBytes);
-  unsigned char* const stage_base = smem + kLutBytes + kSparseLutBytes + (size_t)warp * S * kUnitBytes;
-  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + kLutBytes + kSparseLutBytes + (size_t)kWarps * S * kUnitBytes) + warp * (kMaxSlots + 1);
-  const uint32_t stage_u32 = smem_u32(stage_base);
+  const uint32_t ring_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(warp * S * kUnitBytes);
+  const uint32_t bars_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(kWarps * S * kUnitBytes + warp * S * 8);
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int nV = p.nKB * p.ctas_per_kb;
-  if ((int)blockIdx.x >= nV) return;
 
-  if (lane == 0)
-    for (int s = 0; s <= kMaxSlots; ++s) mbar_init(smem_u32(&bars[s]), 1);
-  mbar_init_fence();
+  // ---- this CTA's K block and, dealt to its warps in turn, its row units ----
+  const int kb = (int)blockIdx.y, slice = (int)blockIdx.x;
+  const int first = slice * p.units_few + min(slice, p.units_extra) + warp;
+  const int end = slice * p.units_few + min(slice, p.units_extra) + p.units_few + (slice < p.units_extra ? 1 : 0);
+  const int ngroups = min(GPB, p.G - GPB * kb);
+
+  if (lane == 0) {
+    for (int s = 0; s < S; ++s) mbar_init(bars_u32 + s * 8, 1);
+    mbar_init_fence();
+  }
   __syncwarp();
 
-  auto share = [&](int v, int& kb, int& first, int& count) {
-    kb = v / p.ctas_per_kb;
-    const int slice = v - kb * p.ctas_per_kb;
-    const int ua = (int)((long long)slice * p.nRU / p.ctas_per_kb);
-    const int ub = (int)((long long)(slice + 1) * p.nRU / p.ctas_per_kb);
-    const int n = ub - ua, q = n / kWarps, r = n - q * kWarps;
-    first = ua + warp * q + min(warp, r);
-    count = q + (warp < r ? 1 : 0);
-  };
-  // n units from `first` into slots slot.., one bulk copy per unit and group; rows past O in the
-  // last unit are never copied (the copy is clipped) and never stored
-  auto stage_units = [&](int kb, int first, int n, int slot, int bar_index) {
+  // ---- constants of the tables: no wait for the launch ahead, and ahead of the staged codes, which would hold them up;
+  // lane = table (base = lane / 16, chunk = lane % 16) ----
+  const int base = lane >> 4, chunk = lane & 15;
+  uint32_t col_half[GPB][4];
+  float col[GPB][8];
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) {
+    const int k0 = (GPB * kb + gi) * 128 + chunk * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) col[gi][j] = 0.f;
+    if (gi < ngroups) {
+      if (GLOBAL) {
+        asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(col_half[gi][0]), "=r"(col_half[gi][1]), "=r"(col_half[gi][2]), "=r"(col_half[gi][3])
+                     : "l"(p.gcol + (size_t)base * p.K + k0));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) col[gi][j] = ldgf(p.cols + (size_t)(k0 + j) * 2 + base);
+      }
+    }
+  }
+  // the refinement's column and its scale: lane = (group, base, column)
+  const int r_gi = GPB == 2 ? lane >> 4 : 0, r_base = (lane >> 3) & 1, r_j = lane & 7;
+  const bool r_live = !GLOBAL && r_gi < ngroups && (GPB == 2 || lane < 16);
+  int r_idx = 0;
+  float r_col = 0.f;
+  if (r_live) {
+    const int g = GPB * kb + r_gi;
+    r_idx = g * 128 + (int)ldg16(p.indices + g * 8 + r_j);
+    r_col = ldgf(p.scols + (size_t)(g * 8 + r_j) * 2 + r_base);
+  }
+  int sal_at[GPB];  // the residual column that a group's contribution carries
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) {
+    const int g = GPB * kb + gi;
+    sal_at[gi] = GLOBAL && gi < ngroups && g < p.n_sal ? (int)ldg32(p.sal_idx + g) : -1;
+  }
+
+  // Staging of this warp's units in order, each into the slot that was read last: one bulk copy per group.  Rows past O in
+  // the last unit are never copied (the copy is clipped) and never stored.
+  int pf_ru = first, pf_slot = 0;
+  auto issue_next = [&]() {
     if (lane == 0) {
-      const int ngroups = min(kBlockGroups, p.G - kBlockGroups * kb);
-      const uint32_t bar = smem_u32(&bars[bar_index]);
-      int total = 0;
-      for (int u = 0; u < n; ++u) total += min(kUnitRows, p.O - (first + u) * kUnitRows) * 32 * ngroups;
-      mbar_expect_tx(bar, (uint32_t)total);
-      for (int u = 0; u < n; ++u) {
-        const int rows = min(kUnitRows, p.O - (first + u) * kUnitRows);
-        for (int gi = 0; gi < ngroups; ++gi)
-          bulk_g2s(stage_u32 + (uint32_t)((slot + u) * kUnitBytes + gi * kGroupBytes),
-                   p.codes + ((size_t)(kBlockGroups * kb + gi) * p.O + (size_t)(first + u) * kUnitRows) * 32, (uint32_t)(rows * 32), bar);
+      const uint32_t bar = bars_u32 + (uint32_t)(pf_slot * 8), dst = ring_u32 + (uint32_t)(pf_slot * kUnitBytes);
+      const uint32_t bytes = (uint32_t)min(kUnitRows, p.O - pf_ru * kUnitRows) * 32u;
+      const uint8_t* const src = p.codes + ((size_t)(GPB * kb) * p.O + (size_t)pf_ru * kUnitRows) * 32;
+      mbar_expect_tx(bar, bytes * (uint32_t)ngroups);
+      bulk_g2s(dst, src, bytes, bar);
+      if (GPB == 2 && ngroups == 2) bulk_g2s(dst + kGroupBytes, src + (size_t)p.O * 32, bytes, bar);
+    }
+    pf_ru += kWarps;
+    pf_slot = pf_slot + 1 == S ? 0 : pf_slot + 1;
+  };
+  if (pf_ru < end) issue_next();
+
+  // Constants of a row in this K block, requested ONE UNIT AHEAD of their use (the first unit's ahead of the wait for the
+  // launch before): requested where they were used, each unit of a warp waited for HBM once more.
+  struct Constants {
+    uint32_t r0, r1, sal[GPB];         // matrix-wide scales: fp16 row scales, bf16 residual values
+    float2 rs[GPB], srs[GPB];          // scales per group: of the bases and of the refinement
+    uint32_t sp[GPB];                  // refinement codes of both bases
+  };
+  auto request = [&](int ru, Constants& c) {
+    const int row = min(ru * kUnitRows + lane, p.O - 1);
+    if (GLOBAL) {
+      c.r0 = ldg16(p.grow + row), c.r1 = ldg16(p.grow + (size_t)p.O + row);
+      const __nv_bfloat16* const sal = p.sal + (size_t)row * p.n_sal + GPB * kb;
+#pragma unroll
+      for (int gi = 0; gi < GPB; ++gi) c.sal[gi] = 0u;
+      if (GPB == 2 && p.sal_pairs) {
+        if (GPB * kb < p.n_sal) {
+          const uint32_t both = ldg32(sal);
+          c.sal[0] = both << 16, c.sal[GPB - 1] = both & 0xffff0000u;
+        }
+      } else {
+#pragma unroll
+        for (int gi = 0; gi < GPB; ++gi)
+          if (gi < ngroups && GPB * kb + gi < p.n_sal) c.sal[gi] = ldg16(sal + gi) << 16;
+      }
+    } else {
+#pragma unroll
+      for (int gi = 0; gi < GPB; ++gi) {
+        c.rs[gi] = c.srs[gi] = make_float2(0.f, 0.f);
+        c.sp[gi] = 0u;
+        if (gi < ngroups) {
+          const size_t at = (size_t)(GPB * kb + gi) * p.O + row;
+          c.rs[gi] = ldgf2(p.rows + at * 2), c.srs[gi] = ldgf2(p.srows + at * 2), c.sp[gi] = ldg16(p.sparse + at * 2);
+        }
       }
     }
   };
+  Constants next;
+  if (first < end) request(first, next);
 
+  // Table addresses and word offsets of the rotated walk, the same for every unit.  Lookups use 32-bit shared-window
+  // addresses: entry * 128 + table offset is ONE dp4a (a byte dot product whose only non-zero weight, 128, sits at the
+  // wanted byte of the staged word).
+  //  planar       row = [base 0: 16 bytes][base 1: 16 bytes]; word (h, ws) holds chunks 4 ws .. 4 ws + 3 of base h
+  //  interleaved  row = 16 words of 16 bits, word c = chunk c of both bases; unshuffled, the 32-bit word w = 4 h + ws is
+  //               [base 0: chunks 2 w, 2 w + 1][base 1: the same]
   const int rb = lane & 3, rw = (lane >> 2) & 3, rh = (lane >> 4) & 1;
-  // Lookups use 32-bit shared-window addresses: entry * 128 + table offset is ONE dp4a (a byte
-  // dot product whose only non-zero weight, 128, sits at the wanted byte of the staged word).
   const uint32_t lut_u32 = smem_u32(lut);
-  uint32_t sel[4];
+  uint32_t sel[4], tables[2][4][4], woff[2][4];
 #pragma unroll
   for (int b = 0; b < 4; ++b) sel[b] = 128u << (8 * ((b + rb) & 3));
-  // Table addresses and word offsets of the rotated walk, the same for every unit: halves of a row (bases), words, bytes.
-  // Formed per look-up they were a third of a unit's instructions; with them in registers, and look-ups summed two at a
-  // time, seven launches of an 8B layer take 43.6 us instead of 44.7 (12288 x 4096: 9.30 -> 9.05, 4096 x 12288: 8.88 -> 8.54).
-  uint32_t tables[2][4][4], woff[2][4];
-  if (!INTERLEAVED) {
 #pragma unroll
-    for (int jh = 0; jh < 2; ++jh)
+  for (int jh = 0; jh < 2; ++jh)
 #pragma unroll
-      for (int jw = 0; jw < 4; ++jw) {
-        const int h = jh ^ rh, ws = (jw + rw) & 3;
-        woff[jh][jw] = (uint32_t)(h * 16 + ws * 4 + lane * 32);
+    for (int jw = 0; jw < 4; ++jw) {
+      const int h = jh ^ rh, ws = (jw + rw) & 3;
+      woff[jh][jw] = (uint32_t)(h * 16 + ws * 4 + lane * 32);
+      asm volatile("" : "+r"(woff[jh][jw]));
 #pragma unroll
-        for (int b = 0; b < 4; ++b) tables[jh][jw][b] = lut_u32 + (uint32_t)(64 * h + 16 * ws + 4 * ((b + rb) & 3));
+      for (int b = 0; b < 4; ++b) {
+        const int at = (b + rb) & 3;
+        tables[jh][jw][b] = lut_u32 + (uint32_t)(INTERLEAVED ? 64 * (at >> 1) + 8 * (4 * h + ws) + 4 * (at & 1) : 64 * h + 16 * ws + 4 * at);
+        asm volatile("" : "+r"(tables[jh][jw][b]));
       }
-  }
-  uint32_t chunk_parity = 0, slot_parity = 0;
-  bool dead = false, first_pass = true;
-  int kb, my_first, my_count;
-  share((int)blockIdx.x, kb, my_first, my_count);
-  if (my_count > 0) stage_units(kb, my_first, min(S, my_count), 0, kMaxSlots);
+    }
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // ---- activations: all requests in one round trip ----
+  uint4 xr[GPB];
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) {
+    xr[gi] = make_uint4(0u, 0u, 0u, 0u);
+    if (gi < ngroups) xr[gi] = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.x) + (GPB * kb + gi) * 128 + chunk * 8);
+  }
+  float sal_x[GPB], r_x = 0.f;
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
+  if (r_live) r_x = load_act(p.x, p.act_dtype, r_idx);
+  for (int s = 1; s < S && pf_ru < end; ++s) issue_next();  // the rest of the ring, behind the activations
+
+  // ---- 32 signed tables per group ----
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) {
+    const uint32_t xw[4] = {xr[gi].x, xr[gi].y, xr[gi].z, xr[gi].w};
+    float v8[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float xv = bits_to_float((unsigned short)((xw[j >> 1] >> (16 * (j & 1))) & 0xffffu), p.act_dtype);
+      v8[j] = GLOBAL ? __fmul_rn(xv, half_bits(col_half[gi][j >> 1] >> (16 * (j & 1)))) : __fmul_rn(xv, col[gi][j]);
+      if (gi >= ngroups) v8[j] = 0.f;  // an odd number of groups: whatever lies in the empty half's slot finds zeros
+    }
+    // entry(p) = sum_b (bit b of p ? +v_b : -v_b) = low-nibble part + high-nibble part.  Warp w
+    // owns the entries whose low nibble is 2w or 2w+1; the sixteen high-nibble parts come from
+    // a tree (one add each), so an entry costs one add and one store.
+    unsigned char* const column = lut + gi * kGroupLutBytes + lane * 4;
+    float hi[16];
+    hi[0] = ((-v8[4] - v8[5]) - v8[6]) - v8[7];
+#pragma unroll
+    for (int h = 1; h < 16; ++h) {
+      const int top = h >= 8 ? 3 : (h >= 4 ? 2 : (h >= 2 ? 1 : 0));
+      hi[h] = hi[h & ~(1 << top)] + 2.f * v8[4 + top];
+    }
+#pragma unroll
+    for (int qq = 0; qq < 16 / kWarps; ++qq) {
+      const int q = warp * (16 / kWarps) + qq;
+      float lo = 0.f;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) lo += ((q >> b) & 1) ? v8[b] : -v8[b];
+#pragma unroll
+      for (int h = 0; h < 16; ++h) *reinterpret_cast<float*>(column + (size_t)(h * 16 + q) * 128) = lo + hi[h];
+    }
+  }
+  if (!GLOBAL) {
+    // two refinement tables per group over its 8 selected columns; warp w fills entries 32w..32w+31
+    const float sv = r_live ? __fmul_rn(r_x, r_col) : 0.f;
+    const int pp = warp * 32 + lane;
+#pragma unroll
+    for (int t = 0; t < 2 * GPB; ++t) {  // (group, base)
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float one = __shfl_sync(0xffffffffu, sv, t * 8 + j);
+        sum += ((pp >> j) & 1) ? one : -one;
+      }
+      sparse_lut[t * 256 + pp] = sum;
+    }
+  }
+  __syncthreads();
 
   // Split over the K blocks: every contribution is ONE 64-bit atomic add carrying the scaled
   // partial sum in fixed point (steps of 2^-26, bits 16..63), an arrival count (bits 0..7) and a
@@ -187,231 +349,102 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     pend_row = -1;
   };
 
-  for (int v = (int)blockIdx.x; v < nV; v += (int)gridDim.x) {
-    if (!first_pass) {
-      __syncthreads();  // everyone has finished reading the previous tables
-      share(v, kb, my_first, my_count);
-      if (!dead && my_count > 0) stage_units(kb, my_first, min(S, my_count), 0, kMaxSlots);
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int ru = first; ru < end; ru += kWarps) {
+    Constants now = next;
+    if (ru + kWarps < end) request(ru + kWarps, next);
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(bars_u32 + (uint32_t)(slot * 8), phase))) {
+      if (lane == 0) atomicExch(p.status, 1u);  // the copy never landed: give up
+      break;
     }
-    first_pass = false;
-    const int ngroups = min(kBlockGroups, p.G - kBlockGroups * kb);
+    const uint32_t unit_u32 = ring_u32 + (uint32_t)(slot * kUnitBytes);
+    constexpr int kSums = GLOBAL ? 1 : GPB;  // matrix-wide scales: the groups of a unit share their sums
+    // planar: [sums of walk half jh]; interleaved: [byte steps 0 and 1 | 2 and 3]
+    uint64_t acc[kSums][2] = {};
+#pragma unroll
+    for (int jh = 0; jh < 2; ++jh)
+#pragma unroll
+      for (int jw = 0; jw < 4; ++jw) {
+        const uint32_t wa = unit_u32 + woff[jh][jw];
+#pragma unroll
+        for (int gi = 0; gi < GPB; ++gi) {
+          uint32_t w, a[4];
+          if (gi == 0)
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(wa));
+          else
+            asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(w) : "r"(wa), "n"(kGroupBytes));
+          if (INTERLEAVED) w = unshuffle(w);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(a[b]) : "r"(w), "r"(sel[b]), "r"(tables[jh][jw][b]));
+          uint64_t& even = acc[GLOBAL ? 0 : gi][INTERLEAVED ? 0 : jh];
+          uint64_t& odd = acc[GLOBAL ? 0 : gi][INTERLEAVED ? 1 : jh];
+          even = gi == 0 ? add2_lds<0>(even, a[0], a[1]) : add2_lds<kGroupLutBytes>(even, a[0], a[1]);
+          odd = gi == 0 ? add2_lds<0>(odd, a[2], a[3]) : add2_lds<kGroupLutBytes>(odd, a[2], a[3]);
+        }
+      }
 
-    float sal_x[kBlockGroups] = {};
-    // ---- 32 signed tables per group: lane = table (base = lane/16, chunk = lane%16), warp = 32 entries ----
+    __syncwarp();
+    if (pf_ru < end) issue_next();
+    if (++slot == S) slot = 0, phase ^= 1u;
+
+    float value = 0.f;
 #pragma unroll
-    for (int gi = 0; gi < kBlockGroups; ++gi) {
-      const int g = kBlockGroups * kb + gi;
-      const int base = lane >> 4, chunk = lane & 15;
-      float v8[8];
-      if (gi < ngroups) {
-        // eight activations (and, with matrix-wide scales, eight fp16 column scales) in one 16-byte load each
-        const int k0 = g * 128 + chunk * 8;
-        const uint4 xr = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.x) + k0);
-        const uint32_t xw[4] = {xr.x, xr.y, xr.z, xr.w};
-        uint32_t cw[4] = {0u, 0u, 0u, 0u};
-        if (GLOBAL) {
-          const uint4 cr = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.gcol) + (size_t)base * p.K + k0);
-          cw[0] = cr.x, cw[1] = cr.y, cw[2] = cr.z, cw[3] = cr.w;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xv = bits_to_float((unsigned short)((xw[j >> 1] >> (16 * (j & 1))) & 0xffffu), p.act_dtype);
-          const float cv = GLOBAL ? __half2float(__ushort_as_half((unsigned short)((cw[j >> 1] >> (16 * (j & 1))) & 0xffffu)))
-                                  : p.cols[(size_t)(k0 + j) * 2 + base];
-          v8[j] = __fmul_rn(xv, cv);
-        }
-      } else {  // an odd number of groups: the second half of the last K block is empty
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v8[j] = 0.f;
+    for (int s = 0; s < kSums; ++s) {
+      float d0, d1;  // the bases' sums
+      if (INTERLEAVED) {
+        float v[4];
+        halves(acc[s][0], v[0], v[1]);
+        halves(acc[s][1], v[2], v[3]);
+        // byte step b served base ((b + rb) & 3) / 2
+        const float near0 = (rb & 1) ? v[0] + v[3] : v[0] + v[1], near1 = (rb & 1) ? v[1] + v[2] : v[2] + v[3];
+        d0 = (rb & 2) ? near1 : near0, d1 = (rb & 2) ? near0 : near1;
+      } else {
+        const float even = sum2(acc[s][0]), odd = sum2(acc[s][1]);
+        d0 = rh ? odd : even, d1 = rh ? even : odd;
       }
-      // the salient input this group's contribution carries (matrix-wide scales): fetched once per group
-      if (GLOBAL && gi < ngroups && g < p.n_sal) sal_x[gi] = load_act(p.x, p.act_dtype, p.sal_idx[g]);
-      // entry(p) = sum_b (bit b of p ? +v_b : -v_b) = low-nibble part + high-nibble part.  Warp w
-      // owns the entries whose low nibble is 2w or 2w+1; the sixteen high-nibble parts come from
-      // a tree (one add each), so an entry costs one add and one store.
-      unsigned char* const column = lut + gi * kGroupLutBytes + lane * 4;
-      float hi[16];
-      hi[0] = ((-v8[4] - v8[5]) - v8[6]) - v8[7];
-#pragma unroll
-      for (int h = 1; h < 16; ++h) {
-        const int top = h >= 8 ? 3 : (h >= 4 ? 2 : (h >= 2 ? 1 : 0));
-        hi[h] = hi[h & ~(1 << top)] + 2.f * v8[4 + top];
-      }
-#pragma unroll
-      for (int qq = 0; qq < 16 / kWarps; ++qq) {
-        const int q = warp * (16 / kWarps) + qq;
-        float lo = 0.f;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) lo += ((q >> b) & 1) ? v8[b] : -v8[b];
-#pragma unroll
-        for (int h = 0; h < 16; ++h) *reinterpret_cast<float*>(column + (size_t)(h * 16 + q) * 128) = lo + hi[h];
-      }
-      if (!GLOBAL && gi < ngroups) {
-        // two refinement tables over the group's 8 selected columns; warp w fills entries 32w..32w+31
-        const int pp = warp * 32 + lane;
-#pragma unroll
-        for (int base2 = 0; base2 < 2; ++base2) {
-          float sum = 0.f;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int idx = p.indices[g * 8 + j];
-            const float sv = __fmul_rn(load_act(p.x, p.act_dtype, g * 128 + idx), p.scols[(size_t)(g * 8 + j) * 2 + base2]);
-            sum += ((pp >> j) & 1) ? sv : -sv;
-          }
-          sparse_lut[gi * 512 + base2 * 256 + pp] = sum;
-        }
+      if (GLOBAL) {
+        value = __fmaf_rn(half_bits(now.r0), d0, value);
+        value = __fmaf_rn(half_bits(now.r1), d1, value);
+      } else {
+        const uint32_t sp = INTERLEAVED ? unshuffle(now.sp[s]) : now.sp[s];
+        const uint32_t p0 = sp & 0xffu, p1 = INTERLEAVED ? sp >> 16 & 0xffu : sp >> 8;
+        value = __fmaf_rn(now.rs[s].x, d0, value);
+        value = __fmaf_rn(now.rs[s].y, d1, value);
+        value = __fmaf_rn(now.srs[s].x, sparse_lut[s * 512 + p0], value);
+        value = __fmaf_rn(now.srs[s].y, sparse_lut[s * 512 + 256 + p1], value);
       }
     }
-    __syncthreads();
-
-    const int chunk_units = min(S, my_count);
-    for (int i = 0; i < my_count; ++i) {
-      const int slot = i % S;
-      const int ru = my_first + i;
-      const int row = ru * kUnitRows + lane;
-      const bool live = row < p.O;
-      float2 rs[kBlockGroups], srs[kBlockGroups];
-      unsigned sp[kBlockGroups] = {};
-      uint32_t g0bits = 0, g1bits = 0;
-      uint32_t sal_bits[kBlockGroups] = {};
+    const int row = ru * kUnitRows + lane;
+    if (GLOBAL) {
+      // the dense residual columns are dealt round-robin over the groups' contributions
 #pragma unroll
-      for (int gi = 0; gi < kBlockGroups; ++gi) {
-        const int g = kBlockGroups * kb + gi;
-        rs[gi] = make_float2(0.f, 0.f);
-        srs[gi] = make_float2(0.f, 0.f);
-        if (GLOBAL && live && gi < ngroups && g < p.n_sal)
-          asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(sal_bits[gi]) : "l"(p.sal + (size_t)row * p.n_sal + g));
-        if (!GLOBAL && live && gi < ngroups) {
-          rs[gi] = *reinterpret_cast<const float2*>(p.rows + ((size_t)g * p.O + row) * 2);
-          srs[gi] = *reinterpret_cast<const float2*>(p.srows + ((size_t)g * p.O + row) * 2);
-          sp[gi] = *reinterpret_cast<const unsigned short*>(p.sparse + ((size_t)g * p.O + row) * 2);
-        }
-      }
-      if (GLOBAL && live) {
-        asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(g0bits) : "l"(p.grow + row));
-        asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(g1bits) : "l"(p.grow + (size_t)p.O + row));
-      }
-
-      bool ok = false;
-      if (!dead) {
-        if (i < chunk_units)
-          ok = mbar_wait_bounded(smem_u32(&bars[kMaxSlots]), chunk_parity);
-        else
-          ok = mbar_wait_bounded(smem_u32(&bars[slot]), (slot_parity >> slot) & 1u);
-      }
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok && !dead) {
-        dead = true;
-        if (lane == 0) atomicExch(p.status, 1u);
-      }
-      if (i >= chunk_units) slot_parity ^= 1u << slot;
-
-      float d0[kBlockGroups] = {}, d1[kBlockGroups] = {};
-      if (!dead) {
-#pragma unroll
-        for (int gi = 0; gi < kBlockGroups; ++gi) {
-          if (gi >= ngroups) break;  // nothing was staged for an empty second group
-          const unsigned char* const buf = stage_base + slot * kUnitBytes + gi * kGroupBytes + lane * 32;
-          const uint32_t buf_u32 = stage_u32 + (uint32_t)(slot * kUnitBytes + gi * kGroupBytes);
-          if (!INTERLEAVED) {
-            // row = [base 0: 16 bytes][base 1: 16 bytes]; steps with jh = 0 serve base rh
-            uint64_t acc[2] = {0ull, 0ull};  // sums of even and odd byte steps
-#pragma unroll
-            for (int jh = 0; jh < 2; ++jh)
-#pragma unroll
-              for (int jw = 0; jw < 4; ++jw) {
-                uint32_t w, a[4];
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(buf_u32 + woff[jh][jw]));
-#pragma unroll
-                for (int b = 0; b < 4; ++b) asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(a[b]) : "r"(w), "r"(sel[b]), "r"(tables[jh][jw][b]));
-                acc[jh] = gi == 0 ? add2_lds<0>(acc[jh], a[0], a[1]) : add2_lds<kGroupLutBytes>(acc[jh], a[0], a[1]);
-                acc[jh] = gi == 0 ? add2_lds<0>(acc[jh], a[2], a[3]) : add2_lds<kGroupLutBytes>(acc[jh], a[2], a[3]);
-              }
-            const float first = sum2(acc[0]), second = sum2(acc[1]);
-            d0[gi] = rh ? second : first;
-            d1[gi] = rh ? first : second;
-          } else {
-            // row = 16 little-endian 16-bit words, word c holds chunk c of both bases, bits
-            // interleaved.  A 32-bit read gives chunks 2w and 2w+1; sub-step b picks
-            // (chunk half, base) = ((b+rb)&1, (b+rb)>>1 & 1).
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int jh = 0; jh < 2; ++jh) {
-#pragma unroll
-              for (int jw = 0; jw < 4; ++jw) {
-                const int w8 = 4 * (jh ^ rh) + ((jw + rw) & 3);
-                const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + w8 * 4);
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                  const int combo = (b + rb) & 3, half = combo & 1, base = combo >> 1;
-                  const uint32_t entry = compact_even((w >> (16 * half)) >> base);
-                  acc[b] += *reinterpret_cast<const float*>(lut + gi * kGroupLutBytes + entry * 128 + 4 * (16 * base + 2 * w8 + half));
-                }
-              }
-            }
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              if ((((b + rb) & 3) >> 1) == 0) d0[gi] += acc[b]; else d1[gi] += acc[b];
-            }
-          }
-        }
-      }
-
-      __syncwarp();
-      if (!dead && i + S < my_count) stage_units(kb, my_first + i + S, 1, slot, slot);
-
-      settle();  // the previous unit's answer has long arrived
-      if (!dead && live) {
-        float value = 0.f;
-        if (GLOBAL) {
-          asm volatile("" : "+r"(g0bits), "+r"(g1bits));  // first use: after the lookups
-          const float r0 = __half2float(__ushort_as_half((unsigned short)g0bits)), r1 = __half2float(__ushort_as_half((unsigned short)g1bits));
-#pragma unroll
-          for (int gi = 0; gi < kBlockGroups; ++gi) {
-            if (gi >= ngroups) break;
-            const int g = kBlockGroups * kb + gi;
-            value = __fmaf_rn(r0, d0[gi], value);
-            value = __fmaf_rn(r1, d1[gi], value);
-            // the dense residual columns are dealt round-robin over the groups' contributions
-            if (g < p.n_sal) {
-              asm volatile("" : "+r"(sal_bits[gi]));
-              value = __fmaf_rn(__uint_as_float(sal_bits[gi] << 16), sal_x[gi], value);
-            }
-            for (int sidx = g + p.G; sidx < p.n_sal; sidx += p.G)  // more salient columns than groups: rare
-              value = __fmaf_rn(__bfloat162float(p.sal[(size_t)row * p.n_sal + sidx]), load_act(p.x, p.act_dtype, p.sal_idx[sidx]), value);
-          }
-        } else {
-#pragma unroll
-          for (int gi = 0; gi < kBlockGroups; ++gi) {
-            if (gi >= ngroups) break;
-            const uint32_t p0 = INTERLEAVED ? compact_even(sp[gi]) : (sp[gi] & 0xffu);
-            const uint32_t p1 = INTERLEAVED ? compact_even(sp[gi] >> 1) : (sp[gi] >> 8);
-            value = __fmaf_rn(rs[gi].x, d0[gi], value);
-            value = __fmaf_rn(rs[gi].y, d1[gi], value);
-            value = __fmaf_rn(srs[gi].x, sparse_lut[gi * 512 + p0], value);
-            value = __fmaf_rn(srs[gi].y, sparse_lut[gi * 512 + 256 + p1], value);
-          }
-        }
-        if (p.nKB == 1) {
-          store_act(p.out, p.act_dtype, row, value);
-        } else {
-          const bool fits = fabsf(value) < 8192.f;  // 255 of them stay inside 48 bits
-          pend_add = fits ? ((unsigned long long)__float2ll_rn(value * 67108864.f) << 16) + 1ull : 257ull;
-          asm volatile("atom.add.relaxed.gpu.global.u64 %0, [%1], %2;" : "=l"(pend_old) : "l"(p.combine + row), "l"(pend_add) : "memory");
-          pend_row = row;
-        }
+      for (int gi = 0; gi < GPB; ++gi) {
+        if (sal_at[gi] >= 0) value = __fmaf_rn(__uint_as_float(now.sal[gi]), sal_x[gi], value);
+        if (p.n_sal > p.G && gi < ngroups && row < p.O)  // more residual columns than groups: rare
+          for (int at = GPB * kb + gi + p.G; at < p.n_sal; at += p.G)
+            value = __fmaf_rn(__bfloat162float(p.sal[(size_t)row * p.n_sal + at]), load_act(p.x, p.act_dtype, p.sal_idx[at]), value);
       }
     }
-    if (my_count > 0) chunk_parity ^= 1u;
+    settle();  // the previous unit's answer has long arrived
+    if (row < p.O) {
+      if (p.nKB == 1) {
+        store_act(p.out, p.act_dtype, row, value);
+      } else {
+        const bool fits = fabsf(value) < 8192.f;  // 255 of them stay inside 48 bits
+        pend_add = fits ? ((unsigned long long)__float2ll_rn(value * 67108864.f) << 16) + 1ull : 257ull;
+        asm volatile("atom.add.relaxed.gpu.global.u64 %0, [%1], %2;" : "=l"(pend_old) : "l"(p.combine + row), "l"(pend_add) : "memory");
+        pend_row = row;
+      }
+    }
   }
-
   settle();
 }
 
 constexpr size_t kCombineOffset = 16384;  // after the status block: one 64-bit word per output row
 
 template <bool INTERLEAVED, bool GLOBAL, int GPB>
-int launch(const BBParams& p, int grid, size_t smem, int max_smem, bool pdl, cudaStream_t stream) {
+int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cudaStream_t stream) {
   static std::mutex lock;
   static bool ready[64] = {};
   int device = 0;
@@ -425,7 +458,7 @@ int launch(const BBParams& p, int grid, size_t smem, int max_smem, bool pdl, cud
     }
   }
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(grid);
+  config.gridDim = grid;
   config.blockDim = dim3(kWarps * 32);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
@@ -456,13 +489,13 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   int c = kCtasPerSm * info->sm_count / p.nKB;
   if (c < 1) c = 1;
   if (c > p.nRU) c = p.nRU;
-  p.ctas_per_kb = c;
-  const int nV = p.nKB * c;
-  const int grid = nV < kCtasPerSm * info->sm_count ? nV : kCtasPerSm * info->sm_count;
+  const dim3 grid(c, p.nKB);
+  p.units_few = p.nRU / c, p.units_extra = p.nRU % c;
+  p.sal_pairs = p.global_mode && p.n_sal % 2 == 0 && aligned(p.sal, 4) ? 1 : 0;
   const int per_warp = ((p.nRU + c - 1) / c + kWarps - 1) / kWarps;
-  const int max_slots = kMaxSlots / gpb;
+  const int max_slots = gpb == 1 ? 4 : (p.global_mode ? 3 : 2);
   p.slots = per_warp < max_slots ? (per_warp < 1 ? 1 : per_warp) : max_slots;
-  const size_t smem = (size_t)gpb * (kGroupLutBytes + kGroupSparseBytes) + (size_t)kWarps * p.slots * gpb * kGroupBytes + (size_t)kWarps * (kMaxSlots + 1) * 8;
+  const size_t smem = (size_t)gpb * (kGroupLutBytes + (p.global_mode ? 0 : kGroupSparseBytes)) + (size_t)kWarps * p.slots * (gpb * kGroupBytes + 8);
   const bool pdl = (flags & FB_W3_NO_PDL) == 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (gpb == 2) {
