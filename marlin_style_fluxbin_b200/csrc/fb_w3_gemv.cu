@@ -114,6 +114,7 @@ struct W3Params {
   int units_per_slice, units_extra;  // nRU / slices and nRU % slices
   int group_partials;  // write scale-multiplied per-group sums instead of reducing
   int same_input;      // FB_W3_SAME_INPUT: no wait at the start, one before the end
+  int early_order;     // the column order is requested ahead of the first weights
 };
 
 // Shared-memory geometry.  Entry p of table t for activation row m lives at byte
@@ -244,9 +245,20 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
   }
   __syncthreads();
 
+  // The column order is part of the weights: this thread's index for the first K block needs no wait.  With one CTA per SM
+  // it is requested ahead of the staged weights, behind which it would arrive later than the activations could be read.
+  // With two, the gathers of all CTAs would then meet at the few L2 lines of x at the same time, and cost more than that.
+  // us, cold, early / late: 1024x4096 (one CTA) 3.13 / 3.35, 1024x12288 5.69 / 6.33; 4096x4096 (two) 4.51 / 4.32, 12288x4096 8.40 / 8.37.
+  const int sb = (int)blockIdx.y, kb_begin = sb * p.S;
+  int el_idx = 0;
+  auto fetch_idx = [&](int kb_) {
+    const int e = kb_ * 256 + (int)threadIdx.x;
+    el_idx = threadIdx.x < 256 && e < p.K ? (int)p.perm[e] : 0;
+  };
+  if (GATHER && p.early_order) fetch_idx(kb_begin);
+
   // Work of this CTA: super-block blockIdx.y (K blocks sb*S ..), the row units [first, first + count)
   // of slice blockIdx.x.  The first nRU % slices slices take one unit more.
-  const int sb = (int)blockIdx.y;
   const int cta_first = (int)blockIdx.x * p.units_per_slice + min((int)blockIdx.x, p.units_extra);
   const int cta_count = p.units_per_slice + ((int)blockIdx.x < p.units_extra ? 1 : 0);
   auto locate = [&](int ru) { return locate_unit(p, ru); };
@@ -285,7 +297,7 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
 
   // This CTA walks the K blocks kb_begin .. kb_begin + nS - 1 over the same rows.  Warp w takes
   // the units cta_first + w, + kWarps, ...; its tasks are numbered K block * my_count + unit.
-  const int kb_begin = sb * p.S, nS = min(p.S, p.nKB - kb_begin);
+  const int nS = min(p.S, p.nKB - kb_begin);
   const int my_count = cta_count > warp ? (cta_count - warp + kWarps - 1) / kWarps : 0;
   const int my_tasks = nS * my_count;
   const int my_first = cta_first + warp, my_end = cta_first + cta_count;
@@ -378,13 +390,7 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
       for (int b = 0; b < 4; ++b) asm volatile("" : "+r"(xl[jh][jw][b]));
     }
 
-  // The column order is part of the weights: this thread's index for the first K block needs no wait.
-  int el_idx = 0;
-  auto fetch_idx = [&](int kb_) {
-    const int e = kb_ * 256 + (int)threadIdx.x;
-    el_idx = threadIdx.x < 256 && e < p.K ? (int)p.perm[e] : 0;
-  };
-  if (GATHER) fetch_idx(kb_begin);
+  if (GATHER && !p.early_order) fetch_idx(kb_begin);
 
   // Everything below reads activations and writes scratch / outputs of this stream.
   if (!p.same_input) {
@@ -812,6 +818,11 @@ Plan make_plan(int m, int nKB, int nRU, const DeviceInfo& info) {
   plan.nSB = (nKB + plan.S - 1) / plan.S;
   int c = ctas_per_sm_for(m) * info.sm_count / plan.nSB;
   if (c < 1) c = 1;
+  // Where one CTA per SM is enough for every warp to have at most one unit (and, with several K blocks a CTA, to leave half of
+  // the warps without), a second one would only take the room in which the next launch can start.  us, one after the
+  // other in a graph, two / one: 1024x4096 3.03 / 2.98, 2048x2048 3.04 / 2.94, 1024x12288 5.97 / 5.77; 2048x12288, seven units a CTA and
+  // three K blocks, 6.46 / 6.65; the seven Linears of an 8B layer, k beside q and v beside k, 35.3 / 34.0.
+  if (const int one = info.sm_count / plan.nSB; one >= 1 && (nRU + one - 1) / one <= (plan.S == 1 ? warps_for(m) : warps_for(m) / 2)) c = one;
   if (c > nRU) c = nRU;
   plan.slices = c;
   plan.smem = smem_bytes(m);
@@ -1004,6 +1015,7 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   if (scratch) bind_scratch(p, scratch);
   const Plan plan = make_plan(m, p.nKB, p.nRU, *info);
   p.S = plan.S;
+  p.early_order = plan.slices * plan.nSB <= info->sm_count ? 1 : 0;
   p.units_per_slice = p.nRU / plan.slices;
   p.units_extra = p.nRU % plan.slices;
   p.nSB = plan.nSB;
