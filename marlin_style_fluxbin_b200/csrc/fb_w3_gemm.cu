@@ -8,23 +8,30 @@
 //   warps 4..19    four warpgroups take turns on groups: a thread dequantises ITS row of the group and puts the 16-bit
 //                  weights into tensor memory (tcgen05.st), where the MMA takes its A operand from: shared
 //                  memory, which the B operand and its copies already load to two thirds, never sees them
-//   warp 1         tcgen05.mma, 128 x tokens x 16
+//   warps 1, 3     tcgen05.mma, 128 x tokens x 16; up to 128 tokens they take turns on groups, each on an accumulator of its
+//                  own, which the epilogue adds up; beyond, warp 3 has nothing to do
 //   warps 20..27   epilogue: accumulator -> outputs
 //
 // Tensor memory: the accumulator (256 columns) and four operand slots of a group (64 columns each).  Two slots
 // and two accumulators of 192 columns, which let the epilogue overlap the next tile, ran 10 % slower: the way
 // from a finished MMA over the refilled slot to the next one is longer than an MMA.  A weight takes one of
 // eight values per (row, group), scale * (code - zero) rounded in the scale's dtype and then in the
-// activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes.
+// activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes, or multiplied out.
 //
-// What bounds it: at 256 tokens a tile the MMA (tensor pipe 86 % active).  Up to 128 tokens a group takes 0.43 us, 840 clocks of 1965 MHz, whatever the
-// tokens (12288 rows, 32 groups less 8), and no unit is near its limit (issue 48 % active, tensor pipe 25 % at 64 tokens, 41 % at 112): counted, the
-// look-ups are 472 of these clocks (59 integer instructions for 32 weights of a row, on pipes of half rate) and, side by side with them, the MMA
-// warp's own course over a group 450 to 500 (two barriers, eight instructions, commits); the rest goes into handing slots over between the two.
-// Either part alone changes nothing while the other stays: with 70 instructions and a branch around the issue both took 600.  The MMA warp looks at both barriers with one instruction, its instructions are predicated on the elected lane
-// (operands stay in uniform registers), and where the activations' ring has as many stages as there are operand slots (up to 192 tokens) one
-// commit releases both.  us on a B200, weights cold, in a graph, before these three -> now: 12288 x 4096 at 64 / 112 / 333 / 512 tokens 18.9 / 21.3 /
-// 38.7 / 45.6 -> 18.8 / 19.9 / 36.0 / 42.4, 4096 x 12288 at 512 52.4 -> 47.8; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 64.
+// What bounds it: at 256 tokens a tile the MMA (tensor pipe 86 % active).  Up to 128 tokens a group took 0.43 us, 840 clocks, whatever the tokens.
+// Clock stamps of a working copy (12288 x 4096, 64 or 112 tokens): the MMA warp's course over a group was about 1000 clocks (barriers 330, eight
+// instructions 470, commits 120; the MMAs themselves end 100 after the last is issued) while each dequantising warpgroup spent 1500 of its 3500
+// clocks per group waiting for a slot.  Two warps that issue, each on its own accumulator, halve that course: 300 to 500 of 3000 clocks are
+// waited for then, and instruction issue of the dequantising warps bounds it.  These were cut as well: values of a row by 16-bit
+// multiplications (500 clocks a group of a warpgroup -> 200), and where scales and activations share a dtype no look-ups at all but a code
+// inside a magic number, two or three 16-bit operations on the idle multiply pipes instead of byte permutes.  A kernel for one issuer and one for
+// two: both loops in one kernel took the MMAs' operands out of uniform registers (twice the time).  The MMA warps look at both barriers with one
+// instruction, their instructions are predicated on the elected lane, and where the activations' ring has as many stages as there are operand
+// slots (up to 192 tokens) one commit releases both.
+// us on a B200, weights cold, in a graph, before -> now, fp16 scales / bf16 scales: 12288 x 4096 at 64 tokens 18.6 -> 16.3 / 19.0 -> 16.9, at 112 19.6 ->
+// 18.1 / 20.0 -> 18.4, at 333 36.9 -> 32.9 / 36.9 -> 31.7, at 512 43.0 -> 41.2 / 43.0 -> 40.9; 4096 x 12288 at 512 48.0 -> 46.2 / 48.5 -> 43.5; 24576 x 4096 at
+// 512 79.9 -> 76.8; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 64.
+// Without effect: a ring of eight plane tiles, scales prefetched into L2, more accumulators for one issuer, polling with pauses, one arrival a warp.
 //
 // A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
 // the CTA ends; it leaves with the status word set and the tensor memory freed.
@@ -70,7 +77,6 @@ struct GemmParams {
   unsigned* status;
   int n, T, G, ldo;
   int tokens, token_tiles, tiles, b_stages;
-  int act_dtype, scale_dtype;
 };
 
 __device__ __forceinline__ void tcgen_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -103,23 +109,46 @@ __device__ __forceinline__ void tmem_load16(uint32_t at, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ unsigned short bits16(float v, int dtype) {
-  return dtype == FB_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+template <bool BF16>
+__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  if (BF16)
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  else
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
 }
-
-// scale * c and scale * (c + 1), rounded in the scale's dtype and then in the activations'
-__device__ __forceinline__ uint32_t two_values(float scale, float c, int scale_dtype, int act_dtype) {
-  float2 v = make_float2(scale * c, scale * (c + 1.f));
-  if (scale_dtype == FB_BF16)
-    v = __bfloat1622float2(__floats2bfloat162_rn(v.x, v.y));
+template <bool BF16>
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  if (BF16)
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   else
-    v = __half22float2(__floats2half2_rn(v.x, v.y));
-  uint32_t bits;
-  if (act_dtype == FB_BF16)
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(bits) : "f"(v.y), "f"(v.x));
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t fma2(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  if (BF16)
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   else
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(bits) : "f"(v.y), "f"(v.x));
-  return bits;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// {low, high} rounded to 16 bits
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(float low, float high) {
+  uint32_t d;
+  if (BF16)
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(high), "f"(low));
+  else
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(high), "f"(low));
+  return d;
+}
+template <bool BF16>
+__device__ __forceinline__ float widen(unsigned short bits) {
+  return BF16 ? __uint_as_float((uint32_t)bits << 16) : __half2float(__ushort_as_half(bits));
 }
 
 // Bytes picked by a selector whose nibbles are below eight (__byte_perm would mask it first).
@@ -159,6 +188,63 @@ __device__ __forceinline__ void look_up(uint32_t p0, uint32_t p1, uint32_t p2, c
   }
 }
 
+// The values of a row's eight codes, scale * (code - zero) rounded in the scale's dtype and then in the activations', split into
+// low and high bytes.  A 16-bit multiplication rounds the exact product once, as the rounding of an fp32 product would.
+template <bool SCALE_BF16, bool ACT_BF16>
+__device__ __forceinline__ void value_table(uint32_t scale_bits, uint32_t zero, uint32_t (&low)[2], uint32_t (&high)[2]) {
+  constexpr uint32_t kCodes[4] = {SCALE_BF16 ? 0x3f800000u : 0x3c000000u, SCALE_BF16 ? 0x40404000u : 0x42004000u, SCALE_BF16 ? 0x40a04080u : 0x45004400u,
+                                  SCALE_BF16 ? 0x40e040c0u : 0x47004600u};  // (0, 1), (2, 3), (4, 5), (6, 7)
+  const float minus_zero = -(float)zero;
+  const uint32_t off = pack2<SCALE_BF16>(minus_zero, minus_zero), scale = scale_bits * 0x10001u;
+  uint32_t v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[q] = mul2<SCALE_BF16>(add2<SCALE_BF16>(kCodes[q], off), scale);
+    if (SCALE_BF16 != ACT_BF16) v[q] = pack2<ACT_BF16>(widen<SCALE_BF16>((unsigned short)v[q]), widen<SCALE_BF16>((unsigned short)(v[q] >> 16)));
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) low[q] = pick(v[2 * q], v[2 * q + 1], 0x6420u), high[q] = pick(v[2 * q], v[2 * q + 1], 0x7531u);
+}
+
+// Scales and activations in one dtype: no table.  A code inside the mantissa of a magic number (128 in bf16, 1024 in fp16: its last
+// place is one) is that number plus the code, or plus 16 times it.  off, off16: -(magic + zero), -(magic / 16 + zero).
+struct RowFactors {
+  uint32_t off, off16, scale;
+};
+template <bool BF16>
+__device__ __forceinline__ bool row_factors(uint32_t scale_bits, uint32_t zero, RowFactors& f) {
+  f.off = zero * 0x10001u + (BF16 ? 0xc300c300u : 0xe400e400u);
+  f.off16 = add2<BF16>(f.off, BF16 ? 0x42f042f0u : 0x63806380u);  // + 120, + 960
+  f.scale = scale_bits * 0x10001u;
+  return zero <= 100u;  // magic + zero has a last place of one
+}
+
+// 32 codes of a row (one word per plane, the high one inverted) -> 16 operand registers, inputs in order.  Nibble i of word j
+// takes the code of input 4 i + j; bytes of two such words are put side by side.
+template <bool BF16>
+__device__ __forceinline__ void multiply(uint32_t p0, uint32_t p1, uint32_t p2, const RowFactors& f, uint32_t* to) {
+  constexpr uint32_t kMagic = BF16 ? 0x43004300u : 0x64006400u, kSixteenth = BF16 ? 0x3d803d80u : 0x2c002c00u;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {  // inputs 4 i, 4 i + 1; 4 i + 2, 4 i + 3
+    const uint32_t a = half ? p0 >> 2 : p0, b = half ? p1 >> 1 : p1 << 1, c = half ? p2 : p2 << 2;
+    uint32_t even, odd;
+    asm("lop3.b32 %0, %1, %2, %3, 0x72;" : "=r"(even) : "r"(blend(a, b, 0x11111111u)), "r"(c), "r"(0x44444444u));  // (a & ~m) | (~b & m)
+    asm("lop3.b32 %0, %1, %2, %3, 0x72;" : "=r"(odd) : "r"(blend(a, b, 0x22222222u)), "r"(c), "r"(0x88888888u));
+    odd >>= 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t w = pick(even, odd, 0x4400u + 0x1111u * k);
+      uint32_t x0, x1;
+      asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(x0) : "r"(w), "r"(0x00070007u), "n"(kMagic));  // (w & m) | magic
+      asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(x1) : "r"(w), "r"(0x00700070u), "n"(kMagic));
+      to[4 * k + half] = mul2<BF16>(add2<BF16>(x0, f.off), f.scale);
+      to[4 * k + 2 + half] = mul2<BF16>(fma2<BF16>(x1, kSixteenth, f.off16), f.scale);
+    }
+  }
+}
+
+// TWO: both MMA warps issue.
+template <bool SCALE_BF16, bool ACT_BF16, bool TWO>
 __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* const planes_s = smem + kBBytes;
@@ -173,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
   if (tid < kBars) {
     const int at = tid - 2 * kMaxBStages;
     const bool by_group = (at >= kPlaneStages && at < 2 * kPlaneStages + kASlots);  // p_empty, a_full: a dequantising warpgroup
-    mbar_init(b_full + 8 * tid, tid == kBars - 1 ? 128 * kEpilogue : by_group ? 128 : 1);
+    mbar_init(b_full + 8 * tid, tid == kBars - 1 ? 128 * kEpilogue : tid == kBars - 2 ? (TWO ? 2 : 1) : by_group ? 128 : 1);  // d_empty, d_full
     mbar_init_fence();
   }
   if (warp == 3) {
@@ -241,22 +327,28 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 || (TWO && warp == 3)) {
     // the whole warp walks the loop and one elected lane issues: operands known to be the same in all lanes go to the
     // tensor core's instructions as they are (issued from a lane's own branch, four of them took 480 clocks)
     // D fp32, A and B in the activation dtype, both K-major
-    const uint32_t format = p.act_dtype == FB_BF16 ? 1u : 0u;
+    const uint32_t format = ACT_BF16 ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (format << 7) | (format << 10) | ((uint32_t)(p.tokens >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
     // K-major, 128-byte swizzle: 8-row groups 1024 bytes apart; 16 inputs are 32 bytes of a row
     const uint64_t b_desc0 = (uint64_t)((smem_u32(smem) >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+    // the groups of a tile that this warp takes: all, or every other one, on an accumulator that is its own
+    constexpr int stride = TWO ? 2 : 1;
+    const int first = TWO && warp == 3 ? 1 : 0;
+    const uint32_t sums = tmem + (TWO && warp == 3 ? kMaxTokens / 2 : 0);
     unsigned step = 0, stage = 0, stage_phase = 0, it = 0;
     for (int tile = blockIdx.x; tile < p.tiles && !dead; tile += gridDim.x, ++it) {
       if (it && !__all_sync(0xffffffffu, mbar_wait_bounded(d_empty, (it - 1) & 1))) {
         dead = true;
         break;
       }
-      for (int g = 0; g < G; ++g, ++step) {
+      if (TWO) step = it * G + first;
+      for (int g = first; g < G; g += stride, step += stride) {
         const unsigned slot = step % kASlots, use = step / kASlots;
+        if (TWO) stage = slot, stage_phase = use & 1;  // as many stages as slots
         // half of the lanes look at either barrier; a vote tells them that both have completed but orders no memory
         // between them, the __syncwarp does: the elected lane may then build on what the barrier of the others released
         const uint32_t full = lane & 1 ? a_full + 8 * slot : b_full + 8 * stage, parity = lane & 1 ? use & 1 : stage_phase;
@@ -270,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
         const uint32_t a = tmem + kAColumn + slot * 64;
         const uint32_t a_done = a_empty + 8 * slot, b_done = b_empty + 8 * stage;
         // the elected lane's predicate sits on the instruction, not on a branch around it: operands stay uniform
-        const uint32_t elect = elected() ? 1u : 0u, later = g > 0 ? 1u : 0u;
+        const uint32_t elect = elected() ? 1u : 0u, later = g > first ? 1u : 0u;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           asm volatile(
@@ -279,16 +371,16 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
               "setp.ne.b32 e, %5, 0;\n\t"
               "setp.ne.b32 p, %4, 0;\n\t"
               "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-              "}\n" ::"r"(tmem),
+              "}\n" ::"r"(sums),
               "r"(a + 8 * i), "l"(b_desc + (i >> 2) * (p.tokens * 8) + 2 * (i & 3)), "r"(idesc), "r"(i ? 1u : later), "r"(elect)
               : "memory");
         if (elect) {
           commit(a_done);
-          if (!paired) commit(b_done);
-          if (g + 1 == G) commit(d_full);
+          if (!TWO && !paired) commit(b_done);
+          if (g + stride >= G) commit(d_full);
         }
         __syncwarp();
-        if (++stage == (unsigned)p.b_stages) stage = 0, stage_phase ^= 1u;
+        if (!TWO && ++stage == (unsigned)p.b_stages) stage = 0, stage_phase ^= 1u;
       }
     }
   } else if (warp >= 4 && warp < 4 + 4 * kDequant) {
@@ -312,15 +404,13 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
       fetch(g);
       for (; g < G; g += kDequant) {
         const unsigned at = count + g, stage = at % kPlaneStages;
-        const float scale = bits_to_float((unsigned short)scale_next, p.scale_dtype);
-        const float zero = (float)zero_next;
+        const uint32_t scale_bits = scale_next, zero = zero_next;
         fetch(g + kDequant);
+        RowFactors factors;
+        // one row of the warp that the short form does not cover sends it to the table
+        const bool table = SCALE_BF16 != ACT_BF16 || !__all_sync(0xffffffffu, row_factors<ACT_BF16>(scale_bits, zero, factors));
         uint32_t low[2], high[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const uint32_t a = two_values(scale, (float)(4 * q) - zero, p.scale_dtype, p.act_dtype), b = two_values(scale, (float)(4 * q + 2) - zero, p.scale_dtype, p.act_dtype);
-          low[q] = __byte_perm(a, b, 0x6420), high[q] = __byte_perm(a, b, 0x7531);
-        }
+        if (table) value_table<SCALE_BF16, ACT_BF16>(scale_bits, zero, low, high);
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full + 8 * stage, (at / kPlaneStages) & 1))) {
           dead = true;
           break;
@@ -333,8 +423,13 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t v[32];
-          look_up(h ? w0.z : w0.x, h ? w1.z : w1.x, h ? w2.z : w2.x, low, high, v);
-          look_up(h ? w0.w : w0.y, h ? w1.w : w1.y, h ? w2.w : w2.y, low, high, v + 16);
+          if (table) {
+            look_up(h ? w0.z : w0.x, h ? w1.z : w1.x, h ? w2.z : w2.x, low, high, v);
+            look_up(h ? w0.w : w0.y, h ? w1.w : w1.y, h ? w2.w : w2.y, low, high, v + 16);
+          } else {
+            multiply<ACT_BF16>(h ? w0.z : w0.x, h ? w1.z : w1.x, h ? w2.z : w2.x, factors, v);
+            multiply<ACT_BF16>(h ? w0.w : w0.y, h ? w1.w : w1.y, h ? w2.w : w2.y, factors, v + 16);
+          }
           if (h == 0) {
             late = use && !__all_sync(0xffffffffu, mbar_wait_bounded(a_empty + 8 * slot, (use - 1) & 1));
             if (late) break;
@@ -380,16 +475,22 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
         uint32_t v[16];
         __syncwarp();
         tmem_load16(tmem + lanes + c, v);
+        if (TWO) {
+          uint32_t w[16];
+          tmem_load16(tmem + lanes + kMaxTokens / 2 + c, w);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
+        }
         if (m.addend) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + bits_to_float(next[i], p.act_dtype));
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + widen<ACT_BF16>(next[i]));
           fetch(c + 16 * kEpilogue);
         }
         if (row < m.O) {
           unsigned short* to = m.out + (size_t)(token0 + c) * p.ldo + row;
 #pragma unroll
           for (int i = 0; i < 16; ++i, to += p.ldo)
-            if (c + i < tokens) *to = bits16(__uint_as_float(v[i]), p.act_dtype);
+            if (c + i < tokens) *to = (unsigned short)pack2<ACT_BF16>(__uint_as_float(v[i]), 0.f);
         }
       }
       __syncwarp();
@@ -405,9 +506,9 @@ __global__ void __launch_bounds__(kThreads, 1) w3_gemm_kernel(const __grid_const
   if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// Tokens of a tile: the tiles go round the SMs, and a round costs 190 + tokens.  One round of 12288 x 4096 measures 18.5 us at 48 tokens, 20.4 at
-// 128, 24.8 at 208 and 27.9 at 256, so that the line is too steep for small tiles; what it picks, of the splits that fit, is all the same within 3 %
-// of the best tile for eight shapes from 3072 x 1024 to 25600 x 5120 at 40 to 1024 tokens (333 of 12288 x 4096: 112 tokens 37.1 us, 128 37.0, 96 50.7).
+// Tokens of a tile: the tiles go round the SMs, and a round costs 190 + tokens.  Too steep a line for small tiles, but of the splits that fit it picks
+// the best in all of eleven shapes from 2560 x 2560 to 25600 x 5120 at 100 to 700 tokens, with scales of either dtype (333 of 12288 x 4096: 112
+// tokens 33.2 us, 176 39.0, 96 45.9; 512 of 6144 x 4096: 176 21.5, 256 25.6, 96 31.3; 512 of 24576 x 4096: 256 76.4, 176 79.7).
 int token_tile(int T, int row_tiles, int sms) {
   int best = 0;
   long long best_cost = 0;
@@ -418,6 +519,24 @@ int token_tile(int T, int row_tiles, int sms) {
     if (!best || cost < best_cost) best = tokens, best_cost = cost;
   }
   return best;
+}
+
+template <bool SCALE_BF16, bool ACT_BF16, bool TWO>
+int launch(const GemmParams& p, int grid, cudaStream_t stream) {
+  static std::mutex lock;
+  static bool ready[64] = {};
+  int device = 0;
+  if (cudaError_t err = cudaGetDevice(&device); err != cudaSuccess) return cuda_fail(err, "cudaGetDevice");
+  if (device < 0 || device >= 64) return fail(FB_ELIMIT, "device ordinal %d outside 0..63", device);
+  {
+    std::lock_guard<std::mutex> guard(lock);
+    if (!ready[device]) {
+      if (cudaError_t err = cudaFuncSetAttribute(w3_gemm_kernel<SCALE_BF16, ACT_BF16, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem); err != cudaSuccess)
+        return cuda_fail(err, "cudaFuncSetAttribute(w3_gemm_kernel)");
+      ready[device] = true;
+    }
+  }
+  return launch_pdl(w3_gemm_kernel<SCALE_BF16, ACT_BF16, TWO>, dim3(grid), dim3(kThreads), kSmem, stream, "w3_gemm_kernel launch", p);
 }
 
 }  // namespace
@@ -437,7 +556,6 @@ extern "C" int fb_w3_gemm(const void* x, int act_dtype, int tokens, const fb_w3_
   if (kSmem > (size_t)info->max_smem_optin) return fail(FB_ELIMIT, "fb_w3_gemm: needs %zu bytes of shared memory", kSmem);
   GemmParams p;
   p.n = n_mats, p.T = tokens, p.G = in_features / 128, p.ldo = out_stride;
-  p.act_dtype = act_dtype, p.scale_dtype = scale_dtype;
   p.status = static_cast<unsigned*>(scratch);
   int row_tiles = 0;
   for (int j = 0; j < n_mats; ++j) {
@@ -463,19 +581,12 @@ extern "C" int fb_w3_gemm(const void* x, int act_dtype, int tokens, const fb_w3_
   if (p.b_stages > kMaxBStages) p.b_stages = kMaxBStages;
   if (!activation_tensor_map(x, tokens, in_features, p.tokens, &p.x_map)) return FB_ECUDA;
 
-  static std::mutex lock;
-  static bool ready[64] = {};
-  int device = 0;
-  if (cudaError_t err = cudaGetDevice(&device); err != cudaSuccess) return cuda_fail(err, "cudaGetDevice");
-  if (device < 0 || device >= 64) return fail(FB_ELIMIT, "device ordinal %d outside 0..63", device);
-  {
-    std::lock_guard<std::mutex> guard(lock);
-    if (!ready[device]) {
-      if (cudaError_t err = cudaFuncSetAttribute(w3_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem); err != cudaSuccess)
-        return cuda_fail(err, "cudaFuncSetAttribute(w3_gemm_kernel)");
-      ready[device] = true;
-    }
-  }
   const int grid = p.tiles < info->sm_count ? p.tiles : info->sm_count;
-  return launch_pdl(w3_gemm_kernel, dim3(grid), dim3(kThreads), kSmem, static_cast<cudaStream_t>(stream), "w3_gemm_kernel launch", p);
+  const cudaStream_t on = static_cast<cudaStream_t>(stream);
+  // two issuers where two accumulators fit and there are as many activation stages as operand slots
+#define FB_LAUNCH(SCALE_BF16, ACT_BF16) \
+  (p.tokens <= kMaxTokens / 2 && p.G > 1 ? launch<SCALE_BF16, ACT_BF16, true>(p, grid, on) : launch<SCALE_BF16, ACT_BF16, false>(p, grid, on))
+  if (scale_dtype == FB_BF16) return act_dtype == FB_BF16 ? FB_LAUNCH(true, true) : FB_LAUNCH(true, false);
+  return act_dtype == FB_BF16 ? FB_LAUNCH(false, true) : FB_LAUNCH(false, false);
+#undef FB_LAUNCH
 }
