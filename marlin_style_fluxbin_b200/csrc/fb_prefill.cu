@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(256) gather_columns_kernel(const unsigned shor
                                                              unsigned short* __restrict__ out, int K) {
   const unsigned short* const row = x + (size_t)blockIdx.x * K;
   unsigned short* const to = out + (size_t)blockIdx.x * K;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
     const uint4 idx = *reinterpret_cast<const uint4*>(perm + k);
     const uint32_t words[4] = {idx.x, idx.y, idx.z, idx.w};
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_prompt_kernel(const unsigned 
   const int index = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (index >= tokens * heads) return;
   const int t = index / heads, head = index - t * heads;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned short* const src = qkv + ((size_t)t * heads + head) * D;
   const uint32_t a = *reinterpret_cast<const uint32_t*>(src + 2 * lane), b = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane);
   if (head >= q_heads + kv_heads) {
@@ -156,27 +158,29 @@ __global__ void __launch_bounds__(256) qknorm_rope_prompt_kernel(const unsigned 
   *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = y1;
 }
 
-// out[t, i] = T(silu(gate_up[t, i])) * gate_up[t, width + i], eight elements per thread.
-__global__ void __launch_bounds__(256) silu_mul_rows_kernel(const unsigned short* __restrict__ gate_up, unsigned short* __restrict__ out, int rows, int width,
-                                                            int out_stride, int dtype) {
-  const int per_row = width / 8;
-  const long long index = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (index >= (long long)rows * per_row) return;
-  const int t = (int)(index / per_row), i = (int)(index - (long long)t * per_row) * 8;
-  const uint4 g = *reinterpret_cast<const uint4*>(gate_up + (size_t)t * 2 * width + i), u = *reinterpret_cast<const uint4*>(gate_up + (size_t)t * 2 * width + width + i);
-  const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
-  uint32_t v[4];
+// out[t, i] = T(silu(gate_up[t, i])) * gate_up[t, width + i], eight elements per thread; a CTA's threads run along one row (a thread's
+// row and column from its index took a 64-bit division: 10.5 us for 512 rows of 12288, 9.7 now, 3.9 TB/s of reads and writes that mostly stay in L2).
+__global__ void __launch_bounds__(256) silu_mul_rows_kernel(const unsigned short* __restrict__ gate_up, unsigned short* __restrict__ out, int width, int out_stride,
+                                                            int dtype) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const size_t t = blockIdx.x;
+  for (long long at = ((long long)blockIdx.y * blockDim.x + threadIdx.x) * 8; at < width; at += (long long)gridDim.y * blockDim.x * 8) {
+    const int i = (int)at;
+    const uint4 g = *reinterpret_cast<const uint4*>(gate_up + (size_t)t * 2 * width + i), u = *reinterpret_cast<const uint4*>(gate_up + (size_t)t * 2 * width + width + i);
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
+    uint32_t v[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    uint32_t both = 0u;
+    for (int k = 0; k < 4; ++k) {
+      uint32_t both = 0u;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float gate = bits_to_float((unsigned short)(gw[k] >> (16 * h)), dtype), up = bits_to_float((unsigned short)(uw[k] >> (16 * h)), dtype);
-      both |= (uint32_t)bits16(round_to(gate / (1.f + __expf(-gate)), dtype) * up, dtype) << (16 * h);
+      for (int h = 0; h < 2; ++h) {
+        const float gate = bits_to_float((unsigned short)(gw[k] >> (16 * h)), dtype), up = bits_to_float((unsigned short)(uw[k] >> (16 * h)), dtype);
+        both |= (uint32_t)bits16(round_to(gate / (1.f + __expf(-gate)), dtype) * up, dtype) << (16 * h);
+      }
+      v[k] = both;
     }
-    v[k] = both;
+    *reinterpret_cast<uint4*>(out + (size_t)t * out_stride + i) = make_uint4(v[0], v[1], v[2], v[3]);
   }
-  *reinterpret_cast<uint4*>(out + (size_t)t * out_stride + i) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
 // *flag (device-visible host memory): 1 if perm is the identity, else 0.
@@ -231,8 +235,7 @@ extern "C" int fb_gather_columns(const void* x, const int16_t* perm, void* out, 
   if (rows < 1 || in_features < 128 || in_features % 128 || in_features > 32767) return fail(FB_ELIMIT, "fb_gather_columns: K=%d must be a multiple of 128 below 32768", in_features);
   if (!aligned(perm, 16) || !aligned(out, 16)) return fail(FB_EINVAL, "fb_gather_columns: perm and out must be 16-byte aligned");
   if (overlaps(out, (size_t)rows * in_features * 2, x, (size_t)rows * in_features * 2)) return fail(FB_EALIAS, "fb_gather_columns: out overlaps x");
-  gather_columns_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(u16(x), perm, u16(out), in_features);
-  return launched("gather_columns launch");
+  return launch_pdl(gather_columns_kernel, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), "gather_columns launch", u16(x), perm, u16(out), in_features);
 }
 
 extern "C" int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, const void* k_weight, const void* cosv, const void* sinv, void* q_out, void* k_cache,
@@ -246,9 +249,8 @@ extern "C" int fb_qknorm_rope_prompt(const void* qkv, const void* q_weight, cons
     return fail(FB_EINVAL, "fb_qknorm_rope_prompt: tensors must be 4-byte aligned");
   const long long warps = (long long)tokens * (q_heads + 2 * kv_heads);
   if (warps > 0x7fffffff) return fail(FB_ELIMIT, "fb_qknorm_rope_prompt: too many tokens");
-  qknorm_rope_prompt_kernel<<<(int)((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(u16(qkv), u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), u16(q_out), u16(k_cache),
-                                                                                                u16(v_cache), tokens, q_heads, kv_heads, max_positions, eps, dtype);
-  return launched("qknorm_rope_prompt launch");
+  return launch_pdl(qknorm_rope_prompt_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, static_cast<cudaStream_t>(stream), "qknorm_rope_prompt launch", u16(qkv),
+                    u16(q_weight), u16(k_weight), u16(cosv), u16(sinv), u16(q_out), u16(k_cache), u16(v_cache), tokens, q_heads, kv_heads, max_positions, eps, dtype);
 }
 
 extern "C" int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int width, int out_stride, int dtype, fb_stream_t stream) {
@@ -256,9 +258,10 @@ extern "C" int fb_silu_mul_rows(const void* gate_up, void* out, int rows, int wi
   if (bad_dtype(dtype)) return fail(FB_EINVAL, "fb_silu_mul_rows: dtype must be FB_F16 or FB_BF16");
   if (rows < 1 || width < 8 || width % 8 || out_stride < width || out_stride % 8) return fail(FB_ELIMIT, "fb_silu_mul_rows: width and stride must be multiples of 8");
   if (!aligned(gate_up, 16) || !aligned(out, 16)) return fail(FB_EINVAL, "fb_silu_mul_rows: tensors must be 16-byte aligned");
-  const long long blocks = ((long long)rows * (width / 8) + 255) / 256;
-  silu_mul_rows_kernel<<<(int)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(u16(gate_up), u16(out), rows, width, out_stride, dtype);
-  return launched("silu_mul_rows launch");
+  const int per_row = width / 8, chunks = (per_row + 255) / 256 < 65535 ? (per_row + 255) / 256 : 65535;
+  const int threads = chunks < 65535 ? ((per_row + chunks - 1) / chunks + 31) / 32 * 32 : 256;
+  return launch_pdl(silu_mul_rows_kernel, dim3(rows, chunks), dim3(threads), 0, static_cast<cudaStream_t>(stream), "silu_mul_rows launch", u16(gate_up), u16(out), width,
+                    out_stride, dtype);
 }
 
 extern "C" int fb_identity_order(const int16_t* perm, int in_features, int* flag, fb_stream_t stream) {
