@@ -247,8 +247,10 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
 
   // The column order is part of the weights: this thread's index for the first K block needs no wait.  With one CTA per SM
   // it is requested ahead of the staged weights, behind which it would arrive later than the activations could be read.
-  // With two, the gathers of all CTAs would then meet at the few L2 lines of x at the same time, and cost more than that.
-  // us, cold, early / late: 1024x4096 (one CTA) 3.13 / 3.35, 1024x12288 5.69 / 6.33; 4096x4096 (two) 4.51 / 4.32, 12288x4096 8.40 / 8.37.
+  // With two, the gathers of all CTAs would then meet at the few L2 lines of x at the same time, and cost more than that; with CTAs
+  // on fewer than half of the SMs there is nothing to get ahead of.
+  // us, cold, early / late: 1024x4096 (one CTA) 3.13 / 3.35, 1024x12288 5.69 / 6.33; 4096x4096 (two) 4.51 / 4.32, 12288x4096 8.40 / 8.37; 128x17408
+  // (56 CTAs, decoded) 8.95 / 8.77.
   const int sb = (int)blockIdx.y, kb_begin = sb * p.S;
   int el_idx = 0;
   auto fetch_idx = [&](int kb_) {
@@ -1015,7 +1017,7 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   if (scratch) bind_scratch(p, scratch);
   const Plan plan = make_plan(m, p.nKB, p.nRU, *info);
   p.S = plan.S;
-  p.early_order = plan.slices * plan.nSB <= info->sm_count ? 1 : 0;
+  p.early_order = plan.slices * plan.nSB <= info->sm_count && 2 * plan.slices * plan.nSB > info->sm_count ? 1 : 0;
   p.units_per_slice = p.nRU / plan.slices;
   p.units_extra = p.nRU % plan.slices;
   p.nSB = plan.nSB;
