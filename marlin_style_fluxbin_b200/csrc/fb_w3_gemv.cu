@@ -47,7 +47,9 @@
 // csrc/lut8_unsigned.cuh:12-27.  Extension over the reference: fp16 or bf16 scales and
 // an optional per-(group,row) zero point, y += scale*(4-zero)*sum(x_group); the rounding
 // correction of the dequantised-weight arithmetic (csrc/w3_lut.cu:105-122) is extended to zero
-// points 3 and 4, the two for which +/-3 are the only inexact products.
+// points 3 and 4, the two for which +/-3 are the only inexact products.  It costs one look-up per eight weights beside the three of the
+// planes (two before, masks of +3 and of -3): us at one row, cold, in a graph, before -> now 1024x4096 3.38 -> 3.08, 4096x4096 4.36 -> 4.13,
+// 12288x4096 9.36 -> 8.55, 4096x12288 10.46 -> 9.76; 12288x4096 at 2 / 3 / 4 rows 15.7 -> 14.4 / 21.6 -> 19.7 / 28.0 -> 25.4.
 #include <mutex>
 #include <new>
 #include <type_traits>
@@ -170,12 +172,21 @@ __device__ __forceinline__ uint64_t fma2_lds(uint64_t acc, uint32_t a0, uint32_t
       : "l"(acc), "r"(a0), "r"(a1), "l"(w));
   return r;
 }
-// Shared-memory load at a 32-bit address plus a compile-time offset (folded into the instruction).
-template <int OFFSET>
-__device__ __forceinline__ float lds_at(uint32_t address) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(address), "n"(OFFSET));
-  return v;
+// {table entry at a0, table entry at a1}, and acc + w * both
+__device__ __forceinline__ uint64_t lds2(uint32_t a0, uint32_t a1) {
+  uint64_t r;
+  asm volatile(
+      "{\n\t.reg .f32 lo, hi;\n\t"
+      "ld.shared.f32 lo, [%1];\n\t"
+      "ld.shared.f32 hi, [%2];\n\t"
+      "mov.b64 %0, {lo, hi};\n\t}"
+      : "=l"(r)
+      : "r"(a0), "r"(a1));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t both, uint64_t w, uint64_t acc) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(both), "l"(w));
+  return acc;
 }
 __device__ __forceinline__ float sum2(uint64_t v) {
   float lo, hi;
@@ -664,23 +675,23 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
       // per activation row and group half: an (even byte step, odd byte step) pair of sums of
       // entry(plane 0) + 2 entry(plane 1) - 4 entry(plane 2)
       uint64_t acc[M][2];
-      float corr[M][2];
+      // with the rounding correction: the planes' sums by themselves, what became of them in a group, and (+3) - (-3)
+      uint64_t each[M][4];
+      float dot[M][2], corr[M][2];
 #pragma unroll
       for (int m = 0; m < M; ++m)
 #pragma unroll
         for (int jh = 0; jh < 2; ++jh) {
-          corr[m][jh] = 0.f;
+          dot[m][jh] = corr[m][jh] = 0.f;
           acc[m][jh] = 0ull;
+          each[m][2 * jh] = each[m][2 * jh + 1] = 0ull;
         }
       const uint64_t two2 = 0x4000000040000000ull, minus_four2 = 0xc0800000c0800000ull;  // {2.f, 2.f}, {-4.f, -4.f}
+      // weights of the planes in (+3) - (-3), by zero point
+      const uint64_t one2 = 0x3f8000003f800000ull, minus_one2 = 0xbf800000bf800000ull;
+      const uint64_t at3[2] = {zp[0] == 3u ? one2 : 0ull, zp[1] == 3u ? one2 : 0ull}, at4[2] = {zp[0] == 3u ? 0ull : minus_one2, zp[1] == 3u ? 0ull : minus_one2};
+      const uint64_t at_f[2] = {zp[0] == 3u ? minus_one2 : one2, zp[1] == 3u ? minus_one2 : one2};
       {
-        // the rounding correction needs the zero points during the lookups (code - zero = +/-3 is
-        // code 7 / 1 at zero point 4 and code 6 / 0 at zero point 3)
-        uint32_t flip[2] = {0u, 0u};
-        if (CORRECT) {
-          flip[0] = zp[0] == 3u ? 0xffffffffu : 0u;
-          flip[1] = zp[1] == 3u ? 0xffffffffu : 0u;
-        }
         // staged words are fetched one (half, word) step ahead of their use, into two register
         // sets used in turn
         auto fetch = [&](int step, uint32_t (&dst)[3]) {
@@ -691,11 +702,40 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
         };
         auto walk = [&](int step, const uint32_t (&w)[3]) {
           const int jh = step >> 2, jw = step & 3;
-          uint32_t plus3 = 0, minus3 = 0;
           if (CORRECT) {
-            const uint32_t low = w[0] ^ flip[jh];
-            plus3 = low & w[1] & ~w[2];   // code - zero = +3 (the stored high plane is inverted)
-            minus3 = low & ~w[1] & w[2];  // code - zero = -3
+            // The rounding correction needs (+3) - (-3) of code - zero.  With one more plane, f = b0 ? b1 : b2', that is f - b2' at zero point 4
+            // and b1 - f at zero point 3: four look-ups summed by themselves, where masks of the two codes took five.
+            uint32_t planes[4] = {w[0], w[1], w[2], 0u};
+            asm("lop3.b32 %0, %1, %2, %3, 0xCA;" : "=r"(planes[3]) : "r"(w[0]), "r"(w[1]), "r"(w[2]));
+#pragma unroll
+            for (int bp = 0; bp < 2; ++bp)
+#pragma unroll
+              for (int pl = 0; pl < 4; ++pl) {
+                const uint32_t a0 = lookup_address(planes[pl], 2 * bp, xl[jh][jw][2 * bp]);
+                const uint32_t a1 = lookup_address(planes[pl], 2 * bp + 1, xl[jh][jw][2 * bp + 1]);
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                  if constexpr (M != 3) {
+                    each[m][pl] = add2_lds(each[m][pl], a0 + (uint32_t)(m * 128), a1 + (uint32_t)(m * 128));
+                  } else {  // twelve sums do not fit the registers (1024 x 4096 7.5 us; in this form 6.4): two a row
+                    const uint64_t both = lds2(a0 + (uint32_t)(m * 128), a1 + (uint32_t)(m * 128));
+                    if (pl < 3) each[m][0] = fma2(both, pl == 0 ? one2 : pl == 1 ? two2 : minus_four2, each[m][0]);
+                    if (pl > 0) each[m][1] = fma2(both, pl == 1 ? at3[jh] : pl == 2 ? at4[jh] : at_f[jh], each[m][1]);
+                  }
+                }
+              }
+            if (jw == 3) {  // the end of a group's half of the walk
+#pragma unroll
+              for (int m = 0; m < M; ++m) {
+                float e[4];
+#pragma unroll
+                for (int pl = 0; pl < 4; ++pl) e[pl] = sum2(each[m][pl]), each[m][pl] = 0ull;
+                dot[m][jh] = M == 3 ? e[0] : e[0] + 2.f * e[1] - 4.f * e[2];
+                const float more = M == 3 ? e[1] : (zp[jh] == 3u ? e[1] - e[3] : e[3] - e[2]);
+                corr[m][jh] = fabsf(dot[m][jh]) <= 3.4028235e38f ? more : 0.f;  // infinite terms (of any code but 4) are all in the dot already
+              }
+            }
+            return;
           }
 #pragma unroll
           for (int bp = 0; bp < 2; ++bp) {  // byte steps 2bp (even) and 2bp + 1 (odd) make one packed add
@@ -707,15 +747,6 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
               for (int m = 0; m < M; ++m) {  // activation row m sits m * 128 bytes further
                 const uint32_t b0 = a0 + (uint32_t)(m * 128), b1 = a1 + (uint32_t)(m * 128);
                 acc[m][jh] = pl == 0 ? add2_lds(acc[m][jh], b0, b1) : fma2_lds(acc[m][jh], b0, b1, pl == 1 ? two2 : minus_four2);
-              }
-            }
-            if (CORRECT) {
-#pragma unroll
-              for (int b = 2 * bp; b < 2 * bp + 2; ++b) {
-                const uint32_t ap = lookup_address(plus3, b, xl[jh][jw][b]);
-                const uint32_t am = lookup_address(minus3, b, xl[jh][jw][b]);
-#pragma unroll
-                for (int m = 0; m < M; ++m) corr[m][jh] += lds_at<0>(ap + (uint32_t)(m * 128)) - lds_at<0>(am + (uint32_t)(m * 128));
               }
             }
           }
@@ -746,7 +777,7 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
         float term[2];
 #pragma unroll
         for (int jh = 0; jh < 2; ++jh) {
-          float d = sum2(acc[m][jh]);
+          float d = CORRECT ? dot[m][jh] : sum2(acc[m][jh]);
           if (any_zeros) d += (4.f - (float)zp[jh]) * sx_cur[m][jh];
           term[jh] = d * sc[jh];
           if (CORRECT) {
