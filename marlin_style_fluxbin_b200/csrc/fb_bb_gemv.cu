@@ -2,7 +2,7 @@
 // packed one bit per weight per base, in groups of 128 inputs.
 //
 // Same skeleton as the W3 GEMV (HBM-bound byte work, see fb_w3_gemv.cu): a K block is TWO groups
-// (one for matrices of fewer than 128 row units);
+// (one for small matrices);
 // a CTA holds 32 signed activation tables per group (2 bases x 16 chunks of 8 inputs, entries are
 // sums of +/- x*col in ascending order) laid out entry-major so that the bank of a lookup is the
 // table number; lane = output row; lanes walk the 32 (base, chunk) pairs of a group in a
@@ -482,9 +482,12 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   p.status = reinterpret_cast<unsigned*>(base);
   p.combine = reinterpret_cast<unsigned long long*>(base + kCombineOffset);
   p.nRU = (p.O + kUnitRows - 1) / kUnitRows;
-  // Two groups per K block halve the per-byte cost of a unit; with few row units the second table
-  // build on the critical path costs more than that saves.
-  const int gpb = p.nRU >= 128 && p.G >= 2 ? 2 : 1;
+  // Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay
+  // once warps have units of one group to spare, more than one each with matrix-wide scales, more than four with scales per group (more
+  // constants per unit either way; two where interleaved codes make a unit longer).  us, one group / two: matrix-wide 2048x4096 (0.9 units a warp) 3.18 / 3.31, 3072x4096 (1.3) 4.10 / 3.62,
+  // 3072x1024 (0.3) 3.38 / 4.60, 1024x12288 (1.3) 4.02 / 3.62; per group 4064x4096 (1.7) 4.23 / 4.45, 2048x12288 (2.6) 5.41 / 5.55, 3072x12288 (3.9)
+  // 6.56 / 6.52; interleaved 4096x4096 (1.7) 5.27 / 5.30, 5120x5120 (2.7) 6.90 / 6.81.
+  const int gpb = p.G >= 2 && p.nRU * p.G > kCtasPerSm * info->sm_count * kWarps * (p.global_mode ? 1 : p.interleaved ? 2 : 4) ? 2 : 1;
   p.nKB = (p.G + gpb - 1) / gpb;
   int c = kCtasPerSm * info->sm_count / p.nKB;
   if (c < 1) c = 1;
