@@ -45,6 +45,7 @@ constexpr int kWarps = 8;
 constexpr int kCtasPerSm = 2;
 constexpr int kGroupLutBytes = 32768;       // 256 entries x 32 tables x 4 B
 constexpr int kGroupSparseBytes = 2048;     // 2 tables x 256 entries
+constexpr int kMaxSalient = 256;            // residual columns
 
 struct BBParams {
   const void* x;
@@ -64,6 +65,7 @@ struct BBParams {
   unsigned* status;
   int O, K, G, nKB, nRU;
   int act_dtype, interleaved, global_mode, n_sal;
+  int more_most, more_full;     // residual columns of a group beyond its first: at most, and groups that have as many
   int sal_pairs;                // the residual values of two groups lie in one aligned 32-bit word
   int slots;                    // staged units per warp
   int units_few, units_extra;   // row units of a slice; slices that have one more
@@ -116,9 +118,11 @@ __device__ __forceinline__ float2 ldgf2(const float* at) {
   asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(at));
   return v;
 }
+__device__ __forceinline__ void prefetch_l2(const void* at) { asm volatile("prefetch.global.L2 [%0];" ::"l"(at)); }
 __device__ __forceinline__ float half_bits(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 
-template <bool INTERLEAVED, bool GLOBAL, int GPB>
+// MORE (matrix-wide scales): a group carries several residual columns.
+template <bool INTERLEAVED, bool GLOBAL, int GPB, bool MORE>
 __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const BBParams p) {
   constexpr int kUnitBytes = GPB * kGroupBytes;  // staged per unit
   constexpr int kLutBytes = GPB * kGroupLutBytes, kSparseLutBytes = GLOBAL ? 0 : GPB * kGroupSparseBytes;
@@ -130,6 +134,8 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   float* const sparse_lut = reinterpret_cast<float*>(smem + kLutBytes);
   const uint32_t ring_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(warp * S * kUnitBytes);
   const uint32_t bars_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(kWarps * S * kUnitBytes + warp * S * 8);
+  // activations of the residual columns beyond one per group (more columns than groups): [group][p.more_most]
+  float* const more_x = reinterpret_cast<float*>(smem + kLutBytes + kSparseLutBytes + kWarps * S * (kUnitBytes + 8));
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -176,11 +182,17 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     r_idx = g * 128 + (int)ldg16(p.indices + g * 8 + r_j);
     r_col = ldgf(p.scols + (size_t)(g * 8 + r_j) * 2 + r_base);
   }
-  int sal_at[GPB];  // the residual column that a group's contribution carries
+  // the residual columns that a group's contribution carries, dealt round-robin: the first, and of the `more` others thread's
+  int sal_at[GPB], more[GPB], more_at[GPB];
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) {
     const int g = GPB * kb + gi;
     sal_at[gi] = GLOBAL && gi < ngroups && g < p.n_sal ? (int)ldg32(p.sal_idx + g) : -1;
+    more[gi] = 0, more_at[gi] = -1;
+    if (MORE && gi < ngroups) {
+      more[gi] = p.more_most - (g < p.more_full ? 0 : 1);
+      if ((int)threadIdx.x < more[gi]) more_at[gi] = (int)ldg32(p.sal_idx + g + ((int)threadIdx.x + 1) * p.G);
+    }
   }
 
   // Staging of this warp's units in order, each into the slot that was read last: one bulk copy per group.  Rows past O in
@@ -237,7 +249,13 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     }
   };
   Constants next;
-  if (first < end) request(first, next);
+  if (first < end) {
+    request(first, next);
+    if (MORE) {  // the rest of a row's residual values, which are read one by one
+      const char* const values = reinterpret_cast<const char*>(p.sal + (size_t)min(first * kUnitRows + lane, p.O - 1) * p.n_sal);
+      for (int at = 0; at < 2 * p.n_sal; at += 32) prefetch_l2(values + at);
+    }
+  }
 
   // Table addresses and word offsets of the rotated walk, the same for every unit.  Lookups use 32-bit shared-window
   // addresses: entry * 128 + table offset is ONE dp4a (a byte dot product whose only non-zero weight, 128, sits at the
@@ -278,6 +296,11 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
   if (r_live) r_x = load_act(p.x, p.act_dtype, r_idx);
+  if (MORE) {
+#pragma unroll
+    for (int gi = 0; gi < GPB; ++gi)
+      if (more_at[gi] >= 0) more_x[gi * p.more_most + (int)threadIdx.x] = load_act(p.x, p.act_dtype, more_at[gi]);
+  }
   for (int s = 1; s < S && pf_ru < end; ++s) issue_next();  // the rest of the ring, behind the activations
 
   // ---- 32 signed tables per group ----
@@ -421,9 +444,14 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
 #pragma unroll
       for (int gi = 0; gi < GPB; ++gi) {
         if (sal_at[gi] >= 0) value = __fmaf_rn(__uint_as_float(now.sal[gi]), sal_x[gi], value);
-        if (p.n_sal > p.G && gi < ngroups && row < p.O)  // more residual columns than groups: rare
+        if (MORE) {
+          const __nv_bfloat16* const from = p.sal + (size_t)min(row, p.O - 1) * p.n_sal + GPB * kb + gi;
+#pragma unroll 4
+          for (int e = 0; e < more[gi]; ++e) value = __fmaf_rn(__bfloat162float(from[(e + 1) * p.G]), more_x[gi * p.more_most + e], value);
+        } else if (p.n_sal > p.G && gi < ngroups && row < p.O) {  // one or two
           for (int at = GPB * kb + gi + p.G; at < p.n_sal; at += p.G)
             value = __fmaf_rn(__bfloat162float(p.sal[(size_t)row * p.n_sal + at]), load_act(p.x, p.act_dtype, p.sal_idx[at]), value);
+        }
       }
     }
     settle();  // the previous unit's answer has long arrived
@@ -443,7 +471,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
 
 constexpr size_t kCombineOffset = 16384;  // after the status block: one 64-bit word per output row
 
-template <bool INTERLEAVED, bool GLOBAL, int GPB>
+template <bool INTERLEAVED, bool GLOBAL, int GPB, bool MORE>
 int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cudaStream_t stream) {
   static std::mutex lock;
   static bool ready[64] = {};
@@ -452,7 +480,7 @@ int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cu
   {
     std::lock_guard<std::mutex> guard(lock);
     if (!ready[device]) {
-      cudaError_t err = cudaFuncSetAttribute(bb_gemv_kernel<INTERLEAVED, GLOBAL, GPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+      cudaError_t err = cudaFuncSetAttribute(bb_gemv_kernel<INTERLEAVED, GLOBAL, GPB, MORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
       if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(bb_gemv_kernel)");
       ready[device] = true;
     }
@@ -467,7 +495,7 @@ int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cu
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = pdl && pdl_allowed() ? 1 : 0;
-  cudaError_t err = cudaLaunchKernelEx(&config, bb_gemv_kernel<INTERLEAVED, GLOBAL, GPB>, p);
+  cudaError_t err = cudaLaunchKernelEx(&config, bb_gemv_kernel<INTERLEAVED, GLOBAL, GPB, MORE>, p);
   if (err != cudaSuccess) return cuda_fail(err, "bb_gemv_kernel launch");
   return FB_OK;
 }
@@ -496,19 +524,28 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   p.units_few = p.nRU / c, p.units_extra = p.nRU % c;
   p.sal_pairs = p.global_mode && p.n_sal % 2 == 0 && aligned(p.sal, 4) ? 1 : 0;
   const int per_warp = ((p.nRU + c - 1) / c + kWarps - 1) / kWarps;
-  const int max_slots = gpb == 1 ? 4 : (p.global_mode ? 3 : 2);
+  // Where a group carries three residual columns and more, up to 1 + more_most (as many do the first more_full groups), their activations
+  // are gathered once per CTA and their values requested ahead; a single one or two are read where they are used, which costs the
+  // others less.  us at 32 columns, gathered / as they are used: 17x128 2.4 / 3.2, 256x512 (8 a group) 2.6 / 3.1, 8192x512 3.5 / 3.8, 512x1024 (4) 2.86 / 2.96,
+  // 2048x2048 (2) 3.10 / 3.09, 5120x2560 (1.6) 4.27 / 4.00.
+  const bool more = p.global_mode && p.n_sal >= 3 * p.G;
+  p.more_most = more ? (p.n_sal - 1) / p.G : 0, p.more_full = more ? p.n_sal - p.more_most * p.G : 0;
+  const size_t more_bytes = (size_t)gpb * p.more_most * sizeof(float);
+  const int max_slots = gpb == 1 ? 4 : (p.global_mode && more_bytes <= 512 ? 3 : 2);  // two CTAs per SM
   p.slots = per_warp < max_slots ? (per_warp < 1 ? 1 : per_warp) : max_slots;
-  const size_t smem = (size_t)gpb * (kGroupLutBytes + (p.global_mode ? 0 : kGroupSparseBytes)) + (size_t)kWarps * p.slots * (gpb * kGroupBytes + 8);
+  const size_t smem = (size_t)gpb * (kGroupLutBytes + (p.global_mode ? 0 : kGroupSparseBytes)) + (size_t)kWarps * p.slots * (gpb * kGroupBytes + 8) + more_bytes;
   const bool pdl = (flags & FB_W3_NO_PDL) == 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (gpb == 2) {
-    if (p.global_mode) return launch<false, true, 2>(p, grid, smem, info->max_smem_optin, pdl, s);
-    if (p.interleaved) return launch<true, false, 2>(p, grid, smem, info->max_smem_optin, pdl, s);
-    return launch<false, false, 2>(p, grid, smem, info->max_smem_optin, pdl, s);
+    if (more) return launch<false, true, 2, true>(p, grid, smem, info->max_smem_optin, pdl, s);
+    if (p.global_mode) return launch<false, true, 2, false>(p, grid, smem, info->max_smem_optin, pdl, s);
+    if (p.interleaved) return launch<true, false, 2, false>(p, grid, smem, info->max_smem_optin, pdl, s);
+    return launch<false, false, 2, false>(p, grid, smem, info->max_smem_optin, pdl, s);
   }
-  if (p.global_mode) return launch<false, true, 1>(p, grid, smem, info->max_smem_optin, pdl, s);
-  if (p.interleaved) return launch<true, false, 1>(p, grid, smem, info->max_smem_optin, pdl, s);
-  return launch<false, false, 1>(p, grid, smem, info->max_smem_optin, pdl, s);
+  if (more) return launch<false, true, 1, true>(p, grid, smem, info->max_smem_optin, pdl, s);
+  if (p.global_mode) return launch<false, true, 1, false>(p, grid, smem, info->max_smem_optin, pdl, s);
+  if (p.interleaved) return launch<true, false, 1, false>(p, grid, smem, info->max_smem_optin, pdl, s);
+  return launch<false, false, 1, false>(p, grid, smem, info->max_smem_optin, pdl, s);
 }
 
 struct BBPrepared : Prepared {
@@ -600,7 +637,7 @@ extern "C" int fb_bb_global_gemv(const void* x, int act_dtype, const uint8_t* co
   if (rc) return rc;
   if (!row_scales || !col_scales) return fail(FB_EINVAL, "fb_bb_global_gemv: scales must be non-null");
   if (!aligned(col_scales, 16)) return fail(FB_EINVAL, "fb_bb_global_gemv: column scales must be 16-byte aligned");
-  if (n_salient < 0 || n_salient > 256 || (n_salient > 0 && (!salient_idx || !salient)))
+  if (n_salient < 0 || n_salient > kMaxSalient || (n_salient > 0 && (!salient_idx || !salient)))
     return fail(FB_EINVAL, "fb_bb_global_gemv: salient columns: 0..256 with index and value tensors");
   if (flags & ~FB_W3_NO_PDL) return fail(FB_EINVAL, "fb_bb_global_gemv: unknown flag bits 0x%x", flags);
   BBParams p = {};

@@ -38,3 +38,11 @@ def test_scales_per_group(o, groups, kernel):
     out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
     _native.bb_gemv(x.cuda(), PackedHybridLinear(payload, kernel=kernel).cuda().layout(), out)
     _check(out, x, decode_layout(convert_artifact(payload, kernel=kernel), torch.float32).double(), groups)
+
+
+@pytest.mark.parametrize("o,groups,salient", ((33, 1, 256), (4099, 2, 255), (12320, 3, 32), (9600, 2, 5)))
+def test_more_residual_columns_than_groups(o, groups, salient):
+    layout, _, x = make_global_case(o, groups * 128, seed=o + groups, n_sal=min(salient, groups * 128))
+    out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    binary_global.global_two_base_m1_out(x.cuda(), {name: value.cuda() for name, value in layout.items()}, out)
+    _check(out, x, binary_global.materialize(layout, torch.float64), groups)
