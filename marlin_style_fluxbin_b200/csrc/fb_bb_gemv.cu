@@ -26,10 +26,10 @@
 // constant is therefore requested before it is needed: column scales and indices at once, ahead of the codes (behind them they
 // arrived after the activations: 5.04 us against 4.39 for 4096 x 4096 with scales per group), a row's scales and residual one
 // unit ahead of their use (requested where they were used, every unit of a warp waited for HBM once more).  A unit
-// costs about 250 instructions (419 before, with the share of a CTA computed by 64-bit divisions, ring slots by a modulo).
+// costs 365 instructions (419 before, with ring slots by a modulo); the share of a CTA takes no 64-bit divisions any more.
 // us on a B200, weights cold, in a graph, before -> now: matrix-wide scales 1024x4096 3.27 -> 2.78, 4096x4096 5.16 -> 3.81,
 // 12288x4096 8.83 -> 7.31, 4096x12288 8.37 -> 6.98; scales per group, planar 4.00 -> 2.82, 6.25 -> 4.39, 9.92 -> 7.62,
-// 9.97 -> 7.62, interleaved 4.35 -> 3.09, 8.50 -> 5.30, 16.5 -> 10.1, 16.5 -> 10.1.
+// 9.97 -> 7.62, interleaved 4.35 -> 3.09, 8.50 -> 5.30, 16.5 -> 10.1, 16.5 -> 10.1 (and 4096x4096 planar 4.24 with one group per K block).
 #include <mutex>
 #include <new>
 
