@@ -250,7 +250,16 @@ __global__ void __launch_bounds__(kThreads, 1) w3_rows_kernel(const __grid_const
   // + 16, which are eight operand words (low half: first, high half: second) ----
   const int items_x = ng * M;
   const int k_in_group = (((int)threadIdx.x >> 1) & 3) * 32 + ((int)threadIdx.x & 1) * 8;
-  auto locate = [&](int i, int& g, int& m) { g = (int)((unsigned)i * p.rows_inv >> 16), m = i - g * M; };
+  // Through a column order row by row: the values that a CTA gathers of a row share sectors (four a sector at a quarter of 4096
+  // inputs), which the L1 holds for a few rows but not for sixteen.  us, cold, in a graph, group by group / row by row, 16 rows: 1024x4096
+  // 15.7 / 8.9, 4096x4096 15.9 / 11.6, 12288x4096 27.0 / 22.6, 4096x12288 38.2 / 33.9; 4 rows 4096x4096 7.2 / 6.8.  In identity order the rows
+  // of a group come first: 2048x2048 at 16 rows 4.17 / 4.28, 4096x4096 6.71 / 6.59.
+  auto locate = [&](int i, int& g, int& m) {
+    if (GATHER)
+      m = (int)((unsigned)(i >> 1) * np_inv >> 16), g = i - m * ng;
+    else
+      g = (int)((unsigned)i * p.rows_inv >> 16), m = i - g * M;
+  };
   uint4 idx_lo = make_uint4(0u, 0u, 0u, 0u), idx_hi = idx_lo, raw_lo = idx_lo, raw_hi = idx_lo;
   auto fetch_idx = [&](int i) {  // the column order is part of the weights: no wait
     int g, m;
