@@ -250,8 +250,9 @@ int fb_w3_finish(const float* partials, int splits, int out_features, void* out,
  * are combined by 64-bit fixed-point integer adds (steps of 2^-26, order-independent, so
  * repeat-exact; a group's term that is not finite or is 8192 or more in magnitude gives NaN).
  * Any O in 1..65536; x and codes 16-byte aligned; scratch zero-filled once and 256-byte aligned, not
- * shared with other kernels, sized by fb_bb_gemv_scratch_bytes(O, K, 0).  Codes, scales and indices (here and
- * below) are constants: they are read ahead of the wait on the launch ahead in the stream.
+ * shared with other kernels, sized by fb_bb_gemv_scratch_bytes(O, K, 0).  The codes (here and
+ * below) are constants: they are read ahead of the wait on the launch ahead in the stream.  All else may be
+ * written by that launch.
  * Replaces the reference's m1_out of the v5 kernels (csrc/m1_v5.cu:132-195); all the
  * reference's kernel names map to this one entry point.
  */

@@ -88,7 +88,10 @@ def workspace_bytes(out_features: int, in_features: int) -> int:
 
 
 def global_two_base_m1_out(x, layout, out):
-    """``out[1,O] = x[1,K] . W^T`` on the current CUDA stream; allocation-free after warm-up."""
+    """``out[1,O] = x[1,K] . W^T`` on the current CUDA stream; allocation-free after warm-up.
+
+    Scales, residual values and indices may be written by what runs directly ahead on the stream.  The codes are read while a launch
+    that releases its dependents early (as this package's do) may still run: they must be complete before that one starts."""
     o, k = validate_layout(layout)
     if tuple(x.shape) != (1, k) or tuple(out.shape) != (1, o) or out.dtype != x.dtype:
         raise ValueError("x/out shape or dtype mismatch")

@@ -22,14 +22,13 @@
 //    residual columns): both groups of a unit share one sum per base; row scales are applied, and the residual
 //    columns dealt, per contribution.
 //
-// What bounds it: the launch chain and, per unit, latencies; a unit carries two thirds of a W3 unit's bytes.  Whatever is
-// constant is therefore requested before it is needed: column scales and indices at once, ahead of the codes (behind them they
-// arrived after the activations: 5.04 us against 4.39 for 4096 x 4096 with scales per group), a row's scales and residual one
-// unit ahead of their use (requested where they were used, every unit of a warp waited for HBM once more).  A unit
-// costs 365 instructions (419 before, with ring slots by a modulo); the share of a CTA takes no 64-bit divisions any more.
-// us on a B200, weights cold, in a graph, before -> now: matrix-wide scales 1024x4096 3.27 -> 2.78, 4096x4096 5.16 -> 3.81,
-// 12288x4096 8.83 -> 7.31, 4096x12288 8.37 -> 6.98; scales per group, planar 4.00 -> 2.82, 6.25 -> 4.39, 9.92 -> 7.62,
-// 9.97 -> 7.62, interleaved 4.35 -> 3.09, 8.50 -> 5.30, 16.5 -> 10.1, 16.5 -> 10.1 (and 4096x4096 planar 4.24 with one group per K block).
+// What bounds it: the launch chain and, per unit, latencies; a unit carries two thirds of a W3 unit's bytes.  Only the codes are read
+// ahead of the wait for the launch ahead, which may write everything else: scales, residual and refinement are brought to the L2
+// before it and requested together with the activations behind it, a row's one unit ahead of their use.
+// us on a B200, weights cold, in a graph, 1024x4096 / 4096x4096 / 12288x4096 / 4096x12288: matrix-wide scales 2.88 / 4.13 / 7.70 / 7.18,
+// scales per group, planar 3.19 / 4.43 / 7.58 / 7.63, interleaved 3.26 / 5.36 / 10.6 / 10.6.  Read ahead of the wait they would take
+// 2.78 / 3.82 / 7.32 / 6.98, 2.85 / 4.24 / 7.63 / 7.63 and 3.09 / 5.27 / 10.1 / 10.1; without the prefetch and the unit ahead, ring
+// slots by a modulo and shares by 64-bit divisions it was 3.27 / 5.15 / 8.82 / 8.43, 4.02 / 6.26 / 9.96 / 9.97 and 4.37 / 8.52 / 16.5 / 16.6.
 #include <mutex>
 #include <new>
 
@@ -104,18 +103,18 @@ __device__ __forceinline__ float sum2(uint64_t v) {
 }
 __device__ __forceinline__ uint32_t ldg16(const void* at) {
   uint32_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(v) : "l"(at));
+  asm volatile("ld.global.u16 %0, [%1];" : "=r"(v) : "l"(at));
   return v;
 }
 __device__ __forceinline__ uint32_t ldg32(const void* at) {
   uint32_t v;
-  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(at));
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(at));
   return v;
 }
 __device__ __forceinline__ float ldgf(const float* at) { return __uint_as_float(ldg32(at)); }
 __device__ __forceinline__ float2 ldgf2(const float* at) {
   float2 v;
-  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(at));
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(at));
   return v;
 }
 __device__ __forceinline__ void prefetch_l2(const void* at) { asm volatile("prefetch.global.L2 [%0];" ::"l"(at)); }
@@ -151,47 +150,29 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   }
   __syncwarp();
 
-  // ---- constants of the tables: no wait for the launch ahead, and ahead of the staged codes, which would hold them up;
-  // lane = table (base = lane / 16, chunk = lane % 16) ----
+  // ---- what the tables are made of beside the activations; lane = table (base = lane / 16, chunk = lane % 16).  A launch ahead may
+  // still write it: ahead of the wait it is only brought to the L2, where such a write meets it ----
   const int base = lane >> 4, chunk = lane & 15;
-  uint32_t col_half[GPB][4];
-  float col[GPB][8];
-#pragma unroll
-  for (int gi = 0; gi < GPB; ++gi) {
-    const int k0 = (GPB * kb + gi) * 128 + chunk * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) col[gi][j] = 0.f;
-    if (gi < ngroups) {
-      if (GLOBAL) {
-        asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(col_half[gi][0]), "=r"(col_half[gi][1]), "=r"(col_half[gi][2]), "=r"(col_half[gi][3])
-                     : "l"(p.gcol + (size_t)base * p.K + k0));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) col[gi][j] = ldgf(p.cols + (size_t)(k0 + j) * 2 + base);
-      }
+  if (warp < ngroups) {
+    const int g = GPB * kb + warp;
+    if (GLOBAL) {  // 128 fp16 of either base, a sector per lane; the residual column that the group's contribution carries first
+      if (lane < 16) prefetch_l2(p.gcol + (size_t)(lane >> 3) * p.K + g * 128 + (lane & 7) * 16);
+      if (lane == 16 && g < p.n_sal) prefetch_l2(p.sal_idx + g);
+    } else {
+      prefetch_l2(p.cols + (size_t)g * 256 + lane * 8);
+      if (lane < 2) prefetch_l2(p.scols + (size_t)g * 16 + lane * 8);
+      if (lane == 2) prefetch_l2(p.indices + g * 8);
     }
   }
-  // the refinement's column and its scale: lane = (group, base, column)
-  const int r_gi = GPB == 2 ? lane >> 4 : 0, r_base = (lane >> 3) & 1, r_j = lane & 7;
-  const bool r_live = !GLOBAL && r_gi < ngroups && (GPB == 2 || lane < 16);
-  int r_idx = 0;
-  float r_col = 0.f;
-  if (r_live) {
-    const int g = GPB * kb + r_gi;
-    r_idx = g * 128 + (int)ldg16(p.indices + g * 8 + r_j);
-    r_col = ldgf(p.scols + (size_t)(g * 8 + r_j) * 2 + r_base);
-  }
-  // the residual columns that a group's contribution carries, dealt round-robin: the first, and of the `more` others thread's
-  int sal_at[GPB], more[GPB], more_at[GPB];
+  // residual columns of a group's contribution, dealt round-robin: the first, and `more` others, one of them this thread's
+  int more[GPB];
+  auto more_column = [&](int gi) { return GPB * kb + gi + ((int)threadIdx.x + 1) * p.G; };
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) {
-    const int g = GPB * kb + gi;
-    sal_at[gi] = GLOBAL && gi < ngroups && g < p.n_sal ? (int)ldg32(p.sal_idx + g) : -1;
-    more[gi] = 0, more_at[gi] = -1;
+    more[gi] = 0;
     if (MORE && gi < ngroups) {
-      more[gi] = p.more_most - (g < p.more_full ? 0 : 1);
-      if ((int)threadIdx.x < more[gi]) more_at[gi] = (int)ldg32(p.sal_idx + g + ((int)threadIdx.x + 1) * p.G);
+      more[gi] = p.more_most - (GPB * kb + gi < p.more_full ? 0 : 1);
+      if ((int)threadIdx.x < more[gi]) prefetch_l2(p.sal_idx + more_column(gi));
     }
   }
 
@@ -212,8 +193,8 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   };
   if (pf_ru < end) issue_next();
 
-  // Constants of a row in this K block, requested ONE UNIT AHEAD of their use (the first unit's ahead of the wait for the
-  // launch before): requested where they were used, each unit of a warp waited for HBM once more.
+  // Constants of a row in this K block, requested ONE UNIT AHEAD of their use (the first unit's together with the activations, brought
+  // to the L2 before): requested where they were used, each unit of a warp waited for HBM once more.
   struct Constants {
     uint32_t r0, r1, sal[GPB];         // matrix-wide scales: fp16 row scales, bf16 residual values
     float2 rs[GPB], srs[GPB];          // scales per group: of the bases and of the refinement
@@ -248,12 +229,23 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       }
     }
   };
-  Constants next;
   if (first < end) {
-    request(first, next);
-    if (MORE) {  // the rest of a row's residual values, which are read one by one
-      const char* const values = reinterpret_cast<const char*>(p.sal + (size_t)min(first * kUnitRows + lane, p.O - 1) * p.n_sal);
-      for (int at = 0; at < 2 * p.n_sal; at += 32) prefetch_l2(values + at);
+    const int row = min(first * kUnitRows + lane, p.O - 1);
+    if (GLOBAL) {
+      prefetch_l2(p.grow + row), prefetch_l2(p.grow + (size_t)p.O + row);
+      const __nv_bfloat16* const sal = p.sal + (size_t)row * p.n_sal;
+      if (MORE) {  // all residual values of the row, which are read one by one
+        for (int at = 0; at < p.n_sal; at += 16) prefetch_l2(sal + at);
+      } else if (GPB * kb < p.n_sal) {
+        prefetch_l2(sal + GPB * kb);
+      }
+    } else {
+#pragma unroll
+      for (int gi = 0; gi < GPB; ++gi)
+        if (gi < ngroups) {
+          const size_t at = ((size_t)(GPB * kb + gi) * p.O + row) * 2;
+          prefetch_l2(p.rows + at), prefetch_l2(p.srows + at), prefetch_l2(p.sparse + at);
+        }
     }
   }
 
@@ -285,13 +277,54 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // ---- activations: all requests in one round trip ----
+  // ---- activations, scales and the first unit's constants: all requests in one round trip ----
   uint4 xr[GPB];
+  uint32_t col_half[GPB][4];
+  float col[GPB][8];
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) {
     xr[gi] = make_uint4(0u, 0u, 0u, 0u);
-    if (gi < ngroups) xr[gi] = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.x) + (GPB * kb + gi) * 128 + chunk * 8);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) col[gi][j] = 0.f;
+    if (gi < ngroups) {
+      const int k0 = (GPB * kb + gi) * 128 + chunk * 8;
+      xr[gi] = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.x) + k0);
+      if (GLOBAL) {
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(col_half[gi][0]), "=r"(col_half[gi][1]), "=r"(col_half[gi][2]), "=r"(col_half[gi][3])
+                     : "l"(p.gcol + (size_t)base * p.K + k0));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) col[gi][j] = ldgf(p.cols + (size_t)(k0 + j) * 2 + base);
+      }
+    }
   }
+  // the refinement's column and its scale: lane = (group, base, column)
+  const int r_gi = GPB == 2 ? lane >> 4 : 0, r_base = (lane >> 3) & 1, r_j = lane & 7;
+  const bool r_live = !GLOBAL && r_gi < ngroups && (GPB == 2 || lane < 16);
+  int r_idx = 0;
+  float r_col = 0.f;
+  if (r_live) {
+    const int g = GPB * kb + r_gi;
+    r_idx = g * 128 + (int)ldg16(p.indices + g * 8 + r_j);
+    r_col = ldgf(p.scols + (size_t)(g * 8 + r_j) * 2 + r_base);
+  }
+  int sal_at[GPB], more_at[GPB];
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) {
+    const int g = GPB * kb + gi;
+    sal_at[gi] = GLOBAL && gi < ngroups && g < p.n_sal ? (int)ldg32(p.sal_idx + g) : -1;
+    more_at[gi] = MORE && (int)threadIdx.x < more[gi] ? (int)ldg32(p.sal_idx + more_column(gi)) : -1;
+  }
+  Constants next;
+  if (first < end) request(first, next);
+  // The rest of the ring, behind these.  The gathers below wait for the indices: the refinement's activation is the last that the tables
+  // wait for, and the ring goes ahead of it (scales per group, 12288x4096 7.92 -> 7.60 us); residual columns come at a unit's end, but the
+  // ring would hold them up by more than that (matrix-wide 4.12 -> 4.17, 12288x4096 7.68 -> 7.96).
+  auto fill_ring = [&]() {
+    for (int s = 1; s < S && pf_ru < end; ++s) issue_next();
+  };
+  if (!GLOBAL) fill_ring();
   float sal_x[GPB], r_x = 0.f;
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
@@ -301,7 +334,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     for (int gi = 0; gi < GPB; ++gi)
       if (more_at[gi] >= 0) more_x[gi * p.more_most + (int)threadIdx.x] = load_act(p.x, p.act_dtype, more_at[gi]);
   }
-  for (int s = 1; s < S && pf_ru < end; ++s) issue_next();  // the rest of the ring, behind the activations
+  if (GLOBAL) fill_ring();
 
   // ---- 32 signed tables per group ----
 #pragma unroll

@@ -221,7 +221,9 @@ def m1_out(x, layout, out, workspace, *, groups_per_split=8, kernel="v1"):
     """Engine-neutral M=1 operator on the current CUDA stream; the caller owns ``out`` and ``workspace``.
 
     fp16/bf16 activations, fp32 accumulation, no allocation after warm-up, only a contiguous
-    ``[1,K]`` input, no hidden fallback.  Returns ``out``.
+    ``[1,K]`` input, no hidden fallback.  The codes are constants (a launch ahead that releases its
+    dependents early must not write them); all other tensors may be written directly ahead.
+    Returns ``out``.
     """
     if kernel not in KERNELS:
         raise ValueError(f"kernel must be one of {KERNELS}")
