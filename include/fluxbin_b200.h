@@ -248,7 +248,8 @@ int fb_w3_finish(const float* partials, int splits, int out_features, void* out,
  * y[o] = sum_g ( r0*d0 + r1*d1 + sr0*s0 + sr1*s1 ), d_b = sum_k sign_b*col_b*x over the group,
  * s_b the same over the group's 8 refined columns; fp32 within a group; the groups (at most 255)
  * are combined by 64-bit fixed-point integer adds (steps of 2^-26, order-independent, so
- * repeat-exact; a group's term that is not finite or is 8192 or more in magnitude gives NaN).
+ * repeat-exact; a group's term that is not finite gives NaN, and so may one of 8192 or more in
+ * magnitude).
  * Any O in 1..65536; x and codes 16-byte aligned; scratch zero-filled once and 256-byte aligned, not
  * shared with other kernels, sized by fb_bb_gemv_scratch_bytes(O, K, 0).  The codes (here and
  * below) are constants: they are read ahead of the wait on the launch ahead in the stream.  All else may be

@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       if (p.nKB == 1) {
         store_act(p.out, p.act_dtype, row, value);
       } else {
-        const bool fits = fabsf(value) < 8192.f;  // 255 of them stay inside 48 bits
+        const bool fits = fabsf(value) < GPB * 8192.f;  // 255 of one group, or 128 of two, stay inside 48 bits
         pend_add = fits ? ((unsigned long long)__float2ll_rn(value * 67108864.f) << 16) + 1ull : 257ull;
         asm volatile("atom.add.relaxed.gpu.global.u64 %0, [%1], %2;" : "=l"(pend_old) : "l"(p.combine + row), "l"(pend_add) : "memory");
         pend_row = row;

@@ -46,3 +46,25 @@ def test_more_residual_columns_than_groups(o, groups, salient):
     out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
     binary_global.global_two_base_m1_out(x.cuda(), {name: value.cuda() for name, value in layout.items()}, out)
     _check(out, x, binary_global.materialize(layout, torch.float64), groups)
+
+
+@pytest.mark.parametrize("o,groups,used,term", ((3104, 32, 2, 6400), (3104, 32, 32, 6400), (4128, 32, 31, 8000), (4064, 96, 96, 8000), (800, 255, 255, 8000), (64, 2, 2, 8000)))
+@pytest.mark.parametrize("mode", ("matrix", "planar", "interleaved"))
+def test_terms_up_to_the_limit(o, groups, used, term, mode):
+    """Terms below 8192 in every group add up, also where a contribution carries two groups: one input a group, all signs positive, and
+    scales that make every product exact."""
+    k = groups * 128
+    x = torch.zeros(1, k, dtype=torch.bfloat16)
+    x[0, :used * 128:128] = term / 128
+    if mode == "matrix":
+        layout = binary_global.make_layout(torch.ones(2, o, k, dtype=torch.int8), torch.full((2, o), 8.0), torch.full((2, k), 8.0), torch.empty(0), torch.empty(o, 0))
+        call = lambda out: binary_global.global_two_base_m1_out(x.cuda(), {name: value.cuda() for name, value in layout.items()}, out)  # noqa: E731
+    else:
+        shape = (groups, o, 2, 16) if mode == "planar" else (groups, o, 32)
+        layout = {"codes": torch.full(shape, 255, dtype=torch.uint8), "rows": torch.full((groups, o, 2), 8.0), "columns": torch.full((groups, 128, 2), 8.0),
+                  "sparse_codes": torch.zeros((groups, o, 2, 1) if mode == "planar" else (groups, o, 2), dtype=torch.uint8), "sparse_rows": torch.zeros(groups, o, 2),
+                  "sparse_columns": torch.zeros(groups, 8, 2), "indices": torch.arange(8, dtype=torch.int16).repeat(groups, 1)}
+        call = lambda out: _native.bb_gemv(x.cuda(), {name: value.cuda() for name, value in layout.items()}, out)  # noqa: E731
+    out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    call(out)
+    assert bool((out == torch.tensor(float(used * term)).bfloat16().cuda()).all())
