@@ -845,17 +845,19 @@ size_t smem_bytes(int m) {
 // ctas_per_sm_for(m) CTAs per SM.  At most kMaxSplits partial sums per output: beyond 16 K blocks one CTA walks
 // several K blocks of its rows in turn.  The SMs are dealt over the super-blocks; the CTAs of a
 // super-block split its row units.
-Plan make_plan(int m, int nKB, int nRU, const DeviceInfo& info) {
+Plan make_plan(int m, int nKB, int nRU, bool gather, const DeviceInfo& info) {
   Plan plan;
   plan.S = (nKB + kMaxSplits - 1) / kMaxSplits;
   plan.nSB = (nKB + plan.S - 1) / plan.S;
   int c = ctas_per_sm_for(m) * info.sm_count / plan.nSB;
   if (c < 1) c = 1;
-  // Where one CTA per SM is enough for every warp to have at most one unit (and, with several K blocks a CTA, to leave half of
-  // the warps without), a second one would only take the room in which the next launch can start.  us, one after the
-  // other in a graph, two / one: 1024x4096 3.03 / 2.98, 2048x2048 3.04 / 2.94, 1024x12288 5.97 / 5.77; 2048x12288, seven units a CTA and
-  // three K blocks, 6.46 / 6.65; the seven Linears of an 8B layer, k beside q and v beside k, 35.3 / 34.0.
-  if (const int one = info.sm_count / plan.nSB; one >= 1 && (nRU + one - 1) / one <= (plan.S == 1 ? warps_for(m) : warps_for(m) / 2)) c = one;
+  // Where one CTA per SM is enough for every warp to have at most one unit (and, with several K blocks a CTA or two rows in identity order, to
+  // leave half of the warps without), a second one would only take the room in which the next launch can start.  us, one after the
+  // other in a graph, two / one: one row 1024x4096 3.05 / 2.92, 2048x2048 3.04 / 2.91, 1024x12288 5.98 / 5.85; 2048x12288, seven units a CTA and
+  // three K blocks, 6.46 / 6.65; the seven Linears of an 8B layer, k beside q and v beside k, 35.3 / 34.0.  Two rows: 1024x4096 (four units a CTA)
+  // 4.73 / 4.66, 2304x4096 (eight) 5.13 / 5.30, with a column order 6.44 / 5.80 and 6.88 / 6.66, 1152x25600 41.7 / 29.0.
+  const int most = plan.S == 1 && (m == 1 || gather) ? warps_for(m) : warps_for(m) / 2;
+  if (const int one = info.sm_count / plan.nSB; one >= 1 && (nRU + one - 1) / one <= most) c = one;
   if (c > nRU) c = nRU;
   plan.slices = c;
   plan.smem = smem_bytes(m);
@@ -1046,7 +1048,7 @@ int run_multi(const void* x, int act_dtype, int m, const fb_w3_matrix_t* matrice
   p.act_dtype = act_dtype;
   p.scale_dtype = scale_dtype;
   if (scratch) bind_scratch(p, scratch);
-  const Plan plan = make_plan(m, p.nKB, p.nRU, *info);
+  const Plan plan = make_plan(m, p.nKB, p.nRU, p.perm != nullptr, *info);
   p.S = plan.S;
   p.early_order = plan.slices * plan.nSB <= info->sm_count && 2 * plan.slices * plan.nSB > info->sm_count ? 1 : 0;
   p.units_per_slice = p.nRU / plan.slices;
