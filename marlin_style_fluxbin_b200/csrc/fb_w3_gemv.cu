@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
   // The column order is part of the weights: this thread's index for the first K block needs no wait.  With one CTA per SM
   // it is requested ahead of the staged weights, behind which it would arrive later than the activations could be read.
   // With two, the gathers of all CTAs would then meet at the few L2 lines of x at the same time, and cost more than that; with CTAs
-  // on fewer than half of the SMs there is nothing to get ahead of.
+  // on fewer than half of the SMs there is nothing to get ahead of.  (One row; several read their order where they use it.)
   // us, cold, early / late: 1024x4096 (one CTA) 3.13 / 3.35, 1024x12288 5.69 / 6.33; 4096x4096 (two) 4.51 / 4.32, 12288x4096 8.40 / 8.37; 128x17408
   // (56 CTAs, decoded) 8.95 / 8.77.
   const int sb = (int)blockIdx.y, kb_begin = sb * p.S;
@@ -717,7 +717,9 @@ __global__ void __launch_bounds__(Geom<M>::kWarps * 32, Geom<M>::kCtasPerSm) w3_
                 for (int m = 0; m < M; ++m) {
                   if constexpr (M != 3) {
                     each[m][pl] = add2_lds(each[m][pl], a0 + (uint32_t)(m * 128), a1 + (uint32_t)(m * 128));
-                  } else {  // twelve sums do not fit the registers (1024 x 4096 7.5 us; in this form 6.4): two a row
+                  } else {
+                    // two sums a row: four spill at three rows (26 bytes) but not at four.  us, four / two, three rows: 1024x4096 7.41 / 7.07, 12288x4096
+                    // 20.8 / 20.4; four rows 9.28 / 9.37, 26.3 / 26.3
                     const uint64_t both = lds2(a0 + (uint32_t)(m * 128), a1 + (uint32_t)(m * 128));
                     if (pl < 3) each[m][0] = fma2(both, pl == 0 ? one2 : pl == 1 ? two2 : minus_four2, each[m][0]);
                     if (pl > 0) each[m][1] = fma2(both, pl == 1 ? at3[jh] : pl == 2 ? at4[jh] : at_f[jh], each[m][1]);
