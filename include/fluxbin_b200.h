@@ -258,6 +258,8 @@ int fb_w3_finish(const float* partials, int splits, int out_features, void* out,
  * reference's kernel names map to this one entry point.
  */
 size_t fb_bb_gemv_scratch_bytes(int out_features, int in_features, int global_scales);
+/* Groups that a contribution carries for a matrix of this size on the current device: 1 or 2, or a negative status. */
+int fb_bb_gemv_block_groups(int out_features, int in_features, int planar, int global_scales);
 int fb_bb_gemv(const void* x, int act_dtype, const uint8_t* codes, int planar, const float* rows,
                const float* cols, const uint8_t* sparse_codes, const float* sparse_rows,
                const float* sparse_cols, const int16_t* indices, void* out, int out_features,

@@ -113,6 +113,8 @@ def library() -> ctypes.CDLL:
         lib.fb_w3_finish.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
         lib.fb_bb_gemv_scratch_bytes.restype = ctypes.c_size_t
         lib.fb_bb_gemv_scratch_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
+        lib.fb_bb_gemv_block_groups.restype = ctypes.c_int
+        lib.fb_bb_gemv_block_groups.argtypes = [ctypes.c_int] * 4
         lib.fb_bb_gemv.restype = ctypes.c_int
         lib.fb_bb_gemv.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int] + [ctypes.c_void_p] * 7 + [
             ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint, ctypes.c_void_p]

@@ -533,6 +533,15 @@ int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cu
   return FB_OK;
 }
 
+// Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay
+// once warps have units of one group to spare, more than one each with matrix-wide scales, more than four with scales per group (more
+// constants per unit either way; two where interleaved codes make a unit longer).  us, one group / two: matrix-wide 2048x4096 (0.9 units a warp) 3.18 / 3.31, 3072x4096 (1.3) 4.10 / 3.62,
+// 3072x1024 (0.3) 3.38 / 4.60, 1024x12288 (1.3) 4.02 / 3.62; per group 4064x4096 (1.7) 4.23 / 4.45, 2048x12288 (2.6) 5.41 / 5.55, 3072x12288 (3.9)
+// 6.56 / 6.52; interleaved 4096x4096 (1.7) 5.27 / 5.30, 5120x5120 (2.7) 6.90 / 6.81.
+int groups_per_block(int groups, int units, bool matrix_wide, bool interleaved, int sms) {
+  return groups >= 2 && units * groups > kCtasPerSm * sms * kWarps * (matrix_wide ? 1 : interleaved ? 2 : 4) ? 2 : 1;
+}
+
 int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_stream_t stream, const char* who) {
   const size_t need = kCombineOffset + (size_t)p.O * sizeof(unsigned long long);
   if (!scratch || scratch_bytes < need) return fail(FB_ESCRATCH, "%s: scratch of %zu bytes needed, %zu given", who, need, scratch_bytes);
@@ -543,12 +552,7 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   p.status = reinterpret_cast<unsigned*>(base);
   p.combine = reinterpret_cast<unsigned long long*>(base + kCombineOffset);
   p.nRU = (p.O + kUnitRows - 1) / kUnitRows;
-  // Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay
-  // once warps have units of one group to spare, more than one each with matrix-wide scales, more than four with scales per group (more
-  // constants per unit either way; two where interleaved codes make a unit longer).  us, one group / two: matrix-wide 2048x4096 (0.9 units a warp) 3.18 / 3.31, 3072x4096 (1.3) 4.10 / 3.62,
-  // 3072x1024 (0.3) 3.38 / 4.60, 1024x12288 (1.3) 4.02 / 3.62; per group 4064x4096 (1.7) 4.23 / 4.45, 2048x12288 (2.6) 5.41 / 5.55, 3072x12288 (3.9)
-  // 6.56 / 6.52; interleaved 4096x4096 (1.7) 5.27 / 5.30, 5120x5120 (2.7) 6.90 / 6.81.
-  const int gpb = p.G >= 2 && p.nRU * p.G > kCtasPerSm * info->sm_count * kWarps * (p.global_mode ? 1 : p.interleaved ? 2 : 4) ? 2 : 1;
+  const int gpb = groups_per_block(p.G, p.nRU, p.global_mode, p.interleaved, info->sm_count);
   p.nKB = (p.G + gpb - 1) / gpb;
   int c = kCtasPerSm * info->sm_count / p.nKB;
   if (c < 1) c = 1;
@@ -613,6 +617,13 @@ extern "C" size_t fb_bb_gemv_scratch_bytes(int out_features, int in_features, in
   if (out_features < 1 || in_features < 128) return 0;
   (void)global_scales;
   return kCombineOffset + (size_t)out_features * sizeof(unsigned long long);
+}
+
+extern "C" int fb_bb_gemv_block_groups(int out_features, int in_features, int planar, int global_scales) {
+  if (out_features < 1 || in_features < 128 || in_features % 128) return fail(FB_ELIMIT, "fb_bb_gemv_block_groups: O=%d, K=%d", out_features, in_features);
+  const DeviceInfo* info = device_info();
+  if (!info) return FB_ECUDA;
+  return groups_per_block(in_features / 128, (out_features + kUnitRows - 1) / kUnitRows, global_scales != 0, !planar, info->sm_count);
 }
 
 namespace {

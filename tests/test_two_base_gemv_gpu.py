@@ -1,4 +1,4 @@
-"""Two-base GEMV at the edges of its units (32 rows), K blocks (one or two groups) and rings, against fp64."""
+"""Two-base GEMV at the edges of its units (32 rows), K blocks (one or two groups, by size) and rings, against fp64."""
 import pytest
 import torch
 
@@ -68,3 +68,45 @@ def test_terms_up_to_the_limit(o, groups, used, term, mode):
     out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
     call(out)
     assert bool((out == torch.tensor(float(used * term)).bfloat16().cuda()).all())
+
+
+def _first_of_two_groups(groups, planar, matrix_wide):
+    """The smallest number of rows whose contributions carry two groups; one unit less must carry one."""
+    count = lambda o: _native.library().fb_bb_gemv_block_groups(o, groups * 128, planar, matrix_wide)  # noqa: E731
+    low, high = 1, 65536  # one group / two
+    assert (count(low), count(high)) == (1, 2)
+    while high - low > 1:
+        middle = (low + high) // 2
+        low, high = (low, middle) if count(middle) == 2 else (middle, high)
+    return high
+
+
+@pytest.mark.parametrize("rows_more", (-1, 0, 18, 31))
+@pytest.mark.parametrize("groups,salient", ((2, 0), (2, 1), (3, 2), (3, 3), (3, 32), (5, 5), (5, 32), (9, 20), (2, 255)))
+def test_matrix_wide_scales_on_either_side_of_two_groups(groups, salient, rows_more):
+    o, k = _first_of_two_groups(groups, 1, 1) + rows_more, groups * 128
+    gen = torch.Generator(device="cuda").manual_seed(o + salient)
+    scale = lambda n: (torch.randn(2, n, device="cuda", generator=gen) * 0.02).abs().half()  # noqa: E731
+    layout = {"codes": torch.randint(0, 256, (groups, o, 2, 16), device="cuda", generator=gen, dtype=torch.uint8), "row_scales": scale(o), "column_scales": scale(k),
+              "salient_indices": torch.randperm(k, device="cuda", generator=gen)[:salient].int(),
+              "salient_values": (torch.randn(o, salient, device="cuda", generator=gen) * 0.05).bfloat16()}
+    x = torch.randn(1, k, device="cuda", generator=gen).bfloat16()
+    out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    binary_global.global_two_base_m1_out(x, layout, out)
+    _check(out, x.cpu(), binary_global.materialize(layout, torch.float64).cpu(), groups)
+
+
+@pytest.mark.parametrize("rows_more", (-1, 0, 18, 31))
+@pytest.mark.parametrize("groups,planar", ((8, 1), (9, 1), (5, 0), (6, 0)))
+def test_scales_per_group_on_either_side_of_two_groups(groups, planar, rows_more):
+    o = _first_of_two_groups(groups, planar, 0) + rows_more
+    gen = torch.Generator(device="cuda").manual_seed(o)
+    normal = lambda *size: torch.randn(*size, device="cuda", generator=gen)  # noqa: E731
+    code = lambda *size: torch.randint(0, 256, size, device="cuda", generator=gen, dtype=torch.uint8)  # noqa: E731
+    layout = {"codes": code(groups, o, 2, 16) if planar else code(groups, o, 32), "rows": normal(groups, o, 2) * 0.1, "columns": normal(groups, 128, 2),
+              "indices": normal(groups, 128).argsort(1)[:, :8].sort(1).values.to(torch.int16).contiguous(),
+              "sparse_codes": code(groups, o, 2, 1) if planar else code(groups, o, 2), "sparse_rows": normal(groups, o, 2) * 0.07, "sparse_columns": normal(groups, 8, 2)}
+    x = normal(1, groups * 128).bfloat16()
+    out = torch.full((1, o), float("nan"), device="cuda", dtype=torch.bfloat16)
+    _native.bb_gemv(x, layout, out)
+    _check(out, x.cpu(), decode_layout(layout, torch.float32).double().cpu(), groups)
