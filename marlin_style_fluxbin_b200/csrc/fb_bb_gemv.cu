@@ -234,7 +234,9 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     if (GLOBAL) {
       prefetch_l2(p.grow + row), prefetch_l2(p.grow + (size_t)p.O + row);
       const __nv_bfloat16* const sal = p.sal + (size_t)row * p.n_sal;
-      if (MORE) {  // all residual values of the row, which are read one by one
+      // A row's residual values are read one by one; up to four sectors of them are requested as a whole.  More would be in every CTA's way:
+      // each K block asks for all of them, past the L1 (255 columns, with / without: 1024x8192 8.03 / 4.56 us, 4096x4096 12.1 / 9.0).
+      if (MORE && p.n_sal <= 64) {
         for (int at = 0; at < p.n_sal; at += 16) prefetch_l2(sal + at);
       } else if (GPB * kb < p.n_sal) {
         prefetch_l2(sal + GPB * kb);
@@ -562,9 +564,9 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   p.sal_pairs = p.global_mode && p.n_sal % 2 == 0 && aligned(p.sal, 4) ? 1 : 0;
   const int per_warp = ((p.nRU + c - 1) / c + kWarps - 1) / kWarps;
   // Where a group carries three residual columns and more, up to 1 + more_most (as many do the first more_full groups), their activations
-  // are gathered once per CTA and their values requested ahead; a single one or two are read where they are used, which costs the
-  // others less.  us at 32 columns, gathered / as they are used: 17x128 2.4 / 3.2, 256x512 (8 a group) 2.6 / 3.1, 8192x512 3.5 / 3.8, 512x1024 (4) 2.86 / 2.96,
-  // 2048x2048 (2) 3.10 / 3.09, 5120x2560 (1.6) 4.27 / 4.00.
+  // are gathered once per CTA and the first unit's values brought to the L2 ahead; a single one or two are read where they are used, which costs
+  // the others less.  us, gathered / as they are used: 32 columns 17x128 2.39 / 2.99, 512x512 (8 a group) 2.81 / 3.15, 16384x512 4.22 / 4.43, 512x1024 (4)
+  // 2.76 / 2.99, 8192x1024 3.90 / 3.76, 2048x2048 (2) 3.35 / 3.22, 5120x2560 (1.6) 4.86 / 4.32; 255 columns 2048x2048 (16) 5.93 / 6.02, 4096x4096 (8) 8.99 / 10.3.
   const bool more = p.global_mode && p.n_sal >= 3 * p.G;
   p.more_most = more ? (p.n_sal - 1) / p.G : 0, p.more_full = more ? p.n_sal - p.more_most * p.G : 0;
   const size_t more_bytes = (size_t)gpb * p.more_most * sizeof(float);
