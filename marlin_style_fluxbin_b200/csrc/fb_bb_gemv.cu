@@ -535,13 +535,14 @@ int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cu
   return FB_OK;
 }
 
-// Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay
-// once warps have units of one group to spare, more than one each with matrix-wide scales, more than four with scales per group (more
-// constants per unit either way; two where interleaved codes make a unit longer).  us, one group / two: matrix-wide 2048x4096 (0.9 units a warp) 3.18 / 3.31, 3072x4096 (1.3) 4.10 / 3.62,
-// 3072x1024 (0.3) 3.38 / 4.60, 1024x12288 (1.3) 4.02 / 3.62; per group 4064x4096 (1.7) 4.23 / 4.45, 2048x12288 (2.6) 5.41 / 5.55, 3072x12288 (3.9)
-// 6.56 / 6.52; interleaved 4096x4096 (1.7) 5.27 / 5.30, 5120x5120 (2.7) 6.90 / 6.81.
+// Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay once warps have
+// units of one group to spare, more than one each with matrix-wide scales, more than four (interleaved: five) with scales per group, which
+// bring more constants per unit either way.  us, one group / two, in brackets units of one group a warp: matrix-wide 2304x4096 (1.0) 3.40 / 3.50,
+// 3072x4096 (1.3) 4.29 / 3.87, 3072x1024 (0.3) 3.48 / 4.53, 1024x12288 (1.3) 4.42 / 3.71; per group 2048x12288 (2.6) 5.53 / 6.04, 3072x12288 (3.9)
+// 6.83 / 6.66, 9472x4096 (4.0) 6.99 / 7.32, 12288x4096 (5.2) 8.24 / 7.85; interleaved 5120x5120 (2.7) 6.91 / 7.45, 8192x5120 (4.3) 9.45 / 9.86,
+// 12288x4096 (5.2) 10.79 / 10.79, 16384x4096 (6.9) 13.3 / 12.7.
 int groups_per_block(int groups, int units, bool matrix_wide, bool interleaved, int sms) {
-  return groups >= 2 && units * groups > kCtasPerSm * sms * kWarps * (matrix_wide ? 1 : interleaved ? 2 : 4) ? 2 : 1;
+  return groups >= 2 && units * groups > kCtasPerSm * sms * kWarps * (matrix_wide ? 1 : interleaved ? 5 : 4) ? 2 : 1;
 }
 
 int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_stream_t stream, const char* who) {
