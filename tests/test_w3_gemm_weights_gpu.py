@@ -1,5 +1,6 @@
-"""Weights of the many-row kernel read out one by one: with the identity as activations an output IS a weight, in every pair of
-dtypes, for every finite scale of 16 bits and for zero points on either side of what the short forms cover."""
+"""Weights of the many-row kernel read out one by one, in every pair of dtypes: with the identity as activations an output IS a weight (scales
+from 1e-30 to where a weight overflows, zero points on either side of what the short forms cover); with a single weight that is not zero in
+a row, every finite scale of 16 bits, where weights are subnormal or infinite too."""
 import pytest
 import torch
 
@@ -36,6 +37,29 @@ def test_every_scale(scale_dtype, act_dtype, zero_points):
     out = torch.empty(k, o, device="cuda", dtype=act_dtype)
     _native.w3_gemm(torch.eye(k, device="cuda", dtype=act_dtype), (layout,), out)
     assert torch.equal(out.T.float(), weights.float())
+
+
+@pytest.mark.parametrize("zero", (None, 3, 0, 7))
+@pytest.mark.parametrize("act_dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("scale_dtype", (torch.bfloat16, torch.float16))
+def test_one_weight_of_every_finite_scale(scale_dtype, act_dtype, zero):
+    from marlin_style_fluxbin_b200 import _native
+
+    o, z = 65536, 4 if zero is None else zero
+    scales = torch.arange(o, device="cuda", dtype=torch.int32).to(torch.int16).view(scale_dtype)
+    scales = torch.where(scales.isfinite(), scales, torch.ones_like(scales)).view(1, o)
+    out = torch.empty(1, o, device="cuda", dtype=act_dtype)
+    for code in range(8):
+        codes = torch.full((128,), z, device="cuda", dtype=torch.int32)
+        codes[16 * code + 3] = code
+        bits = torch.stack((codes & 1, codes >> 1 & 1, 1 - (codes >> 2 & 1)))  # the high plane is stored inverted
+        row = (bits.view(3, 16, 8) << torch.arange(8, device="cuda")).sum(-1).to(torch.uint8)
+        layout = {"planes": row.view(1, 3, 1, 16).expand(1, 3, o, 16).contiguous(), "scales": scales}
+        if zero is not None:
+            layout["zeros"] = torch.full((1, o), zero, device="cuda", dtype=torch.uint8)
+        _native.w3_gemm(torch.ones(1, 128, device="cuda", dtype=act_dtype), (layout,), out)
+        want = (scales.float() * (code - z)).to(scale_dtype).to(act_dtype)  # one factor of eight bits or eleven, one of three: exact in fp32
+        assert torch.equal(out, want), code
 
 
 @pytest.mark.parametrize("o,k,t", ((160, 256, 128), (24576, 256, 128), (24576, 384, 100), (24576, 128, 128), (12288, 640, 333), (256, 640, 129)))
