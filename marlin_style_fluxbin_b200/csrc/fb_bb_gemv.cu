@@ -71,7 +71,7 @@ struct BBParams {
 };
 
 // Two words of eight sign bits per base, interleaved bit by bit, become [base 0: two bytes][base 1: two bytes]: the four
-// steps of a perfect unshuffle.
+// steps of a perfect unshuffle (Warren, Hacker's Delight, 7-2).
 __device__ __forceinline__ uint32_t unshuffle(uint32_t w) {
   uint32_t t;
   t = (w ^ (w >> 1)) & 0x22222222u, w ^= t ^ (t << 1);

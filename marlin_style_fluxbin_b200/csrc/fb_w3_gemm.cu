@@ -18,20 +18,16 @@
 // eight values per (row, group), scale * (code - zero) rounded in the scale's dtype and then in the
 // activations'; they are looked up four at a time by byte permutes whose selector nibbles are the codes, or multiplied out.
 //
-// What bounds it: at 256 tokens a tile the MMA (tensor pipe 86 % active).  Up to 128 tokens a group took 0.43 us, 840 clocks, whatever the tokens.
-// Clock stamps of a working copy (12288 x 4096, 64 or 112 tokens): the MMA warp's course over a group was about 1000 clocks (barriers 330, eight
-// instructions 470, commits 120; the MMAs themselves end 100 after the last is issued) while each dequantising warpgroup spent 1500 of its 3500
-// clocks per group waiting for a slot.  Two warps that issue, each on its own accumulator, halve that course: 300 to 500 of 3000 clocks are
-// waited for then, and instruction issue of the dequantising warps bounds it.  These were cut as well: values of a row by 16-bit
-// multiplications (500 clocks a group of a warpgroup -> 200), and where scales and activations share a dtype no look-ups at all but a code
-// inside a magic number, two or three 16-bit operations on the idle multiply pipes instead of byte permutes.  A kernel for one issuer and one for
-// two: both loops in one kernel took the MMAs' operands out of uniform registers (twice the time).  The MMA warps look at both barriers with one
-// instruction, their instructions are predicated on the elected lane, and where the activations' ring has as many stages as there are operand
-// slots (up to 192 tokens) one commit releases both.
-// us on a B200, weights cold, in a graph, before -> now, fp16 scales / bf16 scales: 12288 x 4096 at 64 tokens 18.6 -> 16.3 / 19.0 -> 16.9, at 112 19.6 ->
-// 18.1 / 20.0 -> 18.4, at 333 36.9 -> 32.9 / 36.9 -> 31.7, at 512 43.0 -> 41.2 / 43.0 -> 40.9; 4096 x 12288 at 512 48.0 -> 46.2 / 48.5 -> 43.5; 24576 x 4096 at
-// 512 79.9 -> 76.8; chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 64.
-// Without effect: a ring of eight plane tiles, scales prefetched into L2, more accumulators for one issuer, polling with pauses, one arrival a warp.
+// What bounds it: at 256 tokens a tile the MMA (tensor pipe 86 % active); up to 128 instruction issue of the dequantising warps, whatever the
+// tokens.  Two warps issue there because one's course over a group (1000 clocks: two barriers 330, eight instructions 470, commits 120) would hold
+// the four warpgroups up for 1500 of their 3500 clocks a group; with two they wait 300 to 500.  One issuer and two are kernels of their own: both
+// loops in one took the MMAs' operands out of uniform registers (twice the time).  The values of a row come from 16-bit multiplications (200 clocks a
+// group of a warpgroup, fp32 ones took 500); where scales and activations share a dtype there is no table but a code inside a magic number,
+// on the idle multiply pipes.  The MMA warps look at both barriers with one instruction, their instructions are predicated on the elected lane, and
+// where the activations' ring has as many stages as there are operand slots (up to 192 tokens) one commit releases both.
+// us on a B200, weights cold, in a graph, fp16 / bf16 scales (in brackets with one issuer and a table of fp32 products): 12288 x 4096 at 64 tokens
+// 16.3 / 16.9 (18.6 / 19.0), at 112 18.1 / 18.4 (19.6 / 20.0), at 333 32.9 / 31.7 (36.9 / 36.9), at 512 41.2 / 40.9 (43.0 / 43.0); 4096 x 12288 at 512
+// 46.2 / 43.5 (48.0 / 48.5); 24576 x 4096 at 512 76.8 (79.9); chunks of the dense weight, 12288 x 4096 at 64 / 512: 39 / 62.
 //
 // A role whose wait expires gives up after two seconds in which the rings stood still, so what is in flight has landed when
 // the CTA ends; it leaves with the status word set and the tensor memory freed.
@@ -207,7 +203,8 @@ __device__ __forceinline__ void value_table(uint32_t scale_bits, uint32_t zero, 
 }
 
 // Scales and activations in one dtype: no table.  A code inside the mantissa of a magic number (128 in bf16, 1024 in fp16: its last
-// place is one) is that number plus the code, or plus 16 times it.  off, off16: -(magic + zero), -(magic / 16 + zero).
+// place is one) is that number plus the code, or plus 16 times it: the published way to make 16-bit floats of small integers (Kim et al.,
+// "Who Says Elephants Can't Run", 2022), here on words of three interleaved planes.  off, off16: -(magic + zero), -(magic / 16 + zero).
 struct RowFactors {
   uint32_t off, off16, scale;
 };

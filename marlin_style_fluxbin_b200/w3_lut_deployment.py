@@ -29,10 +29,11 @@ DENSE_CHUNK_BYTES = 52 << 20
 
 def fused_gemm_pays(rows: int, out_features: int) -> bool:
     """Whether ``rows`` activation rows go through the kernel that dequantises into tensor memory rather than through dense
-    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy.  us in a graph, weights cold, this / chunks, 512 rows:
-    1024 x 4096 18.6 / 12.7, 2048 x 4096 19.5 / 17.4, 2048 x 12288 47.4 / 36.4, 3072 x 4096 20.3 / 20.0, 3072 x 12288 47.5 / 57.0, 4096 x 4096
-    21.2 / 23.9; 64 rows: 3072 x 4096 17.7 / 15.5, 4096 x 4096 20.2 / 18.4, 3072 x 12288 44.6 / 51.9, 12288 x 4096 19.2 / 39.3.  Beyond a thousand
-    rows the chunks, dequantised once for all of them, catch up: 2048 rows of 12288 x 1024 59 / 50, of 12288 x 4096 157 / 160."""
+    chunks.  One tile of it walks all of K, so a narrow matrix keeps few SMs busy.  us in a graph, weights cold, bf16 activations, fp16 scales, this / chunks,
+    512 rows: 512 x 4096 15.5 / 11.5, 1024 x 4096 15.6 / 12.9, 2048 x 4096 16.7 / 16.9, 2048 x 12288 40.0 / 35.7, 3072 x 4096 17.8 / 19.2, 3072 x 12288
+    41.7 / 55.9, 4096 x 4096 18.7 / 22.4, 12288 x 4096 42.3 / 61.9; 64 rows: 2048 x 4096 15.4 / 14.1, 3072 x 4096 15.6 / 15.3, 4096 x 4096 15.7 / 16.3,
+    12288 x 4096 16.4 / 38.8 (bf16 scales: 0.5 to 1.5 less for this below 256 rows).  Beyond a thousand rows the chunks, dequantised once for all of them, catch up where K is short: 2048
+    rows of 12288 x 1024 49.5 / 48.4, but of 12288 x 4096 154 / 166.  Nor does the line follow K on its other side: 512 rows of 1024 x 1024 take 6.9 / 8.1."""
     return rows <= 1024 and out_features > 2048 and out_features % 32 == 0
 
 ROW_TILES = (256, 512, 1024)
