@@ -16,6 +16,7 @@ from typing import Mapping
 
 import torch
 from torch import nn
+from torch.multiprocessing.reductions import StorageWeakRef
 from torch.nn import functional as F
 
 from . import _native
@@ -202,19 +203,31 @@ def load_extension(kernel="v1"):
     return SimpleNamespace(m1_out=native_m1_out)
 
 
-_LOOKUP_CACHE: dict[int, torch.Tensor] = {}
+# (device, address, shape, strides) of a lookup -> its storage, its version and what was read from it
+_LOOKUP_CACHE: dict[tuple, tuple[StorageWeakRef, int, torch.Tensor]] = {}
+_RETIRED_INDICES: list[torch.Tensor] = []  # of lookups that are gone: a captured graph may still read them
 
 
 def _indices_from_lookup(lookup: torch.Tensor) -> torch.Tensor:
-    """Recover the sorted ``[G,8]`` column indices from a ``[G,128]`` position lookup (cached per tensor)."""
-    key = lookup.data_ptr()
-    cached = _LOOKUP_CACHE.get(key)
-    if cached is None or cached.shape[0] != lookup.shape[0] or cached.device != lookup.device:
+    """Recover the sorted ``[G,8]`` column indices from a ``[G,128]`` position lookup.
+
+    Kept as long as the lookup's storage lives and nothing has written it in place (an inference tensor does not
+    count its writes: it must stay as it is).  After a write they change where they lie, so that captured calls follow."""
+    key = (lookup.device, lookup.data_ptr(), lookup.shape, lookup.stride())
+    version = -1 if lookup.is_inference() else lookup._version
+    storage, seen, kept = _LOOKUP_CACHE.get(key, (None, None, None))
+    indices = kept
+    if storage is None or storage.expired() or seen != version:
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("first use of a lookup tensor must happen before graph capture")
-        cached = torch.nonzero(lookup >= 0)[:, 1].reshape(lookup.shape[0], 8).to(torch.int16).contiguous()
-        _LOOKUP_CACHE[key] = cached
-    return cached
+        with torch.inference_mode(False), torch.no_grad():  # a tensor that may be written later
+            indices = torch.nonzero(lookup >= 0)[:, 1].reshape(lookup.shape[0], 8).to(torch.int16).contiguous()
+            if storage is not None and storage.expired():
+                _RETIRED_INDICES.append(kept)
+            elif storage is not None:
+                indices = kept.copy_(indices)
+        _LOOKUP_CACHE[key] = (StorageWeakRef(lookup.untyped_storage()), version, indices)
+    return indices
 
 
 def m1_out(x, layout, out, workspace, *, groups_per_split=8, kernel="v1"):

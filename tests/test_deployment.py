@@ -93,6 +93,29 @@ def test_all_65536_interleaved_patterns_and_planar_roundtrip():
     assert workspace_shape(17, 384, 4, kernel="v4") == (3 * 272 + 17,) and workspace_shape(17, 384, 4) == (1, 17)
 
 
+def test_indices_follow_the_lookup_they_were_read_from(monkeypatch):
+    """Neither a write in place nor another lookup at the address of one that is gone gets the indices of what lay there."""
+    from marlin_style_fluxbin_b200.deployment import _indices_from_lookup
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)  # without a GPU it raises
+    first, second = (convert_artifact(make_payload(7, 3, seed=seed)) for seed in (1, 2))
+    lookup = first["lookup"].clone()
+    indices = _indices_from_lookup(lookup)
+    assert torch.equal(indices, first["indices"]) and _indices_from_lookup(lookup) is indices
+    lookup.copy_(second["lookup"])
+    assert _indices_from_lookup(lookup) is indices and torch.equal(indices, second["indices"])
+    memory = first["lookup"].numpy().copy()
+    assert torch.equal(_indices_from_lookup(torch.from_numpy(memory)), first["indices"])
+    memory[:] = second["lookup"].numpy()
+    assert torch.equal(_indices_from_lookup(torch.from_numpy(memory)), second["indices"])
+    written = first["lookup"].clone()
+    with torch.inference_mode():
+        assert torch.equal(_indices_from_lookup(second["lookup"].clone()), second["indices"])
+        assert torch.equal(_indices_from_lookup(written), first["indices"])
+    written.copy_(second["lookup"])
+    assert torch.equal(_indices_from_lookup(written), second["indices"])
+
+
 def test_fail_closed_payload_contract():
     for field, mutate in (("refinement_indices", lambda x: x.fill_(128)), ("refinement_indices", lambda x: x.zero_()),
                           ("global_row_scales", lambda x: x.fill_(float("nan"))), ("global_column_scales", lambda x: x.half()),
