@@ -25,8 +25,8 @@
 // What bounds it: the launch chain and, per unit, latencies; a unit carries two thirds of a W3 unit's bytes.  Only the codes are read
 // ahead of the wait for the launch ahead, which may write everything else: scales, residual and refinement are brought to the L2
 // before it and requested together with the activations behind it, a row's one unit ahead of their use.
-// us on a B200, weights cold, in a graph, 1024x4096 / 4096x4096 / 12288x4096 / 4096x12288: matrix-wide scales 2.88 / 4.13 / 7.70 / 7.18,
-// scales per group, planar 3.19 / 4.43 / 7.58 / 7.63, interleaved 3.26 / 5.36 / 10.6 / 10.6.  Read ahead of the wait they would take
+// us on a B200, weights cold, in a graph, 1024x4096 / 4096x4096 / 12288x4096 / 4096x12288: matrix-wide scales 2.77 / 3.93 / 7.58 / 7.06,
+// scales per group, planar 3.17 / 4.32 / 7.63 / 7.67, interleaved 3.25 / 5.33 / 10.6 / 10.6.  Read ahead of the wait they would take
 // 2.78 / 3.82 / 7.32 / 6.98, 2.85 / 4.24 / 7.63 / 7.63 and 3.09 / 5.27 / 10.1 / 10.1; without the prefetch and the unit ahead, ring
 // slots by a modulo and shares by 64-bit divisions it was 3.27 / 5.15 / 8.82 / 8.43, 4.02 / 6.26 / 9.96 / 9.97 and 4.37 / 8.52 / 16.5 / 16.6.
 #include <mutex>
@@ -320,23 +320,11 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   }
   Constants next;
   if (first < end) request(first, next);
-  // The rest of the ring, behind these.  The gathers below wait for the indices: the refinement's activation is the last that the tables
-  // wait for, and the ring goes ahead of it (scales per group, 12288x4096 7.92 -> 7.60 us); residual columns come at a unit's end, but the
-  // ring would hold them up by more than that (matrix-wide 4.12 -> 4.17, 12288x4096 7.68 -> 7.96).
-  auto fill_ring = [&]() {
-    for (int s = 1; s < S && pf_ru < end; ++s) issue_next();
-  };
-  if (!GLOBAL) fill_ring();
-  float sal_x[GPB], r_x = 0.f;
-#pragma unroll
-  for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
+  // The rest of the ring goes behind these and ahead of the gathers, which wait for the indices (scales per group, 12288x4096 7.60 us; behind
+  // them 7.92).
+  for (int s = 1; s < S && pf_ru < end; ++s) issue_next();
+  float r_x = 0.f;
   if (r_live) r_x = load_act(p.x, p.act_dtype, r_idx);
-  if (MORE) {
-#pragma unroll
-    for (int gi = 0; gi < GPB; ++gi)
-      if (more_at[gi] >= 0) more_x[gi * p.more_most + (int)threadIdx.x] = load_act(p.x, p.act_dtype, more_at[gi]);
-  }
-  if (GLOBAL) fill_ring();
 
   // ---- 32 signed tables per group ----
 #pragma unroll
@@ -384,6 +372,15 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       }
       sparse_lut[t * 256 + pp] = sum;
     }
+  }
+  // residual columns come at a unit's end: gathered ahead of the tables they held those up (4096x4096 4.12 us, here 3.93)
+  float sal_x[GPB];
+#pragma unroll
+  for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
+  if (MORE) {
+#pragma unroll
+    for (int gi = 0; gi < GPB; ++gi)
+      if (more_at[gi] >= 0) more_x[gi * p.more_most + (int)threadIdx.x] = load_act(p.x, p.act_dtype, more_at[gi]);
   }
   __syncthreads();
 
