@@ -25,8 +25,8 @@
 // What bounds it: the launch chain and, per unit, latencies; a unit carries two thirds of a W3 unit's bytes.  Only the codes are read
 // ahead of the wait for the launch ahead, which may write everything else: scales, residual and refinement are brought to the L2
 // before it and requested together with the activations behind it, a row's one unit ahead of their use.
-// us on a B200, weights cold, in a graph, 1024x4096 / 4096x4096 / 12288x4096 / 4096x12288: matrix-wide scales 2.77 / 3.93 / 7.58 / 7.06,
-// scales per group, planar 3.17 / 4.32 / 7.63 / 7.67, interleaved 3.25 / 5.33 / 10.6 / 10.6.  Read ahead of the wait they would take
+// us on a B200, weights cold, in a graph, 1024x4096 / 4096x4096 / 12288x4096 / 4096x12288: matrix-wide scales 2.78 / 3.97 / 7.58 / 7.11,
+// scales per group, planar 3.18 / 4.35 / 7.63 / 7.69, interleaved 3.26 / 5.36 / 10.6 / 10.6.  Read ahead of the wait they would take
 // 2.78 / 3.82 / 7.32 / 6.98, 2.85 / 4.24 / 7.63 / 7.63 and 3.09 / 5.27 / 10.1 / 10.1; without the prefetch and the unit ahead, ring
 // slots by a modulo and shares by 64-bit divisions it was 3.27 / 5.15 / 8.82 / 8.43, 4.02 / 6.26 / 9.96 / 9.97 and 4.37 / 8.52 / 16.5 / 16.6.
 #include <mutex>
@@ -64,7 +64,7 @@ struct BBParams {
   unsigned* status;
   int O, K, G, nKB, nRU;
   int act_dtype, interleaved, global_mode, n_sal;
-  int more_most, more_full;     // residual columns of a group beyond its first: at most, and groups that have as many
+  int sal_most, sal_full;       // residual columns of a group whose activations are gathered: at most, and groups that have as many
   int sal_pairs;                // the residual values of two groups lie in one aligned 32-bit word
   int slots;                    // staged units per warp
   int units_few, units_extra;   // row units of a slice; slices that have one more
@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   float* const sparse_lut = reinterpret_cast<float*>(smem + kLutBytes);
   const uint32_t ring_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(warp * S * kUnitBytes);
   const uint32_t bars_u32 = smem_u32(smem + kLutBytes + kSparseLutBytes) + (uint32_t)(kWarps * S * kUnitBytes + warp * S * 8);
-  // activations of the residual columns beyond one per group (more columns than groups): [group][p.more_most]
-  float* const more_x = reinterpret_cast<float*>(smem + kLutBytes + kSparseLutBytes + kWarps * S * (kUnitBytes + 8));
+  // activations of the residual columns where a group carries several: [group][p.sal_most]
+  float* const sal_x = reinterpret_cast<float*>(smem + kLutBytes + kSparseLutBytes + kWarps * S * (kUnitBytes + 8));
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -155,24 +155,25 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
   const int base = lane >> 4, chunk = lane & 15;
   if (warp < ngroups) {
     const int g = GPB * kb + warp;
-    if (GLOBAL) {  // 128 fp16 of either base, a sector per lane; the residual column that the group's contribution carries first
+    if (GLOBAL) {  // 128 fp16 of either base, a sector per lane; a single residual column
       if (lane < 16) prefetch_l2(p.gcol + (size_t)(lane >> 3) * p.K + g * 128 + (lane & 7) * 16);
-      if (lane == 16 && g < p.n_sal) prefetch_l2(p.sal_idx + g);
+      if (!MORE && lane == 16 && g < p.n_sal) prefetch_l2(p.sal_idx + g);
     } else {
       prefetch_l2(p.cols + (size_t)g * 256 + lane * 8);
       if (lane < 2) prefetch_l2(p.scols + (size_t)g * 16 + lane * 8);
       if (lane == 2) prefetch_l2(p.indices + g * 8);
     }
   }
-  // residual columns of a group's contribution, dealt round-robin: the first, and `more` others, one of them this thread's
-  int more[GPB];
-  auto more_column = [&](int gi) { return GPB * kb + gi + ((int)threadIdx.x + 1) * p.G; };
+  // residual columns of a group's contribution, dealt round-robin: with MORE a thread gathers one of them, else all threads the first
+  int sal_count[GPB];
+  auto sal_column = [&](int gi) { return GPB * kb + gi + (MORE ? (int)threadIdx.x * p.G : 0); };
+  auto gathers = [&](int gi) { return (MORE ? (int)threadIdx.x : 0) < sal_count[gi]; };
 #pragma unroll
   for (int gi = 0; gi < GPB; ++gi) {
-    more[gi] = 0;
-    if (MORE && gi < ngroups) {
-      more[gi] = p.more_most - (GPB * kb + gi < p.more_full ? 0 : 1);
-      if ((int)threadIdx.x < more[gi]) prefetch_l2(p.sal_idx + more_column(gi));
+    sal_count[gi] = 0;
+    if (GLOBAL && gi < ngroups) {
+      sal_count[gi] = max(0, p.sal_most - (GPB * kb + gi < p.sal_full ? 0 : 1));
+      if (MORE && (int)threadIdx.x < sal_count[gi]) prefetch_l2(p.sal_idx + sal_column(gi));
     }
   }
 
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       prefetch_l2(p.grow + row), prefetch_l2(p.grow + (size_t)p.O + row);
       const __nv_bfloat16* const sal = p.sal + (size_t)row * p.n_sal;
       // A row's residual values are read one by one; up to four sectors of them are requested as a whole.  More would be in every CTA's way:
-      // each K block asks for all of them, past the L1 (255 columns, with / without: 1024x8192 8.03 / 4.56 us, 4096x4096 12.1 / 9.0).
+      // each K block asks for all of them, past the L1 (255 columns, with / without: 1024x8192 8.03 / 4.42 us, 4096x4096 12.1 / 8.8).
       if (MORE && p.n_sal <= 64) {
         for (int at = 0; at < p.n_sal; at += 16) prefetch_l2(sal + at);
       } else if (GPB * kb < p.n_sal) {
@@ -311,18 +312,23 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
     r_idx = g * 128 + (int)ldg16(p.indices + g * 8 + r_j);
     r_col = ldgf(p.scols + (size_t)(g * 8 + r_j) * 2 + r_base);
   }
-  int sal_at[GPB], more_at[GPB];
+  int sal_at[GPB];
 #pragma unroll
-  for (int gi = 0; gi < GPB; ++gi) {
-    const int g = GPB * kb + gi;
-    sal_at[gi] = GLOBAL && gi < ngroups && g < p.n_sal ? (int)ldg32(p.sal_idx + g) : -1;
-    more_at[gi] = MORE && (int)threadIdx.x < more[gi] ? (int)ldg32(p.sal_idx + more_column(gi)) : -1;
-  }
+  for (int gi = 0; gi < GPB; ++gi) sal_at[gi] = gathers(gi) ? (int)ldg32(p.sal_idx + sal_column(gi)) : -1;
   Constants next;
   if (first < end) request(first, next);
   // The rest of the ring goes behind these and ahead of the gathers, which wait for the indices (scales per group, 12288x4096 7.60 us; behind
   // them 7.92).
   for (int s = 1; s < S && pf_ru < end; ++s) issue_next();
+  // The residual columns' activations: where a group carries several, few warps gather them, ahead of the tables (12288x1024 4.53 us; behind them
+  // 4.72, the first column by all warps 5.47).  A single one is gathered by all, behind the tables, which it would hold up (4096x4096
+  // 4.05 us; ahead of them 4.13).
+  float gathered[GPB];
+  auto gather = [&]() {
+#pragma unroll
+    for (int gi = 0; gi < GPB; ++gi) gathered[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
+  };
+  if (MORE) gather();
   float r_x = 0.f;
   if (r_live) r_x = load_act(p.x, p.act_dtype, r_idx);
 
@@ -373,14 +379,11 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       sparse_lut[t * 256 + pp] = sum;
     }
   }
-  // residual columns come at a unit's end: gathered ahead of the tables they held those up (4096x4096 4.12 us, here 3.93)
-  float sal_x[GPB];
-#pragma unroll
-  for (int gi = 0; gi < GPB; ++gi) sal_x[gi] = sal_at[gi] >= 0 ? load_act(p.x, p.act_dtype, sal_at[gi]) : 0.f;
+  if (!MORE) gather();
   if (MORE) {
 #pragma unroll
     for (int gi = 0; gi < GPB; ++gi)
-      if (more_at[gi] >= 0) more_x[gi * p.more_most + (int)threadIdx.x] = load_act(p.x, p.act_dtype, more_at[gi]);
+      if (sal_at[gi] >= 0) sal_x[gi * p.sal_most + (int)threadIdx.x] = gathered[gi];
   }
   __syncthreads();
 
@@ -475,11 +478,11 @@ __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm) bb_gemv_kernel(const 
       // the dense residual columns are dealt round-robin over the groups' contributions
 #pragma unroll
       for (int gi = 0; gi < GPB; ++gi) {
-        if (sal_at[gi] >= 0) value = __fmaf_rn(__uint_as_float(now.sal[gi]), sal_x[gi], value);
+        if (sal_count[gi] > 0) value = __fmaf_rn(__uint_as_float(now.sal[gi]), MORE ? sal_x[gi * p.sal_most] : gathered[gi], value);
         if (MORE) {
           const __nv_bfloat16* const from = p.sal + (size_t)min(row, p.O - 1) * p.n_sal + GPB * kb + gi;
 #pragma unroll 4
-          for (int e = 0; e < more[gi]; ++e) value = __fmaf_rn(__bfloat162float(from[(e + 1) * p.G]), more_x[gi * p.more_most + e], value);
+          for (int e = 1; e < sal_count[gi]; ++e) value = __fmaf_rn(__bfloat162float(from[e * p.G]), sal_x[gi * p.sal_most + e], value);
         } else if (p.n_sal > p.G && gi < ngroups && row < p.O) {  // one or two
           for (int at = GPB * kb + gi + p.G; at < p.n_sal; at += p.G)
             value = __fmaf_rn(__bfloat162float(p.sal[(size_t)row * p.n_sal + at]), load_act(p.x, p.act_dtype, p.sal_idx[at]), value);
@@ -534,8 +537,8 @@ int launch(const BBParams& p, dim3 grid, size_t smem, int max_smem, bool pdl, cu
 
 // Two groups per K block halve the per-byte cost of a unit and double the tables to build ahead of the first: they pay once warps have
 // units of one group to spare, more than one each with matrix-wide scales, more than four (interleaved: five) with scales per group, which
-// bring more constants per unit either way.  us, one group / two, in brackets units of one group a warp: matrix-wide 2304x4096 (1.0) 3.40 / 3.50,
-// 3072x4096 (1.3) 4.29 / 3.87, 3072x1024 (0.3) 3.48 / 4.53, 1024x12288 (1.3) 4.42 / 3.71; per group 2048x12288 (2.6) 5.53 / 6.04, 3072x12288 (3.9)
+// bring more constants per unit either way.  us, one group / two, in brackets units of one group a warp: matrix-wide 2304x4096 (1.0) 3.29 / 3.59,
+// 3072x4096 (1.3) 4.14 / 3.89, 3072x1024 (0.3) 3.02 / 3.81, 1024x12288 (1.3) 4.10 / 3.74; per group 2048x12288 (2.6) 5.53 / 6.04, 3072x12288 (3.9)
 // 6.83 / 6.66, 9472x4096 (4.0) 6.99 / 7.32, 12288x4096 (5.2) 8.24 / 7.85; interleaved 5120x5120 (2.7) 6.91 / 7.45, 8192x5120 (4.3) 9.45 / 9.86,
 // 12288x4096 (5.2) 10.79 / 10.79, 16384x4096 (6.9) 13.3 / 12.7.
 int groups_per_block(int groups, int units, bool matrix_wide, bool interleaved, int sms) {
@@ -561,16 +564,17 @@ int run(BBParams& p, void* scratch, size_t scratch_bytes, unsigned flags, fb_str
   p.units_few = p.nRU / c, p.units_extra = p.nRU % c;
   p.sal_pairs = p.global_mode && p.n_sal % 2 == 0 && aligned(p.sal, 4) ? 1 : 0;
   const int per_warp = ((p.nRU + c - 1) / c + kWarps - 1) / kWarps;
-  // Where a group carries three residual columns and more, up to 1 + more_most (as many do the first more_full groups), their activations
-  // are gathered once per CTA and the first unit's values brought to the L2 ahead; a single one or two are read where they are used, which costs
-  // the others less.  us, gathered / as they are used: 32 columns 17x128 2.39 / 2.99, 512x512 (8 a group) 2.81 / 3.15, 16384x512 4.22 / 4.43, 512x1024 (4)
-  // 2.76 / 2.99, 8192x1024 3.90 / 3.76, 2048x2048 (2) 3.35 / 3.22, 5120x2560 (1.6) 4.86 / 4.32; 255 columns 2048x2048 (16) 5.93 / 6.02, 4096x4096 (8) 8.99 / 10.3.
+  // Where a group carries three residual columns and more, their activations are gathered once per CTA; a second one is read where it is
+  // used, which costs about the same.  us, gathered / as they are used: 32 columns 17x128 2.32 / 2.93, 512x512 (8 a group) 2.68 / 3.10, 16384x512 3.94 / 4.31, 512x1024 (4)
+  // 2.70 / 2.93, 8192x1024 3.41 / 3.62, 8192x1280 (3.2) 4.20 / 4.94, 2048x2048 (2) 2.96 / 3.02, 5120x2560 (1.6) 4.17 / 4.17; 255 columns 2048x2048 (16) 5.51 / 5.86, 4096x4096
+  // (8) 8.79 / 10.2.
   const bool more = p.global_mode && p.n_sal >= 3 * p.G;
-  p.more_most = more ? (p.n_sal - 1) / p.G : 0, p.more_full = more ? p.n_sal - p.more_most * p.G : 0;
-  const size_t more_bytes = (size_t)gpb * p.more_most * sizeof(float);
-  const int max_slots = gpb == 1 ? 4 : (p.global_mode && more_bytes <= 512 ? 3 : 2);  // two CTAs per SM
+  p.sal_most = !p.global_mode || p.n_sal == 0 ? 0 : more ? (p.n_sal - 1) / p.G + 1 : 1;
+  p.sal_full = p.n_sal - (p.sal_most > 1 ? (p.sal_most - 1) * p.G : 0);
+  const size_t sal_bytes = more ? (size_t)gpb * p.sal_most * sizeof(float) : 0;
+  const int max_slots = gpb == 1 ? 4 : (p.global_mode && sal_bytes <= 512 ? 3 : 2);  // two CTAs per SM
   p.slots = per_warp < max_slots ? (per_warp < 1 ? 1 : per_warp) : max_slots;
-  const size_t smem = (size_t)gpb * (kGroupLutBytes + (p.global_mode ? 0 : kGroupSparseBytes)) + (size_t)kWarps * p.slots * (gpb * kGroupBytes + 8) + more_bytes;
+  const size_t smem = (size_t)gpb * (kGroupLutBytes + (p.global_mode ? 0 : kGroupSparseBytes)) + (size_t)kWarps * p.slots * (gpb * kGroupBytes + 8) + sal_bytes;
   const bool pdl = (flags & FB_W3_NO_PDL) == 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (gpb == 2) {
